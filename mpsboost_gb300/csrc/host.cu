@@ -770,6 +770,11 @@ struct mpsb_cuda_trainer {
 
   int grid(int per_sm) const { return b->sm_count * per_sm; }
 
+  // The most nodes depth level d can hold, over all trees.
+  uint32_t level_nodes(uint32_t d) const {
+    return uint32_t(std::min<uint64_t>(dev.max_level_nodes, uint64_t(n_trees) << std::min<uint32_t>(d, 31)));
+  }
+
   // Captured rounds bake in the launch shape: drop them after a change.
   void reset_graphs() {
     for (int i = 0; i < 2; ++i) {
@@ -835,7 +840,7 @@ struct mpsb_cuda_trainer {
         CK(launch_subtract(dev, grid(8), s)); ++k;
       }
       if (depth > 0) {
-        CK(launch_split_scan(dev, parity, grid(4), s)); k += split_scan_kernels(dev);
+        CK(launch_split_scan(dev, parity, level_nodes(d), grid(4), s)); k += split_scan_kernels(dev);
       }
       CK(launch_finalize(dev, parity, d, s)); ++k;
       if (d + 1 < depth) {
@@ -868,7 +873,7 @@ struct mpsb_cuda_trainer {
     }
     CK(launch_root_stats(dev, s)); ++k;
     if (depth > 0) {
-      CK(launch_split_scan(dev, 0, grid(4), s)); k += split_scan_kernels(dev);
+      CK(launch_split_scan(dev, 0, n_trees, grid(4), s)); k += split_scan_kernels(dev);
     }
     CK(launch_leafwise_init(dev, s)); ++k;
     for (uint32_t step = 0; step < lw_steps && depth > 0; ++step) {
@@ -876,8 +881,8 @@ struct mpsb_cuda_trainer {
       CK(launch_partition(dev, grid(4), s)); k += kPartitionKernels;
       CK(launch_zero_build_slots(dev, grid(8), s)); ++k;
       CK(launch_hist_build(build_view(), hcfg, grid(1), s)); ++k;
-      CK(launch_subtract(dev, grid(8), s)); ++k;
-      CK(launch_split_scan(dev, 1, grid(4), s)); k += split_scan_kernels(dev);
+      if (!dev.fused_sub) { CK(launch_subtract(dev, grid(8), s)); ++k; }
+      CK(launch_split_scan(dev, 1, 2 * n_trees, grid(4), s)); k += split_scan_kernels(dev);
       CK(launch_leafwise_merge(dev, s)); ++k;
     }
     CK(launch_leafwise_finish(dev, s)); ++k;
@@ -1064,9 +1069,10 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.bins_block_stride = kBlockFeatures;
   a.bins_fm = ds->bins_fm.as<uint8_t>();
   a.slots = ds->slots;
-  // Level-wise growth on u8 datasets: the split scan forms each sibling's histogram
-  // (MPSB_FUSED_SUB=0: subtract_kernel does).
-  a.fused_sub = ds->slots == uint32_t(kSlots) && p->growth_strategy != 1;
+  a.scan_two_phase = p->split_strategy == 0 && p->reg_alpha == 0.0 && p->reg_lambda > 0.0;
+  // The split scan forms each sibling's histogram (MPSB_FUSED_SUB=0: subtract_kernel
+  // does); the one-launch scan on level-wise u8 datasets only.
+  a.fused_sub = a.scan_two_phase || (ds->slots == uint32_t(kSlots) && p->growth_strategy != 1);
   if (const char* v = std::getenv("MPSB_FUSED_SUB")) a.fused_sub = a.fused_sub && std::atoi(v) != 0;
   a.bins16 = ds->bins16.as<uint16_t>();
   a.bins16_fm = ds->bins16_fm.as<uint16_t>();
@@ -1270,10 +1276,10 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
     a.node_path[q] = t->alloc<uint32_t>(size_t(a.max_level_nodes) * W);
     a.node_allowed[q] = t->alloc<uint32_t>(size_t(a.max_level_nodes) * W);
   }
-  a.partial = t->alloc<SplitRec>(size_t(a.max_level_nodes) * a.n_fchunks);
+  a.partial_stride = a.scan_two_phase ? 1u : a.n_fchunks;
+  a.partial = t->alloc<SplitRec>(size_t(a.max_level_nodes) * a.partial_stride);
   a.node_screen = t->alloc<uint32_t>(a.max_level_nodes);
-  a.chunk_screen = t->alloc<uint32_t>(size_t(a.max_level_nodes) * a.n_fchunks);
-  a.scan_two_phase = p->split_strategy == 0 && p->reg_alpha == 0.0 && p->reg_lambda > 0.0;
+  if (a.scan_two_phase) a.feature_screen = t->alloc<uint32_t>(size_t(a.max_level_nodes) * F);
   a.build = t->alloc<BuildEntry>(a.max_level_nodes);
   a.build_prefix = t->alloc<uint32_t>(a.max_level_nodes + 1);
   a.sub = t->alloc<SubEntry>(a.max_level_nodes);

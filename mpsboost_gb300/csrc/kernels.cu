@@ -10,9 +10,11 @@
 //                  (TreeTrainingAccess::Create, tree_structure.cpp:104-116).
 //   subtract       SubtractHistograms (tree_histogram.cpp:16-66): exact int64 in fixed
 //                  mode, FP64 with the Hessian clamp in float mode.
-//   split_scan     FindBestSplit (tree_split.cpp:142-234): one warp per (node, feature),
-//                  warp-shuffle prefix over the 256 slots, FP64 gains with both missing
-//                  directions, random threshold, monotone and interaction rules.
+//   split_screen, split_exact, split_scan
+//                  FindBestSplit (tree_split.cpp:142-234): prefix sums over a feature's
+//                  slots, FP64 gains with both missing directions, random threshold,
+//                  monotone and interaction rules; where an FP32 screen can rule candidates
+//                  out, in two launches (screen, then the FP64 gains of what is left).
 //   finalize       the per-level bookkeeping of TrainLevelWiseRegressionTree
 //                  (tree.cpp:67-145): acceptance under max_leaves, ApplySplit
 //                  (tree_structure.cpp:118-148), smaller-child selection, next level.
@@ -595,43 +597,45 @@ __device__ __forceinline__ double image(typename Stat<FIXED>::V v, double inv) {
   else return v;
 }
 
-// ConsiderMissingDirection (tree_split.cpp:65-115) + MonotonicBoundsForSplit
-// (tree_monotonic.cpp:12-58).
+// ConsiderMissingDirection (tree_split.cpp:65-115): the FP64 gain of one candidate; false
+// where the reference rejects it.
 template <bool FIXED>
-__device__ __forceinline__ void consider(const TreeParams& p, const Stat<FIXED>& cl,
-                                         const Stat<FIXED>& cr, double inv_g, double inv_h,
-                                         int8_t mono, double plo, double phi, uint32_t feature,
-                                         uint32_t threshold, uint32_t default_left,
-                                         SplitRec& best, uint32_t& err) {
-  if (cl.count < p.min_samples_leaf || cr.count < p.min_samples_leaf) return;
+__device__ __forceinline__ bool exact_gain(const TreeParams& p, const Stat<FIXED>& cl,
+                                           const Stat<FIXED>& cr, double inv_g, double inv_h,
+                                           int8_t mono, double plo, double phi, double* gain_out,
+                                           uint32_t& err) {
+  if (cl.count < p.min_samples_leaf || cr.count < p.min_samples_leaf) return false;
   const double lh = image<FIXED>(cl.h, inv_h), rh = image<FIXED>(cr.h, inv_h);
-  if (lh < p.min_child_weight || rh < p.min_child_weight || lh <= 0.0 || rh <= 0.0) return;
+  if (lh < p.min_child_weight || rh < p.min_child_weight || lh <= 0.0 || rh <= 0.0) return false;
   const double lg = image<FIXED>(cl.g, inv_g), rg = image<FIXED>(cr.g, inv_g);
   double gain;
   if (!split_gain(lg, lh, rg, rh, p, &gain)) {
     err |= kErrNonFinite;
-    return;
+    return false;
   }
-  if (gain <= 0.0 || gain < p.min_gain_to_split) return;
-  double ll = plo, lu = phi, rl = plo, ru = phi;
+  if (gain <= 0.0 || gain < p.min_gain_to_split) return false;
   if (mono != 0) {
     double lv, rv;
     if (!leaf_weight(lg, lh, p, &lv) || !leaf_weight(rg, rh, p, &rv)) {
       err |= kErrNonFinite;
-      return;
+      return false;
     }
     lv = clamp_bounds(lv, plo, phi);
     rv = clamp_bounds(rv, plo, phi);
-    if (mono > 0) {
-      if (lv > rv) return;
-      lu = (rv < lu) ? rv : lu;  // std::min(lu, rv)
-      rl = (rl < lv) ? lv : rl;  // std::max(rl, lv)
-    } else {
-      if (lv < rv) return;
-      ll = (ll < rv) ? rv : ll;  // std::max(ll, rv)
-      ru = (lv < ru) ? lv : ru;  // std::min(ru, lv)
-    }
+    if (mono > 0 ? lv > rv : lv < rv) return false;
   }
+  *gain_out = gain;
+  return true;
+}
+
+// The record of an accepted candidate, with MonotonicBoundsForSplit (tree_monotonic.cpp:
+// 12-58); the leaf weights repeat exact_gain's operations.
+template <bool FIXED>
+__device__ __forceinline__ SplitRec split_record(const TreeParams& p, const Stat<FIXED>& cl,
+                                                 const Stat<FIXED>& cr, double inv_g, double inv_h,
+                                                 int8_t mono, double plo, double phi, double gain,
+                                                 uint32_t feature, uint32_t threshold,
+                                                 uint32_t default_left) {
   SplitRec c;
   c.gain = gain;
   c.valid = 1;
@@ -648,15 +652,128 @@ __device__ __forceinline__ void consider(const TreeParams& p, const Stat<FIXED>&
   } else {
     c.lqg = c.lqh = c.rqg = c.rqh = 0;
   }
-  c.lg = lg;
-  c.lh = lh;
-  c.rg = rg;
-  c.rh = rh;
-  c.ll = ll;
-  c.lu = lu;
-  c.rl = rl;
-  c.ru = ru;
+  c.lg = image<FIXED>(cl.g, inv_g);
+  c.lh = image<FIXED>(cl.h, inv_h);
+  c.rg = image<FIXED>(cr.g, inv_g);
+  c.rh = image<FIXED>(cr.h, inv_h);
+  c.ll = c.rl = plo;
+  c.lu = c.ru = phi;
+  if (mono != 0) {
+    double lv = 0.0, rv = 0.0;
+    leaf_weight(c.lg, c.lh, p, &lv);
+    leaf_weight(c.rg, c.rh, p, &rv);
+    lv = clamp_bounds(lv, plo, phi);
+    rv = clamp_bounds(rv, plo, phi);
+    if (mono > 0) {
+      c.lu = (rv < c.lu) ? rv : c.lu;  // std::min(lu, rv)
+      c.rl = (c.rl < lv) ? lv : c.rl;  // std::max(rl, lv)
+    } else {
+      c.ll = (c.ll < rv) ? rv : c.ll;  // std::max(ll, rv)
+      c.ru = (lv < c.ru) ? lv : c.ru;  // std::min(ru, lv)
+    }
+  }
+  return c;
+}
+
+template <bool FIXED>
+__device__ __forceinline__ void consider(const TreeParams& p, const Stat<FIXED>& cl,
+                                         const Stat<FIXED>& cr, double inv_g, double inv_h,
+                                         int8_t mono, double plo, double phi, uint32_t feature,
+                                         uint32_t threshold, uint32_t default_left,
+                                         SplitRec& best, uint32_t& err) {
+  double gain;
+  if (!exact_gain<FIXED>(p, cl, cr, inv_g, inv_h, mono, plo, phi, &gain, err)) return;
+  const SplitRec c = split_record<FIXED>(p, cl, cr, inv_g, inv_h, mono, plo, phi, gain, feature,
+                                         threshold, default_left);
   if (better_split(c, best)) best = c;
+}
+
+// ---- FP32 screen ---------------------------------------------------------------------
+// Every eligible candidate's score S = gL^2/(hL+lambda) + gR^2/(hR+lambda) is computed in
+// FP32 with relative error <= 15u (u = 2^-24; each int64 -> FP32 conversion below is within
+// 3u, lambda is rounded once, the approximate reciprocal is within 2u). A candidate whose
+// FP32 score is below M(1 - 2^-18), M the best FP32 score of a certainly eligible candidate
+// of the node, then has an exact score at least 30u*M below that candidate's, far outside
+// the FP64 evaluation's own rounding (a few 2^-53 * M, the parent score included), so its
+// FP64 gain is strictly lower and it cannot win. Only the rest -- and candidates whose
+// min_child_weight test or score is too close to call in FP32 -- run the FP64 evaluation of
+// the reference. The score is quadratic only without reg_alpha, the admissible set monotone
+// in it only without monotone constraints, and random thresholds leave one candidate: the
+// screen is off for those, and where lambda in hessian quanta leaves a safe range.
+//
+// Fixed point scores the quantized sums themselves: with lambda and min_child_weight taken
+// times 2^kh (a power of two: no rounding), every score of a node is the real one times the
+// same power of two, so the comparisons are the same and no sum is scaled. Sums stay below
+// 2^62 and an eligible hessian sum is at least 1, so no square, reciprocal or sum leaves the
+// FP32 normal range (a zero gradient scores 0).
+struct ScreenScale {
+  bool on;  // the screen applies to this feature of this node
+  float lambda, mcw_lo, mcw_hi;
+};
+
+template <bool FIXED>
+__device__ __forceinline__ ScreenScale screen_scale(const TreeParams& P, int8_t mono, int kh) {
+  ScreenScale s;
+  s.on = P.screen_params != 0 && mono == 0;
+  float unit = 1.0f;
+  if constexpr (FIXED) {
+    s.on = s.on && kh >= -120 && kh <= 120;
+    unit = s.on ? __int_as_float((127 + kh) << 23) : 1.0f;
+  }
+  s.lambda = P.screen_lambda * unit;
+  if (FIXED && !(s.lambda <= 0x1p100f)) s.on = false;
+  // Without a minimum no sum is rejected or close to it.
+  s.mcw_lo = P.screen_mcw_on ? P.screen_mcw_lo * unit : -1.0f;
+  s.mcw_hi = P.screen_mcw_on ? P.screen_mcw_hi * unit : -1.0f;
+  return s;
+}
+
+// m as hi * 2^32 + lo: float(hi) and float(lo) are each within u, and the fused
+// multiply-add rounds once more, so the result is within 3u (no cancellation: both parts
+// are non-negative). The conversions run on the FP32 pipe.
+__device__ __forceinline__ float u64_to_f32_3u(unsigned long long m) {
+  return __fmaf_rn(u32_to_f32_rn(uint32_t(m >> 32)), 4294967296.0f, u32_to_f32_rn(uint32_t(m)));
+}
+
+// 1/y within 2u for a normal y below 2^126.
+__device__ __forceinline__ float rcp_approx(float y) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return r;
+}
+
+// 0: rejected by the FP64 test before any arithmetic (no error flag either);
+// 1: admissible, FP32 score in *s32; 2: too close to call. msl: min_samples_leaf, at most
+// 2^32 - 1 (no node holds more rows).
+template <bool FIXED>
+__device__ __forceinline__ int screen_classify(uint32_t msl, const ScreenScale& sc,
+                                               const Stat<FIXED>& cl, const Stat<FIXED>& cr,
+                                               float* s32) {
+  if (min(cl.count, cr.count) < msl) return 0;
+  if constexpr (FIXED) {
+    if (!(cl.h > 0) || !(cr.h > 0)) return 0;  // image > 0 iff q > 0
+    const float lh = u64_to_f32_3u((unsigned long long)cl.h), rh = u64_to_f32_3u((unsigned long long)cr.h);
+    const float least = fminf(lh, rh);
+    if (least < sc.mcw_lo) return 0;
+    const float lg = u64_to_f32_3u((unsigned long long)(cl.g < 0 ? -cl.g : cl.g));
+    const float rg = u64_to_f32_3u((unsigned long long)(cr.g < 0 ? -cr.g : cr.g));
+    *s32 = __fmaf_rn(lg * lg, rcp_approx(lh + sc.lambda), (rg * rg) * rcp_approx(rh + sc.lambda));
+    return least <= sc.mcw_hi ? 2 : 1;
+  } else {
+    if (!f64_finite(cl.h) || !f64_finite(cr.h) || !f64_finite(cl.g) || !f64_finite(cr.g)) return 2;
+    if (!(cl.h > 0) || !(cr.h > 0)) return 0;
+    const float lh = f64_to_f32_rn(cl.h), rh = f64_to_f32_rn(cr.h);
+    const float least = fminf(lh, rh);
+    if (least < sc.mcw_lo) return 0;
+    const float lg = f64_to_f32_rn(cl.g), rg = f64_to_f32_rn(cr.g);
+    const float score = screen_div(lg * lg, lh + sc.lambda) + screen_div(rg * rg, rh + sc.lambda);
+    *s32 = score;
+    return (least <= sc.mcw_hi || !isfinite(score)) ? 2 : 1;
+  }
+}
+
+__device__ __forceinline__ uint32_t min_leaf_rows(const TreeParams& P) {
+  return uint32_t(P.min_samples_leaf < 0xFFFFFFFFull ? P.min_samples_leaf : 0xFFFFFFFFull);
 }
 
 // One warp per (node, feature); a CTA covers one node and blockDim/32 features and
@@ -675,11 +792,10 @@ struct ScanCand {
 // (word 0 count, 1 g, 2 h): the lane's eight slots read conflict-free.
 constexpr size_t kScanHistBytes = size_t(kSlots) * 3 * sizeof(unsigned long long);
 
-// Shared memory per warp: its best split, its staged histogram and (exact phase) its FP64
-// queue.
-template <bool FIXED, bool SCREEN>
+// Shared memory per warp: its best split, its staged histogram and its FP64 queue.
+template <bool FIXED>
 constexpr size_t scan_smem_per_warp() {
-  return sizeof(SplitRec) + kScanHistBytes + (SCREEN ? 0 : kScanQueue * sizeof(ScanCand<FIXED>));
+  return sizeof(SplitRec) + kScanHistBytes + kScanQueue * sizeof(ScanCand<FIXED>);
 }
 
 // Copies a feature's histogram (kSlots x {count, g, h} 64-bit words, 6 KB, 16-byte
@@ -807,65 +923,40 @@ __device__ __forceinline__ void stage_few_slots(unsigned long long* slot_hist,
   __syncwarp();
 }
 
-// Bit 31 of a chunk's screen word: some feature of the chunk is evaluated exactly whatever
-// the node's maximum (its screen is off, or a candidate is too close to call in FP32).
-// The low bits hold the chunk's best certainly admissible FP32 score (a non-negative
-// float's bits).
-constexpr uint32_t kChunkExact = 0x80000000u;
-
-// The split scan of a level, one warp per (node, feature), a CTA per (node, chunk of
-// blockDim/32 features). With the FP32 screen on (best-split strategy, no reg_alpha,
-// reg_lambda > 0) it runs in two launches:
-//  SCREEN: each warp forms its feature's prefix sums and the FP32 scores of its
-//    candidates, raises the node's running maximum of certainly admissible scores
-//    (node_screen, atomicMax on the float bits) and writes its chunk's maximum and exact
-//    flag (chunk_screen).
-//  EXACT: with the node's final maximum M, a chunk whose candidates all score below
-//    M(1 - 2^-18) and holds nothing to evaluate exactly writes "no split" at once; the
-//    other chunks evaluate in FP64, as the reference does, every candidate at or above
-//    that cut and every close call. A candidate below the cut has a strictly lower exact
-//    gain than the admissible candidate that scored M, which its own chunk evaluates, so
-//    it can win neither its chunk nor the node.
-// EXACT alone (screen off, or no node maxima: the per-feature entry point) screens each
-// feature against its own maximum. Each chunk's best split goes to partial[node][chunk].
+// The split scan of a level in one launch, one warp per (node, feature), a CTA per (node,
+// chunk of blockDim/32 features): where the two-launch scan below does not apply (no FP32
+// screen, or the per-feature entry point, which needs every feature's best split). A
+// feature the screen does apply to is screened against its own maximum. Each chunk's best
+// split goes to partial[node][chunk].
 //
 // WIDE (a dataset with more than kSlots slots per feature): each warp walks its feature's
 // slots in pages of kSlots, first for the total count and the missing slot (the last
 // page's slot kMissingSlot), then per scan pass page by page with the left prefix carried
 // from page to page; thresholds are numbered across pages.
-template <bool FIXED, bool SCREEN, bool WIDE>
+template <bool FIXED, bool WIDE>
 __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev a, int parity) {
   using V = typename Stat<FIXED>::V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   SplitRec* warp_best = reinterpret_cast<SplitRec*>(smem_raw);
-  uint32_t* warp_screen = reinterpret_cast<uint32_t*>(smem_raw);  // SCREEN: [warp]
   unsigned long long* s_hist =
       reinterpret_cast<unsigned long long*>(smem_raw + sizeof(SplitRec) * nwarps);
   ScanCand<FIXED>* s_queue = reinterpret_cast<ScanCand<FIXED>*>(
       smem_raw + (sizeof(SplitRec) + kScanHistBytes) * nwarps);
   static_assert(sizeof(SplitRec) % 8 == 0, "staged words and queue entries stay 8-byte aligned");
-  __shared__ uint32_t s_list[32], s_listed;  // two-phase exact launch: a batch's items to evaluate
   const TreeParams& P = a.params;
   const uint32_t n_chunks = a.n_fchunks;
   const uint32_t n_nodes = a.ctl->n_nodes;
   const uint32_t items = n_nodes * n_chunks;
-  const bool two_phase = !SCREEN && a.node_screen != nullptr && a.scan_two_phase != 0;
-  // The level's first launch forms the siblings' histograms (u8 datasets).
-  const bool fuse_sub = !WIDE && a.fused_sub != 0 && (SCREEN || !two_phase);
-  // Launch-wide screen constants (FP64 tests and conversions stay out of the item loop).
-  const bool screen_params = P.screen_params != 0;
-  const float lam32 = P.screen_lambda;
-  const bool mcw_on = P.screen_mcw_on != 0;
-  const float mcw_lo = P.screen_mcw_lo, mcw_hi = P.screen_mcw_hi;
+  const bool fuse_sub = !WIDE && a.fused_sub != 0;  // the launch forms the siblings' histograms
   // The work on one (node, chunk) item; every thread of the CTA calls it.
   auto eval_item = [&](uint32_t item) {
     const uint32_t i = item / n_chunks, c = item % n_chunks;
     const NodeRec node = a.nodes[parity][i];
     const uint32_t f = c * uint32_t(nwarps) + uint32_t(warp);
     const double inv_g = a.trees[node.tree].inv_g, inv_h = a.trees[node.tree].inv_h;
-    const int st_kg = a.trees[node.tree].kg, st_kh = a.trees[node.tree].kh;
+    const int st_kh = a.trees[node.tree].kh;
     SplitRec best;
     best.valid = 0;
     best.gain = 0.0;
@@ -873,8 +964,7 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
     best.threshold = 0;
     best.default_left = 1;
     uint32_t err = 0;
-    float best32 = -1.0f;  // SCREEN: best certainly admissible FP32 score of the feature
-    bool exact = false;    // SCREEN: the feature needs the exact pass whatever the cut
+    float best32 = -1.0f;  // best certainly admissible FP32 score of the feature
     // A node with fewer than 2 * min_samples_leaf rows has no admissible split.
     bool active = f < a.features && node.count >= 2 * P.min_samples_leaf;
     if (active) {
@@ -1007,56 +1097,10 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
                       a.feature_rank ? a.feature_rank[size_t(node.tree) * a.features + f] : f,
                       node.node_index, node.depth, nb - 1)
                 : 0xffffffffu;
-        // Exact FP32 pre-screen. Every eligible candidate's score S = gL^2/(hL+lambda) +
-        // gR^2/(hR+lambda) is computed in FP32 with relative error <= 14u (u = 2^-24; each
-        // int64 -> FP32 conversion below is within 3u, lambda is rounded once, a division
-        // within 2u). A candidate whose FP32 score is below M(1 - 2^-18), M the best FP32
-        // score of a certainly eligible candidate of the node, then has an exact score at
-        // least 30u*M below that candidate's, far outside the FP64 evaluation's own
-        // rounding (a few 2^-53 * M, the parent score included), so its FP64 gain is
-        // strictly lower and it cannot win. Only the rest -- and candidates whose
-        // min_child_weight test or score is too close to call in FP32 -- run the FP64
-        // evaluation of the reference. The score is quadratic only without reg_alpha, the
-        // admissible set monotone in it only without monotone constraints, and random
-        // thresholds leave one candidate: the screen is off for those, and where 2^-k
-        // leaves the FP32 normal range.
-        const bool screen = screen_params && mono == 0 &&
-                            (!FIXED || (st_kg >= -120 && st_kg <= 120 && st_kh >= -120 && st_kh <= 120));
-        // 2^-k exactly, built from the exponent field.
-        const float inv_g32 = FIXED && screen ? __int_as_float((127 - st_kg) << 23) : 1.0f;
-        const float inv_h32 = FIXED && screen ? __int_as_float((127 - st_kh) << 23) : 1.0f;
-        // |v| as hi * 2^32 + lo: float(hi) and float(lo) are each within u, and the fused
-        // multiply-add rounds once more, so the result is within 3u of v (no cancellation:
-        // both parts are non-negative). The conversions run on the FP32 pipe.
-        auto to32 = [&](V v, float inv32) -> float {
-          if constexpr (FIXED) {
-            const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
-            const float f = __fmaf_rn(u32_to_f32_rn(uint32_t(m >> 32)), 4294967296.0f,
-                                      u32_to_f32_rn(uint32_t(m)));
-            return (v < 0 ? -f : f) * inv32;
-          } else {
-            return f64_to_f32_rn(v);
-          }
-        };
-        // 0: rejected by the FP64 test before any arithmetic (no error flag either);
-        // 1: admissible, FP32 score in *s32; 2: too close to call.
+        const ScreenScale scale = screen_scale<FIXED>(P, mono, st_kh);
+        const bool screen = scale.on;
         auto classify = [&](const Stat<FIXED>& cl, const Stat<FIXED>& cr, float* s32) -> int {
-          if (cl.count < P.min_samples_leaf || cr.count < P.min_samples_leaf) return 0;
-          if constexpr (!FIXED) {
-            if (!f64_finite(cl.h) || !f64_finite(cr.h) || !f64_finite(cl.g) || !f64_finite(cr.g)) return 2;
-          }
-          if (!(cl.h > 0) || !(cr.h > 0)) return 0;  // fixed point: image > 0 iff q > 0
-          const float lh = to32(cl.h, inv_h32), rh = to32(cr.h, inv_h32);
-          int cls = 1;
-          if (mcw_on) {
-            if (lh < mcw_lo || rh < mcw_lo) return 0;
-            if (lh <= mcw_hi || rh <= mcw_hi) cls = 2;
-          }
-          const float lg = to32(cl.g, inv_g32), rg = to32(cr.g, inv_g32);
-          const float sc = screen_div(lg * lg, lh + lam32) + screen_div(rg * rg, rh + lam32);
-          if (!isfinite(sc)) cls = 2;
-          *s32 = sc;
-          return cls;
+          return screen_classify<FIXED>(min_leaf_rows(P), scale, cl, cr, s32);
         };
         // Visits every (threshold, missing direction) step of the lane's 8 slots of the
         // staged page (the left prefix before them `cin`, the page's first threshold
@@ -1123,7 +1167,7 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
             }
           }
         };
-        // The lane's best certainly admissible FP32 score; close calls set `exact`.
+        // The lane's best certainly admissible FP32 score.
         auto screen_scores = [&]() {
           for_pages([&](const Stat<FIXED>& cin, uint32_t base, bool last) {
             scan_candidates(cin, base, last, [&](bool cand, const Stat<FIXED>& cl,
@@ -1132,26 +1176,16 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
               float sc = 0.0f;
               const int cls = classify(cl, cr, &sc);
               if (cls == 1) best32 = fmaxf(best32, sc);
-              if (cls == 2) exact = true;
             });
           });
           for (int off = 16; off > 0; off >>= 1)
             best32 = fmaxf(best32, __shfl_xor_sync(0xffffffffu, best32, off));
         };
-        if constexpr (SCREEN) {
-          if (screen) screen_scores();
-          else exact = true;
-        } else {
+        {
           float cut = -1.0f;
           if (screen) {
-            float m;
-            if (two_phase) {
-              m = __uint_as_float(a.node_screen[i]);
-            } else {
-              screen_scores();
-              m = best32;
-            }
-            cut = m >= 1e-30f ? m * (1.0f - 0x1p-18f) : -1.0f;
+            screen_scores();
+            cut = best32 >= 1e-30f ? best32 * (1.0f - 0x1p-18f) : -1.0f;
           }
           // Candidates that pass the screen queue up, and the warp evaluates them in FP64
           // one per lane: the narrow FP64 pipe runs one pass per 32 survivors instead of
@@ -1197,22 +1231,7 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
       }
     }
     if (err) raise(a.ctl, err);
-    if constexpr (SCREEN) {
-      exact = __any_sync(0xffffffffu, exact);
-      if (lane == 0) {
-        if (best32 >= 1e-30f) atomicMax(a.node_screen + i, __float_as_uint(best32));
-        warp_screen[warp] = (exact ? kChunkExact : 0u) | (best32 > 0.0f ? __float_as_uint(best32) : 0u);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        uint32_t word = 0;
-        for (int w = 0; w < nwarps; ++w)
-          word = (word & kChunkExact) | (warp_screen[w] & kChunkExact) |
-                 max(word & ~kChunkExact, warp_screen[w] & ~kChunkExact);
-        a.chunk_screen[size_t(i) * n_chunks + c] = word;
-      }
-      __syncthreads();
-    } else {
+    {
       // Warp argmax (all lanes share the feature): every lane ends with the winner's id.
       uint32_t win = uint32_t(lane);
       {
@@ -1251,45 +1270,482 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
       __syncthreads();
     }
   };
-  if (two_phase) {
-    // Batches of 32 consecutive items: warp 0 tests them against their nodes' final screen
-    // maxima, one lane each, writes "no split" for the chunks below the cut and lists the
-    // rest, which the CTA then evaluates in turn. At the deep levels most chunks are below
-    // the cut, and a CTA that tested them one at a time waited on a global load and two
-    // barriers per chunk.
-    const uint32_t n_batches = (items + 31u) / 32u;
-    for (uint32_t bt = blockIdx.x; bt < n_batches; bt += gridDim.x) {
-      if (warp == 0) {
-        const uint32_t item = bt * 32u + uint32_t(lane);
-        bool keep = false;
-        if (item < items) {
-          const uint32_t i = item / n_chunks, c = item % n_chunks;
-          const uint32_t cs = a.chunk_screen[size_t(i) * n_chunks + c];
-          const float m = __uint_as_float(a.node_screen[i]);
-          keep = (cs & kChunkExact) || !(m >= 1e-30f) || !(__uint_as_float(cs) < m * (1.0f - 0x1p-18f));
-          if (!keep) {
-            SplitRec none;
-            none.valid = 0;
-            none.gain = 0.0;
-            none.feature = c * uint32_t(nwarps);
-            none.threshold = 0;
-            none.default_left = 1;
-            a.partial[size_t(i) * n_chunks + c] = none;
-          }
-        }
-        const uint32_t ballot = __ballot_sync(0xffffffffu, keep);
-        if (keep) s_list[__popc(ballot & ((1u << lane) - 1u))] = item;
-        if (lane == 0) s_listed = uint32_t(__popc(ballot));
+  for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) eval_item(item);
+  (void)sizeof(V);
+}
+
+// ---- Split scan in two launches ---------------------------------------------------------
+// Where the FP32 screen applies (best-split strategy, no reg_alpha, reg_lambda > 0):
+//  split_screen_kernel forms every (node, feature)'s prefix sums and the FP32 scores of its
+//    candidates, raises the node's maximum of certainly admissible scores (node_screen,
+//    atomicMax on the float bits) and writes the feature's own (feature_screen).
+//  split_exact_kernel, with the node's final maximum M, evaluates in FP64, as the reference
+//    does, the features that hold a candidate at or above M(1 - 2^-18) or one to evaluate
+//    whatever the maximum, and of those features the candidates at or above that cut and
+//    the close calls. A candidate below the cut has a strictly lower exact gain than the
+//    admissible candidate that scored M, so it cannot win the node. partial[node] is the
+//    node's best split.
+// Both give a page of kSlots slots to a CTA, two neighbouring slots per thread (48
+// contiguous bytes, three 16-byte loads): a block-wide prefix sum, then each thread
+// evaluates its own thresholds' candidates. One slot per thread spends half its
+// instructions on the prefix sum, eight (a warp per page) load 192-byte strides and leave a
+// shallow level's few features to few warps. Threads past the feature's bins load and
+// evaluate nothing, so a feature of few bins costs little.
+constexpr int kScanCta = kSlots / 2;
+constexpr int kScanCtaWarps = kScanCta / 32;
+constexpr uint32_t kScanFeaturesPerItem = 8;  // at most; fewer where that leaves SMs idle
+
+// A feature_screen word: 0 (no candidate), or the best certainly admissible FP32 score's
+// bits (at least 1), with kFeatureExact set where the feature is evaluated exactly whatever
+// the node's maximum (its screen is off, or a candidate is too close to call in FP32).
+constexpr uint32_t kFeatureExact = 0x80000000u;
+
+// The warps' totals of a page, exchanged through shared memory, and the missing slot.
+template <bool FIXED>
+struct PageTotals {
+  typename Stat<FIXED>::V g[kScanCtaWarps], h[kScanCtaWarps];
+  typename Stat<FIXED>::V miss_g, miss_h;
+  uint32_t count[kScanCtaWarps], miss_count;
+};
+
+template <bool FIXED>
+__device__ __forceinline__ Stat<FIXED> warp_inclusive(Stat<FIXED> x, int lane) {
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const Stat<FIXED> y = shfl_up_stat<FIXED>(x, off);
+    if (lane >= off) x = stat_add<FIXED>(y, x);
+  }
+  return x;
+}
+
+// Block-wide inclusive prefix of one value per thread; *total gets the page's sum. One
+// barrier; `t` may be written again after the CTA's next barrier.
+template <bool FIXED>
+__device__ __forceinline__ Stat<FIXED> page_prefix(const Stat<FIXED>& own, PageTotals<FIXED>& t,
+                                                   Stat<FIXED>* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Stat<FIXED> incl = warp_inclusive<FIXED>(own, lane);
+  if (lane == 31) {
+    t.count[warp] = incl.count;
+    t.g[warp] = incl.g;
+    t.h[warp] = incl.h;
+  }
+  __syncthreads();
+  Stat<FIXED> before = stat_zero<FIXED>(), all = stat_zero<FIXED>();
+#pragma unroll
+  for (int q = 0; q < kScanCtaWarps; ++q) {
+    if (q == warp) before = all;
+    Stat<FIXED> w;
+    w.count = t.count[q];
+    w.g = t.g[q];
+    w.h = t.h[q];
+    all = stat_add<FIXED>(all, w);
+  }
+  *total = all;
+  return stat_add<FIXED>(before, incl);
+}
+
+// The raw words of a thread's two slots (count, g, h of the even one, then of the odd one),
+// and the built sibling's where the histogram is formed on the way.
+struct SlotWords {
+  unsigned long long own[6], built[6];
+};
+
+__device__ __forceinline__ void load_pair(unsigned long long (&w)[6], const unsigned long long* src) {
+  const ulonglong2* v = reinterpret_cast<const ulonglong2*>(src);  // 48-byte pairs of a 16-byte aligned slot
+  const ulonglong2 x = v[0], y = v[1], z = v[2];
+  w[0] = x.x;
+  w[1] = x.y;
+  w[2] = y.x;
+  w[3] = y.y;
+  w[4] = z.x;
+  w[5] = z.y;
+}
+
+template <bool FIXED>
+__device__ __forceinline__ Stat<FIXED> slot_stat(unsigned long long c, unsigned long long g,
+                                                 unsigned long long h, uint32_t& err) {
+  Stat<FIXED> b;
+  b.count = uint32_t(c);
+  if (c >> 32) err |= kErrCountMismatch;  // a node holds fewer than 2^32 rows
+  if constexpr (FIXED) {
+    b.g = (long long)g;
+    b.h = (long long)h;
+  } else {
+    b.g = __longlong_as_double((long long)g);
+    b.h = __longlong_as_double((long long)h);
+    if (!isfinite(b.g) || !isfinite(b.h) || b.h < 0.0) err |= kErrNonFinite;
+  }
+  return b;
+}
+
+// What the scans need of a node, its tree and the launch.
+template <bool FIXED>
+struct ScanNode {
+  uint32_t slot, sub_from;
+  Stat<FIXED> parent;
+  double inv_h;
+};
+
+template <bool FIXED>
+__device__ __forceinline__ ScanNode<FIXED> scan_node(const NodeRec& node, double inv_h) {
+  ScanNode<FIXED> s;
+  s.slot = node.slot;
+  s.sub_from = node.sub_from;
+  s.parent.count = uint32_t(node.count);
+  if constexpr (FIXED) {
+    s.parent.g = node.qg;
+    s.parent.h = node.qh;
+  } else {
+    s.parent.g = node.g;
+    s.parent.h = node.h;
+  }
+  s.inv_h = inv_h;
+  return s;
+}
+
+// The missing rows' statistics never exceed the node's (tree_split.cpp:186-189).
+template <bool FIXED>
+__device__ __forceinline__ bool missing_above(const Stat<FIXED>& miss, const Stat<FIXED>& parent,
+                                              double inv_h) {
+  if (miss.count > parent.count) return true;
+  if constexpr (FIXED) {
+    // The images q * 2^-k compare as the quantized sums while those convert exactly.
+    const long long lim = 1ll << 53;
+    return (miss.h > -lim && miss.h < lim && parent.h > -lim && parent.h < lim)
+               ? miss.h > parent.h
+               : images_above(miss.h, parent.h, inv_h);
+  } else {
+    return miss.h > parent.h;
+  }
+}
+
+// Whether a page-`p` pair holds anything: every slot from the feature's bin count on is
+// empty, but for the missing rows' (the last of all, odd: the second of its pair).
+__device__ __forceinline__ bool pair_held(uint32_t s, uint32_t nb, bool hm, uint32_t S) {
+  return s < nb || (hm && s + 2 == S);
+}
+
+// Words of the pair that starts at slot s (zeros where both slots are empty).
+template <bool FIXED, bool SUB>
+__device__ __forceinline__ SlotWords load_slots(const TrainerDev& a, const ScanNode<FIXED>& node,
+                                                uint32_t f, uint32_t nb, bool hm, uint32_t S, uint32_t s) {
+  SlotWords w{};
+  if (pair_held(s, nb, hm, S)) {
+    load_pair(w.own, a.hist + ((size_t(node.slot) * a.features + f) * S + s) * 3);
+    if (SUB && node.sub_from != 0)
+      load_pair(w.built, a.hist + ((size_t(node.sub_from - 1) * a.features + f) * S + s) * 3);
+  }
+  return w;
+}
+
+// One feature of one node, every thread of the CTA: calls visit(left, right, threshold,
+// default_left) for each candidate of the thread's slots. `first` holds page 0's words of
+// the thread's pair. SUB (the level's first launch): a sibling's histogram is formed as
+// parent minus built child on the way, with subtract_kernel's checks, and written back.
+template <bool FIXED, bool WIDE, bool SUB, class Visit>
+__device__ __forceinline__ void scan_feature(const TrainerDev& a, const ScanNode<FIXED>& node,
+                                             uint32_t f, uint32_t nb, bool hm, const SlotWords& first,
+                                             PageTotals<FIXED>* totals, uint32_t& buf, uint32_t& err,
+                                             Visit&& visit) {
+  const uint32_t S = WIDE ? a.slots : uint32_t(kSlots);
+  const uint32_t pages = WIDE ? S / uint32_t(kSlots) : 1u;
+  const bool sub = SUB && node.sub_from != 0;
+  Stat<FIXED> miss = stat_zero<FIXED>(), carry = stat_zero<FIXED>();
+  if (WIDE && hm) {  // the last page's last slot, needed from the first page on
+    uint32_t ignored = 0;
+    SlotWords w = load_slots<FIXED, SUB>(a, node, f, nb, hm, S, S - 2);
+#pragma unroll
+    for (uint32_t k = 3; k < 6; ++k)
+      if (sub) w.own[k] = sibling_word<FIXED>(w.own[k], w.built[k], k - 3, ignored);
+    miss = slot_stat<FIXED>(w.own[3], w.own[4], w.own[5], ignored);
+  }
+  for (uint32_t p = 0; p < pages; ++p) {
+    const uint32_t s = p * uint32_t(kSlots) + 2 * threadIdx.x;
+    SlotWords w = first;
+    if (WIDE && p > 0) w = load_slots<FIXED, SUB>(a, node, f, nb, hm, S, s);
+    if (sub && pair_held(s, nb, hm, S)) {
+#pragma unroll
+      for (uint32_t k = 0; k < 6; ++k) w.own[k] = sibling_word<FIXED>(w.own[k], w.built[k], k % 3, err);
+      ulonglong2* out = reinterpret_cast<ulonglong2*>(
+          a.hist + ((size_t(node.slot) * a.features + f) * S + s) * 3);
+      out[0] = make_ulonglong2(w.own[0], w.own[1]);
+      out[1] = make_ulonglong2(w.own[2], w.own[3]);
+      out[2] = make_ulonglong2(w.own[4], w.own[5]);
+    }
+    const Stat<FIXED> b0 = slot_stat<FIXED>(w.own[0], w.own[1], w.own[2], err);
+    Stat<FIXED> b1 = slot_stat<FIXED>(w.own[3], w.own[4], w.own[5], err);
+    PageTotals<FIXED>& t = totals[buf];
+    buf ^= 1u;
+    if (hm && s + 2 == S) {
+      t.miss_count = b1.count;
+      t.miss_g = b1.g;
+      t.miss_h = b1.h;
+      b1 = stat_zero<FIXED>();
+    }
+    Stat<FIXED> total;
+    const Stat<FIXED> left1 =
+        stat_add<FIXED>(carry, page_prefix<FIXED>(stat_add<FIXED>(b0, b1), t, &total));
+    carry = stat_add<FIXED>(carry, total);
+    if (!WIDE && hm) {
+      miss.count = t.miss_count;
+      miss.g = t.miss_g;
+      miss.h = t.miss_h;
+    }
+    if (p + 1 == pages && carry.count + miss.count != node.parent.count) {
+      err |= kErrCountMismatch;
+      if (!WIDE) return;  // the same in every thread
+    }
+    if (p == 0 && nb >= 2 && missing_above<FIXED>(miss, node.parent, node.inv_h)) err |= kErrMissing;
+    const Stat<FIXED> nmp = stat_sub<FIXED>(node.parent, miss);
+    // A threshold's candidates. An empty bin's repeat threshold s-1's statistics exactly and
+    // lose the tie to them (IsBetterSplit prefers the lower threshold).
+    auto at = [&](uint32_t th, const Stat<FIXED>& left, bool empty_bin) {
+      if (th + 1 >= nb || (empty_bin && th > 0)) return;
+      if (left.count > nmp.count) {
+        err |= kErrPrefix;
+        return;
       }
+      const Stat<FIXED> right = stat_sub<FIXED>(nmp, left);
+      if (left.count == 0 && right.count == 0) return;
+      visit(stat_add<FIXED>(left, miss), right, th, 1u);
+      if (miss.count != 0) visit(left, stat_add<FIXED>(right, miss), th, 0u);
+    };
+    at(s, stat_sub<FIXED>(left1, b1), b0.count == 0);
+    at(s + 1, left1, b1.count == 0);
+  }
+}
+
+template <bool FIXED, bool WIDE>
+__global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(TrainerDev a, int parity) {
+  __shared__ PageTotals<FIXED> s_totals[2];
+  __shared__ uint32_t s_word[2][kScanFeaturesPerItem][kScanCtaWarps];
+  const TreeParams& P = a.params;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t F = a.features, S = WIDE ? a.slots : uint32_t(kSlots);
+  const uint32_t msl = min_leaf_rows(P);
+  const uint32_t n_nodes = a.ctl->n_nodes;
+  // An item: up to kScanFeaturesPerItem features of one node, fewer while the level has
+  // fewer (node, feature) pairs than that many per CTA.
+  const uint64_t pairs = uint64_t(n_nodes) * F;
+  const uint32_t per = uint32_t(min(uint64_t(kScanFeaturesPerItem), max(uint64_t(1), pairs / gridDim.x)));
+  const uint32_t chunks = ceil_div(F, per);
+  const uint32_t items = n_nodes * chunks;
+  uint32_t buf = 0, ib = 0, err = 0;
+  for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, ib ^= 1u) {
+    const uint32_t i = item / chunks, f0 = (item - i * chunks) * per;
+    const uint32_t nf = min(per, F - f0);
+    const NodeRec& rec = a.nodes[parity][i];
+    const TreeState& tree = a.trees[rec.tree];
+    const ScanNode<FIXED> node = scan_node<FIXED>(rec, tree.inv_h);
+    const int kh = tree.kh;
+    // A node with fewer than 2 * min_samples_leaf rows has no admissible split.
+    const bool usable = rec.count >= 2 * P.min_samples_leaf;
+    const uint32_t* allowed = a.node_allowed[parity] + size_t(i) * P.path_words;
+    auto active = [&](uint32_t k) -> bool {
+      return k < nf && usable && ((allowed[(f0 + k) >> 5] >> ((f0 + k) & 31)) & 1u);
+    };
+    bool act = active(0);
+    uint32_t nb = act ? a.bin_count[f0] : 0u;
+    bool hm = act && a.has_missing[f0] != 0;
+    SlotWords w = !WIDE && act ? load_slots<FIXED, true>(a, node, f0, nb, hm, S, 2 * threadIdx.x) : SlotWords{};
+    for (uint32_t k = 0; k < nf; ++k) {
+      // The next feature's words are in flight while this one is scanned (a wide feature's
+      // pages are many and its registers fewer: its own words only).
+      const uint32_t f = f0 + k;
+      const bool act_next = active(k + 1);
+      const uint32_t nb_next = act_next ? a.bin_count[f + 1] : 0u;
+      const bool hm_next = act_next && a.has_missing[f + 1] != 0;
+      const SlotWords w_next = !WIDE && act_next
+                                   ? load_slots<FIXED, true>(a, node, f + 1, nb_next, hm_next, S, 2 * threadIdx.x)
+                                   : SlotWords{};
+      if (WIDE && act) w = load_slots<FIXED, true>(a, node, f, nb, hm, S, 2 * threadIdx.x);
+      uint32_t word = 0, exact = 0;
+      if (act) {  // the same in every thread
+        const ScreenScale scale = screen_scale<FIXED>(P, P.has_monotonic ? a.monotonic[f] : int8_t(0), kh);
+        scan_feature<FIXED, WIDE, true>(
+            a, node, f, nb, hm, w, s_totals, buf, err,
+            [&](const Stat<FIXED>& cl, const Stat<FIXED>& cr, uint32_t, uint32_t) {
+              if (!scale.on) {
+                exact = kFeatureExact;
+                return;
+              }
+              float score = 0.0f;
+              const int cls = screen_classify<FIXED>(msl, scale, cl, cr, &score);
+              if (cls == 1) word = max(word, max(__float_as_uint(score), 1u));
+              if (cls == 2) exact = kFeatureExact;
+            });
+      }
+      word = __reduce_max_sync(0xffffffffu, word);
+      if (__any_sync(0xffffffffu, exact != 0)) word |= kFeatureExact;
+      if (lane == 0) s_word[ib][k][warp] = word;
+      act = act_next;
+      nb = nb_next;
+      hm = hm_next;
+      w = w_next;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t best = 0, flag = 0;
+      if (uint32_t(lane) < nf) {
+#pragma unroll
+        for (int q = 0; q < kScanCtaWarps; ++q) {
+          const uint32_t v = s_word[ib][lane][q];
+          best = max(best, v & ~kFeatureExact);
+          flag |= v & kFeatureExact;
+        }
+        a.feature_screen[size_t(i) * F + f0 + lane] = best | flag;
+      }
+      best = __reduce_max_sync(0xffffffffu, best);
+      if (lane == 0 && __uint_as_float(best) >= 1e-30f) atomicMax(a.node_screen + i, best);
+    }
+  }
+  if (err) raise(a.ctl, err);
+}
+
+// One CTA per node.
+template <bool FIXED, bool WIDE>
+__global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, int parity) {
+  __shared__ PageTotals<FIXED> s_totals[2];
+  __shared__ uint32_t s_list[kScanCta], s_listed;
+  __shared__ double s_gain[kScanCtaWarps];
+  __shared__ uint32_t s_key[kScanCtaWarps][5];  // valid, feature, threshold, default_left, thread
+  const TreeParams& P = a.params;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t F = a.features, S = WIDE ? a.slots : uint32_t(kSlots);
+  const uint32_t msl = min_leaf_rows(P);
+  const uint32_t n_nodes = a.ctl->n_nodes;
+  uint32_t buf = 0, err = 0;
+  for (uint32_t i = blockIdx.x; i < n_nodes; i += gridDim.x) {
+    const NodeRec& rec = a.nodes[parity][i];
+    const TreeState& tree = a.trees[rec.tree];
+    const double inv_g = tree.inv_g, inv_h = tree.inv_h;
+    const ScanNode<FIXED> node = scan_node<FIXED>(rec, inv_h);
+    const double lo = rec.lo, hi = rec.hi;
+    const float m = __uint_as_float(a.node_screen[i]);
+    const float cut = m >= 1e-30f ? m * (1.0f - 0x1p-18f) : -1.0f;
+    // The thread's best candidate.
+    uint32_t valid = 0, feature = 0, threshold = 0, default_left = 0;
+    double gain = 0.0;
+    Stat<FIXED> cl = stat_zero<FIXED>(), cr = stat_zero<FIXED>();
+    for (uint32_t base = 0; base < F; base += kScanCta) {
+      if (threadIdx.x == 0) s_listed = 0;
+      __syncthreads();
+      const uint32_t mine = base + threadIdx.x;
+      const uint32_t word = mine < F ? a.feature_screen[size_t(i) * F + mine] : 0u;
+      if (word != 0 && ((word & kFeatureExact) || !(__uint_as_float(word) < cut)))
+        s_list[atomicAdd(&s_listed, 1u)] = mine;  // any order: the best split is unique
       __syncthreads();
       const uint32_t listed = s_listed;
-      for (uint32_t k = 0; k < listed; ++k) eval_item(s_list[k]);
-      __syncthreads();  // the list is rewritten by the next batch
+      for (uint32_t k = 0; k < listed; ++k) {
+        const uint32_t f = s_list[k];
+        const uint32_t nb = a.bin_count[f];
+        const bool hm = a.has_missing[f] != 0;
+        const int8_t mono = P.has_monotonic ? a.monotonic[f] : int8_t(0);
+        const ScreenScale scale = screen_scale<FIXED>(P, mono, tree.kh);
+        const SlotWords w = load_slots<FIXED, false>(a, node, f, nb, hm, S, 2 * threadIdx.x);
+        scan_feature<FIXED, WIDE, false>(
+            a, node, f, nb, hm, w, s_totals, buf, err,
+            [&](const Stat<FIXED>& l, const Stat<FIXED>& r, uint32_t t, uint32_t dl) {
+              if (scale.on && cut > 0.0f) {
+                float score = 0.0f;
+                const int cls = screen_classify<FIXED>(msl, scale, l, r, &score);
+                if (!(cls == 2 || (cls == 1 && score >= cut))) return;
+              }
+              double g;
+              if (!exact_gain<FIXED>(P, l, r, inv_g, inv_h, mono, lo, hi, &g, err)) return;
+              bool take = !valid;
+              if (!take) {
+                if (g != gain) take = g > gain;
+                else if (f != feature) take = f < feature;
+                else if (t != threshold) take = t < threshold;
+                else take = dl > default_left;
+              }
+              if (take) {
+                valid = 1;
+                gain = g;
+                feature = f;
+                threshold = t;
+                default_left = dl;
+                cl = l;
+                cr = r;
+              }
+            });
+      }
+      __syncthreads();  // the list is rewritten
     }
-  } else {
-    for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) eval_item(item);
+    // The CTA's best: a warp argmax, then over the warps.
+    uint32_t win = threadIdx.x;
+    {
+      double g = gain;
+      uint32_t v = valid, f = feature, t = threshold, dl = default_left;
+      if (__any_sync(0xffffffffu, v != 0)) {
+        for (int off = 16; off > 0; off >>= 1) {
+          const double og = __shfl_xor_sync(0xffffffffu, g, off);
+          const uint32_t ov = __shfl_xor_sync(0xffffffffu, v, off);
+          const uint32_t of = __shfl_xor_sync(0xffffffffu, f, off);
+          const uint32_t ot = __shfl_xor_sync(0xffffffffu, t, off);
+          const uint32_t od = __shfl_xor_sync(0xffffffffu, dl, off);
+          const uint32_t ow = __shfl_xor_sync(0xffffffffu, win, off);
+          bool take;
+          if (ov != v) take = ov > v;
+          else if (!v) take = ow < win;
+          else if (og != g) take = og > g;
+          else if (of != f) take = of < f;
+          else if (ot != t) take = ot < t;
+          else if (od != dl) take = od > dl;
+          else take = ow < win;
+          if (take) {
+            g = og;
+            v = ov;
+            f = of;
+            t = ot;
+            dl = od;
+            win = ow;
+          }
+        }
+      }
+      if (lane == 0) {
+        s_gain[warp] = g;
+        s_key[warp][0] = v;
+        s_key[warp][1] = f;
+        s_key[warp][2] = t;
+        s_key[warp][3] = dl;
+        s_key[warp][4] = win;
+      }
+    }
+    __syncthreads();
+    int bw = -1;
+#pragma unroll
+    for (int q = 0; q < kScanCtaWarps; ++q) {
+      if (!s_key[q][0]) continue;
+      bool take = bw < 0;
+      if (!take) {
+        if (s_gain[q] != s_gain[bw]) take = s_gain[q] > s_gain[bw];
+        else if (s_key[q][1] != s_key[bw][1]) take = s_key[q][1] < s_key[bw][1];
+        else if (s_key[q][2] != s_key[bw][2]) take = s_key[q][2] < s_key[bw][2];
+        else take = s_key[q][3] > s_key[bw][3];
+      }
+      if (take) bw = q;
+    }
+    if (bw < 0) {
+      if (threadIdx.x == 0) {
+        SplitRec none;
+        none.valid = 0;
+        none.gain = 0.0;
+        none.feature = 0;
+        none.threshold = 0;
+        none.default_left = 1;
+        a.partial[i] = none;
+      }
+    } else if (threadIdx.x == s_key[bw][4]) {
+      const int8_t mono = P.has_monotonic ? a.monotonic[feature] : int8_t(0);
+      a.partial[i] = split_record<FIXED>(P, cl, cr, inv_g, inv_h, mono, lo, hi, gain, feature,
+                                         threshold, default_left);
+    }
+    __syncthreads();  // the argmax arrays and the list are rewritten by the next node
   }
-  (void)sizeof(V);
+  if (err) raise(a.ctl, err);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1332,12 +1788,12 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
   for (uint32_t t = threadIdx.x; t < a.n_trees; t += blockDim.x) tree_acc[t] = 0;
   __syncthreads();
 
-  // Phase A0: one warp per node merges the best splits of the node's feature chunks into
-  // chunk 0's record (lanes read chunks in parallel; the features of different chunks
+  // Phase A0 (a scan that left one record per feature chunk): one warp per node merges them
+  // into the first record (lanes read chunks in parallel; the features of different chunks
   // differ, so the total order of better_split has a unique winner among valid records).
-  if (depth < P.max_depth) {  // nodes at max_depth never split (tree.cpp:152-154)
+  const uint32_t nfc = a.partial_stride;
+  if (depth < P.max_depth && nfc > 1) {  // nodes at max_depth never split (tree.cpp:152-154)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const uint32_t nfc = a.n_fchunks;
     for (uint32_t i = warp; i < n; i += nw) {
       SplitRec* rec = a.partial + size_t(i) * nfc;
       uint32_t mine = lane < int(nfc) ? uint32_t(lane) : 0u;
@@ -1390,7 +1846,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
     bool first = false;
     if (i < n) {
       if (depth < P.max_depth) {
-        const SplitRec& b = a.partial[size_t(i) * a.n_fchunks];
+        const SplitRec& b = a.partial[size_t(i) * a.partial_stride];
         v[0] = b.valid;
         if (b.valid) v[1] = uint32_t(((b.lcount <= b.rcount ? b.lcount : b.rcount) + 255) / 256);
       }
@@ -1439,7 +1895,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       const bool acc = a.scratch_flags[i] && (a.trees[tree].leaf_count + within < P.max_leaves);
       v[0] = acc;
       if (acc) {
-        const SplitRec& b = a.partial[size_t(i) * a.n_fchunks];
+        const SplitRec& b = a.partial[size_t(i) * a.partial_stride];
         const uint32_t built = uint32_t(b.lcount <= b.rcount ? b.lcount : b.rcount);
         if (!last) {
           v[1] = ceil_div(built, item_rows);
@@ -1485,7 +1941,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
     TreeNodeOut* tn = a.tree_nodes + size_t(t) * a.max_tree_nodes;
     const bool acc = a.scratch_flags[i] != 0;
     if (acc) {
-      const SplitRec b = a.partial[size_t(i) * a.n_fchunks];
+      const SplitRec b = a.partial[size_t(i) * a.partial_stride];
       const uint32_t k = a.scratch_prefix[i];
       const uint32_t kt = k - tree_acc_base[t];
       atomicAdd(&tree_acc[t], 1u);
@@ -1537,8 +1993,8 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
         R.hi = b.ru;
         L.tree = R.tree = t;
         L.depth = R.depth = node.depth + 1;
-        // The sibling of the built child keeps the parent's slot; u8 datasets subtract in
-        // the next level's split scan (fused_sub), wide ones with subtract_kernel.
+        // The sibling of the built child keeps the parent's slot, from which the next
+        // level's split scan (fused_sub) or subtract_kernel subtracts the built child's.
         L.sub_from = (a.fused_sub && !build_left) ? new_slot + 1 : 0;
         R.sub_from = (a.fused_sub && build_left) ? new_slot + 1 : 0;
         next[2 * k] = L;
@@ -1849,9 +2305,9 @@ __global__ void __launch_bounds__(kPartThreads) partition_scatter_kernel(Trainer
 // scan of the children, merge (the children's best splits into the active lists).
 // ------------------------------------------------------------------------------------
 __device__ SplitRec merged_split(const TrainerDev& a, uint32_t i) {
-  SplitRec b = a.partial[size_t(i) * a.n_fchunks];
-  for (uint32_t c = 1; c < a.n_fchunks; ++c) {
-    const SplitRec x = a.partial[size_t(i) * a.n_fchunks + c];
+  SplitRec b = a.partial[size_t(i) * a.partial_stride];
+  for (uint32_t c = 1; c < a.partial_stride; ++c) {
+    const SplitRec x = a.partial[size_t(i) * a.partial_stride + c];
     if (better_split(x, b)) b = x;
   }
   return b;
@@ -1975,7 +2431,8 @@ __global__ void __launch_bounds__(1024) leafwise_select_kernel(TrainerDev a) {
           n.hi = left ? b.lu : b.ru;
           n.tree = t;
           n.depth = depth;
-          n.sub_from = 0;  // leaf-wise steps subtract with subtract_kernel
+          // As in finalize: the sibling of the built child keeps the parent's slot.
+          n.sub_from = (a.fused_sub && grow && left != build_left) ? new_slot + 1 : 0;
           kid[k].best = no_split();
           kid[k].parity = np;
           kid[k].scanned = grow ? 0u : 1u;
@@ -2501,41 +2958,48 @@ cudaError_t launch_subtract(const TrainerDev& a, int grid, cudaStream_t s) {
   subtract_kernel<<<grid, 256, 0, s>>>(a);
   return cudaGetLastError();
 }
-template <bool FIXED, bool SCREEN, bool WIDE>
-cudaError_t launch_scan_shape(const TrainerDev& a, int parity, int grid, int threads, cudaStream_t s) {
-  const size_t smem = scan_smem_per_warp<FIXED, SCREEN>() * size_t(threads / 32);
+template <bool FIXED, bool WIDE>
+cudaError_t launch_scan_one(const TrainerDev& a, int parity, int grid, int threads, cudaStream_t s) {
+  const size_t smem = scan_smem_per_warp<FIXED>() * size_t(threads / 32);
   static std::atomic<unsigned long long> configured{0};  // one bit per device
-  const cudaError_t err = opt_in_dynamic_smem(configured, split_scan_kernel<FIXED, SCREEN, WIDE>,
-                                              scan_smem_per_warp<FIXED, SCREEN>() * (kScanThreadsMax / 32));
+  const cudaError_t err = opt_in_dynamic_smem(configured, split_scan_kernel<FIXED, WIDE>,
+                                              scan_smem_per_warp<FIXED>() * (kScanThreadsMax / 32));
   if (err != cudaSuccess) return err;
-  split_scan_kernel<FIXED, SCREEN, WIDE><<<grid, threads, smem, s>>>(a, parity);
+  split_scan_kernel<FIXED, WIDE><<<grid, threads, smem, s>>>(a, parity);
   return cudaGetLastError();
 }
-template <bool FIXED, bool SCREEN>
-cudaError_t launch_scan_variant(const TrainerDev& a, int parity, int grid, int threads, cudaStream_t s) {
-  if (a.slots == uint32_t(kSlots)) return launch_scan_shape<FIXED, SCREEN, false>(a, parity, grid, threads, s);
-  if (a.slots < uint32_t(kSlots) || a.slots % uint32_t(kSlots)) return cudaErrorInvalidValue;
-  return launch_scan_shape<FIXED, SCREEN, true>(a, parity, grid, threads, s);
+template <bool FIXED, bool WIDE>
+cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes, cudaStream_t s) {
+  const uint64_t resident = uint64_t(a.sm_count ? a.sm_count : 152) * 6;
+  const uint32_t screen = uint32_t(std::min<uint64_t>(resident, uint64_t(max_nodes) * a.features));
+  split_screen_kernel<FIXED, WIDE><<<screen, kScanCta, 0, s>>>(a, parity);
+  const cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  const uint32_t exact = uint32_t(std::min<uint64_t>(resident, max_nodes));
+  split_exact_kernel<FIXED, WIDE><<<exact, kScanCta, 0, s>>>(a, parity);
+  return cudaGetLastError();
 }
 
 uint32_t split_scan_kernels(const TrainerDev& a) {
   return a.node_screen && a.scan_two_phase ? 2u : 1u;
 }
 
-cudaError_t launch_split_scan(const TrainerDev& a, int parity, int grid, cudaStream_t s) {
-  const int threads = int(a.scan_threads);
-  if (threads < 32 || threads > kScanThreadsMax || threads % 32) return cudaErrorInvalidValue;
-  const bool fixed = a.mode == kModeFixed;
+cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, int grid, cudaStream_t s) {
+  const bool fixed = a.mode == kModeFixed, wide = a.slots != uint32_t(kSlots);
+  if (a.slots < uint32_t(kSlots) || a.slots % uint32_t(kSlots) || max_nodes == 0) return cudaErrorInvalidValue;
   if (split_scan_kernels(a) == 2) {
     // node_screen was cleared by the level's zero_build_slots_kernel.
-    cudaError_t err;
-    // The screen phase holds about half the registers: twice the CTAs.
-    err = fixed ? launch_scan_variant<true, true>(a, parity, 2 * grid, threads, s)
-                : launch_scan_variant<false, true>(a, parity, 2 * grid, threads, s);
-    if (err != cudaSuccess) return err;
+    if (fixed) return wide ? launch_scan_two<true, true>(a, parity, max_nodes, s)
+                           : launch_scan_two<true, false>(a, parity, max_nodes, s);
+    return wide ? launch_scan_two<false, true>(a, parity, max_nodes, s)
+                : launch_scan_two<false, false>(a, parity, max_nodes, s);
   }
-  return fixed ? launch_scan_variant<true, false>(a, parity, grid, threads, s)
-               : launch_scan_variant<false, false>(a, parity, grid, threads, s);
+  const int threads = int(a.scan_threads);
+  if (threads < 32 || threads > kScanThreadsMax || threads % 32) return cudaErrorInvalidValue;
+  if (fixed) return wide ? launch_scan_one<true, true>(a, parity, grid, threads, s)
+                         : launch_scan_one<true, false>(a, parity, grid, threads, s);
+  return wide ? launch_scan_one<false, true>(a, parity, grid, threads, s)
+              : launch_scan_one<false, false>(a, parity, grid, threads, s);
 }
 cudaError_t launch_leafwise_init(const TrainerDev& a, cudaStream_t s) {
   leafwise_init_kernel<<<1, 256, 0, s>>>(a);

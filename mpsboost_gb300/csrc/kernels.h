@@ -63,17 +63,18 @@ struct TrainerDev {
   uint32_t* node_path[2];       // [max_level_nodes][path_words]
   uint32_t* node_allowed[2];    // [max_level_nodes][path_words]
   uint32_t max_level_nodes;
-  SplitRec* partial;            // [max_level_nodes][n_fchunks]
-  // Two-phase split scan (scan_two_phase: the FP32 screen applies): [max_level_nodes]
+  SplitRec* partial;            // [max_level_nodes][partial_stride]
+  uint32_t partial_stride;      // records per node: 1 (two-launch scan) or n_fchunks
+  // Two-launch split scan (scan_two_phase: the FP32 screen applies): [max_level_nodes]
   // maximum FP32 screen score of each node's certainly admissible candidates (float
   // bits; zeroed by each level's zero_build_slots_kernel, which every scan of the trainer
-  // follows) and [max_level_nodes][n_fchunks] each chunk's maximum
-  // and exact flag. Null node_screen: one launch, each feature screened on its own (the
-  // per-feature entry point needs every feature's best split).
+  // follows) and [max_level_nodes][features] each feature's maximum and exact flag. Null
+  // node_screen: one launch, each feature screened on its own (the per-feature entry point
+  // needs every feature's best split).
   uint32_t* node_screen;
-  uint32_t* chunk_screen;
+  uint32_t* feature_screen;
   uint32_t scan_two_phase;
-  uint32_t n_fchunks;           // feature chunks of the split scan (32 features each)
+  uint32_t n_fchunks;           // feature chunks of the one-launch split scan (a warp each feature)
   BuildEntry* build;            // [max_level_nodes]
   uint32_t* build_prefix;       // [max_level_nodes + 1] chunk prefix
   SubEntry* sub;                // [max_level_nodes]
@@ -101,7 +102,7 @@ struct TrainerDev {
   uint32_t n_classes;           // native softmax: K classes, one tree per class in turn;
                                 // preds holds the margins [K][n_rows] and the round
                                 // counter modulo K is the class of the current tree
-  uint32_t scan_threads;        // block size of the split scan (multiple of 32)
+  uint32_t scan_threads;        // block size of the one-launch split scan (multiple of 32)
   uint32_t fused_sub;           // level-wise siblings are subtracted by the split scan
                                 // (NodeRec::sub_from), not by subtract_kernel
   // finalize scratch
@@ -177,7 +178,9 @@ cudaError_t launch_leafwise_finish(const TrainerDev& a, cudaStream_t stream);
 // into the roots' slots (after a gradient-only build).
 cudaError_t launch_root_cache(const TrainerDev& a, int save, int grid, cudaStream_t stream);
 cudaError_t launch_subtract(const TrainerDev& a, int grid, cudaStream_t stream);
-cudaError_t launch_split_scan(const TrainerDev& a, int parity, int grid, cudaStream_t stream);
+// max_nodes: a bound on the nodes the launch scans (ctl->n_nodes), from the level.
+cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, int grid,
+                              cudaStream_t stream);
 uint32_t split_scan_kernels(const TrainerDev& a);  // launches per launch_split_scan
 cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, cudaStream_t stream);
 cudaError_t launch_partition(const TrainerDev& a, int grid, cudaStream_t stream);

@@ -274,11 +274,12 @@ int mpsb_cuda_scan_splits(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     a.max_tree_nodes = 1;
     a.scan_threads = 32;  // one feature per CTA: partial[f] is feature f's best split
     a.n_fchunks = F;
+    a.partial_stride = F;
     a.partial = ss.alloc<SplitRec>(F);
     CK(launch_root_stats(a, s));
     const uint32_t one = 1;
     CK(cudaMemcpyAsync(&a.ctl->n_nodes, &one, sizeof one, cudaMemcpyHostToDevice, s));
-    CK(launch_split_scan(a, 0, b->sm_count * 8, s));
+    CK(launch_split_scan(a, 0, 1, b->sm_count * 8, s));
     check_ctl(a, s);
     std::vector<SplitRec> rec(F);
     CK(cudaMemcpy(rec.data(), a.partial, F * sizeof(SplitRec), cudaMemcpyDeviceToHost));
