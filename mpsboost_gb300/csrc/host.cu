@@ -850,7 +850,7 @@ struct mpsb_cuda_trainer {
         CK(cudaStreamWaitEvent(side, fork_ev, 0));
         CK(launch_zero_build_slots(dev, grid(8), side)); ++k;
         CK(cudaEventRecord(zero_ev, side));
-        CK(launch_partition(dev, grid(4), s)); k += kPartitionKernels;
+        CK(launch_partition(dev, level_nodes(d), grid(4), s)); k += partition_kernels(dev, level_nodes(d));
       }
     }
     CK(launch_apply_leaves(dev, grid(8), s)); k += 2;
@@ -878,7 +878,7 @@ struct mpsb_cuda_trainer {
     CK(launch_leafwise_init(dev, s)); ++k;
     for (uint32_t step = 0; step < lw_steps && depth > 0; ++step) {
       CK(launch_leafwise_select(dev, s)); ++k;
-      CK(launch_partition(dev, grid(4), s)); k += kPartitionKernels;
+      CK(launch_partition(dev, n_trees, grid(4), s)); k += partition_kernels(dev, n_trees);
       CK(launch_zero_build_slots(dev, grid(8), s)); ++k;
       CK(launch_hist_build(build_view(), hcfg, grid(1), s)); ++k;
       if (!dev.fused_sub) { CK(launch_subtract(dev, grid(8), s)); ++k; }

@@ -2293,6 +2293,143 @@ __global__ void __launch_bounds__(kPartThreads) partition_scatter_kernel(Trainer
   if (err) raise(a.ctl, err);
 }
 
+// One launch for levels of few rows: a thread-block cluster per split node. Each CTA routes
+// a contiguous part of the node's rows (flags in shared memory), the CTAs read each other's
+// left counts through distributed shared memory, and each writes its part. Bound by the
+// latency of its two passes over the part; the three launches above, which spread a node's
+// rows over the whole GPU, cost 20 us on a 100,000-row node where this takes one launch.
+constexpr int kClusterThreads = 1024;
+constexpr uint32_t kClusterPartRows = 65536;  // rows per CTA (flag words in shared memory)
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_ctas() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The u32 at shared address `addr` of the cluster's CTA `rank`.
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr, uint32_t rank) {
+  uint32_t remote, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];\n" : "=r"(v) : "r"(remote) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(kClusterThreads) partition_cluster_kernel(TrainerDev a) {
+  constexpr uint32_t kWords = kClusterPartRows / 32;
+  constexpr int kUnroll = 4;
+  __shared__ uint32_t s_flags[kWords], s_prefix[kWords];
+  __shared__ uint32_t s_scan[33], s_left;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t rank = cluster_rank(), ctas = cluster_ctas();
+  const uint32_t n_part = a.ctl->n_part;
+  uint32_t err = 0;
+  for (uint32_t e = blockIdx.x / ctas; e < n_part; e += gridDim.x / ctas) {  // the cluster's nodes
+    const PartEntry pe = a.part[e];
+    // The CTA's rows: [start, start + count), whole 32-row words.
+    const uint32_t per = ceil_div(ceil_div(pe.seg_cnt, ctas), 32u) * 32u;
+    const uint32_t start = min(rank * per, pe.seg_cnt);
+    uint32_t count = min(per, pe.seg_cnt - start);
+    if (count > kClusterPartRows) {  // the launch is chosen for nodes that fit
+      err |= kErrCapacity;
+      count = 0;
+    }
+    const size_t src_off = (size_t(pe.tree) * 2 + pe.parity) * a.seg_stride + pe.seg_off + start;
+    const size_t dst_off = (size_t(pe.tree) * 2 + (pe.parity ^ 1)) * a.seg_stride + pe.seg_off;
+    const uint32_t* src = a.rows + src_off;
+    uint32_t* dst = a.rows + dst_off;
+    const uint32_t words = ceil_div(count, 32u);
+    for (uint32_t p0 = 0; p0 < words * 32u; p0 += kUnroll * kClusterThreads) {
+      uint32_t r[kUnroll];
+#pragma unroll
+      for (int k = 0; k < kUnroll; ++k) {
+        const uint32_t p = p0 + uint32_t(k * kClusterThreads) + threadIdx.x;
+        r[k] = p < count ? __ldg(src + p) : 0xffffffffu;
+      }
+      bool left[kUnroll];
+#pragma unroll
+      for (int k = 0; k < kUnroll; ++k)
+        left[k] = r[k] < a.n_rows && row_goes_left(a, r[k], pe.feature, pe.threshold, pe.default_left);
+#pragma unroll
+      for (int k = 0; k < kUnroll; ++k) {
+        const uint32_t word = __ballot_sync(0xffffffffu, left[k]);
+        const uint32_t w = (p0 + uint32_t(k * kClusterThreads)) / 32u + uint32_t(warp);
+        if (lane == 0 && w < words) s_flags[w] = word;
+      }
+    }
+    __syncthreads();
+    // Exclusive prefix of the words' left rows, a run of neighbouring words per thread.
+    {
+      constexpr uint32_t kRun = kWords / kClusterThreads;
+      uint32_t c[kRun], v[1] = {0}, tot[1];
+#pragma unroll
+      for (uint32_t q = 0; q < kRun; ++q) {
+        const uint32_t w = threadIdx.x * kRun + q;
+        c[q] = w < words ? uint32_t(__popc(s_flags[w])) : 0u;
+        v[0] += c[q];
+      }
+      block_scan<1>(v, tot, s_scan);
+      uint32_t run = v[0];
+#pragma unroll
+      for (uint32_t q = 0; q < kRun; ++q) {
+        const uint32_t w = threadIdx.x * kRun + q;
+        if (w < words) s_prefix[w] = run;
+        run += c[q];
+      }
+      if (threadIdx.x == 0) s_left = tot[0];
+    }
+    cluster_barrier();  // every CTA's left count (and this CTA's prefix) is written
+    uint32_t left_before = 0, left_all = 0;
+    {
+      const uint32_t mine = uint32_t(lane) < ctas
+                                ? ld_cluster_u32(static_cast<uint32_t>(__cvta_generic_to_shared(&s_left)), uint32_t(lane))
+                                : 0u;
+      left_all = __reduce_add_sync(0xffffffffu, mine);
+      left_before = __reduce_add_sync(0xffffffffu, uint32_t(lane) < rank ? mine : 0u);
+    }
+    if (left_all != pe.lcount) err |= kErrPartition;
+    if (rank == 0 && threadIdx.x == 0) atomicAdd(&a.ctl->rows_partitioned, (unsigned long long)pe.seg_cnt);
+    const uint32_t right_before = start - left_before;
+    const float2* gh_src = a.gh_ordered ? a.gh + src_off : nullptr;
+    float2* gh_dst = a.gh_ordered ? a.gh + dst_off : nullptr;
+    for (uint32_t p0 = 0; p0 < count; p0 += kUnroll * kClusterThreads) {
+      uint32_t r[kUnroll];
+      float2 g[kUnroll];
+#pragma unroll
+      for (int k = 0; k < kUnroll; ++k) {
+        const uint32_t p = p0 + uint32_t(k * kClusterThreads) + threadIdx.x;
+        r[k] = p < count ? __ldg(src + p) : 0u;
+        g[k] = (p < count && a.gh_ordered) ? __ldg(gh_src + p) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int k = 0; k < kUnroll; ++k) {
+        const uint32_t p = p0 + uint32_t(k * kClusterThreads) + threadIdx.x;
+        if (p >= count) continue;
+        const uint32_t word = s_flags[p >> 5];
+        const uint32_t lpos = s_prefix[p >> 5] + uint32_t(__popc(word & ((1u << lane) - 1u)));
+        const bool left = (word >> lane) & 1u;
+        const uint32_t rel = left ? left_before + lpos : pe.lcount + right_before + (p - lpos);
+        if (rel < pe.seg_cnt) {  // always true when the counts agree
+          dst[rel] = r[k];
+          if (a.gh_ordered) gh_dst[rel] = g[k];
+        } else {
+          err |= kErrPartition;
+        }
+      }
+    }
+    // No CTA exits or rewrites its count and flags while another reads the count.
+    cluster_barrier();
+  }
+  if (err) raise(a.ctl, err);
+}
+
 // ------------------------------------------------------------------------------------
 // Leaf-wise growth (TrainLeafWiseRegressionTree, tree_leafwise.cpp:56-142)
 //
@@ -3021,7 +3158,42 @@ cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, cud
   finalize_kernel<<<1, 1024, 0, s>>>(a, parity, depth);
   return cudaGetLastError();
 }
-cudaError_t launch_partition(const TrainerDev& a, int grid, cudaStream_t s) {
+// CTAs per node of the cluster launch for a level of at most max_nodes split nodes over
+// `rows` rows in all (0: the three launches). As many as fit the GPU at once (one of these
+// CTAs per SM), up to the 16 of a non-portable cluster; not where that leaves a thread more
+// than 48 rows on average.
+static uint32_t partition_cluster_ctas(const TrainerDev& a, uint32_t max_nodes, uint64_t rows) {
+  const uint32_t sms = a.sm_count ? a.sm_count : 152;
+  uint32_t ctas = 16;
+  while (ctas > 1 && uint64_t(max_nodes) * ctas > sms) ctas >>= 1;
+  if (uint64_t(a.seg_stride) > uint64_t(ctas) * kClusterPartRows) return 0;  // the largest node possible
+  const uint64_t threads = std::min<uint64_t>(uint64_t(max_nodes) * ctas, sms) * kClusterThreads;
+  return rows <= 48 * threads ? ctas : 0;
+}
+
+uint32_t partition_kernels(const TrainerDev& a, uint32_t max_nodes) {
+  return partition_cluster_ctas(a, max_nodes, uint64_t(a.n_trees) * a.seg_stride) ? 1u : 3u;
+}
+
+cudaError_t launch_partition(const TrainerDev& a, uint32_t max_nodes, int grid, cudaStream_t s) {
+  if (const uint32_t ctas = partition_cluster_ctas(a, max_nodes, uint64_t(a.n_trees) * a.seg_stride)) {
+    static std::atomic<unsigned long long> configured{0};  // one bit per device
+    cudaError_t err = allow_large_clusters(configured, partition_cluster_kernel);
+    if (err != cudaSuccess) return err;
+    const uint32_t sms = a.sm_count ? a.sm_count : 152;
+    const uint32_t clusters = std::min(max_nodes, std::max(1u, sms / ctas));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(clusters * ctas);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, partition_cluster_kernel, a);
+  }
   partition_count_kernel<<<grid, kPartThreads, 0, s>>>(a);
   partition_scan_kernel<<<grid, 1024, 0, s>>>(a);
   partition_scatter_kernel<<<grid, kPartThreads, 0, s>>>(a);

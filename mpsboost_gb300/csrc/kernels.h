@@ -183,7 +183,9 @@ cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_node
                               cudaStream_t stream);
 uint32_t split_scan_kernels(const TrainerDev& a);  // launches per launch_split_scan
 cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, cudaStream_t stream);
-cudaError_t launch_partition(const TrainerDev& a, int grid, cudaStream_t stream);
+// max_nodes: a bound on the nodes the launch partitions (ctl->n_part).
+cudaError_t launch_partition(const TrainerDev& a, uint32_t max_nodes, int grid, cudaStream_t stream);
+uint32_t partition_kernels(const TrainerDev& a, uint32_t max_nodes);  // launches per launch_partition
 cudaError_t launch_partition_count(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_partition_finish(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_apply_leaves(const TrainerDev& a, int grid, cudaStream_t stream);
@@ -233,7 +235,17 @@ inline cudaError_t opt_in_dynamic_smem(std::atomic<unsigned long long>& devices,
   return err;
 }
 
-// Number of kernels each launch_* helper enqueues (launch accounting).
-constexpr int kPartitionKernels = 3;
+// Allows `kernel` clusters of more than the portable 8 CTAs, once per device as above.
+template <typename Kernel>
+inline cudaError_t allow_large_clusters(std::atomic<unsigned long long>& devices, Kernel kernel) {
+  int device = 0;
+  cudaError_t err = cudaGetDevice(&device);
+  if (err != cudaSuccess) return err;
+  const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
+  if (bit && (devices.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (err == cudaSuccess && bit) devices.fetch_or(bit, std::memory_order_acq_rel);
+  return err;
+}
 
 }  // namespace mpsb

@@ -42,3 +42,13 @@ def test_split_scan_edges(backend, port, bins, features, nan, leaves):
     growth = dict(growth_strategy="leaf_wise", max_leaves=leaves) if leaves else {}
     assert_equals_replica(backend, port, x, y, w, bins, n_estimators=2, learning_rate=0.3, max_depth=5,
                           min_samples_leaf=4, min_child_weight=2.0, **growth)
+
+
+# Rows around the 32-row flag words, a CTA's 1,024 rows, 16 CTAs of a cluster and their
+# 48 rows per thread (786,432: the last single-launch partition of a root, and one past it).
+@pytest.mark.parametrize("rows", [33, 511, 1025, 16 * 1024 - 1, 16 * 1024 + 1, 70_001, 786_432, 786_433])
+def test_partition_edges(backend, port, rows):
+    x = seeded_matrix(rows, rows, 3, 0.05, integer_columns=1)
+    y, w = targets(x, rows)
+    assert_equals_replica(backend, port, x, y, w, 64, n_estimators=2, learning_rate=0.3, max_depth=4,
+                          min_samples_leaf=2)
