@@ -842,7 +842,7 @@ struct mpsb_cuda_trainer {
       if (depth > 0) {
         CK(launch_split_scan(dev, parity, level_nodes(d), grid(4), s)); k += split_scan_kernels(dev);
       }
-      CK(launch_finalize(dev, parity, d, s)); ++k;
+      CK(launch_finalize(dev, parity, d, level_nodes(d), s)); ++k;
       if (d + 1 < depth) {
         // The next level's build slots (named by the finalize) are cleared on the side
         // stream while the partition moves the rows.

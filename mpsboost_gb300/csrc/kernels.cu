@@ -1774,6 +1774,25 @@ __device__ bool bounded_leaf(const TreeParams& p, double g, double h, double lo,
   return true;
 }
 
+// InteractionAllowsFeature (tree_interactions.cpp:32-45) of a child: word w of its allowed
+// features from its path words.
+__device__ __forceinline__ uint32_t allowed_word(const TrainerDev& a, const uint32_t* path,
+                                                 uint32_t tree, uint32_t w) {
+  const TreeParams& P = a.params;
+  uint32_t allowed = 0xffffffffu;
+  if (P.n_groups > 0) {
+    allowed = 0;
+    for (uint32_t g = 0; g < P.n_groups; ++g) {
+      bool subset = true;
+      for (uint32_t u = 0; u < P.path_words && subset; ++u)
+        subset = (path[u] & ~a.group_masks[g * P.path_words + u]) == 0;
+      if (subset) allowed |= a.group_masks[g * P.path_words + w];
+    }
+  }
+  if (a.tree_feature_masks != nullptr) allowed &= a.tree_feature_masks[tree * P.path_words + w];
+  return allowed;
+}
+
 __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity, uint32_t depth) {
   __shared__ uint32_t sh[33 * 6];
   Control* ctl = a.ctl;
@@ -2006,19 +2025,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
           a.node_path[parity ^ 1][(2 * k + 1) * W + w] = path;
         }
         for (uint32_t w = 0; w < W; ++w) {
-          uint32_t allowed = 0xffffffffu;
-          if (P.n_groups > 0) {  // InteractionAllowsFeature (tree_interactions.cpp:32-45)
-            allowed = 0;
-            for (uint32_t g = 0; g < P.n_groups; ++g) {
-              bool subset = true;
-              for (uint32_t u = 0; u < W && subset; ++u) {
-                const uint32_t gm = a.group_masks[g * W + u];
-                subset = (a.node_path[parity ^ 1][(2 * k) * W + u] & ~gm) == 0;
-              }
-              if (subset) allowed |= a.group_masks[g * W + w];
-            }
-          }
-          if (a.tree_feature_masks != nullptr) allowed &= a.tree_feature_masks[t * W + w];
+          const uint32_t allowed = allowed_word(a, a.node_path[parity ^ 1] + size_t(2 * k) * W, t, w);
           a.node_allowed[parity ^ 1][(2 * k) * W + w] = allowed;
           a.node_allowed[parity ^ 1][(2 * k + 1) * W + w] = allowed;
         }
@@ -2121,6 +2128,238 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       ctl->hist_items = carry6[1] * a.nfb;
       ctl->part_chunks = carry6[2];
       ctl->split_items = 2 * n_acc * a.n_fchunks;
+      ctl->item_rows = item_rows;
+    }
+    ctl->hist_counter = 0;
+  }
+}
+
+// The finalize of a level with at most one node per thread (up to kNodeFinalizeMax): a
+// node's record, split and prefixes stay in its thread's registers, where the general
+// kernel walks the nodes in five passes that each read back from global memory what the
+// pass before wrote. Latency-bound: a chain of three loads (counts, records, tree state),
+// two block scans and the stores.
+constexpr uint32_t kNodeFinalizeMax = 512;
+
+__global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(TrainerDev a, int parity,
+                                                                          uint32_t depth) {
+  __shared__ uint32_t sh[33 * 6];
+  __shared__ uint32_t s_valid_base[kNodeFinalizeMax], s_acc_base[kNodeFinalizeMax + 1];
+  __shared__ uint32_t s_node_of[kNodeFinalizeMax];  // accepted split k: its node
+  Control* ctl = a.ctl;
+  const TreeParams& P = a.params;
+  const uint32_t n = ctl->n_nodes;
+  const uint32_t free_top = ctl->free_top;
+  const uint32_t leafseg_base = ctl->n_leafseg, leafchunk_base = ctl->leaf_chunks;
+  const uint32_t W = P.path_words;
+  const bool last = depth + 1 >= P.max_depth;  // children are leaves
+  const uint32_t i = threadIdx.x;
+  uint32_t err = 0;
+  if (n > blockDim.x) {  // the launch covers the level's bound
+    if (i == 0) raise(ctl, kErrCapacity);
+    return;
+  }
+  NodeRec node;
+  SplitRec b;
+  node.tree = 0;
+  node.seg_cnt = 0;
+  b.valid = 0;
+  uint32_t leaf_count = 0, tree_nodes = 0;
+  bool first = false;
+  double lv = 0.0, rv = 0.0;
+  if (i < n) {
+    node = a.nodes[parity][i];
+    if (depth < P.max_depth) b = a.partial[size_t(i) * a.partial_stride];  // else: tree.cpp:152-154
+    first = i == 0 || a.nodes[parity][i - 1].tree != node.tree;
+    leaf_count = a.trees[node.tree].leaf_count;
+    tree_nodes = a.trees[node.tree].n_tree_nodes;
+  }
+  const uint32_t built = b.valid ? uint32_t(b.lcount <= b.rcount ? b.lcount : b.rcount) : 0u;
+  // Valid splits before the node and, through its tree's ordinal in the level, before its
+  // tree's first node; rows the next level builds.
+  uint32_t v3[3] = {b.valid ? 1u : 0u, (built + 255) / 256, first ? 1u : 0u}, tot3[3];
+  block_scan<3>(v3, tot3, sh);
+  const uint32_t ord = first ? v3[2] : (i < n ? v3[2] - 1 : 0u);
+  if (first) s_valid_base[ord] = v3[0];
+  __syncthreads();
+  const uint32_t base_per_sm = a.items_per_sm ? a.items_per_sm : 3u;
+  const uint32_t level_per_sm = n >= 8 ? base_per_sm + 1 : (base_per_sm > 2 ? base_per_sm - 1 : base_per_sm);
+  const uint32_t item_rows =
+      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(tot3[1]) * 256, a.nfb, a.sm_count, level_per_sm);
+  const bool acc = i < n && b.valid && (leaf_count + (v3[0] - s_valid_base[ord]) < P.max_leaves);
+  const bool leafseg = i < n && (!acc || last);
+  // 0 accepted, 1 build chunks, 2 partition chunks, 3 leaf segments, 4 leaf chunks, 5 freed.
+  uint32_t v[6] = {acc ? 1u : 0u,
+                   acc && !last ? ceil_div(built, item_rows) : 0u,
+                   acc && !last ? ceil_div(node.seg_cnt, kPartChunk) : 0u,
+                   leafseg ? 1u : 0u,
+                   leafseg ? ceil_div(node.seg_cnt, kApplyChunk) : 0u,
+                   i < n && !acc && !last ? 1u : 0u};
+  uint32_t tot[6];
+  block_scan<6>(v, tot, sh);
+  const uint32_t n_acc = tot[0], k = v[0];
+  if (first) s_acc_base[ord] = k;
+  if (i == 0) s_acc_base[tot3[2]] = n_acc;
+  if (acc) s_node_of[k] = i;
+  const uint32_t new_slot = acc && !last ? a.free_stack[free_top - 1 - k] : 0u;
+  if (acc) {
+    if (!bounded_leaf(P, b.lg, b.lh, b.ll, b.lu, &lv)) err |= kErrNonFinite;
+    if (!bounded_leaf(P, b.rg, b.rh, b.rl, b.ru, &rv)) err |= kErrNonFinite;
+  }
+  __syncthreads();  // also: the new slots are read before stopped nodes return theirs
+  if (i < n) {
+    const uint32_t t = node.tree;
+    TreeNodeOut* tn = a.tree_nodes + size_t(t) * a.max_tree_nodes;
+    LeafSeg ls;
+    ls.tree = t;
+    ls.parity = uint32_t(parity);
+    ls.seg_off = node.seg_off;
+    ls.seg_cnt = node.seg_cnt;
+    ls.split = 0;
+    ls.feature = ls.threshold = ls.default_left = 0;
+    ls.value = ls.left_value = ls.right_value = 0.0;
+    const uint32_t li = tree_nodes + 2 * (k - s_acc_base[ord]), ri = li + 1;
+    const bool room = !acc || ri < a.max_tree_nodes;
+    if (!room) err |= kErrCapacity;
+    if (acc && room) {
+      write_leaf(&tn[li], lv);
+      write_leaf(&tn[ri], rv);
+      TreeNodeOut& pn = tn[node.node_index];
+      pn.feature_index = b.feature;
+      pn.threshold_bin = b.threshold;
+      pn.left_child = li;
+      pn.right_child = ri;
+      pn.leaf_value = 0.0;
+      pn.gain = b.gain;
+      pn.default_left = uint8_t(b.default_left);
+      pn.flags = 0;
+      if (b.lcount + b.rcount != node.seg_cnt) err |= kErrPartition;
+      if (!last) {
+        const bool build_left = b.lcount <= b.rcount;
+        NodeRec c;  // the left child, then the right one
+        c.tree = t;
+        c.depth = node.depth + 1;
+        c.seg_off = node.seg_off;
+        c.seg_cnt = uint32_t(b.lcount);
+        c.node_index = li;
+        c.slot = build_left ? new_slot : node.slot;
+        c.count = b.lcount;
+        c.qg = b.lqg;
+        c.qh = b.lqh;
+        c.g = b.lg;
+        c.h = b.lh;
+        c.lo = b.ll;
+        c.hi = b.lu;
+        // The sibling of the built child keeps the parent's slot, from which the next
+        // level's split scan (fused_sub) or subtract_kernel subtracts the built child's.
+        c.sub_from = (a.fused_sub && !build_left) ? new_slot + 1 : 0;
+        a.nodes[parity ^ 1][2 * k] = c;
+        BuildEntry be;
+        be.tree = t;
+        be.parity = uint32_t(parity ^ 1);
+        be.seg_off = node.seg_off;
+        be.seg_cnt = uint32_t(b.lcount);
+        be.slot = new_slot;
+        be.pad = 0;
+        c.seg_off = node.seg_off + uint32_t(b.lcount);
+        c.seg_cnt = uint32_t(b.rcount);
+        c.node_index = ri;
+        c.slot = build_left ? node.slot : new_slot;
+        c.count = b.rcount;
+        c.qg = b.rqg;
+        c.qh = b.rqh;
+        c.g = b.rg;
+        c.h = b.rh;
+        c.lo = b.rl;
+        c.hi = b.ru;
+        c.sub_from = (a.fused_sub && build_left) ? new_slot + 1 : 0;
+        a.nodes[parity ^ 1][2 * k + 1] = c;
+        if (!build_left) {
+          be.seg_off = c.seg_off;
+          be.seg_cnt = c.seg_cnt;
+        }
+        a.build[k] = be;
+        a.build_prefix[k] = v[1];
+        a.sub[k] = SubEntry{node.slot, new_slot};
+        PartEntry pe;
+        pe.tree = t;
+        pe.parity = uint32_t(parity);
+        pe.seg_off = node.seg_off;
+        pe.seg_cnt = node.seg_cnt;
+        pe.feature = b.feature;
+        pe.threshold = b.threshold;
+        pe.default_left = b.default_left;
+        pe.lcount = uint32_t(b.lcount);
+        a.part[k] = pe;
+        a.part_prefix[k] = v[2];
+        if (P.n_groups > 0) {
+          uint32_t* path = a.node_path[parity ^ 1] + size_t(2 * k) * W;
+          for (uint32_t w = 0; w < W; ++w) {
+            uint32_t word = a.node_path[parity][size_t(i) * W + w];
+            if ((b.feature >> 5) == w) word |= 1u << (b.feature & 31);
+            path[w] = path[W + w] = word;
+          }
+          for (uint32_t w = 0; w < W; ++w) {
+            const uint32_t word = allowed_word(a, path, t, w);
+            a.node_allowed[parity ^ 1][size_t(2 * k) * W + w] = word;
+            a.node_allowed[parity ^ 1][size_t(2 * k + 1) * W + w] = word;
+          }
+        }
+      } else {
+        ls.split = 1;
+        ls.feature = b.feature;
+        ls.threshold = b.threshold;
+        ls.default_left = b.default_left;
+        ls.left_value = lv;
+        ls.right_value = rv;
+      }
+    } else if (!acc) {
+      ls.value = tn[node.node_index].leaf_value;  // the node's rows keep the current leaf value
+      if (!last) a.free_stack[free_top - n_acc + v[5]] = node.slot;
+    }
+    if (leafseg) {
+      const uint32_t at = leafseg_base + v[3];
+      if (at < a.max_leafsegs) {
+        a.leafseg[at] = ls;
+        a.leaf_prefix[at] = leafchunk_base + v[4];
+      } else {
+        err |= kErrCapacity;
+      }
+    }
+    if (first) {
+      const uint32_t mine = s_acc_base[ord + 1] - s_acc_base[ord];
+      a.trees[t].n_tree_nodes = tree_nodes + 2 * mine;
+      a.trees[t].leaf_count = leaf_count + mine;
+    }
+  }
+  // Without interaction groups a child's allowed features are its tree's (all, or a
+  // forest tree's subset); its path is not needed.
+  if (!last && P.n_groups == 0)
+    for (uint32_t idx = i; idx < 2 * n_acc * W; idx += blockDim.x) {
+      uint32_t word = 0xffffffffu;
+      if (a.tree_feature_masks != nullptr) {
+        const uint32_t t = a.nodes[parity][s_node_of[idx / (2 * W)]].tree;
+        word = a.tree_feature_masks[size_t(t) * W + idx % W];
+      }
+      a.node_allowed[parity ^ 1][idx] = word;
+    }
+  if (err) raise(ctl, err);
+  if (i == 0) {
+    ctl->n_leafseg = leafseg_base + tot[3];
+    ctl->leaf_chunks = leafchunk_base + tot[4];
+    if (leafseg_base + tot[3] <= a.max_leafsegs) a.leaf_prefix[leafseg_base + tot[3]] = leafchunk_base + tot[4];
+    const uint32_t acc_next = last ? 0u : n_acc;
+    ctl->n_nodes = 2 * acc_next;
+    ctl->n_build = acc_next;
+    ctl->n_sub = acc_next;
+    ctl->n_part = acc_next;
+    ctl->hist_items = last ? 0u : tot[1] * a.nfb;
+    ctl->part_chunks = last ? 0u : tot[2];
+    ctl->split_items = 2 * acc_next * a.n_fchunks;
+    if (!last) {
+      ctl->free_top = free_top - n_acc + (n - n_acc);
+      a.build_prefix[n_acc] = tot[1];
+      a.part_prefix[n_acc] = tot[2];
       ctl->item_rows = item_rows;
     }
     ctl->hist_counter = 0;
@@ -3154,8 +3393,12 @@ cudaError_t launch_leafwise_finish(const TrainerDev& a, cudaStream_t s) {
   leafwise_finish_kernel<<<1, 32, 0, s>>>(a);
   return cudaGetLastError();
 }
-cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, cudaStream_t s) {
-  finalize_kernel<<<1, 1024, 0, s>>>(a, parity, depth);
+cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, uint32_t max_nodes,
+                            cudaStream_t s) {
+  if (max_nodes <= kNodeFinalizeMax && a.partial_stride == 1)
+    finalize_nodes_kernel<<<1, (max_nodes + 31) / 32 * 32, 0, s>>>(a, parity, depth);
+  else
+    finalize_kernel<<<1, 1024, 0, s>>>(a, parity, depth);
   return cudaGetLastError();
 }
 // CTAs per node of the cluster launch for a level of at most max_nodes split nodes over

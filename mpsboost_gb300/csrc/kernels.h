@@ -182,7 +182,9 @@ cudaError_t launch_subtract(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, int grid,
                               cudaStream_t stream);
 uint32_t split_scan_kernels(const TrainerDev& a);  // launches per launch_split_scan
-cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, cudaStream_t stream);
+// max_nodes: a bound on the level's nodes (ctl->n_nodes).
+cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, uint32_t max_nodes,
+                            cudaStream_t stream);
 // max_nodes: a bound on the nodes the launch partitions (ctl->n_part).
 cudaError_t launch_partition(const TrainerDev& a, uint32_t max_nodes, int grid, cudaStream_t stream);
 uint32_t partition_kernels(const TrainerDev& a, uint32_t max_nodes);  // launches per launch_partition
