@@ -840,7 +840,7 @@ struct mpsb_cuda_trainer {
         CK(launch_subtract(dev, grid(8), s)); ++k;
       }
       if (depth > 0) {
-        CK(launch_split_scan(dev, parity, level_nodes(d), grid(4), s)); k += split_scan_kernels(dev);
+        CK(launch_split_scan(dev, parity, level_nodes(d), false, grid(4), s)); k += split_scan_kernels(dev);
       }
       CK(launch_finalize(dev, parity, d, level_nodes(d), s)); ++k;
       if (d + 1 < depth) {
@@ -873,17 +873,23 @@ struct mpsb_cuda_trainer {
     }
     CK(launch_root_stats(dev, s)); ++k;
     if (depth > 0) {
-      CK(launch_split_scan(dev, 0, n_trees, grid(4), s)); k += split_scan_kernels(dev);
+      CK(launch_split_scan(dev, 0, n_trees, false, grid(4), s)); k += split_scan_kernels(dev);
     }
     CK(launch_leafwise_init(dev, s)); ++k;
     for (uint32_t step = 0; step < lw_steps && depth > 0; ++step) {
       CK(launch_leafwise_select(dev, s)); ++k;
+      // The built child's slot is cleared beside the partition, as between levels.
+      CK(cudaEventRecord(fork_ev, s));
+      CK(cudaStreamWaitEvent(side, fork_ev, 0));
+      CK(launch_zero_build_slots(dev, grid(8), side)); ++k;
+      CK(cudaEventRecord(zero_ev, side));
       CK(launch_partition(dev, n_trees, grid(4), s)); k += partition_kernels(dev, n_trees);
-      CK(launch_zero_build_slots(dev, grid(8), s)); ++k;
+      CK(cudaStreamWaitEvent(s, zero_ev, 0));
       CK(launch_hist_build(build_view(), hcfg, grid(1), s)); ++k;
       if (!dev.fused_sub) { CK(launch_subtract(dev, grid(8), s)); ++k; }
-      CK(launch_split_scan(dev, 1, 2 * n_trees, grid(4), s)); k += split_scan_kernels(dev);
-      CK(launch_leafwise_merge(dev, s)); ++k;
+      const uint32_t scans = split_scan_kernels(dev);
+      CK(launch_split_scan(dev, 1, 2 * n_trees, true, grid(4), s)); k += scans;
+      if (scans == 1) { CK(launch_leafwise_merge(dev, s)); ++k; }
     }
     CK(launch_leafwise_finish(dev, s)); ++k;
     return k;

@@ -776,6 +776,15 @@ __device__ __forceinline__ uint32_t min_leaf_rows(const TreeParams& P) {
   return uint32_t(P.min_samples_leaf < 0xFFFFFFFFull ? P.min_samples_leaf : 0xFFFFFFFFull);
 }
 
+__device__ __forceinline__ SplitRec no_split() {
+  SplitRec b;
+  b.gain = 0.0;
+  b.valid = 0;
+  b.feature = b.threshold = 0;
+  b.default_left = 1;
+  return b;
+}
+
 // One warp per (node, feature); a CTA covers one node and blockDim/32 features and
 // writes the best split of its features to partial[node][chunk].
 constexpr int kScanThreadsMax = 512;
@@ -1603,9 +1612,10 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
   if (err) raise(a.ctl, err);
 }
 
-// One CTA per node.
+// One CTA per node. to_active: a leaf-wise step, whose nodes' splits go to their active
+// leaves.
 template <bool FIXED, bool WIDE>
-__global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, int parity) {
+__global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, int parity, bool to_active) {
   __shared__ PageTotals<FIXED> s_totals[2];
   __shared__ uint32_t s_list[kScanCta], s_listed;
   __shared__ double s_gain[kScanCtaWarps];
@@ -1728,20 +1738,19 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
       }
       if (take) bw = q;
     }
+    SplitRec* out = a.partial + i;
+    if (to_active) {
+      const uint32_t at = a.lw_scan_map[i];
+      LeafActive& leaf = a.lw_active[size_t(at >> 16) * a.lw_cap + (at & 0xFFFFu)];
+      out = &leaf.best;
+      if (threadIdx.x == 0) leaf.scanned = 1;
+    }
     if (bw < 0) {
-      if (threadIdx.x == 0) {
-        SplitRec none;
-        none.valid = 0;
-        none.gain = 0.0;
-        none.feature = 0;
-        none.threshold = 0;
-        none.default_left = 1;
-        a.partial[i] = none;
-      }
+      if (threadIdx.x == 0) *out = no_split();
     } else if (threadIdx.x == s_key[bw][4]) {
       const int8_t mono = P.has_monotonic ? a.monotonic[feature] : int8_t(0);
-      a.partial[i] = split_record<FIXED>(P, cl, cr, inv_g, inv_h, mono, lo, hi, gain, feature,
-                                         threshold, default_left);
+      *out = split_record<FIXED>(P, cl, cr, inv_g, inv_h, mono, lo, hi, gain, feature, threshold,
+                                 default_left);
     }
     __syncthreads();  // the argmax arrays and the list are rewritten by the next node
   }
@@ -2689,15 +2698,6 @@ __device__ SplitRec merged_split(const TrainerDev& a, uint32_t i) {
   return b;
 }
 
-__device__ __forceinline__ SplitRec no_split() {
-  SplitRec b;
-  b.gain = 0.0;
-  b.valid = 0;
-  b.feature = b.threshold = 0;
-  b.default_left = 1;
-  return b;
-}
-
 // Root of every tree becomes its first active leaf (after the level-0 split scan).
 __global__ void leafwise_init_kernel(TrainerDev a) {
   const TreeParams& P = a.params;
@@ -2721,215 +2721,263 @@ __global__ void leafwise_init_kernel(TrainerDev a) {
   }
 }
 
-__global__ void __launch_bounds__(1024) leafwise_select_kernel(TrainerDev a) {
+// A warp per tree, kSelectTrees at a time: the lanes compare the active leaves and copy the
+// records, where one thread walked them before (29 us a step at 31 leaves).
+constexpr uint32_t kSelectTrees = 8;
+
+__global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(TrainerDev a) {
   __shared__ uint32_t sh[33 * 3];
   __shared__ unsigned long long built_rows;
   const TreeParams& P = a.params;
   const uint32_t W = P.path_words, cap = a.lw_cap, S = a.lw_slot_cap;
-  const uint32_t t = threadIdx.x;
-  if (t == 0) built_rows = 0;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) built_rows = 0;
   __syncthreads();
   uint32_t err = 0;
-  bool split = false, build = false;
-  uint32_t n_scan = 0, kid_at[2] = {0, 0};
-  PartEntry pe{};
-  BuildEntry be{};
-  SubEntry se{};
-  if (t < a.n_trees && !a.lw_done[t]) {
-    LeafActive* act = a.lw_active + size_t(t) * cap;
-    uint32_t* path = a.lw_path + size_t(t) * cap * W;
-    uint32_t* allowed = a.lw_allowed + size_t(t) * cap * W;
-    TreeState& ts = a.trees[t];
-    const uint32_t cnt = a.lw_count[t];
-    int best = -1;
-    if (cnt > a.lw_max_active) {
-      err |= kErrLeafQueue;
-    } else if (ts.leaf_count < a.lw_max_leaves) {
-      for (uint32_t j = 0; j < cnt; ++j) {  // IsBetterLeafWiseCandidate (tree_leafwise.cpp:16-27)
-        const LeafActive& l = act[j];
-        if (l.node.depth >= P.max_depth || !l.scanned || !l.best.valid) continue;
-        if (best < 0 || l.best.gain > act[best].best.gain ||
-            (l.best.gain == act[best].best.gain && l.node.node_index < act[best].node.node_index))
-          best = int(j);
-      }
-    }
-    if (best < 0) {
-      a.lw_done[t] = 1;
-    } else {
-      const LeafActive c = act[best];
-      const SplitRec& b = c.best;
-      TreeNodeOut* tn = a.tree_nodes + size_t(t) * a.max_tree_nodes;
-      const uint32_t li = ts.n_tree_nodes, ri = li + 1;
-      const uint32_t depth = c.node.depth + 1;
-      const bool grow = depth < P.max_depth;
-      if (ri >= a.max_tree_nodes || cnt + 2 > cap || (grow && a.lw_slot_top[t] == 0)) {
-        err |= kErrCapacity;
-        a.lw_done[t] = 1;
-      } else {
-        // ApplySplit (tree_structure.cpp:118-148).
-        double lv = 0.0, rv = 0.0;
-        if (!bounded_leaf(P, b.lg, b.lh, b.ll, b.lu, &lv)) err |= kErrNonFinite;
-        if (!bounded_leaf(P, b.rg, b.rh, b.rl, b.ru, &rv)) err |= kErrNonFinite;
-        write_leaf(&tn[li], lv);
-        write_leaf(&tn[ri], rv);
-        TreeNodeOut& pn = tn[c.node.node_index];
-        pn.feature_index = b.feature;
-        pn.threshold_bin = b.threshold;
-        pn.left_child = li;
-        pn.right_child = ri;
-        pn.leaf_value = 0.0;
-        pn.gain = b.gain;
-        pn.default_left = uint8_t(b.default_left);
-        pn.flags = 0;
-        ts.n_tree_nodes += 2;
-        ts.leaf_count += 1;
-        if (b.lcount + b.rcount != c.node.seg_cnt) err |= kErrPartition;
-        // Children in the other row buffer: left rows, then right rows (the partition).
-        const uint32_t np = c.parity ^ 1u;
-        const bool build_left = b.lcount <= b.rcount;
-        uint32_t new_slot = 0xffffffffu;
-        if (grow) new_slot = a.lw_slots[size_t(t) * S + --a.lw_slot_top[t]];
-        else a.lw_slots[size_t(t) * S + a.lw_slot_top[t]++] = c.node.slot;  // no child histograms
-        LeafActive kid[2];
-        for (int k = 0; k < 2; ++k) {
-          NodeRec& n = kid[k].node;
-          const bool left = k == 0;
-          n.seg_off = left ? c.node.seg_off : c.node.seg_off + uint32_t(b.lcount);
-          n.seg_cnt = uint32_t(left ? b.lcount : b.rcount);
-          n.node_index = left ? li : ri;
-          n.slot = !grow ? 0xffffffffu : ((left == build_left) ? new_slot : c.node.slot);
-          n.count = left ? b.lcount : b.rcount;
-          n.qg = left ? b.lqg : b.rqg;
-          n.qh = left ? b.lqh : b.rqh;
-          n.g = left ? b.lg : b.rg;
-          n.h = left ? b.lh : b.rh;
-          n.lo = left ? b.ll : b.rl;
-          n.hi = left ? b.lu : b.ru;
-          n.tree = t;
-          n.depth = depth;
-          // As in finalize: the sibling of the built child keeps the parent's slot.
-          n.sub_from = (a.fused_sub && grow && left != build_left) ? new_slot + 1 : 0;
-          kid[k].best = no_split();
-          kid[k].parity = np;
-          kid[k].scanned = grow ? 0u : 1u;
-        }
-        // Children's path and allowed words go to positions cnt, cnt + 1 (free), the
-        // chosen leaf's place takes the last leaf, then the children move down by one.
-        for (int k = 0; k < 2; ++k)
-          for (uint32_t w = 0; w < W; ++w) {
-            uint32_t pw = path[size_t(best) * W + w];
-            if ((b.feature >> 5) == w) pw |= 1u << (b.feature & 31);
-            path[size_t(cnt + k) * W + w] = pw;
+  uint32_t n_part = 0, n_build = 0, n_scan = 0;  // entries of the rounds before
+  for (uint32_t base = 0; base < a.n_trees; base += blockDim.x / 32) {
+    const uint32_t t = base + warp;
+    bool split = false, build = false;
+    uint32_t last = 0;
+    PartEntry pe{};
+    BuildEntry be{};
+    SubEntry se{};
+    LeafActive kid[2];
+    if (t < a.n_trees && !a.lw_done[t]) {  // the same in the whole warp
+      LeafActive* act = a.lw_active + size_t(t) * cap;
+      uint32_t* path = a.lw_path + size_t(t) * cap * W;
+      uint32_t* allowed = a.lw_allowed + size_t(t) * cap * W;
+      TreeState& ts = a.trees[t];
+      const uint32_t cnt = a.lw_count[t], leaf_count = ts.leaf_count, tree_nodes = ts.n_tree_nodes;
+      uint32_t best = 0xffffffffu, best_node = 0xffffffffu;
+      double best_gain = 0.0;
+      if (cnt > a.lw_max_active) {
+        err |= kErrLeafQueue;
+      } else if (leaf_count < a.lw_max_leaves) {
+        // IsBetterLeafWiseCandidate (tree_leafwise.cpp:16-27): the larger gain, then the
+        // smaller node index.
+        for (uint32_t j = lane; j < cnt; j += 32) {
+          const LeafActive& l = act[j];
+          const uint32_t d = l.node.depth, sc = l.scanned, va = l.best.valid, ni = l.node.node_index;
+          const double g = l.best.gain;
+          if (d >= P.max_depth || !sc || !va) continue;
+          if (best == 0xffffffffu || g > best_gain || (g == best_gain && ni < best_node)) {
+            best = j;
+            best_gain = g;
+            best_node = ni;
           }
-        for (uint32_t w = 0; w < W; ++w) {
-          uint32_t al = 0xffffffffu;
-          if (P.n_groups > 0) {  // InteractionAllowsFeature (tree_interactions.cpp:32-45)
-            al = 0;
-            for (uint32_t g = 0; g < P.n_groups; ++g) {
-              bool subset = true;
-              for (uint32_t u = 0; u < W && subset; ++u)
-                subset = (path[size_t(cnt) * W + u] & ~a.group_masks[g * W + u]) == 0;
-              if (subset) al |= a.group_masks[g * W + w];
+        }
+        for (int off = 16; off > 0; off >>= 1) {
+          const uint32_t ob = __shfl_xor_sync(0xffffffffu, best, off);
+          const uint32_t on = __shfl_xor_sync(0xffffffffu, best_node, off);
+          const double og = __shfl_xor_sync(0xffffffffu, best_gain, off);
+          if (ob != 0xffffffffu &&
+              (best == 0xffffffffu || og > best_gain || (og == best_gain && on < best_node))) {
+            best = ob;
+            best_gain = og;
+            best_node = on;
+          }
+        }
+      }
+      if (best == 0xffffffffu) {
+        if (lane == 0) a.lw_done[t] = 1;
+      } else {
+        const LeafActive c = act[best];  // every lane (the loads broadcast)
+        const SplitRec& b = c.best;
+        TreeNodeOut* tn = a.tree_nodes + size_t(t) * a.max_tree_nodes;
+        const uint32_t li = tree_nodes, ri = li + 1;
+        const uint32_t depth = c.node.depth + 1;
+        const bool grow = depth < P.max_depth;
+        const uint32_t slot_top = a.lw_slot_top[t];
+        if (ri >= a.max_tree_nodes || cnt + 2 > cap || (grow && slot_top == 0)) {
+          err |= kErrCapacity;
+          if (lane == 0) a.lw_done[t] = 1;
+        } else {
+          // ApplySplit (tree_structure.cpp:118-148).
+          double lv = 0.0, rv = 0.0;
+          if (!bounded_leaf(P, b.lg, b.lh, b.ll, b.lu, &lv)) err |= kErrNonFinite;
+          if (!bounded_leaf(P, b.rg, b.rh, b.rl, b.ru, &rv)) err |= kErrNonFinite;
+          if (b.lcount + b.rcount != c.node.seg_cnt) err |= kErrPartition;
+          // Children in the other row buffer: left rows, then right rows (the partition).
+          const uint32_t np = c.parity ^ 1u;
+          const bool build_left = b.lcount <= b.rcount;
+          const uint32_t new_slot = grow ? a.lw_slots[size_t(t) * S + slot_top - 1] : 0xffffffffu;
+          if (lane == 0) {
+            write_leaf(&tn[li], lv);
+            write_leaf(&tn[ri], rv);
+            TreeNodeOut& pn = tn[c.node.node_index];
+            pn.feature_index = b.feature;
+            pn.threshold_bin = b.threshold;
+            pn.left_child = li;
+            pn.right_child = ri;
+            pn.leaf_value = 0.0;
+            pn.gain = b.gain;
+            pn.default_left = uint8_t(b.default_left);
+            pn.flags = 0;
+            ts.n_tree_nodes = tree_nodes + 2;
+            ts.leaf_count = leaf_count + 1;
+            // A leaf at max_depth has no child histograms: its slot is free again.
+            if (!grow) a.lw_slots[size_t(t) * S + slot_top] = c.node.slot;
+            a.lw_slot_top[t] = grow ? slot_top - 1 : slot_top + 1;
+          }
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            NodeRec& n = kid[k].node;
+            const bool left = k == 0;
+            n.seg_off = left ? c.node.seg_off : c.node.seg_off + uint32_t(b.lcount);
+            n.seg_cnt = uint32_t(left ? b.lcount : b.rcount);
+            n.node_index = left ? li : ri;
+            n.slot = !grow ? 0xffffffffu : ((left == build_left) ? new_slot : c.node.slot);
+            n.count = left ? b.lcount : b.rcount;
+            n.qg = left ? b.lqg : b.rqg;
+            n.qh = left ? b.lqh : b.rqh;
+            n.g = left ? b.lg : b.rg;
+            n.h = left ? b.lh : b.rh;
+            n.lo = left ? b.ll : b.rl;
+            n.hi = left ? b.lu : b.ru;
+            n.tree = t;
+            n.depth = depth;
+            // As in finalize: the sibling of the built child keeps the parent's slot.
+            n.sub_from = (a.fused_sub && grow && left != build_left) ? new_slot + 1 : 0;
+            kid[k].best = no_split();
+            kid[k].parity = np;
+            kid[k].scanned = grow ? 0u : 1u;
+          }
+          last = cnt - 1;
+          if (P.n_groups > 0) {
+            // Children's path and allowed words go to positions cnt, cnt + 1 (free), the
+            // chosen leaf's place takes the last leaf, then the children move down by one.
+            if (lane == 0) {
+              for (uint32_t k = 0; k < 2; ++k)
+                for (uint32_t w = 0; w < W; ++w) {
+                  uint32_t pw = path[size_t(best) * W + w];
+                  if ((b.feature >> 5) == w) pw |= 1u << (b.feature & 31);
+                  path[size_t(cnt + k) * W + w] = pw;
+                }
+              for (uint32_t w = 0; w < W; ++w) {
+                const uint32_t al = allowed_word(a, path + size_t(cnt) * W, t, w);
+                allowed[size_t(cnt) * W + w] = al;
+                allowed[size_t(cnt + 1) * W + w] = al;
+              }
+              for (uint32_t w = 0; w < W && best != last; ++w) {
+                path[size_t(best) * W + w] = path[size_t(last) * W + w];
+                allowed[size_t(best) * W + w] = allowed[size_t(last) * W + w];
+              }
+              for (uint32_t k = 0; k < 2; ++k)
+                for (uint32_t w = 0; w < W; ++w) {
+                  path[size_t(last + k) * W + w] = path[size_t(cnt + k) * W + w];
+                  allowed[size_t(last + k) * W + w] = allowed[size_t(cnt + k) * W + w];
+                }
             }
           }
-          if (a.tree_feature_masks != nullptr) al &= a.tree_feature_masks[t * W + w];
-          allowed[size_t(cnt) * W + w] = al;
-          allowed[size_t(cnt + 1) * W + w] = al;
-        }
-        const uint32_t last = cnt - 1;
-        if (uint32_t(best) != last) {
-          act[best] = act[last];
-          for (uint32_t w = 0; w < W; ++w) {
-            path[size_t(best) * W + w] = path[size_t(last) * W + w];
-            allowed[size_t(best) * W + w] = allowed[size_t(last) * W + w];
+          if (best != last) {  // the chosen leaf's place takes the last leaf, word by word
+            static_assert(sizeof(LeafActive) % 8 == 0, "a warp copies 8-byte words");
+            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(act + last);
+            unsigned long long* dst = reinterpret_cast<unsigned long long*>(act + best);
+            for (uint32_t q = lane; q < sizeof(LeafActive) / 8; q += 32) dst[q] = src[q];
           }
-        }
-        for (int k = 0; k < 2; ++k) {
-          act[last + k] = kid[k];
-          for (uint32_t w = 0; w < W; ++w) {
-            path[size_t(last + k) * W + w] = path[size_t(cnt + k) * W + w];
-            allowed[size_t(last + k) * W + w] = allowed[size_t(cnt + k) * W + w];
+          __syncwarp();
+          if (lane < 2) act[last + lane] = lane == 0 ? kid[0] : kid[1];
+          // Room for both children (tree_leafwise.cpp:130-134).
+          const bool full = !(cnt - 1 + 2 <= a.lw_max_active || leaf_count + 1 >= a.lw_max_leaves);
+          if (full) err |= kErrLeafQueue;
+          if (lane == 0) {
+            a.lw_count[t] = cnt + 1;
+            if (full) a.lw_done[t] = 1;
           }
-        }
-        a.lw_count[t] = cnt + 1;
-        // Room for both children (tree_leafwise.cpp:130-134).
-        if (!(cnt - 1 + 2 <= a.lw_max_active || ts.leaf_count >= a.lw_max_leaves)) {
-          err |= kErrLeafQueue;
-          a.lw_done[t] = 1;
-        }
-        split = true;
-        pe.tree = t;
-        pe.parity = c.parity;
-        pe.seg_off = c.node.seg_off;
-        pe.seg_cnt = c.node.seg_cnt;
-        pe.feature = b.feature;
-        pe.threshold = b.threshold;
-        pe.default_left = b.default_left;
-        pe.lcount = uint32_t(b.lcount);
-        if (grow) {
-          build = true;
-          be.tree = t;
-          be.parity = np;
-          be.seg_off = build_left ? kid[0].node.seg_off : kid[1].node.seg_off;
-          be.seg_cnt = build_left ? kid[0].node.seg_cnt : kid[1].node.seg_cnt;
-          be.slot = new_slot;
-          be.pad = 0;
-          se.parent_slot = c.node.slot;
-          se.built_slot = new_slot;
-          atomicAdd(&built_rows, (unsigned long long)be.seg_cnt);
-          n_scan = 2;
-          kid_at[0] = last;
-          kid_at[1] = last + 1;
+          split = true;
+          pe.tree = t;
+          pe.parity = c.parity;
+          pe.seg_off = c.node.seg_off;
+          pe.seg_cnt = c.node.seg_cnt;
+          pe.feature = b.feature;
+          pe.threshold = b.threshold;
+          pe.default_left = b.default_left;
+          pe.lcount = uint32_t(b.lcount);
+          if (grow) {
+            build = true;
+            be.tree = t;
+            be.parity = np;
+            be.seg_off = build_left ? kid[0].node.seg_off : kid[1].node.seg_off;
+            be.seg_cnt = build_left ? kid[0].node.seg_cnt : kid[1].node.seg_cnt;
+            be.slot = new_slot;
+            be.pad = 0;
+            se.parent_slot = c.node.slot;
+            se.built_slot = new_slot;
+            if (lane == 0) atomicAdd(&built_rows, (unsigned long long)be.seg_cnt);
+          }
         }
       }
     }
+    const bool lead = lane == 0;  // the warp's entries
+    uint32_t v[2] = {lead && split ? 1u : 0u, lead && build ? 1u : 0u}, tot[2];
+    block_scan<2>(v, tot, sh);
+    const uint32_t at_part = n_part + __shfl_sync(0xffffffffu, v[0], 0);
+    const uint32_t at_build = n_build + __shfl_sync(0xffffffffu, v[1], 0);
+    if (lead && split) a.part[at_part] = pe;
+    if (build) {
+      // Both children of a grown leaf are scanned: two scan entries per build entry.
+      if (lead) {
+        a.build[at_build] = be;
+        a.sub[at_build] = se;
+      }
+      if (lane < 2) {
+        a.nodes[1][2 * at_build + lane] = lane == 0 ? kid[0].node : kid[1].node;
+        a.lw_scan_map[2 * at_build + lane] = (t << 16) | (last + lane);
+      }
+      for (uint32_t w = lane; w < 2 * W; w += 32) {
+        const uint32_t word = w < W ? w : w - W;
+        uint32_t al = 0xffffffffu;
+        if (P.n_groups > 0) al = a.lw_allowed[(size_t(t) * cap + last) * W + word];
+        else if (a.tree_feature_masks != nullptr) al = a.tree_feature_masks[t * W + word];
+        a.node_allowed[1][size_t(2 * at_build) * W + w] = al;
+      }
+    }
+    n_part += tot[0];
+    n_build += tot[1];
+    n_scan += 2 * tot[1];
   }
   if (err) raise(a.ctl, err);
-  uint32_t v[3] = {split ? 1u : 0u, build ? 1u : 0u, n_scan};
-  uint32_t tot[3];
-  block_scan<3>(v, tot, sh);
-  if (split) a.part[v[0]] = pe;
-  if (build) {
-    a.build[v[1]] = be;
-    a.sub[v[1]] = se;
-  }
-  for (uint32_t k = 0; k < n_scan; ++k) {
-    const uint32_t s = v[2] + k;
-    a.nodes[1][s] = a.lw_active[size_t(t) * cap + kid_at[k]].node;
-    for (uint32_t w = 0; w < W; ++w)
-      a.node_allowed[1][size_t(s) * W + w] = a.lw_allowed[(size_t(t) * cap + kid_at[k]) * W + w];
-    a.lw_scan_map[s] = (t << 16) | kid_at[k];
-  }
   __syncthreads();
-  if (threadIdx.x == 0) {  // work lists of the step (few entries: one per tree)
+  if (warp == 0) {  // work lists of the step, 32 entries at a time
     Control* ctl = a.ctl;
-    uint32_t acc = 0;
-    for (uint32_t e = 0; e < tot[0]; ++e) {
-      a.part_prefix[e] = acc;
-      acc += ceil_div(a.part[e].seg_cnt, kPartChunk);
-    }
-    a.part_prefix[tot[0]] = acc;
-    ctl->n_part = tot[0];
-    ctl->part_chunks = acc;
     const uint32_t item_rows =
         a.item_rows ? a.item_rows : adaptive_item_rows(built_rows, a.nfb, a.sm_count, a.items_per_sm);
-    acc = 0;
-    for (uint32_t e = 0; e < tot[1]; ++e) {
-      a.build_prefix[e] = acc;
-      acc += ceil_div(a.build[e].seg_cnt, item_rows);
+    auto prefix = [&](uint32_t n, uint32_t* out, auto&& chunks_of) -> uint32_t {
+      uint32_t acc = 0;
+      for (uint32_t e0 = 0; e0 < n; e0 += 32) {
+        const uint32_t e = e0 + lane;
+        const uint32_t own = e < n ? chunks_of(e) : 0u;
+        uint32_t x = own;
+        for (int off = 1; off < 32; off <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+          if (lane >= uint32_t(off)) x += y;
+        }
+        if (e < n) out[e] = acc + x - own;
+        acc += __shfl_sync(0xffffffffu, x, 31);
+      }
+      if (lane == 0) out[n] = acc;
+      return acc;
+    };
+    const uint32_t part_chunks =
+        prefix(n_part, a.part_prefix, [&](uint32_t e) { return ceil_div(a.part[e].seg_cnt, kPartChunk); });
+    const uint32_t build_chunks =
+        prefix(n_build, a.build_prefix, [&](uint32_t e) { return ceil_div(a.build[e].seg_cnt, item_rows); });
+    if (lane == 0) {
+      ctl->n_part = n_part;
+      ctl->part_chunks = part_chunks;
+      ctl->n_build = n_build;
+      ctl->n_sub = n_build;
+      ctl->hist_items = build_chunks * a.nfb;
+      ctl->hist_counter = 0;
+      ctl->item_rows = item_rows;
+      ctl->n_nodes = n_scan;
+      ctl->split_items = n_scan * a.n_fchunks;
     }
-    a.build_prefix[tot[1]] = acc;
-    ctl->n_build = tot[1];
-    ctl->n_sub = tot[1];
-    ctl->hist_items = acc * a.nfb;
-    ctl->hist_counter = 0;
-    ctl->item_rows = item_rows;
-    ctl->n_nodes = tot[2];
-    ctl->split_items = tot[2] * a.n_fchunks;
   }
 }
 
-// The children's best splits into their active entries.
+// The children's best splits into their active entries (after a one-launch scan).
 __global__ void leafwise_merge_kernel(TrainerDev a) {
   for (uint32_t s = threadIdx.x; s < a.ctl->n_nodes; s += blockDim.x) {
     const uint32_t m = a.lw_scan_map[s];
@@ -2939,40 +2987,55 @@ __global__ void leafwise_merge_kernel(TrainerDev a) {
   }
 }
 
-// Every active leaf becomes a leaf segment of the prediction update.
+// Every active leaf becomes a leaf segment of the prediction update: one warp, a leaf per
+// lane.
 __global__ void leafwise_finish_kernel(TrainerDev a) {
-  if (threadIdx.x != 0) return;
+  const uint32_t lane = threadIdx.x;
   Control* ctl = a.ctl;
   uint32_t n = 0, chunks = 0, err = 0;
   for (uint32_t t = 0; t < a.n_trees; ++t) {
     const LeafActive* act = a.lw_active + size_t(t) * a.lw_cap;
     const TreeNodeOut* tn = a.tree_nodes + size_t(t) * a.max_tree_nodes;
-    for (uint32_t j = 0; j < a.lw_count[t]; ++j) {
-      if (n >= a.max_leafsegs) {
-        err |= kErrCapacity;
-        break;
+    const uint32_t count = a.lw_count[t];
+    for (uint32_t j0 = 0; j0 < count; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      LeafSeg ls{};
+      if (j < count) {
+        ls.tree = t;
+        ls.parity = act[j].parity;
+        ls.seg_off = act[j].node.seg_off;
+        ls.seg_cnt = act[j].node.seg_cnt;
+        ls.value = tn[act[j].node.node_index].leaf_value;
       }
-      LeafSeg ls;
-      ls.tree = t;
-      ls.parity = act[j].parity;
-      ls.seg_off = act[j].node.seg_off;
-      ls.seg_cnt = act[j].node.seg_cnt;
-      ls.split = 0;
-      ls.feature = ls.threshold = ls.default_left = 0;
-      ls.value = tn[act[j].node.node_index].leaf_value;
-      ls.left_value = ls.right_value = 0.0;
-      a.leafseg[n] = ls;
-      a.leaf_prefix[n] = chunks;
-      chunks += ceil_div(ls.seg_cnt, kApplyChunk);
-      ++n;
+      const uint32_t own = j < count ? ceil_div(ls.seg_cnt, kApplyChunk) : 0u;
+      uint32_t x = own;
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= uint32_t(off)) x += y;
+      }
+      if (j < count) {
+        if (n + lane < a.max_leafsegs) {
+          a.leafseg[n + lane] = ls;
+          a.leaf_prefix[n + lane] = chunks + x - own;
+        } else {
+          err |= kErrCapacity;
+        }
+      }
+      n += min(32u, count - j0);
+      chunks += __shfl_sync(0xffffffffu, x, 31);
     }
   }
-  a.leaf_prefix[n] = chunks;
-  ctl->n_leafseg = n;
-  ctl->leaf_chunks = chunks;
-  ctl->n_nodes = ctl->n_build = ctl->n_sub = ctl->n_part = 0;
-  ctl->hist_items = ctl->part_chunks = ctl->split_items = 0;
-  if (err) raise(ctl, err);
+  if (__any_sync(0xffffffffu, err != 0)) {
+    if (lane == 0) raise(ctl, kErrCapacity);
+    n = min(n, a.max_leafsegs);
+  }
+  if (lane == 0) {
+    a.leaf_prefix[n] = chunks;
+    ctl->n_leafseg = n;
+    ctl->leaf_chunks = chunks;
+    ctl->n_nodes = ctl->n_build = ctl->n_sub = ctl->n_part = 0;
+    ctl->hist_items = ctl->part_chunks = ctl->split_items = 0;
+  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -3345,14 +3408,15 @@ cudaError_t launch_scan_one(const TrainerDev& a, int parity, int grid, int threa
   return cudaGetLastError();
 }
 template <bool FIXED, bool WIDE>
-cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes, cudaStream_t s) {
+cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes, bool to_active,
+                            cudaStream_t s) {
   const uint64_t resident = uint64_t(a.sm_count ? a.sm_count : 152) * 6;
   const uint32_t screen = uint32_t(std::min<uint64_t>(resident, uint64_t(max_nodes) * a.features));
   split_screen_kernel<FIXED, WIDE><<<screen, kScanCta, 0, s>>>(a, parity);
   const cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   const uint32_t exact = uint32_t(std::min<uint64_t>(resident, max_nodes));
-  split_exact_kernel<FIXED, WIDE><<<exact, kScanCta, 0, s>>>(a, parity);
+  split_exact_kernel<FIXED, WIDE><<<exact, kScanCta, 0, s>>>(a, parity, to_active);
   return cudaGetLastError();
 }
 
@@ -3360,15 +3424,16 @@ uint32_t split_scan_kernels(const TrainerDev& a) {
   return a.node_screen && a.scan_two_phase ? 2u : 1u;
 }
 
-cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, int grid, cudaStream_t s) {
+cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, bool to_active,
+                              int grid, cudaStream_t s) {
   const bool fixed = a.mode == kModeFixed, wide = a.slots != uint32_t(kSlots);
   if (a.slots < uint32_t(kSlots) || a.slots % uint32_t(kSlots) || max_nodes == 0) return cudaErrorInvalidValue;
   if (split_scan_kernels(a) == 2) {
     // node_screen was cleared by the level's zero_build_slots_kernel.
-    if (fixed) return wide ? launch_scan_two<true, true>(a, parity, max_nodes, s)
-                           : launch_scan_two<true, false>(a, parity, max_nodes, s);
-    return wide ? launch_scan_two<false, true>(a, parity, max_nodes, s)
-                : launch_scan_two<false, false>(a, parity, max_nodes, s);
+    if (fixed) return wide ? launch_scan_two<true, true>(a, parity, max_nodes, to_active, s)
+                           : launch_scan_two<true, false>(a, parity, max_nodes, to_active, s);
+    return wide ? launch_scan_two<false, true>(a, parity, max_nodes, to_active, s)
+                : launch_scan_two<false, false>(a, parity, max_nodes, to_active, s);
   }
   const int threads = int(a.scan_threads);
   if (threads < 32 || threads > kScanThreadsMax || threads % 32) return cudaErrorInvalidValue;
@@ -3382,7 +3447,7 @@ cudaError_t launch_leafwise_init(const TrainerDev& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t launch_leafwise_select(const TrainerDev& a, cudaStream_t s) {
-  leafwise_select_kernel<<<1, 1024, 0, s>>>(a);
+  leafwise_select_kernel<<<1, 32 * std::min(a.n_trees, kSelectTrees), 0, s>>>(a);
   return cudaGetLastError();
 }
 cudaError_t launch_leafwise_merge(const TrainerDev& a, cudaStream_t s) {

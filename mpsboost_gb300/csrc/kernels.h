@@ -179,8 +179,10 @@ cudaError_t launch_leafwise_finish(const TrainerDev& a, cudaStream_t stream);
 cudaError_t launch_root_cache(const TrainerDev& a, int save, int grid, cudaStream_t stream);
 cudaError_t launch_subtract(const TrainerDev& a, int grid, cudaStream_t stream);
 // max_nodes: a bound on the nodes the launch scans (ctl->n_nodes), from the level.
-cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, int grid,
-                              cudaStream_t stream);
+// to_active: a leaf-wise step; a two-launch scan writes its nodes' splits to their active
+// leaves (after a one-launch scan launch_leafwise_merge does).
+cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, bool to_active,
+                              int grid, cudaStream_t stream);
 uint32_t split_scan_kernels(const TrainerDev& a);  // launches per launch_split_scan
 // max_nodes: a bound on the level's nodes (ctl->n_nodes).
 cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, uint32_t max_nodes,
