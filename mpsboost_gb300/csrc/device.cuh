@@ -323,6 +323,89 @@ __device__ __forceinline__ float f64_to_f32_rn(double x) {
   return __uint_as_float(sign | uint32_t(rne_shift(m, s)));  // a carry gives 2^-126 exactly
 }
 
+// ---- The logistic function on the integer pipe ---------------------------------------
+// The FP64 pipe's two lanes per clock made the FP64 exp and division of a logistic row cost
+// about 100 us per million rows. e^-t is computed in 64-bit fixed point by the usual table
+// reduction (Tang, "Table-driven implementation of the exponential function", 1989):
+// t log2(e) = k + i/16 + j/256 + r, e^-t = 2^-k 2^(-i/16) 2^(-j/256) e^(-r ln 2), the last
+// factor by its Taylor series (r ln 2 < 0.0028: five terms leave 2^-60); 1/(1+e^-t) by one
+// third-order Newton step from an FP32 reciprocal. Every result is within 2^-56.5
+// relative of the exact value (checked against 60-digit arithmetic), then rounded once to
+// the 53 bits of a double, where an FP64 evaluation rounds several times.
+struct Fixed64 {  // value m * 2^-64 * 2^-k, m >= 2^60
+  unsigned long long m;
+  int k;
+};
+
+// 2^(-i/16) and 2^(-j/256), times 2^64, rounded (2^64 itself saturated).
+static __device__ const unsigned long long kExp2Sixteenths[16] = {
+    0xFFFFFFFFFFFFFFFFull, 0xF5257D152486CC2Cull, 0xEAC0C6E7DD24392Full, 0xE0CCDEEC2A94E111ull,
+    0xD744FCCAD69D6AF4ull, 0xCE248C151F8480E4ull, 0xC5672A115506DADDull, 0xBD08A39F580C36BFull,
+    0xB504F333F9DE6484ull, 0xAD583EEA42A14AC6ull, 0xA5FED6A9B15138EAull, 0x9EF5326091A111AEull,
+    0x9837F0518DB8A96Full, 0x91C3D373AB11C336ull, 0x8B95C1E3EA8BD6E7ull, 0x85AAC367CC487B15ull};
+static __device__ const unsigned long long kExp2Fine[16] = {
+    0xFFFFFFFFFFFFFFFFull, 0xFF4ECB59511EC8A5ull, 0xFE9E115C7B8F884Cull, 0xFDEDD1B496A89F35ull,
+    0xFD3E0C0CF486C175ull, 0xFC8EC01121E447BBull, 0xFBDFED6CE5F09C49ull, 0xFB3193CC4227C3F4ull,
+    0xFA83B2DB722A033Aull, 0xF9D64A46EB939F35ull, 0xF92959BB5DD4BA74ull, 0xF87CE0E5B2094D9Cull,
+    0xF7D0DF730AD13BB9ull, 0xF7255510C4288239ull, 0xF67A416C733F846Eull, 0xF5CFA433E6537290ull};
+
+// The nearest double (ties to even) of a Fixed64.
+__device__ __forceinline__ double fixed64_to_f64(const Fixed64& v) {
+  const int lz = __clzll((long long)v.m);
+  const unsigned long long m = v.m << lz;
+  unsigned long long d = m >> 11;
+  const uint32_t rem = uint32_t(m) & 0x7FFu;
+  d += (rem > 0x400u || (rem == 0x400u && (d & 1ull))) ? 1ull : 0ull;
+  return __longlong_as_double((long long)((((unsigned long long)(1022 - 1 - lz - v.k)) << 52) + d));
+}
+
+// e^-t for 0 <= t <= kExpFixedMax.
+constexpr double kExpFixedMax = 40.0;
+__device__ __forceinline__ Fixed64 exp_neg_fixed(double t) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(t);
+  const int shift = int(bits >> 52) - 1017;  // t in units of 2^-58
+  const unsigned long long mant = (bits & ((1ull << 52) - 1ull)) | (1ull << 52);
+  const unsigned long long T = shift >= 0 ? mant << shift : (shift > -64 ? mant >> -shift : 0ull);
+  const unsigned long long u = __umul64hi(T, 0xB8AA3B295C17F0BCull);  // log2(e) * 2^63: units of 2^-57
+  const unsigned long long f = u << 7;
+  const unsigned long long z = __umul64hi(f << 8, 0xB17217F7D1CF79ACull);  // r ln 2 * 2^72
+  const uint32_t zh = uint32_t(z >> 32);
+  // 1 - x + x^2/2 - x^3/6 + x^4/24 - x^5/120, x = z * 2^-72, by Horner's rule; the inner
+  // terms in 32 bits.
+  const uint32_t a4 = 0xFFFFFFFFu - __umulhi(zh, 0xFFFFFFFFu / 1280u);
+  const uint32_t a3 = 0xFFFFFFFFu - __umulhi(zh >> 10, a4);
+  const unsigned long long a2 =
+      ~__umul64hi(__umul64hi(z, 0xFFFFFFFFFFFFFFFFull / 768ull), (unsigned long long)a3 << 32);
+  const unsigned long long a1 = ~__umul64hi(z >> 9, a2);
+  const unsigned long long tail = ~(__umul64hi(z, a1) >> 8);
+  const unsigned long long lead =
+      __umul64hi(__ldg(kExp2Sixteenths + (f >> 60)), __ldg(kExp2Fine + ((f >> 56) & 15u)));
+  return Fixed64{__umul64hi(lead, tail), int(u >> 57)};
+}
+
+// e^-t (t >= 0), rounded once.
+__device__ __forceinline__ double exp_neg(double t) {
+  return t <= kExpFixedMax ? fixed64_to_f64(exp_neg_fixed(t)) : exp(-t);
+}
+
+// With e = e^-t, 0 <= t <= kExpFixedMax: *small = e/(1+e), *big = 1/(1+e), *product their
+// product.
+__device__ __forceinline__ void logistic_fixed(double t, double* small, double* big, double* product) {
+  const Fixed64 e = exp_neg_fixed(t);
+  const unsigned long long D = (1ull << 63) + (e.k < 63 ? e.m >> (e.k + 1) : 0ull);  // (1+e) * 2^63
+  float r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(__uint2float_rn(uint32_t(D >> 32)) * 0x1p-31f));
+  const unsigned long long R0 = __float2uint_rz(r0 * 4294967296.0f);  // saturates below 2^32
+  // d = 1 - D R0 (below 2^-20), R = R0 (1 + d + d^2).
+  const long long d = (long long)((1ull << 63) - __umul64hi(D, R0 << 32));
+  const long long c = d + (((d >> 16) * (d >> 16)) >> 31);
+  const unsigned long long R = (R0 << 32) + (unsigned long long)__mul64hi((long long)(R0 << 31), c << 2);
+  const unsigned long long q = __umul64hi(e.m, R);
+  *big = fixed64_to_f64(Fixed64{R, 0});
+  *small = fixed64_to_f64(Fixed64{q, e.k});
+  *product = fixed64_to_f64(Fixed64{__umul64hi(q, R), e.k});
+}
+
 // round_half_even(x * 2^k) for a finite float x, exactly, with integer arithmetic only.
 // Equals llrint(ldexp((double)x, k)) whenever the result fits in int64 (the scale rule
 // guarantees |result| < 2^62).

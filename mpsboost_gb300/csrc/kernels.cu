@@ -142,6 +142,15 @@ __device__ __forceinline__ bool objective_pair(uint32_t objective, double y, dou
       return f64_finite(*g);
     case 1: {
       if (y != 0.0 && y != 1.0) return false;
+      const double t = __longlong_as_double(__double_as_longlong(p) & 0x7FFFFFFFFFFFFFFFll);  // |p|
+      if (t <= kExpFixedMax) {
+        // The label's side needs no subtraction: g = prob or -(1 - prob).
+        double small, big;
+        logistic_fixed(t, &small, &big, h);
+        const bool negative = __double_as_longlong(p) < 0;
+        *g = y == 0.0 ? (negative ? small : big) : (negative ? -big : -small);
+        return true;
+      }
       const double prob = logistic_probability(p);
       *g = __dadd_rn(prob, -y);
       *h = __dmul_rn(prob, __dadd_rn(1.0, -prob));
@@ -189,7 +198,7 @@ __device__ __forceinline__ bool softmax_pair(const TrainerDev& a, double label, 
   }
   double normalizer = 0.0, target_exp = 0.0;
   for (uint32_t k = 0; k < K; ++k) {
-    const double e = exp(__dadd_rn(a.preds[size_t(k) * a.n_rows + row], -maximum));
+    const double e = exp_neg(__dadd_rn(maximum, -a.preds[size_t(k) * a.n_rows + row]));
     normalizer = __dadd_rn(normalizer, e);
     if (k == target) target_exp = e;
   }

@@ -3,6 +3,9 @@ replica (every tree node and training prediction)."""
 
 from __future__ import annotations
 
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -52,3 +55,30 @@ def test_partition_edges(backend, port, rows):
     y, w = targets(x, rows)
     assert_equals_replica(backend, port, x, y, w, 64, n_estimators=2, learning_rate=0.3, max_depth=4,
                           min_samples_leaf=2)
+
+
+# A histogram cell of 2,047 rows (the packed limbs' largest), one past it, and multiples of
+# 2,048 (whose count fields read 0), in a block with continuous features; unweighted fits
+# build two packed words, weighted ones four.
+@pytest.mark.parametrize("heavy", [2047, 2048, 4096, 6144])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_packed_limb_overflow(backend, port, heavy, weighted):
+    x = seeded_matrix(heavy, 10_000, 34, 0.0)
+    x[:, 1] = 1.0
+    x[:heavy, 1] = 0.0
+    x[:, 33] = np.arange(10_000) % 3 == 0
+    y, w = targets(x, heavy)
+    assert_equals_replica(backend, port, x, y, w if weighted else None, 255, n_estimators=3, learning_rate=0.3,
+                          max_depth=4, min_samples_leaf=2)
+
+
+def test_integer_pipe_logistic_within_half_an_ulp(tmp_path):
+    """e^-t and the logistic function's pieces on the integer pipe against long double."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = tmp_path / "logistic_check"
+    subprocess.run(["nvcc", "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17",
+                    "-I", os.path.join(root, "mpsboost_gb300", "csrc"), "-I", os.path.join(root, "include"),
+                    os.path.join(root, "tests", "native", "logistic_check.cu"), "-o", str(exe)],
+                   check=True)
+    run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stdout + run.stderr
