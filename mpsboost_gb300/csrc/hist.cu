@@ -487,7 +487,35 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 // This thread's bulk operations are complete (their global writes performed).
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 
-template <int MODE, int THREADS>
+// Packed limbs (fixed-point modes with counts): per cell, with N rows of values q < 2^30,
+//  word 0  sum of q_g mod 2^32                     (the value's low 32 bits, no split)
+//  kModeFixed:   word 1  sum of q_h mod 2^32
+//                word 2  sum of floor(q_g / 2^21), signed
+//                word 3  sum of floor(q_h / 2^21) * 2^11 + 1: the count below it
+//  kModeFixedCG: word 1  sum of floor(q_g / 2^21) * 2^11 + 1 (signed, mod 2^32)
+// While N <= 2047 the count field cannot carry, the high sums stay inside their fields
+// (2^9 * 2047 < 2^20), and since 0 <= sum q - 2^21 * sum floor(q / 2^21) < N * 2^21 <= 2^32
+// the two words give sum q exactly. A cell past 2047 rows loses a multiple of 2048 from its
+// count field, so a feature's count fields add up to the item's rows exactly when no cell
+// of the feature passed; an item that fails this check is built again with split limbs.
+// That is four reductions per cell instead of five (two instead of three) of the shared
+// reduction rate that bounds the kernel.
+constexpr uint32_t kPackCountBits = 11;
+constexpr uint32_t kPackCountMask = (1u << kPackCountBits) - 1u;
+constexpr int kPackShift = 21;
+
+template <int MODE>
+__host__ __device__ constexpr bool can_pack() { return MODE == kModeFixed || MODE == kModeFixedCG; }
+template <int MODE>
+__host__ __device__ constexpr int packed_words() { return MODE == kModeFixed ? 4 : 2; }
+
+// The exact sum from its value mod 2^32 and the sum of its rows' high parts.
+__device__ __forceinline__ unsigned long long packed_sum(uint32_t low, int32_t high) {
+  const long long near = (long long)high * (1ll << kPackShift);
+  return (unsigned long long)(near + (long long)(low - uint32_t(near)));
+}
+
+template <int MODE, int THREADS, bool PACKED>
 __device__ __forceinline__ void flush_cta_histogram_bulk(const TrainerDev& a, const BuildEntry& e, uint32_t fb,
                                                          const unsigned char* hist_smem,
                                                          unsigned long long* staging, long long q_unit_h,
@@ -512,7 +540,17 @@ __device__ __forceinline__ void flush_cta_histogram_bulk(const TrainerDev& a, co
       for (uint32_t j = 0; j < kFlushBins; ++j) {
         const uint32_t idx = (b0 + j) * kBlockFeatures + lane;
         unsigned long long c, g, h;
-        if constexpr (MODE == kModeFixed) {
+        if constexpr (PACKED && MODE == kModeFixed) {
+          const uint32_t hc = w[3 * CELLS + idx];
+          c = hc & kPackCountMask;
+          g = packed_sum(w[idx], int32_t(w[2 * CELLS + idx]));
+          h = packed_sum(w[CELLS + idx], int32_t(hc >> kPackCountBits));
+        } else if constexpr (PACKED) {
+          const uint32_t gc = w[CELLS + idx];
+          c = gc & kPackCountMask;
+          g = packed_sum(w[idx], int32_t(gc) >> kPackCountBits);
+          h = (unsigned long long)((long long)c * q_unit_h);
+        } else if constexpr (MODE == kModeFixed) {
           c = w[idx];
           g = (unsigned long long)((long long)int32_t(w[2 * CELLS + idx]) * 65536 + (long long)w[CELLS + idx]);
           h = (unsigned long long)((long long)w[4 * CELLS + idx] * 65536 + (long long)w[3 * CELLS + idx]);
@@ -544,9 +582,17 @@ __device__ __forceinline__ void flush_cta_histogram_bulk(const TrainerDev& a, co
   }
 }
 
+// Items of a (depth level, feature block) build with packed limbs while at most one in
+// kPackFailCost of them has failed the check (limb_votes: passed, failed, kept over the
+// trainer's rounds). A failed item costs about two, a passed one saves a fifth to a third,
+// so the break-even is one failure in three to five; a block with a heavy cell (a feature
+// of few bins, many missing rows) fails its first items and stays on split limbs.
+constexpr uint32_t kPackFailCost = 8;
+
 // A work item's description, prepared one item ahead by one warp.
 struct ItemDesc {
   uint32_t item, limit, fb, row_begin, row_count;
+  uint32_t packed;  // build with packed limbs first
   int kg, kh;
   BuildEntry e;
 };
@@ -580,6 +626,11 @@ __device__ __forceinline__ void fetch_item_warp(const TrainerDev& a, uint32_t la
     d.row_count = d.row_begin < d.e.seg_cnt ? min(item_rows, d.e.seg_cnt - d.row_begin) : 0u;
     d.kg = a.trees[d.e.tree].kg;
     d.kh = a.trees[d.e.tree].kh;
+    if (a.limb_votes) {
+      const volatile uint32_t* votes = a.limb_votes + 2 * d.fb;  // other CTAs add to them
+      const uint32_t passed = votes[0], failed = votes[1];
+      d.packed = failed * kPackFailCost <= passed + 2 * kPackFailCost;
+    }
   }
   if (lane == 0) *out = d;
 }
@@ -615,8 +666,17 @@ __global__ void __launch_bounds__(THREADS, 1) hist_build_direct_kernel(TrainerDe
   const uint32_t lb = lane & 3u;
   const uint32_t byte_sel = (0u ^ lb) | ((1u ^ lb) << 4) | ((2u ^ lb) << 8) | ((3u ^ lb) << 12);
 
+  auto zero = [&](int words16) {
+    uint4* z = reinterpret_cast<uint4*>(hist_smem);
+    for (int i = tid; i < words16; i += THREADS) z[i] = make_uint4(0, 0, 0, 0);
+  };
+  constexpr int kSplitWords16 = int(HistSmem<MODE>::kBytes / 16);
+  constexpr int kPackedWords16 = can_pack<MODE>() ? packed_words<MODE>() * CELLS / 4 : kSplitWords16;
+  uint32_t* s_ok = reinterpret_cast<uint32_t*>(s_desc + 1);  // [kBlockFeatures] count sums, then the verdict
   if (warp == kFlushWarps) fetch_item_warp(a, lane, s_desc);
+  zero(kSplitWords16);  // beside the first item's chain of loads
   __syncthreads();
+  bool zeroed = true;
   // With hist_base 128-byte aligned, hist_base + 4 (lane ^ i) = (hist_base + 4 lane) ^ 4 i
   // (4 lane and 4 i stay below 128), one instruction per reduction round.
   const bool aligned = (hist_base & 127u) == 0u;  // CTA-uniform
@@ -636,11 +696,10 @@ __global__ void __launch_bounds__(THREADS, 1) hist_build_direct_kernel(TrainerDe
     const int kg = d.kg;
     const int kh = d.kh;
     const long long q_unit_h = MODE == kModeFixedCG ? quantize_f32(1.0f, kh) : 0ll;
-    {
-      uint4* z = reinterpret_cast<uint4*>(hist_smem);
-      const int words = int(HistSmem<MODE>::kBytes / 16);
-      for (int i = tid; i < words; i += THREADS) z[i] = make_uint4(0, 0, 0, 0);
-    }
+    bool packed = can_pack<MODE>() && d.packed != 0;  // CTA-uniform
+    if (!zeroed) zero(packed ? kPackedWords16 : kSplitWords16);
+    zeroed = false;
+    if (packed && tid < kBlockFeatures) s_ok[tid] = 0;
     __syncthreads();  // also: every thread holds this item's description
 
     const uint32_t ngroups = (row_count + 31u) / 32u;
@@ -661,96 +720,137 @@ __global__ void __launch_bounds__(THREADS, 1) hist_build_direct_kernel(TrainerDe
       if (k >= my || pos >= row_count) return make_float2(0.f, 0.f);
       return gh_seg ? __ldg(gh_seg + pos) : __ldg(gh_row + r);
     };
-    // Ring of the next PF groups' bins and pairs; the row id of group k + PF is loaded
-    // one iteration before its bins.
-    Bins32 bq[PF];
-    float2 gq[PF];
+    // Reduces the item's rows into the CTA histogram, in packed or split limbs.
+    auto accumulate = [&](auto packed_tag) {
+      constexpr bool PACKED = decltype(packed_tag)::value;
+      // Ring of the next PF groups' bins and pairs; the row id of group k + PF is loaded
+      // one iteration before its bins.
+      Bins32 bq[PF];
+      float2 gq[PF];
 #pragma unroll
-    for (int j = 0; j < PF; ++j) {
-      const uint32_t r = row_at(uint32_t(j));
-      bq[j] = bins_at(uint32_t(j), r);
-      gq[j] = gh_at(uint32_t(j), r);
-    }
-    uint32_t r_ahead = row_at(PF);
-    for (uint32_t k = 0; k < my; ++k) {
-      const uint32_t r_next = row_at(k + PF + 1);
-      const Bins32 b_new = bins_at(k + PF, r_ahead);
-      const float2 g_new = gh_at(k + PF, r_ahead);
-      const Bins32& b0 = bq[0];
-      const float2& g0 = gq[0];
-      if (pos_of(k) < row_count) {
-        // Limbs of the row's quantized values (|q| <= 2^30): unsigned low 16 bits and the
-        // signed high part.
-        uint32_t glo, ghi, hlo = 0, hhi = 0;
-        {
-          const long long qg = quantize_f32(g0.x, kg);
-          glo = uint32_t(qg) & 0xFFFFu;
-          ghi = uint32_t(int32_t(qg >> 16));
-          if constexpr (MODE == kModeFixed) {
-            const long long qh = quantize_f32(g0.y, kh);
-            hlo = uint32_t(qh) & 0xFFFFu;
-            hhi = uint32_t(qh >> 16);
-          }
-        }
-        // w[k] = word k ^ lw of the row's block with its bytes permuted by lb: byte i of w
-        // is byte i ^ lane of the block (feature i ^ lane).
-        uint32_t w[8];
-#pragma unroll
-        for (uint32_t k8 = 0; k8 < 8; ++k8) w[k8] = b0.w[k8];
-#pragma unroll
-        for (uint32_t bit = 1; bit < 8; bit <<= 1) {
-          const bool swap = (lw & bit) != 0;  // per lane: selects, no divergence
-#pragma unroll
-          for (uint32_t k8 = 0; k8 < 8; ++k8)
-            if ((k8 & bit) == 0) {
-              const uint32_t x = w[k8], y = w[k8 | bit];
-              w[k8] = swap ? y : x;
-              w[k8 | bit] = swap ? x : y;
-            }
-        }
-#pragma unroll
-        for (uint32_t k8 = 0; k8 < 8; ++k8) w[k8] = __byte_perm(w[k8], 0u, byte_sel);
-        auto reduce_row = [&](auto aligned_tag) {
-          constexpr bool ALIGNED = decltype(aligned_tag)::value;
-#pragma unroll
-          for (uint32_t i = 0; i < 32; ++i) {
-            const uint32_t bin = (w[i >> 2] >> (8u * (i & 3u))) & 0xFFu;
-            const uint32_t cell = ALIGNED ? (lane_base ^ (i << 2)) : hist_base + ((lane ^ i) << 2);
-            const uint32_t addr = cell + (bin << 7);  // bin * kBlockFeatures * 4 bytes
-            if constexpr (MODE == kModeFixed) {
-              red_shared_u32<0>(addr, 1u);
-              red_shared_u32<1u * CELLS * 4u>(addr, glo);
-              red_shared_u32<2u * CELLS * 4u>(addr, ghi);
-              red_shared_u32<3u * CELLS * 4u>(addr, hlo);
-              red_shared_u32<4u * CELLS * 4u>(addr, hhi);
+      for (int j = 0; j < PF; ++j) {
+        const uint32_t r = row_at(uint32_t(j));
+        bq[j] = bins_at(uint32_t(j), r);
+        gq[j] = gh_at(uint32_t(j), r);
+      }
+      uint32_t r_ahead = row_at(PF);
+      for (uint32_t k = 0; k < my; ++k) {
+        const uint32_t r_next = row_at(k + PF + 1);
+        const Bins32 b_new = bins_at(k + PF, r_ahead);
+        const float2 g_new = gh_at(k + PF, r_ahead);
+        const Bins32& b0 = bq[0];
+        const float2& g0 = gq[0];
+        if (pos_of(k) < row_count) {
+          // The words the row adds to each of its cells (word 0 first). Split limbs
+          // (|q| <= 2^30): unsigned low 16 bits and the signed high part.
+          uint32_t v0, v1, v2 = 0, v3 = 0, v4 = 0;
+          {
+            const long long qg = quantize_f32(g0.x, kg);
+            if constexpr (PACKED) {
+              v0 = uint32_t(qg);
+              const int32_t high = int32_t(qg >> kPackShift);
+              if constexpr (MODE == kModeFixed) {
+                const long long qh = quantize_f32(g0.y, kh);
+                v1 = uint32_t(qh);
+                v2 = uint32_t(high);
+                v3 = (uint32_t(qh >> kPackShift) << kPackCountBits) | 1u;
+              } else {
+                v1 = (uint32_t(high) << kPackCountBits) | 1u;
+              }
             } else if constexpr (MODE == kModeFixedG) {
-              red_shared_u32<0>(addr, glo);
-              red_shared_u32<1u * CELLS * 4u>(addr, ghi);
+              v0 = uint32_t(qg) & 0xFFFFu;
+              v1 = uint32_t(int32_t(qg >> 16));
             } else {
-              red_shared_u32<0>(addr, 1u);
-              red_shared_u32<1u * CELLS * 4u>(addr, glo);
-              red_shared_u32<2u * CELLS * 4u>(addr, ghi);
+              v0 = 1u;
+              v1 = uint32_t(qg) & 0xFFFFu;
+              v2 = uint32_t(int32_t(qg >> 16));
+              if constexpr (MODE == kModeFixed) {
+                const long long qh = quantize_f32(g0.y, kh);
+                v3 = uint32_t(qh) & 0xFFFFu;
+                v4 = uint32_t(qh >> 16);
+              }
             }
           }
-        };
-        if (aligned) reduce_row(std::true_type{});
-        else reduce_row(std::false_type{});
-      }
+          // w[k] = word k ^ lw of the row's block with its bytes permuted by lb: byte i of w
+          // is byte i ^ lane of the block (feature i ^ lane).
+          uint32_t w[8];
 #pragma unroll
-      for (int j = 0; j + 1 < PF; ++j) {
-        bq[j] = bq[j + 1];
-        gq[j] = gq[j + 1];
+          for (uint32_t k8 = 0; k8 < 8; ++k8) w[k8] = b0.w[k8];
+#pragma unroll
+          for (uint32_t bit = 1; bit < 8; bit <<= 1) {
+            const bool swap = (lw & bit) != 0;  // per lane: selects, no divergence
+#pragma unroll
+            for (uint32_t k8 = 0; k8 < 8; ++k8)
+              if ((k8 & bit) == 0) {
+                const uint32_t x = w[k8], y = w[k8 | bit];
+                w[k8] = swap ? y : x;
+                w[k8 | bit] = swap ? x : y;
+              }
+          }
+#pragma unroll
+          for (uint32_t k8 = 0; k8 < 8; ++k8) w[k8] = __byte_perm(w[k8], 0u, byte_sel);
+          auto reduce_row = [&](auto aligned_tag) {
+            constexpr bool ALIGNED = decltype(aligned_tag)::value;
+            constexpr int WORDS = PACKED ? packed_words<MODE>() : int(HistSmem<MODE>::kBytes / (4 * CELLS));
+#pragma unroll
+            for (uint32_t i = 0; i < 32; ++i) {
+              const uint32_t bin = (w[i >> 2] >> (8u * (i & 3u))) & 0xFFu;
+              const uint32_t cell = ALIGNED ? (lane_base ^ (i << 2)) : hist_base + ((lane ^ i) << 2);
+              const uint32_t addr = cell + (bin << 7);  // bin * kBlockFeatures * 4 bytes
+              red_shared_u32<0>(addr, v0);
+              red_shared_u32<1u * CELLS * 4u>(addr, v1);
+              if constexpr (WORDS > 2) red_shared_u32<2u * CELLS * 4u>(addr, v2);
+              if constexpr (WORDS > 3) red_shared_u32<3u * CELLS * 4u>(addr, v3);
+              if constexpr (WORDS > 4) red_shared_u32<4u * CELLS * 4u>(addr, v4);
+            }
+          };
+          if (aligned) reduce_row(std::true_type{});
+          else reduce_row(std::false_type{});
+        }
+#pragma unroll
+        for (int j = 0; j + 1 < PF; ++j) {
+          bq[j] = bq[j + 1];
+          gq[j] = gq[j + 1];
+        }
+        bq[PF - 1] = b_new;
+        gq[PF - 1] = g_new;
+        r_ahead = r_next;
       }
-      bq[PF - 1] = b_new;
-      gq[PF - 1] = g_new;
-      r_ahead = r_next;
+    };
+    if constexpr (can_pack<MODE>()) {
+      if (packed) {
+        accumulate(std::true_type{});
+        __syncthreads();
+        if (row_count > kPackCountMask) {
+          // Each feature's count fields, lane = feature, bins over the warps.
+          const uint32_t* counts = reinterpret_cast<const uint32_t*>(hist_smem) + (packed_words<MODE>() - 1) * CELLS;
+          uint32_t sum = 0;
+          for (uint32_t b = uint32_t(warp); b < kSlots; b += WARPS) sum += counts[b * kBlockFeatures + lane] & kPackCountMask;
+          atomicAdd(s_ok + lane, sum);
+          __syncthreads();
+          // Padding features of the last block hold every row in bin 0: they are not flushed.
+          const bool good = fb * kBlockFeatures + lane >= a.features || s_ok[lane] == row_count;
+          packed = __all_sync(0xffffffffu, good);  // the same in every warp
+          if (tid == 0) atomicAdd(a.limb_votes + 2 * fb + (packed ? 0 : 1), 1u);
+          if (!packed) {
+            __syncthreads();
+            zero(kSplitWords16);
+            __syncthreads();
+          }
+        }
+      }
     }
-    __syncthreads();
+    if (!packed) {
+      accumulate(std::false_type{});
+      __syncthreads();
+    }
     // The next item's description is fetched while the flush warps work.
     if (warp == kFlushWarps) fetch_item_warp(a, lane, s_desc);
-    flush_cta_histogram_bulk<MODE, THREADS>(
-        a, e, fb, hist_smem, reinterpret_cast<unsigned long long*>(hist_smem + HistSmem<MODE>::kBytes),
-        q_unit_h, row_count);
+    unsigned long long* staging = reinterpret_cast<unsigned long long*>(hist_smem + HistSmem<MODE>::kBytes);
+    if (can_pack<MODE>() && packed)
+      flush_cta_histogram_bulk<MODE, THREADS, true>(a, e, fb, hist_smem, staging, q_unit_h, row_count);
+    else
+      flush_cta_histogram_bulk<MODE, THREADS, false>(a, e, fb, hist_smem, staging, q_unit_h, row_count);
     __syncthreads();
   }
   bulk_wait_all();  // this thread's bulk reductions have reached the slots
@@ -759,7 +859,7 @@ __global__ void __launch_bounds__(THREADS, 1) hist_build_direct_kernel(TrainerDe
 template <int MODE, int THREADS, int PF = 2>
 cudaError_t launch_direct(const TrainerDev& a, int grid, cudaStream_t stream) {
   static_assert(kBlockFeatures * 4 == 128, "a bin row of the CTA histogram is 128 bytes");
-  const size_t smem = HistSmem<MODE>::kBytes + kFlushBytes + (sizeof(ItemDesc) + 15) / 16 * 16;
+  const size_t smem = HistSmem<MODE>::kBytes + kFlushBytes + (sizeof(ItemDesc) + kBlockFeatures * 4 + 15) / 16 * 16;
   static std::atomic<unsigned long long> configured{0};  // one bit per device
   const cudaError_t err = opt_in_dynamic_smem(configured, hist_build_direct_kernel<MODE, THREADS, PF>, smem);
   if (err != cudaSuccess) return err;

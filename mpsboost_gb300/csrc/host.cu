@@ -742,6 +742,7 @@ struct mpsb_cuda_trainer {
   std::vector<uint64_t> level_cells_total;
   uint32_t rounds_enqueued = 0;
   uint32_t blocked_levels = 2;  // levels built from the column-blocked bins
+  uint32_t* limb_votes = nullptr;  // [levels][nfb][2] (device): TrainerDev::limb_votes by level
   mpsb_cuda_stats stats{};
   uint64_t kernels_per_round[2] = {0, 0};
   uint64_t cells_base = 0, rows_base = 0, part_base = 0;
@@ -885,7 +886,7 @@ struct mpsb_cuda_trainer {
       CK(cudaEventRecord(zero_ev, side));
       CK(launch_partition(dev, n_trees, grid(4), s)); k += partition_kernels(dev, n_trees);
       CK(cudaStreamWaitEvent(s, zero_ev, 0));
-      CK(launch_hist_build(build_view(), hcfg, grid(1), s)); ++k;
+      CK(launch_hist_build(step_view(), hcfg, grid(1), s)); ++k;
       if (!dev.fused_sub) { CK(launch_subtract(dev, grid(8), s)); ++k; }
       const uint32_t scans = split_scan_kernels(dev);
       CK(launch_split_scan(dev, 1, 2 * n_trees, true, grid(4), s)); k += scans;
@@ -902,11 +903,19 @@ struct mpsb_cuda_trainer {
     return v;
   }
 
+  // A leaf-wise step's view: the packed-limb votes of level 1 stand for every step.
+  TrainerDev step_view() const {
+    TrainerDev v = build_view();
+    if (limb_votes) v.limb_votes = limb_votes + size_t(2) * dev.nfb;
+    return v;
+  }
+
   // Dense levels (every row of a node close to the next) read the column-blocked copy of
   // the bins, whose 32-byte block rows are consecutive; sparse levels read the padded
   // row-major copy, whose 128-byte row line serves all feature blocks through L2.
   TrainerDev level_view(uint32_t d) const {
     TrainerDev v = build_view();
+    if (limb_votes) v.limb_votes = limb_votes + size_t(2) * dev.nfb * d;
     if (d < blocked_levels) {
       v.bins = ds->bins_blocked.as<uint8_t>();
       v.bins_row_stride = kBlockFeatures;
@@ -1307,6 +1316,13 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.tree_nodes = t->alloc<TreeNodeOut>(size_t(T) * tree_nodes);
   a.ctl = t->alloc<Control>(1);
   CK(cudaMemsetAsync(a.ctl, 0, sizeof(Control), s));
+  // Packed histogram limbs (MPSB_PACKED=0: split limbs only).
+  const char* packed = std::getenv("MPSB_PACKED");
+  if (a.mode == kModeFixed && ds->slots == uint32_t(kSlots) && !(packed && std::atoi(packed) == 0)) {
+    const size_t votes = size_t(std::max<uint32_t>(D, 2)) * ds->nfb * 2;
+    t->limb_votes = t->alloc<uint32_t>(votes);
+    CK(cudaMemsetAsync(t->limb_votes, 0, votes * sizeof(uint32_t), s));
+  }
   a.scratch_flags = t->alloc<uint32_t>(a.max_level_nodes);
   a.scratch_prefix = t->alloc<uint32_t>(a.max_level_nodes);
   a.scratch_aux = t->alloc<uint32_t>(a.max_level_nodes);

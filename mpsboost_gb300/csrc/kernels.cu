@@ -37,9 +37,11 @@ __device__ __forceinline__ void raise(Control* ctl, uint32_t bits) { atomicOr(&c
 __device__ __forceinline__ uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 // Rows per histogram work item for a level that builds `rows` rows: about per_sm (default
-// three) items per SM, a multiple of 512, within [4096, kItemRowsMax]. Where the
+// three) items per SM, a multiple of 512, within [1024, kItemRowsMax]. Where the
 // kItemRowsMax cap forces more items, their number is raised to the next multiple of the
-// SM count, so that the persistent CTAs end the level together.
+// SM count, so that the persistent CTAs end the level together. At the lower end an item's
+// reductions (about 1.5 us) weigh as much as its flush: 100,000 x 32, depth 6, 50 trees
+// take 17.5, 17.3, 17.7 and 18.7 ms with items of 512, 1,024, 2,048 and 4,096 rows.
 __device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, uint32_t nfb, uint32_t sms,
                                                       uint32_t per_sm) {
   const uint64_t n_sm = sms ? sms : 152;
@@ -48,7 +50,7 @@ __device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, uint32_t n
   if (target < min_items) target = (min_items + n_sm - 1) / n_sm * n_sm;
   uint64_t per = (rows * nfb + target - 1) / target;
   per = (per + 511) / 512 * 512;
-  if (per < 4096) per = 4096;
+  if (per < 1024) per = 1024;
   if (per > kItemRowsMax) per = kItemRowsMax;
   return uint32_t(per);
 }

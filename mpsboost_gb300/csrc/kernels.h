@@ -93,6 +93,8 @@ struct TrainerDev {
   TreeNodeOut* tree_nodes;      // [n_trees][max_tree_nodes]
   uint32_t max_tree_nodes;
   Control* ctl;
+  uint32_t* limb_votes;         // [nfb][2] of the launch's depth level: work items that passed
+                                // and failed the packed-limb check (null: split limbs only)
   uint32_t item_rows;           // rows per histogram work item (<= kItemRowsMax); 0: the
                                 // level's adaptive value ctl->item_rows
   uint32_t sm_count;
