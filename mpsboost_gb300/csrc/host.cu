@@ -200,6 +200,11 @@ RowSums row_sums_checked(const double* w, const double* y, uint64_t n, int label
 RowSums row_sums(const double* w, const double* y, uint64_t n, int label_mode, const char* name) {
   if (n == 0) throw TrainingError("labels must be non-empty");
   const int mode = y ? label_mode : 0;
+  if (!w && !mode) {  // n unit weights: their sum is n exactly
+    RowSums r;
+    r.total = double(n);
+    return r;
+  }
   std::atomic<bool> bad{false};
   const uint32_t workers = uint32_t(std::min<uint64_t>(
       std::max(1u, std::min(16u, std::thread::hardware_concurrency())), (n + (1u << 20) - 1) >> 20));
@@ -258,6 +263,14 @@ int label_mode_of(uint32_t objective) {
   return 0;
 }
 
+// The logistic base score of a positive weight total.
+double logistic_base(double pos, double total) {
+  const double eps = 1e-15;
+  double prob = pos / total;
+  prob = std::min(1.0 - eps, std::max(eps, prob));
+  return std::log(prob / (1.0 - prob));
+}
+
 // InitialBaseScore (trainer.cpp:68-176) on host FP64 in row order. `cls` >= 0 selects the
 // one-vs-rest binary labels (label == cls). `pre`: this fit's row sums, when they carry
 // the label sum of the objective (cls < 0).
@@ -285,10 +298,7 @@ double base_score(const mpsb_train_params& p, const double* y, const double* w, 
         if (l == 1.0) { pos += W(i); continue; }
         throw TrainingError("binary-logistic labels must be 0 or 1");
       }
-      const double eps = 1e-15;
-      double prob = pos / total;
-      prob = std::min(1.0 - eps, std::max(eps, prob));
-      return std::log(prob / (1.0 - prob));
+      return logistic_base(pos, total);
     }
     case MPSB_QUANTILE: {
       std::vector<std::pair<double, double>> o(n);
@@ -1186,13 +1196,29 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
     a.weights = d_w;
   }
 
+  // Unweighted class fits: the rows of each class, counted on the device. With a label that
+  // is no class id the host passes below report it.
+  std::vector<unsigned long long> class_rows;
+  if (!weights && !forest && (softmax_classes || p->objective == MPSB_BINARY_LOGISTIC)) {
+    const uint32_t K = softmax_classes ? softmax_classes : (t->ovr ? n_classes : 2u);
+    if (K <= kLabelCountMax) {
+      unsigned long long* d_counts = t->alloc<unsigned long long>(K + 1);
+      CK(cudaMemsetAsync(d_counts, 0, (K + 1) * sizeof(unsigned long long), s));
+      CK(launch_label_counts(d_labels, n, K, d_counts, s));
+      class_rows.resize(K + 1);
+      CK(cudaMemcpyAsync(class_rows.data(), d_counts, (K + 1) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+      if (class_rows[K] != 0) class_rows.clear();
+    }
+  }
   if (softmax_classes) {
     // Margins [K][n] from the class priors (WeightedClassBaseScores,
     // multiclass_trainer.cpp:39-67); labels must be class ids (22-37).
     const uint32_t K = softmax_classes;
     const double total = sums.total;
     std::vector<double> cw(K, 0.0);
-    for (uint64_t i = 0; i < n; ++i) {
+    for (uint32_t k = 0; k < K && !class_rows.empty(); ++k) cw[k] = double(class_rows[k]);
+    for (uint64_t i = 0; i < n && class_rows.empty(); ++i) {
       const double y = labels[i];
       if (!std::isfinite(y)) throw TrainingError("softmax labels must be finite");
       if (std::floor(y) != y || y < 0.0 || y >= double(K))
@@ -1213,7 +1239,9 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   if (!softmax_classes) a.preds = t->alloc<double>(size_t(T) * n);
   for (uint32_t k = 0; k < T && !softmax_classes; ++k) {
     t->base_scores[k] = forest ? forest->base_scores[k]
-                               : base_score(*p, labels, weights, n, t->ovr ? int64_t(k) : -1, &sums);
+                        : !class_rows.empty()
+                            ? logistic_base(double(class_rows[t->ovr ? k : 1u]), sums.total)
+                            : base_score(*p, labels, weights, n, t->ovr ? int64_t(k) : -1, &sums);
     CK(launch_fill_f64(a.preds + size_t(k) * n, n, t->base_scores[k], s));
   }
   trace.mark("base scores, predictions");
@@ -1631,11 +1659,12 @@ int mpsb_cuda_train_ovr(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
                         mpsb_cuda_model** out) {
   return guard([&] {
     if (n_classes < 2) throw TrainingError("one-vs-rest needs at least two classes");
+    bool ids = true;
     for (uint64_t i = 0; i < n; ++i) {
       const double y = labels[i];
-      if (!(y >= 0.0 && y < double(n_classes) && std::floor(y) == y))
-        throw TrainingError("one-vs-rest labels must be class ids in [0, n_classes)");
+      ids &= (y >= 0.0) & (y < double(n_classes)) & (std::floor(y) == y);
     }
+    if (!ids) throw TrainingError("one-vs-rest labels must be class ids in [0, n_classes)");
     std::unique_ptr<mpsb_cuda_trainer> t(new mpsb_cuda_trainer);
     setup_trainer(t.get(), b, ds, labels, weights, n, p, options, n_classes);
     t->run(p->n_estimators);

@@ -3152,6 +3152,25 @@ __global__ void round_end_kernel(TrainerDev a) {
   if (threadIdx.x == 0) *a.round_counter = round + 1;
 }
 
+// Rows of each class id 0..classes-1 (counts[classes]: rows whose label is none of them).
+// The class priors and the logistic base score of an unweighted fit are these whole
+// numbers, in any order of addition. HBM-bound (8 B per row); shared-memory counters per
+// CTA.
+__global__ void __launch_bounds__(256) label_counts_kernel(const double* labels, uint64_t n, uint32_t classes,
+                                                           unsigned long long* counts) {
+  extern __shared__ uint32_t s_counts[];  // [classes + 1]
+  for (uint32_t k = threadIdx.x; k <= classes; k += blockDim.x) s_counts[k] = 0;
+  __syncthreads();
+  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
+    const double y = labels[i];
+    const bool id = y >= 0.0 && y < double(classes) && floor(y) == y;
+    atomicAdd(s_counts + (id ? uint32_t(y) : classes), 1u);
+  }
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k <= classes; k += blockDim.x)
+    if (s_counts[k]) atomicAdd(counts + k, (unsigned long long)s_counts[k]);
+}
+
 // ------------------------------------------------------------------------------------
 // Standalone entries
 // ------------------------------------------------------------------------------------
@@ -3544,6 +3563,13 @@ cudaError_t launch_apply_leaves(const TrainerDev& a, int grid, cudaStream_t s) {
 }
 cudaError_t launch_round_end(const TrainerDev& a, cudaStream_t s) {
   round_end_kernel<<<1, 256, 0, s>>>(a);
+  return cudaGetLastError();
+}
+cudaError_t launch_label_counts(const double* labels, uint64_t n, uint32_t classes, unsigned long long* counts,
+                                cudaStream_t s) {
+  if (n == 0 || classes > kLabelCountMax) return cudaErrorInvalidValue;
+  const unsigned grid = unsigned(std::min<uint64_t>((n + 1023) / 1024, 152ull * 8));
+  label_counts_kernel<<<grid, 256, (classes + 1) * sizeof(uint32_t), s>>>(labels, n, classes, counts);
   return cudaGetLastError();
 }
 cudaError_t launch_squared_error(const double* labels, const double* preds, uint64_t n,

@@ -196,6 +196,10 @@ cudaError_t launch_partition_count(const TrainerDev& a, int grid, cudaStream_t s
 cudaError_t launch_partition_finish(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_apply_leaves(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_round_end(const TrainerDev& a, cudaStream_t stream);
+// counts [classes + 1], zeroed by the caller: rows per class id, then rows of no class.
+constexpr uint32_t kLabelCountMax = 8192;  // classes (32 KB of shared counters)
+cudaError_t launch_label_counts(const double* labels, uint64_t n, uint32_t classes, unsigned long long* counts,
+                                cudaStream_t stream);
 cudaError_t launch_squared_error(const double* labels, const double* preds, uint64_t n,
                                  double* out_pairs, uint32_t* error, cudaStream_t stream);
 // Bins from the u8 feature-major copy (missing rows at 255), or with bins16_fm set from

@@ -82,3 +82,26 @@ def test_integer_pipe_logistic_within_half_an_ulp(tmp_path):
                    check=True)
     run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
     assert run.returncode == 0, run.stdout + run.stderr
+
+
+# Unweighted class fits count their labels on the device: rows around a CTA's 1,024 and a
+# label that is no class id.
+@pytest.mark.parametrize("rows", [40, 1023, 1025, 300_001])
+@pytest.mark.parametrize("classes", [2, 7])
+def test_class_counts_give_the_base_scores(backend, rows, classes):
+    x = seeded_matrix(rows, rows, 2)
+    y = np.random.default_rng(rows).integers(0, classes, rows).astype(np.float64)
+    y[:classes] = np.arange(classes)
+    binned = mb.quantize_dense(x, 16)
+    params = dict(n_estimators=1, max_depth=2, learning_rate=0.5)
+    share = [np.count_nonzero(y == k) / rows for k in range(classes)]
+    got = [m.base_score for m in mb.train_ovr(backend, binned, y, classes, **params)]
+    np.testing.assert_allclose(got, [np.log(p / (1 - p)) for p in share], rtol=1e-15, atol=1e-15)
+    soft = mb.train_softmax(backend, binned, y, classes, **params)
+    np.testing.assert_allclose(soft.base_scores, np.log(share), rtol=1e-15)
+    y[-1] = 0.5
+    with pytest.raises(mb.TrainingError, match="0 or 1" if classes == 2 else "class ids"):
+        if classes == 2:
+            mb.train_regressor(backend, binned, y, objective="binary_logistic", **params)
+        else:
+            mb.train_softmax(backend, binned, y, classes, **params)
