@@ -16,7 +16,6 @@ constexpr int kMissingSlot = 255;    // bin value of a missing row (features wit
 constexpr int kBlockFeatures = 32;   // features per column block of the bin matrix
 constexpr uint32_t kItemRowsMax = 65536;  // rows of one histogram work item (limb bound)
 constexpr uint32_t kPartChunk = 4096;     // rows per partition chunk
-constexpr uint32_t kApplyChunk = 4096;    // rows per leaf-application chunk
 
 // kModeFixedG: fixed point, gradient limbs only (a root build whose count and hessian
 // histograms are restored from the fit's first round).
@@ -179,6 +178,8 @@ struct Control {
   uint32_t free_top;       // histogram-slot free stack
   uint32_t split_items;    // nodes x feature chunks
   uint32_t item_rows;      // rows per histogram work item of the current level
+  uint32_t round;          // the round in progress
+  uint32_t grad_ticket;    // CTAs of the gradient launch that have finished
   unsigned long long cells;       // cumulative row x feature cells built (accounting)
   unsigned long long rows_built;
   unsigned long long rows_partitioned;  // rows routed by partitions (accounting)

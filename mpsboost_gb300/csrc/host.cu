@@ -812,23 +812,23 @@ struct mpsb_cuda_trainer {
   uint64_t enqueue_round(bool record_events, bool root_gradient_only) {
     cudaStream_t s = b->stream;
     uint64_t k = 0;
-    CK(launch_round_begin(dev, s)); ++k;
-    CK(launch_gradients(dev, std::max(1, std::min(grid(4), int((dev.seg_stride + 255) / 256))), s)); ++k;
-    CK(launch_round_setup(dev, s)); ++k;
+    // The roots' slots are cleared beside the gradients.
+    CK(cudaEventRecord(fork_ev, s));
+    CK(cudaStreamWaitEvent(side, fork_ev, 0));
+    CK(launch_zero_root_slots(dev, root_gradient_only, grid(8), side)); ++k;
+    CK(cudaEventRecord(zero_ev, side));
+    CK(launch_gradients(dev, root_gradient_only,
+                        std::max(1, std::min(grid(4), int((dev.seg_stride + 255) / 256))), s)); ++k;
+    CK(cudaStreamWaitEvent(s, zero_ev, 0));
     if (leafwise) {
       k += enqueue_leafwise(root_gradient_only);
       CK(launch_apply_leaves(dev, grid(8), s)); k += 2;
-      CK(launch_round_end(dev, s)); ++k;
       return k;
     }
     const uint32_t levels = std::max<uint32_t>(depth, 1);
     for (uint32_t d = 0; d < levels; ++d) {
       const int parity = int(d & 1);
-      if (d == 0) {
-        CK(launch_zero_build_slots(dev, grid(8), s)); ++k;
-      } else {
-        CK(cudaStreamWaitEvent(s, zero_ev, 0));  // this level's slots were cleared beside the partition
-      }
+      if (d > 0) CK(cudaStreamWaitEvent(s, zero_ev, 0));  // its slots were cleared beside the partition
       if (record_events) CK(cudaEventRecord(events[2 * d], s));
       if (options & MPSB_OPT_PER_NODE) {
         k += enqueue_hist_per_node(d);
@@ -843,15 +843,12 @@ struct mpsb_cuda_trainer {
                            cudaMemcpyDeviceToDevice, s));
       }
       if (d == 0) {
-        if (root_reuse) {
-          CK(launch_root_cache(dev, root_gradient_only ? 0 : 1, grid(4), s)); ++k;
-        }
-        CK(launch_root_stats(dev, s)); ++k;
+        k += enqueue_root_stats(root_gradient_only);
       } else if (!dev.fused_sub) {
         CK(launch_subtract(dev, grid(8), s)); ++k;
       }
       if (depth > 0) {
-        CK(launch_split_scan(dev, parity, level_nodes(d), false, grid(4), s)); k += split_scan_kernels(dev);
+        CK(launch_split_scan(dev, parity, level_nodes(d), d == 0 ? ScanKind::kRoot : ScanKind::kLevel, grid(4), s)); k += split_scan_kernels(dev);
       }
       CK(launch_finalize(dev, parity, d, level_nodes(d), s)); ++k;
       if (d + 1 < depth) {
@@ -865,7 +862,19 @@ struct mpsb_cuda_trainer {
       }
     }
     CK(launch_apply_leaves(dev, grid(8), s)); k += 2;
-    CK(launch_round_end(dev, s)); ++k;
+    return k;
+  }
+
+  // After the roots' histograms: their cache in a fit's first round, and their statistics
+  // where the split scan does not form them.
+  uint64_t enqueue_root_stats(bool root_gradient_only) {
+    uint64_t k = 0;
+    if (root_reuse && !root_gradient_only) {
+      CK(launch_root_cache(dev, grid(4), b->stream)); ++k;
+    }
+    if (depth == 0 || !scan_forms_root(dev)) {
+      CK(launch_root_stats(dev, b->stream)); ++k;
+    }
     return k;
   }
 
@@ -875,16 +884,12 @@ struct mpsb_cuda_trainer {
   uint64_t enqueue_leafwise(bool root_gradient_only) {
     cudaStream_t s = b->stream;
     uint64_t k = 0;
-    CK(launch_zero_build_slots(dev, grid(8), s)); ++k;
     TrainerDev view = level_view(0);
     if (root_gradient_only) view.mode = kModeFixedG;
     CK(launch_hist_build(view, hcfg, grid(1), s)); ++k;
-    if (root_reuse) {
-      CK(launch_root_cache(dev, root_gradient_only ? 0 : 1, grid(4), s)); ++k;
-    }
-    CK(launch_root_stats(dev, s)); ++k;
+    k += enqueue_root_stats(root_gradient_only);
     if (depth > 0) {
-      CK(launch_split_scan(dev, 0, n_trees, false, grid(4), s)); k += split_scan_kernels(dev);
+      CK(launch_split_scan(dev, 0, n_trees, ScanKind::kRoot, grid(4), s)); k += split_scan_kernels(dev);
     }
     CK(launch_leafwise_init(dev, s)); ++k;
     for (uint32_t step = 0; step < lw_steps && depth > 0; ++step) {
@@ -899,7 +904,7 @@ struct mpsb_cuda_trainer {
       CK(launch_hist_build(step_view(), hcfg, grid(1), s)); ++k;
       if (!dev.fused_sub) { CK(launch_subtract(dev, grid(8), s)); ++k; }
       const uint32_t scans = split_scan_kernels(dev);
-      CK(launch_split_scan(dev, 1, 2 * n_trees, true, grid(4), s)); k += scans;
+      CK(launch_split_scan(dev, 1, 2 * n_trees, ScanKind::kActive, grid(4), s)); k += scans;
       if (scans == 1) { CK(launch_leafwise_merge(dev, s)); ++k; }
     }
     CK(launch_leafwise_finish(dev, s)); ++k;
@@ -1289,6 +1294,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.gh_ordered = 1;
   a.rows = t->alloc<uint32_t>(size_t(T) * 2 * seg_rows);
   a.trees = t->alloc<TreeState>(T);
+  CK(cudaMemsetAsync(a.trees, 0, size_t(T) * sizeof(TreeState), s));
   a.max_level_nodes = uint32_t(T * level_nodes);
   a.n_slots = a.max_level_nodes;
   if (t->leafwise) {
@@ -1333,6 +1339,8 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.part_offsets = t->alloc<uint32_t>(a.max_part_chunks);
   a.part_flags = t->alloc<uint32_t>(size_t(a.max_part_chunks) * (kPartChunk / 32));
   a.max_leafsegs = uint32_t(T * (leaves + 1));
+  // Leaf chunks of 4,096 rows; a quarter of that where they would leave SMs idle.
+  a.apply_chunk = uint64_t(T) * seg_rows <= (1u << 20) ? 1024u : 4096u;
   a.leafseg = t->alloc<LeafSeg>(a.max_leafsegs);
   a.leaf_prefix = t->alloc<uint32_t>(a.max_leafsegs + 1);
   if (!a.skip_apply) {

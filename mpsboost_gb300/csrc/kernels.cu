@@ -3,11 +3,14 @@
 //   gradients      ComputeObjectiveGradients + ApplySampleWeights (trainer.cpp:178-216),
 //                  FP64 math rounded once to FP32 pairs, plus per-tree max|g| / max h for
 //                  the fixed-point scales.
-//   round_setup    fixed-point exponents, root node, level-0 build list.
-//   root_cache     the roots' count and hessian histograms kept from a fit's first round
+//                  The last CTA sets the round up: fixed-point exponents, root nodes,
+//                  level-0 build list.
+//   zero_slots     clears a level's histogram slots; root slots start from the count and
+//                  hessian histograms that root_cache kept from a fit's first round
 //                  (objectives whose hessian does not depend on the prediction).
 //   root_stats     root statistics from the root histogram; root leaf value
-//                  (TreeTrainingAccess::Create, tree_structure.cpp:104-116).
+//                  (TreeTrainingAccess::Create, tree_structure.cpp:104-116), where the
+//                  root's split scan does not form them.
 //   subtract       SubtractHistograms (tree_histogram.cpp:16-66): exact int64 in fixed
 //                  mode, FP64 with the Hessian clamp in float mode.
 //   split_screen, split_exact, split_scan
@@ -20,8 +23,9 @@
 //                  (tree_structure.cpp:118-148), smaller-child selection, next level.
 //   partition      PrepareSplitRows' stable partition (tree_split.cpp:273-289) as a
 //                  ballot/popc compaction: count, per-node scan, scatter.
-//   apply_leaves   predictions += lr * leaf (trainer.cpp:256-262) from the final row
-//                  segments: no tree traversal.
+//   apply_leaves, apply_steps
+//                  predictions += lr * leaf (trainer.cpp:256-262) from the final row
+//                  segments: no tree traversal; the round's trees into the model.
 #include <algorithm>
 #include <cfloat>
 #include <type_traits>
@@ -57,9 +61,13 @@ __device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, uint32_t n
 
 // Exponent e with x < 2^e (frexp convention) of a positive finite float.
 __device__ __forceinline__ int exponent_above(float x) {
-  int e;
-  frexpf(x, &e);
-  return e;
+  const uint32_t bits = __float_as_uint(x), field = bits >> 23;
+  return field ? int(field) - 126 : 32 - __clz(int(bits)) - 149;
+}
+
+// 2^k for -1022 <= k <= 1023.
+__device__ __forceinline__ double exp2_int(int k) {
+  return __longlong_as_double((long long)(1023 + k) << 52);
 }
 
 // Block-wide exclusive scan of N values per thread. `sh` holds >= 33*N words.
@@ -104,24 +112,8 @@ __device__ void block_scan(uint32_t (&v)[N], uint32_t (&total)[N], uint32_t* sh)
 }
 
 // ------------------------------------------------------------------------------------
-// Round begin / gradients / setup
+// Gradients and round setup
 // ------------------------------------------------------------------------------------
-__global__ void round_begin_kernel(TrainerDev a) {
-  for (uint32_t i = threadIdx.x; i < a.n_slots; i += blockDim.x) a.free_stack[i] = a.n_slots - 1 - i;
-  for (uint32_t t = threadIdx.x; t < a.n_trees; t += blockDim.x) {
-    a.trees[t].max_abs_g_bits = 0;
-    a.trees[t].max_h_bits = 0;
-    a.trees[t].n_tree_nodes = 1;
-    a.trees[t].leaf_count = 1;
-  }
-  if (threadIdx.x == 0) {
-    a.ctl->free_top = a.n_slots;
-    a.ctl->n_leafseg = 0;
-    a.ctl->leaf_chunks = 0;
-    a.leaf_prefix[0] = 0;
-  }
-}
-
 __device__ __forceinline__ double logistic_probability(double m) {  // objective.cpp:309-317
   if (m >= 0.0) {
     const double e = exp(-m);
@@ -223,12 +215,100 @@ __device__ __forceinline__ bool f64_negative(double x) {
   return b < 0 && (b & 0x7FFFFFFFFFFFFFFFll) != 0;
 }
 
+__device__ __forceinline__ uint32_t root_rows(const TrainerDev& a, uint32_t t) {
+  return a.sample_rows ? a.sample_count[t] : a.n_rows;
+}
+
+// The round's start, by one CTA once every gradient is known: fixed-point exponents, slots,
+// root nodes and the level-0 build list. Tree t's root takes slot t. g_only: the roots'
+// count and hessian histograms come from the fit's first round.
+__device__ __noinline__ void round_setup(const TrainerDev& a, bool g_only) {
+  for (uint32_t i = threadIdx.x; i < a.n_slots; i += blockDim.x) a.free_stack[i] = a.n_slots - 1 - i;
+  if (threadIdx.x == 0) {  // trees are few: serial prefix of the roots' work items
+    uint64_t total = 0;
+    for (uint32_t t = 0; t < a.n_trees; ++t) total += root_rows(a, t);
+    const uint32_t item_rows =
+        a.item_rows ? a.item_rows : adaptive_item_rows(total, a.nfb, a.sm_count, a.items_per_sm);
+    uint32_t acc = 0;
+    for (uint32_t t = 0; t < a.n_trees; ++t) {
+      a.build_prefix[t] = acc;
+      acc += ceil_div(root_rows(a, t), item_rows);
+    }
+    a.build_prefix[a.n_trees] = acc;
+    a.ctl->free_top = a.n_slots - a.n_trees;
+    a.ctl->n_leafseg = 0;
+    a.ctl->leaf_chunks = 0;
+    a.leaf_prefix[0] = 0;
+    a.ctl->round = *a.round_counter;
+    a.ctl->n_nodes = a.n_trees;
+    a.ctl->n_build = a.n_trees;
+    a.ctl->n_sub = 0;
+    a.ctl->n_part = 0;
+    a.ctl->hist_items = acc * a.nfb;
+    a.ctl->hist_counter = 0;
+    a.ctl->split_items = a.n_trees * a.n_fchunks;
+    a.ctl->item_rows = item_rows;
+  }
+  if (threadIdx.x >= 32) {  // beside warp 0's work items
+    for (uint32_t t = threadIdx.x - 32; t < a.n_trees; t += blockDim.x - 32) {
+      TreeState& s = a.trees[t];
+      const float mg = __uint_as_float(__ldcg(&s.max_abs_g_bits)), mh = __uint_as_float(__ldcg(&s.max_h_bits));
+      s.max_abs_g_bits = s.max_h_bits = 0;  // the next round's maxima start here
+      s.n_tree_nodes = 1;
+      s.leaf_count = 1;
+      // every row's |q| <= 2^30: the histogram's 32-bit limb sums cannot overflow
+      s.kg = mg > 0.0f ? 30 - exponent_above(mg) : 0;
+      s.kh = mh > 0.0f ? 30 - exponent_above(mh) : 0;
+      s.inv_g = exp2_int(-s.kg);  // |k| <= 179: a float's exponent and the 30 bits
+      s.inv_h = exp2_int(-s.kh);
+      if (g_only && a.root_cache_kh[t] != s.kh) raise(a.ctl, kErrRootCache);
+      const uint32_t slot = t;
+      const uint32_t cnt = root_rows(a, t);
+      NodeRec r;
+      r.seg_off = 0;
+      r.seg_cnt = cnt;
+      r.node_index = 0;
+      r.slot = slot;
+      r.count = 0;
+      r.qg = r.qh = 0;
+      r.g = r.h = 0.0;
+      r.lo = -INFINITY;
+      r.hi = INFINITY;
+      r.tree = t;
+      r.depth = 0;
+      r.sub_from = 0;
+      a.nodes[0][t] = r;
+      for (uint32_t w = 0; w < a.params.path_words; ++w) {
+        uint32_t allowed = 0xffffffffu;
+        if (a.params.n_groups > 0) {  // empty path: any group containing the feature
+          allowed = 0;
+          for (uint32_t g = 0; g < a.params.n_groups; ++g)
+            allowed |= a.group_masks[g * a.params.path_words + w];
+        }
+        if (a.tree_feature_masks != nullptr)
+          allowed &= a.tree_feature_masks[t * a.params.path_words + w];
+        a.node_path[0][t * a.params.path_words + w] = 0;
+        a.node_allowed[0][t * a.params.path_words + w] = allowed;
+      }
+      BuildEntry e;
+      e.tree = t;
+      e.parity = 0;
+      e.seg_off = 0;
+      e.seg_cnt = cnt;
+      e.slot = slot;
+      e.pad = 0;
+      a.build[t] = e;
+    }
+  }
+}
+
 // grid = (x, n_trees): blockIdx.y is the tree, so a block's maxima belong to one tree.
 // SQ: squared error without softmax classes only; the instantiation leaves out the other
 // objectives' code, so it needs fewer registers and more rows are in flight per SM.
+// The last CTA to finish sets the round up.
 template <bool SQ>
-__global__ void __launch_bounds__(256) gradients_kernel(TrainerDev a) {
-  __shared__ uint32_t sg[8], shh[8];
+__global__ void __launch_bounds__(256, SQ ? 8 : 4) gradients_kernel(const __grid_constant__ TrainerDev a, bool g_only) {
+  __shared__ uint32_t sg[8], shh[8], s_last;
   const uint32_t t = blockIdx.y;
   const size_t tree_off = size_t(t) * a.n_rows;
   // Squared error and quantile have h = 1, so h * w = w exactly.
@@ -302,140 +382,98 @@ __global__ void __launch_bounds__(256) gradients_kernel(TrainerDev a) {
     }
     atomicMax(&a.trees[t].max_abs_g_bits, mg);
     atomicMax(&a.trees[t].max_h_bits, mh);
+    __threadfence();
+    s_last = atomicAdd(&a.ctl->grad_ticket, 1u) == gridDim.x * gridDim.y - 1 ? 1u : 0u;
   }
   if (bad) raise(a.ctl, kErrGradient);
-}
-
-__device__ __forceinline__ uint32_t root_rows(const TrainerDev& a, uint32_t t) {
-  return a.sample_rows ? a.sample_count[t] : a.n_rows;
-}
-
-__global__ void round_setup_kernel(TrainerDev a) {
-  if (threadIdx.x == 0) {  // trees are few: serial prefix of the roots' work items
-    uint64_t total = 0;
-    for (uint32_t t = 0; t < a.n_trees; ++t) total += root_rows(a, t);
-    const uint32_t item_rows =
-        a.item_rows ? a.item_rows : adaptive_item_rows(total, a.nfb, a.sm_count, a.items_per_sm);
-    uint32_t acc = 0;
-    for (uint32_t t = 0; t < a.n_trees; ++t) {
-      a.build_prefix[t] = acc;
-      acc += ceil_div(root_rows(a, t), item_rows);
-    }
-    a.build_prefix[a.n_trees] = acc;
-    a.ctl->free_top = a.n_slots - a.n_trees;
-    a.ctl->n_nodes = a.n_trees;
-    a.ctl->n_build = a.n_trees;
-    a.ctl->n_sub = 0;
-    a.ctl->n_part = 0;
-    a.ctl->hist_items = acc * a.nfb;
-    a.ctl->hist_counter = 0;
-    a.ctl->split_items = a.n_trees * a.n_fchunks;
-    a.ctl->item_rows = item_rows;
-  }
-  for (uint32_t base = 0; base < a.n_trees; base += blockDim.x) {
-    const uint32_t t = base + threadIdx.x;
-    if (t < a.n_trees) {
-      TreeState& s = a.trees[t];
-      const float mg = __uint_as_float(s.max_abs_g_bits), mh = __uint_as_float(s.max_h_bits);
-      // every row's |q| <= 2^30: the histogram's 32-bit limb sums cannot overflow
-      s.kg = mg > 0.0f ? 30 - exponent_above(mg) : 0;
-      s.kh = mh > 0.0f ? 30 - exponent_above(mh) : 0;
-      s.inv_g = ldexp(1.0, -s.kg);
-      s.inv_h = ldexp(1.0, -s.kh);
-      const uint32_t slot = a.free_stack[a.n_slots - 1 - t];
-      const uint32_t cnt = root_rows(a, t);
-      NodeRec r;
-      r.seg_off = 0;
-      r.seg_cnt = cnt;
-      r.node_index = 0;
-      r.slot = slot;
-      r.count = 0;
-      r.qg = r.qh = 0;
-      r.g = r.h = 0.0;
-      r.lo = -INFINITY;
-      r.hi = INFINITY;
-      r.tree = t;
-      r.depth = 0;
-      r.sub_from = 0;
-      a.nodes[0][t] = r;
-      for (uint32_t w = 0; w < a.params.path_words; ++w) {
-        uint32_t allowed = 0xffffffffu;
-        if (a.params.n_groups > 0) {  // empty path: any group containing the feature
-          allowed = 0;
-          for (uint32_t g = 0; g < a.params.n_groups; ++g)
-            allowed |= a.group_masks[g * a.params.path_words + w];
-        }
-        if (a.tree_feature_masks != nullptr)
-          allowed &= a.tree_feature_masks[t * a.params.path_words + w];
-        a.node_path[0][t * a.params.path_words + w] = 0;
-        a.node_allowed[0][t * a.params.path_words + w] = allowed;
-      }
-      BuildEntry e;
-      e.tree = t;
-      e.parity = 0;
-      e.seg_off = 0;
-      e.seg_cnt = cnt;
-      e.slot = slot;
-      e.pad = 0;
-      a.build[t] = e;
-    }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    if (threadIdx.x == 0) a.ctl->grad_ticket = 0;
+    round_setup(a, g_only);
   }
 }
 
-// Zero the histogram slots of the current build list.
-__global__ void zero_build_slots_kernel(TrainerDev a) {
+// Clears the histogram slots of the current build list (kZeroBuilt) or of the trees' roots
+// (kZeroRoots: tree t's slot t, before the round's lists exist, beside the gradients).
+// kRestoreRoots: the root of every tree holds all rows in every round, so its count
+// histogram never changes, and when the hessian does not depend on the prediction (squared
+// error and quantile: h = weight) neither does its hessian histogram, nor the hessian scale.
+// The first round of a fit builds the roots in full and saves those two words per cell;
+// later rounds start the roots from them and build only the gradient limbs. The hessian
+// scale is checked by the round's setup.
+enum : int { kZeroBuilt = 0, kZeroRoots = 1, kRestoreRoots = 2 };
+
+__global__ void zero_slots_kernel(TrainerDev a, int what) {
   // The level's split scan publishes node maxima into node_screen: clear them first.
   if (a.node_screen)
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.max_level_nodes; i += gridDim.x * blockDim.x)
       a.node_screen[i] = 0u;
   const uint64_t words_per_slot = uint64_t(a.features) * a.slots * 3;
-  const uint64_t total = uint64_t(a.ctl->n_build) * (words_per_slot / 2);
+  if (what == kRestoreRoots) {
+    // Pairs of cells: their two {count, hessian} words each, into 48 bytes.
+    const uint64_t total = uint64_t(a.n_trees) * (words_per_slot / 6);
+    for (uint64_t idx = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; idx < total;
+         idx += uint64_t(gridDim.x) * blockDim.x) {
+      const ulonglong2* cache = reinterpret_cast<const ulonglong2*>(a.root_cache + idx * 4);
+      const ulonglong2 c0 = cache[0], c1 = cache[1];
+      ulonglong2* out = reinterpret_cast<ulonglong2*>(a.hist + idx * 6);  // tree t's root slot is t
+      out[0] = make_ulonglong2(c0.x, 0);
+      out[1] = make_ulonglong2(c0.y, c1.x);
+      out[2] = make_ulonglong2(0, c1.y);
+    }
+    return;
+  }
+  const uint64_t total = uint64_t(what == kZeroBuilt ? a.ctl->n_build : a.n_trees) * (words_per_slot / 2);
   for (uint64_t idx = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; idx < total;
        idx += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t e = uint32_t(idx / (words_per_slot / 2));
-    const uint64_t w = idx % (words_per_slot / 2);
+    const uint64_t w = idx - e * (words_per_slot / 2);
     if (a.tree_feature_masks) {
       // A forest tree reads only its own features' histograms (and feature 0's, for the
       // root statistics): the others are neither cleared nor subtracted nor scanned.
       const uint32_t f = uint32_t(w * 2 / (a.slots * 3));
-      const uint32_t mask = a.tree_feature_masks[size_t(a.build[e].tree) * a.params.path_words + (f >> 5)];
+      const uint32_t tree = what == kZeroBuilt ? a.build[e].tree : e;
+      const uint32_t mask = a.tree_feature_masks[size_t(tree) * a.params.path_words + (f >> 5)];
       if (f != 0 && !((mask >> (f & 31)) & 1u)) continue;
     }
-    reinterpret_cast<ulonglong2*>(a.hist + a.build[e].slot * words_per_slot)[w] =
-        make_ulonglong2(0, 0);
+    const uint32_t slot = what == kZeroBuilt ? a.build[e].slot : e;
+    reinterpret_cast<ulonglong2*>(a.hist + slot * words_per_slot)[w] = make_ulonglong2(0, 0);
   }
 }
 
-// The root of every tree holds all rows in every round, so its count histogram never
-// changes, and when the hessian does not depend on the prediction (squared error and
-// quantile: h = weight) neither does its hessian histogram, nor the hessian scale. The
-// first round of a fit builds the roots in full and saves those two words per cell; later
-// rounds build only the gradient limbs and restore them. The hessian scale is checked.
-__global__ void root_cache_kernel(TrainerDev a, int save) {
+// Saves the roots' count and hessian words of a fit's first round (kRestoreRoots).
+__global__ void root_cache_kernel(TrainerDev a) {
   const uint64_t per_tree = uint64_t(a.features) * a.slots;
   const uint64_t total = per_tree * a.n_trees;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < total;
        i += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t t = uint32_t(i / per_tree);
-    const uint64_t cell = i % per_tree;
-    unsigned long long* slot = a.hist + (uint64_t(a.build[t].slot) * per_tree + cell) * 3;
-    unsigned long long* c = a.root_cache + i * 2;
-    if (save) {
-      c[0] = slot[0];
-      c[1] = slot[2];
-      if (cell == 0) a.root_cache_kh[t] = a.trees[t].kh;
-    } else {
-      if (a.root_cache_kh[t] != a.trees[t].kh) {
-        if (cell == 0) raise(a.ctl, kErrRootCache);
-        continue;
-      }
-      slot[0] = c[0];
-      slot[2] = c[1];
-    }
+    const unsigned long long* slot = a.hist + i * 3;  // tree t's root slot is t
+    a.root_cache[i * 2] = slot[0];
+    a.root_cache[i * 2 + 1] = slot[2];
+    if (i % per_tree == 0) a.root_cache_kh[i / per_tree] = a.trees[i / per_tree].kh;
   }
 }
 
-// Root statistics: the total of feature 0's slots (all rows, exact in fixed mode).
+// The root's leaf: tree t's node 0 (TreeTrainingAccess::Create, tree_structure.cpp:104-116).
+__device__ __forceinline__ void write_root_leaf(const TrainerDev& a, uint32_t t, double g, double h) {
+  double leaf = 0.0;
+  if (!leaf_weight(g, h, a.params, &leaf)) raise(a.ctl, kErrNonFinite);
+  TreeNodeOut n;
+  n.feature_index = 0;
+  n.threshold_bin = 0;
+  n.left_child = 0xffffffffu;
+  n.right_child = 0xffffffffu;
+  n.leaf_value = leaf;
+  n.gain = 0.0;
+  n.default_left = 1;
+  n.flags = 1;
+  for (int k = 0; k < 6; ++k) n.reserved[k] = 0;
+  a.tree_nodes[size_t(t) * a.max_tree_nodes] = n;
+}
+
+// Root statistics: the total of feature 0's slots (all rows, exact in fixed mode), where
+// the root's split scan does not form them itself.
 __global__ void root_stats_kernel(TrainerDev a) {
   const int lane = threadIdx.x & 31;
   for (uint32_t t = threadIdx.x >> 5; t < a.n_trees; t += blockDim.x >> 5) {
@@ -471,19 +509,7 @@ __global__ void root_stats_kernel(TrainerDev a) {
         r.h = h;
       }
       if (cnt != r.seg_cnt) raise(a.ctl, kErrCountMismatch);
-      double leaf = 0.0;
-      if (!leaf_weight(r.g, r.h, a.params, &leaf)) raise(a.ctl, kErrNonFinite);
-      TreeNodeOut n;
-      n.feature_index = 0;
-      n.threshold_bin = 0;
-      n.left_child = 0xffffffffu;
-      n.right_child = 0xffffffffu;
-      n.leaf_value = leaf;
-      n.gain = 0.0;
-      n.default_left = 1;
-      n.flags = 1;
-      for (int k = 0; k < 6; ++k) n.reserved[k] = 0;
-      a.tree_nodes[size_t(t) * a.max_tree_nodes] = n;
+      write_root_leaf(a, t, r.g, r.h);
     }
   }
 }
@@ -1463,8 +1489,10 @@ __device__ __forceinline__ SlotWords load_slots(const TrainerDev& a, const ScanN
 // default_left) for each candidate of the thread's slots. `first` holds page 0's words of
 // the thread's pair. SUB (the level's first launch): a sibling's histogram is formed as
 // parent minus built child on the way, with subtract_kernel's checks, and written back.
-template <bool FIXED, bool WIDE, bool SUB, class Visit>
-__device__ __forceinline__ void scan_feature(const TrainerDev& a, const ScanNode<FIXED>& node,
+// ROOT: the node's statistics are the feature's own totals (every feature of a root holds
+// all of its rows, so in fixed point they are the same), which it leaves in node.parent.
+template <bool FIXED, bool WIDE, bool SUB, bool ROOT, class Visit>
+__device__ __forceinline__ void scan_feature(const TrainerDev& a, ScanNode<FIXED>& node,
                                              uint32_t f, uint32_t nb, bool hm, const SlotWords& first,
                                              PageTotals<FIXED>* totals, uint32_t& buf, uint32_t& err,
                                              Visit&& visit) {
@@ -1512,6 +1540,14 @@ __device__ __forceinline__ void scan_feature(const TrainerDev& a, const ScanNode
       miss.g = t.miss_g;
       miss.h = t.miss_h;
     }
+    if constexpr (ROOT) {  // one page
+      const uint32_t rows = node.parent.count;
+      node.parent = stat_add<FIXED>(carry, miss);
+      if (node.parent.count != rows) {
+        err |= kErrCountMismatch;
+        return;  // the same in every thread
+      }
+    }
     if (p + 1 == pages && carry.count + miss.count != node.parent.count) {
       err |= kErrCountMismatch;
       if (!WIDE) return;  // the same in every thread
@@ -1536,8 +1572,9 @@ __device__ __forceinline__ void scan_feature(const TrainerDev& a, const ScanNode
   }
 }
 
-template <bool FIXED, bool WIDE>
+template <bool FIXED, bool WIDE, bool ROOT>
 __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(TrainerDev a, int parity) {
+  static_assert(!ROOT || (FIXED && !WIDE), "the features' totals are the same in fixed point only");
   __shared__ PageTotals<FIXED> s_totals[2];
   __shared__ uint32_t s_word[2][kScanFeaturesPerItem][kScanCtaWarps];
   const TreeParams& P = a.params;
@@ -1555,12 +1592,14 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
   for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, ib ^= 1u) {
     const uint32_t i = item / chunks, f0 = (item - i * chunks) * per;
     const uint32_t nf = min(per, F - f0);
-    const NodeRec& rec = a.nodes[parity][i];
+    NodeRec& rec = a.nodes[parity][i];
     const TreeState& tree = a.trees[rec.tree];
-    const ScanNode<FIXED> node = scan_node<FIXED>(rec, tree.inv_h);
+    ScanNode<FIXED> node = scan_node<FIXED>(rec, tree.inv_h);
+    if constexpr (ROOT) node.parent.count = rec.seg_cnt;
     const int kh = tree.kh;
-    // A node with fewer than 2 * min_samples_leaf rows has no admissible split.
-    const bool usable = rec.count >= 2 * P.min_samples_leaf;
+    // A node with fewer than 2 * min_samples_leaf rows has no admissible split (a root's
+    // statistics are formed all the same).
+    const bool usable = ROOT || rec.count >= 2 * P.min_samples_leaf;
     const uint32_t* allowed = a.node_allowed[parity] + size_t(i) * P.path_words;
     auto active = [&](uint32_t k) -> bool {
       return k < nf && usable && ((allowed[(f0 + k) >> 5] >> ((f0 + k) & 31)) & 1u);
@@ -1583,7 +1622,7 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
       uint32_t word = 0, exact = 0;
       if (act) {  // the same in every thread
         const ScreenScale scale = screen_scale<FIXED>(P, P.has_monotonic ? a.monotonic[f] : int8_t(0), kh);
-        scan_feature<FIXED, WIDE, true>(
+        scan_feature<FIXED, WIDE, true, ROOT>(
             a, node, f, nb, hm, w, s_totals, buf, err,
             [&](const Stat<FIXED>& cl, const Stat<FIXED>& cr, uint32_t, uint32_t) {
               if (!scale.on) {
@@ -1595,6 +1634,22 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
               if (cls == 1) word = max(word, max(__float_as_uint(score), 1u));
               if (cls == 2) exact = kFeatureExact;
             });
+        if constexpr (ROOT) {
+          if (threadIdx.x == 0) {
+            // The tree's first allowed feature writes the root's record and leaf.
+            bool lead = (allowed[f >> 5] & ((1u << (f & 31)) - 1u)) == 0;
+            for (uint32_t q = 0; q < (f >> 5); ++q) lead = lead && allowed[q] == 0;
+            if (lead) {
+              rec.count = node.parent.count;
+              rec.qg = node.parent.g;
+              rec.qh = node.parent.h;
+              rec.g = q_image(node.parent.g, tree.inv_g);
+              rec.h = q_image(node.parent.h, tree.inv_h);
+              write_root_leaf(a, rec.tree, rec.g, rec.h);
+            }
+          }
+          node.parent.count = rec.seg_cnt;
+        }
       }
       word = __reduce_max_sync(0xffffffffu, word);
       if (__any_sync(0xffffffffu, exact != 0)) word |= kFeatureExact;
@@ -1641,7 +1696,7 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
     const NodeRec& rec = a.nodes[parity][i];
     const TreeState& tree = a.trees[rec.tree];
     const double inv_g = tree.inv_g, inv_h = tree.inv_h;
-    const ScanNode<FIXED> node = scan_node<FIXED>(rec, inv_h);
+    ScanNode<FIXED> node = scan_node<FIXED>(rec, inv_h);
     const double lo = rec.lo, hi = rec.hi;
     const float m = __uint_as_float(a.node_screen[i]);
     const float cut = m >= 1e-30f ? m * (1.0f - 0x1p-18f) : -1.0f;
@@ -1665,7 +1720,7 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
         const int8_t mono = P.has_monotonic ? a.monotonic[f] : int8_t(0);
         const ScreenScale scale = screen_scale<FIXED>(P, mono, tree.kh);
         const SlotWords w = load_slots<FIXED, false>(a, node, f, nb, hm, S, 2 * threadIdx.x);
-        scan_feature<FIXED, WIDE, false>(
+        scan_feature<FIXED, WIDE, false, false>(
             a, node, f, nb, hm, w, s_totals, buf, err,
             [&](const Stat<FIXED>& l, const Stat<FIXED>& r, uint32_t t, uint32_t dl) {
               if (scale.on && cut > 0.0f) {
@@ -1943,7 +1998,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       }
       const bool leafseg = !acc || last;
       v[3] = leafseg;
-      v[4] = leafseg ? ceil_div(node.seg_cnt, kApplyChunk) : 0;
+      v[4] = leafseg ? ceil_div(node.seg_cnt, a.apply_chunk) : 0;
       v[5] = (!acc && !last) ? 1u : 0u;
     }
     const uint32_t own0 = v[0];
@@ -2213,7 +2268,7 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
                    acc && !last ? ceil_div(built, item_rows) : 0u,
                    acc && !last ? ceil_div(node.seg_cnt, kPartChunk) : 0u,
                    leafseg ? 1u : 0u,
-                   leafseg ? ceil_div(node.seg_cnt, kApplyChunk) : 0u,
+                   leafseg ? ceil_div(node.seg_cnt, a.apply_chunk) : 0u,
                    i < n && !acc && !last ? 1u : 0u};
   uint32_t tot[6];
   block_scan<6>(v, tot, sh);
@@ -3018,7 +3073,7 @@ __global__ void leafwise_finish_kernel(TrainerDev a) {
         ls.seg_cnt = act[j].node.seg_cnt;
         ls.value = tn[act[j].node.node_index].leaf_value;
       }
-      const uint32_t own = j < count ? ceil_div(ls.seg_cnt, kApplyChunk) : 0u;
+      const uint32_t own = j < count ? ceil_div(ls.seg_cnt, a.apply_chunk) : 0u;
       uint32_t x = own;
       for (int off = 1; off < 32; off <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
@@ -3060,7 +3115,25 @@ __global__ void leafwise_finish_kernel(TrainerDev a) {
 // streams instead of one 32-byte sector each way per row.
 constexpr uint32_t kNoLeaf = 0xffffffffu;
 
+// The launch also ends the round: each tree's nodes go to the model, and the round counter
+// moves on (the launches after it read the round from ctl).
 __global__ void __launch_bounds__(256, 4) apply_leaves_kernel(TrainerDev a) {
+  const uint32_t round = a.ctl->round;
+  if (round < a.max_rounds) {
+    static_assert(sizeof(TreeNodeOut) % 8 == 0, "nodes are copied as 8-byte words");
+    for (uint32_t t = blockIdx.x; t < a.n_trees; t += gridDim.x) {
+      const uint32_t cnt = a.trees[t].n_tree_nodes;
+      const unsigned long long* src =
+          reinterpret_cast<const unsigned long long*>(a.tree_nodes + size_t(t) * a.max_tree_nodes);
+      unsigned long long* dst = reinterpret_cast<unsigned long long*>(
+          a.model_nodes + (size_t(round) * a.n_trees + t) * a.max_tree_nodes);
+      for (uint32_t i = threadIdx.x; i < cnt * uint32_t(sizeof(TreeNodeOut) / 8); i += blockDim.x) dst[i] = src[i];
+      if (threadIdx.x == 0) a.model_counts[size_t(round) * a.n_trees + t] = cnt;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.round_counter = round + 1;
+  } else if (blockIdx.x == 0 && threadIdx.x == 0) {
+    raise(a.ctl, kErrCapacity);
+  }
   if (a.skip_apply) return;  // forest trees: no training predictions
   const double lr = a.params.learning_rate;
   uint32_t err = 0;
@@ -3069,8 +3142,8 @@ __global__ void __launch_bounds__(256, 4) apply_leaves_kernel(TrainerDev a) {
   for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
     const uint32_t s = find_entry(a.leaf_prefix, n_seg, c);
     const LeafSeg ls = a.leafseg[s];
-    const uint32_t start = (c - a.leaf_prefix[s]) * kApplyChunk;
-    const uint32_t count = min(kApplyChunk, ls.seg_cnt - start);
+    const uint32_t start = (c - a.leaf_prefix[s]) * a.apply_chunk;
+    const uint32_t count = min(a.apply_chunk, ls.seg_cnt - start);
     const uint32_t* rows = a.rows + (size_t(ls.tree) * 2 + ls.parity) * a.seg_stride + ls.seg_off + start;
     uint32_t* leaf_of = a.leaf_of + size_t(ls.tree) * a.n_rows;
     if (start == 0 && threadIdx.x == 0) {
@@ -3115,7 +3188,7 @@ __global__ void __launch_bounds__(256) apply_steps_kernel(TrainerDev a) {
   uint32_t err = 0;
   const uint32_t steps = 2 * a.ctl->n_leafseg;
   // Softmax trees update the margins of the current round's class.
-  const uint32_t klass = a.n_classes ? *a.round_counter % a.n_classes : 0u;
+  const uint32_t klass = a.n_classes ? a.ctl->round % a.n_classes : 0u;
   const size_t total = size_t(a.n_trees) * a.n_rows;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += size_t(gridDim.x) * blockDim.x) {
@@ -3133,23 +3206,6 @@ __global__ void __launch_bounds__(256) apply_steps_kernel(TrainerDev a) {
     pred[r] = out;
   }
   if (err) raise(a.ctl, err);
-}
-
-__global__ void round_end_kernel(TrainerDev a) {
-  const uint32_t round = *a.round_counter;
-  if (round >= a.max_rounds) {
-    if (threadIdx.x == 0) raise(a.ctl, kErrCapacity);
-    return;
-  }
-  for (uint32_t t = 0; t < a.n_trees; ++t) {
-    const uint32_t cnt = a.trees[t].n_tree_nodes;
-    const TreeNodeOut* src = a.tree_nodes + size_t(t) * a.max_tree_nodes;
-    TreeNodeOut* dst = a.model_nodes + (size_t(round) * a.n_trees + t) * a.max_tree_nodes;
-    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) dst[i] = src[i];
-    if (threadIdx.x == 0) a.model_counts[size_t(round) * a.n_trees + t] = cnt;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) *a.round_counter = round + 1;
 }
 
 // Rows of each class id 0..classes-1 (counts[classes]: rows whose label is none of them).
@@ -3396,36 +3452,38 @@ __global__ void pack_bins16_kernel(const void* src, uint32_t width, const uint8_
 
 }  // namespace
 
-cudaError_t launch_round_begin(const TrainerDev& a, cudaStream_t s) {
-  round_begin_kernel<<<1, 1024, 0, s>>>(a);
-  return cudaGetLastError();
-}
-cudaError_t launch_gradients(const TrainerDev& a, int grid, cudaStream_t s) {
+cudaError_t launch_gradients(const TrainerDev& a, bool g_only, int grid, cudaStream_t s) {
   if (a.objective == 0 && !a.n_classes)  // twice the CTAs: twice as many fit on an SM
-    gradients_kernel<true><<<dim3(2 * grid, a.n_trees), 256, 0, s>>>(a);
+    gradients_kernel<true><<<dim3(2 * grid, a.n_trees), 256, 0, s>>>(a, g_only);
   else
-    gradients_kernel<false><<<dim3(grid, a.n_trees), 256, 0, s>>>(a);
-  return cudaGetLastError();
-}
-cudaError_t launch_round_setup(const TrainerDev& a, cudaStream_t s) {
-  round_setup_kernel<<<1, 1024, 0, s>>>(a);
+    gradients_kernel<false><<<dim3(grid, a.n_trees), 256, 0, s>>>(a, g_only);
   return cudaGetLastError();
 }
 cudaError_t launch_zero_build_slots(const TrainerDev& a, int grid, cudaStream_t s) {
-  zero_build_slots_kernel<<<grid, 256, 0, s>>>(a);
+  zero_slots_kernel<<<grid, 256, 0, s>>>(a, int(kZeroBuilt));
+  return cudaGetLastError();
+}
+cudaError_t launch_zero_root_slots(const TrainerDev& a, bool g_only, int grid, cudaStream_t s) {
+  zero_slots_kernel<<<grid, 256, 0, s>>>(a, int(g_only ? kRestoreRoots : kZeroRoots));
   return cudaGetLastError();
 }
 cudaError_t launch_root_stats(const TrainerDev& a, cudaStream_t s) {
   root_stats_kernel<<<1, 1024, 0, s>>>(a);
   return cudaGetLastError();
 }
-cudaError_t launch_root_cache(const TrainerDev& a, int save, int grid, cudaStream_t s) {
-  root_cache_kernel<<<grid, 256, 0, s>>>(a, save);
+cudaError_t launch_root_cache(const TrainerDev& a, int grid, cudaStream_t s) {
+  root_cache_kernel<<<grid, 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 cudaError_t launch_subtract(const TrainerDev& a, int grid, cudaStream_t s) {
   subtract_kernel<<<grid, 256, 0, s>>>(a);
   return cudaGetLastError();
+}
+uint32_t split_scan_kernels(const TrainerDev& a) {
+  return a.node_screen && a.scan_two_phase ? 2u : 1u;
+}
+bool scan_forms_root(const TrainerDev& a) {
+  return split_scan_kernels(a) == 2 && a.mode == kModeFixed && a.slots == uint32_t(kSlots);
 }
 template <bool FIXED, bool WIDE>
 cudaError_t launch_scan_one(const TrainerDev& a, int parity, int grid, int threads, cudaStream_t s) {
@@ -3438,32 +3496,36 @@ cudaError_t launch_scan_one(const TrainerDev& a, int parity, int grid, int threa
   return cudaGetLastError();
 }
 template <bool FIXED, bool WIDE>
-cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes, bool to_active,
+cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind,
                             cudaStream_t s) {
   const uint64_t resident = uint64_t(a.sm_count ? a.sm_count : 152) * 6;
   const uint32_t screen = uint32_t(std::min<uint64_t>(resident, uint64_t(max_nodes) * a.features));
-  split_screen_kernel<FIXED, WIDE><<<screen, kScanCta, 0, s>>>(a, parity);
+  if constexpr (FIXED && !WIDE) {
+    if (kind == ScanKind::kRoot && scan_forms_root(a))
+      split_screen_kernel<true, false, true><<<screen, kScanCta, 0, s>>>(a, parity);
+    else
+      split_screen_kernel<true, false, false><<<screen, kScanCta, 0, s>>>(a, parity);
+  } else {
+    split_screen_kernel<FIXED, WIDE, false><<<screen, kScanCta, 0, s>>>(a, parity);
+  }
   const cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   const uint32_t exact = uint32_t(std::min<uint64_t>(resident, max_nodes));
-  split_exact_kernel<FIXED, WIDE><<<exact, kScanCta, 0, s>>>(a, parity, to_active);
+  split_exact_kernel<FIXED, WIDE><<<exact, kScanCta, 0, s>>>(a, parity, kind == ScanKind::kActive);
   return cudaGetLastError();
 }
 
-uint32_t split_scan_kernels(const TrainerDev& a) {
-  return a.node_screen && a.scan_two_phase ? 2u : 1u;
-}
 
-cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, bool to_active,
+cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind,
                               int grid, cudaStream_t s) {
   const bool fixed = a.mode == kModeFixed, wide = a.slots != uint32_t(kSlots);
   if (a.slots < uint32_t(kSlots) || a.slots % uint32_t(kSlots) || max_nodes == 0) return cudaErrorInvalidValue;
   if (split_scan_kernels(a) == 2) {
-    // node_screen was cleared by the level's zero_build_slots_kernel.
-    if (fixed) return wide ? launch_scan_two<true, true>(a, parity, max_nodes, to_active, s)
-                           : launch_scan_two<true, false>(a, parity, max_nodes, to_active, s);
-    return wide ? launch_scan_two<false, true>(a, parity, max_nodes, to_active, s)
-                : launch_scan_two<false, false>(a, parity, max_nodes, to_active, s);
+    // node_screen was cleared by the level's zero_slots_kernel.
+    if (fixed) return wide ? launch_scan_two<true, true>(a, parity, max_nodes, kind, s)
+                           : launch_scan_two<true, false>(a, parity, max_nodes, kind, s);
+    return wide ? launch_scan_two<false, true>(a, parity, max_nodes, kind, s)
+                : launch_scan_two<false, false>(a, parity, max_nodes, kind, s);
   }
   const int threads = int(a.scan_threads);
   if (threads < 32 || threads > kScanThreadsMax || threads % 32) return cudaErrorInvalidValue;
@@ -3559,10 +3621,6 @@ cudaError_t launch_fill_f64(double* dst, uint64_t n, double value, cudaStream_t 
 cudaError_t launch_apply_leaves(const TrainerDev& a, int grid, cudaStream_t s) {
   apply_leaves_kernel<<<grid, 256, 0, s>>>(a);
   apply_steps_kernel<<<grid, 256, 0, s>>>(a);
-  return cudaGetLastError();
-}
-cudaError_t launch_round_end(const TrainerDev& a, cudaStream_t s) {
-  round_end_kernel<<<1, 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 cudaError_t launch_label_counts(const double* labels, uint64_t n, uint32_t classes, unsigned long long* counts,

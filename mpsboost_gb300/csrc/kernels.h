@@ -67,7 +67,7 @@ struct TrainerDev {
   uint32_t partial_stride;      // records per node: 1 (two-launch scan) or n_fchunks
   // Two-launch split scan (scan_two_phase: the FP32 screen applies): [max_level_nodes]
   // maximum FP32 screen score of each node's certainly admissible candidates (float
-  // bits; zeroed by each level's zero_build_slots_kernel, which every scan of the trainer
+  // bits; zeroed by each level's zero_slots_kernel, which every scan of the trainer
   // follows) and [max_level_nodes][features] each feature's maximum and exact flag. Null
   // node_screen: one launch, each feature screened on its own (the per-feature entry point
   // needs every feature's best split).
@@ -89,6 +89,7 @@ struct TrainerDev {
                                 // round (kNoLeaf between rounds)
   double* leaf_steps;           // [2 * max_leafsegs]: lr x leaf value per (segment, side)
   uint32_t* leaf_prefix;        // [max_leafsegs + 1]
+  uint32_t apply_chunk;         // rows per leaf-application chunk
   uint32_t max_leafsegs;
   TreeNodeOut* tree_nodes;      // [n_trees][max_tree_nodes]
   uint32_t max_tree_nodes;
@@ -164,10 +165,12 @@ bool encode_bins_tmap(CUtensorMap* map, const uint8_t* bins, uint64_t row_stride
 cudaError_t launch_hist_build(const TrainerDev& a, const HistConfig& cfg, int grid,
                               cudaStream_t stream);
 cudaError_t launch_fill_f64(double* dst, uint64_t n, double value, cudaStream_t stream);
-cudaError_t launch_round_begin(const TrainerDev& a, cudaStream_t stream);
-cudaError_t launch_gradients(const TrainerDev& a, int grid, cudaStream_t stream);
-cudaError_t launch_round_setup(const TrainerDev& a, cudaStream_t stream);
+// Gradients, then the round's setup. g_only: the roots' count and hessian histograms come
+// from the fit's first round.
+cudaError_t launch_gradients(const TrainerDev& a, bool g_only, int grid, cudaStream_t stream);
 cudaError_t launch_zero_build_slots(const TrainerDev& a, int grid, cudaStream_t stream);
+// The roots' slots: cleared, or (g_only) started from the kept count and hessian words.
+cudaError_t launch_zero_root_slots(const TrainerDev& a, bool g_only, int grid, cudaStream_t stream);
 cudaError_t launch_root_stats(const TrainerDev& a, cudaStream_t stream);
 // Leaf-wise growth: after the root's split scan (init), per step (select before the
 // partition / histogram / subtraction / split scan of the chosen leaves' children, merge
@@ -176,14 +179,16 @@ cudaError_t launch_leafwise_init(const TrainerDev& a, cudaStream_t stream);
 cudaError_t launch_leafwise_select(const TrainerDev& a, cudaStream_t stream);
 cudaError_t launch_leafwise_merge(const TrainerDev& a, cudaStream_t stream);
 cudaError_t launch_leafwise_finish(const TrainerDev& a, cudaStream_t stream);
-// save != 0: copy the roots' count and hessian words into root_cache; else restore them
-// into the roots' slots (after a gradient-only build).
-cudaError_t launch_root_cache(const TrainerDev& a, int save, int grid, cudaStream_t stream);
+// Copies the roots' count and hessian words into root_cache.
+cudaError_t launch_root_cache(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_subtract(const TrainerDev& a, int grid, cudaStream_t stream);
 // max_nodes: a bound on the nodes the launch scans (ctl->n_nodes), from the level.
-// to_active: a leaf-wise step; a two-launch scan writes its nodes' splits to their active
-// leaves (after a one-launch scan launch_leafwise_merge does).
-cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, bool to_active,
+// kRoot: level 0, whose statistics the scan forms where scan_forms_root (else
+// launch_root_stats has). kActive: a leaf-wise step; a two-launch scan writes its nodes'
+// splits to their active leaves (after a one-launch scan launch_leafwise_merge does).
+enum class ScanKind { kRoot, kLevel, kActive };
+bool scan_forms_root(const TrainerDev& a);
+cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind,
                               int grid, cudaStream_t stream);
 uint32_t split_scan_kernels(const TrainerDev& a);  // launches per launch_split_scan
 // max_nodes: a bound on the level's nodes (ctl->n_nodes).
@@ -195,7 +200,6 @@ uint32_t partition_kernels(const TrainerDev& a, uint32_t max_nodes);  // launche
 cudaError_t launch_partition_count(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_partition_finish(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_apply_leaves(const TrainerDev& a, int grid, cudaStream_t stream);
-cudaError_t launch_round_end(const TrainerDev& a, cudaStream_t stream);
 // counts [classes + 1], zeroed by the caller: rows per class id, then rows of no class.
 constexpr uint32_t kLabelCountMax = 8192;  // classes (32 KB of shared counters)
 cudaError_t launch_label_counts(const double* labels, uint64_t n, uint32_t classes, unsigned long long* counts,
