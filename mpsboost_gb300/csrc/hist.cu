@@ -470,7 +470,9 @@ __device__ __forceinline__ Bins32 ld_nc_na_v8(const void* p) {
 // feature's 8 cells (conflict-free), writes their 24 words into its row of the warp's
 // staging tile in the slot's order, and hands the row to one 192-byte
 // `cp.reduce.async.bulk ... .add.u64`, which L2 applies a sector at a time instead of as
-// 24 single-word atomics. All-zero rows are skipped. Every thread of the CTA calls it.
+// 24 single-word atomics. All-zero rows are skipped. `single`: no other item adds to the
+// node's slot, which was not cleared, so every row is stored instead. Every thread of the
+// CTA calls it.
 constexpr int kFlushWarps = 8;
 constexpr int kFlushBins = 8;
 constexpr int kFlushRowWords = kFlushBins * 3 + 2;  // a feature's 24 words, padded to 16 bytes
@@ -479,6 +481,10 @@ constexpr size_t kFlushBytes = size_t(kFlushWarps) * kBlockFeatures * kFlushRowW
 __device__ __forceinline__ void bulk_reduce_add_u64(void* gdst, uint32_t ssrc, uint32_t bytes) {
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;\n" ::"l"(gdst),
                "r"(ssrc), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* gdst, uint32_t ssrc, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(gdst), "r"(ssrc), "r"(bytes)
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
@@ -519,7 +525,7 @@ template <int MODE, int THREADS, bool PACKED>
 __device__ __forceinline__ void flush_cta_histogram_bulk(const TrainerDev& a, const BuildEntry& e, uint32_t fb,
                                                          const unsigned char* hist_smem,
                                                          unsigned long long* staging, long long q_unit_h,
-                                                         uint32_t row_count) {
+                                                         uint32_t row_count, bool single) {
   static_assert(THREADS / 32 > kFlushWarps, "flush warps and a spare warp");
   constexpr int CELLS = kSlots * kBlockFeatures;
   const int tid = threadIdx.x;
@@ -568,9 +574,11 @@ __device__ __forceinline__ void flush_cta_histogram_bulk(const TrainerDev& a, co
         row[3 * j + 2] = h;
         any |= c | g | h;
       }
-      if (lane < width && any != 0ull) {
+      if (lane < width && (single || any != 0ull)) {
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the row's stores before the bulk read
-        bulk_reduce_add_u64(dst_base + (size_t(lane) * kSlots + b0) * 3, row_addr, kFlushBins * 3 * 8);
+        unsigned long long* dst = dst_base + (size_t(lane) * kSlots + b0) * 3;
+        if (single) bulk_store(dst, row_addr, kFlushBins * 3 * 8);
+        else bulk_reduce_add_u64(dst, row_addr, kFlushBins * 3 * 8);
         bulk_commit();
       }
     }
@@ -593,6 +601,7 @@ constexpr uint32_t kPackFailCost = 8;
 struct ItemDesc {
   uint32_t item, limit, fb, row_begin, row_count;
   uint32_t packed;  // build with packed limbs first
+  uint32_t single;  // the node's only row chunk: its cells are stored, not added
   int kg, kh;
   BuildEntry e;
 };
@@ -626,6 +635,7 @@ __device__ __forceinline__ void fetch_item_warp(const TrainerDev& a, uint32_t la
     d.row_count = d.row_begin < d.e.seg_cnt ? min(item_rows, d.e.seg_cnt - d.row_begin) : 0u;
     d.kg = a.trees[d.e.tree].kg;
     d.kh = a.trees[d.e.tree].kh;
+    d.single = a.store_single && a.build_prefix[lo + 1] - a.build_prefix[lo] == 1;
     if (a.limb_votes) {
       const volatile uint32_t* votes = a.limb_votes + 2 * d.fb;  // other CTAs add to them
       const uint32_t passed = votes[0], failed = votes[1];
@@ -848,9 +858,9 @@ __global__ void __launch_bounds__(THREADS, 1) hist_build_direct_kernel(TrainerDe
     if (warp == kFlushWarps) fetch_item_warp(a, lane, s_desc);
     unsigned long long* staging = reinterpret_cast<unsigned long long*>(hist_smem + HistSmem<MODE>::kBytes);
     if (can_pack<MODE>() && packed)
-      flush_cta_histogram_bulk<MODE, THREADS, true>(a, e, fb, hist_smem, staging, q_unit_h, row_count);
+      flush_cta_histogram_bulk<MODE, THREADS, true>(a, e, fb, hist_smem, staging, q_unit_h, row_count, d.single != 0);
     else
-      flush_cta_histogram_bulk<MODE, THREADS, false>(a, e, fb, hist_smem, staging, q_unit_h, row_count);
+      flush_cta_histogram_bulk<MODE, THREADS, false>(a, e, fb, hist_smem, staging, q_unit_h, row_count, d.single != 0);
     __syncthreads();
   }
   bulk_wait_all();  // this thread's bulk reductions have reached the slots

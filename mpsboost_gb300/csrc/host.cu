@@ -848,7 +848,8 @@ struct mpsb_cuda_trainer {
         CK(launch_subtract(dev, grid(8), s)); ++k;
       }
       if (depth > 0) {
-        CK(launch_split_scan(dev, parity, level_nodes(d), d == 0 ? ScanKind::kRoot : ScanKind::kLevel, grid(4), s)); k += split_scan_kernels(dev);
+        CK(launch_split_scan(dev, parity, level_nodes(d), d == 0 ? ScanKind::kRoot : ScanKind::kLevel, d + 1 == depth,
+                             grid(4), s)); k += split_scan_kernels(dev);
       }
       CK(launch_finalize(dev, parity, d, level_nodes(d), s)); ++k;
       if (d + 1 < depth) {
@@ -889,7 +890,7 @@ struct mpsb_cuda_trainer {
     CK(launch_hist_build(view, hcfg, grid(1), s)); ++k;
     k += enqueue_root_stats(root_gradient_only);
     if (depth > 0) {
-      CK(launch_split_scan(dev, 0, n_trees, ScanKind::kRoot, grid(4), s)); k += split_scan_kernels(dev);
+      CK(launch_split_scan(dev, 0, n_trees, ScanKind::kRoot, false, grid(4), s)); k += split_scan_kernels(dev);
     }
     CK(launch_leafwise_init(dev, s)); ++k;
     for (uint32_t step = 0; step < lw_steps && depth > 0; ++step) {
@@ -904,7 +905,7 @@ struct mpsb_cuda_trainer {
       CK(launch_hist_build(step_view(), hcfg, grid(1), s)); ++k;
       if (!dev.fused_sub) { CK(launch_subtract(dev, grid(8), s)); ++k; }
       const uint32_t scans = split_scan_kernels(dev);
-      CK(launch_split_scan(dev, 1, 2 * n_trees, ScanKind::kActive, grid(4), s)); k += scans;
+      CK(launch_split_scan(dev, 1, 2 * n_trees, ScanKind::kActive, false, grid(4), s)); k += scans;
       if (scans == 1) { CK(launch_leafwise_merge(dev, s)); ++k; }
     }
     CK(launch_leafwise_finish(dev, s)); ++k;
@@ -931,6 +932,7 @@ struct mpsb_cuda_trainer {
   TrainerDev level_view(uint32_t d) const {
     TrainerDev v = build_view();
     if (limb_votes) v.limb_votes = limb_votes + size_t(2) * dev.nfb * d;
+    if (d == 0) v.store_single = 0;
     if (d < blocked_levels) {
       v.bins = ds->bins_blocked.as<uint8_t>();
       v.bins_row_stride = kBlockFeatures;
@@ -1190,6 +1192,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   cudaStream_t s = b->stream;
   const uint32_t W = tp.path_words;
 
+  a.store_single = a.mode == kModeFixed && ds->slots == uint32_t(kSlots) && t->hcfg.direct && !t->hcfg.bins_tmap;
   trace.mark("parameters, root cache");
   // inputs
   double* d_labels = t->alloc<double>(n);

@@ -429,6 +429,8 @@ __global__ void zero_slots_kernel(TrainerDev a, int what) {
        idx += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t e = uint32_t(idx / (words_per_slot / 2));
     const uint64_t w = idx - e * (words_per_slot / 2);
+    // A node of one row chunk is stored by its work items, not added.
+    if (what == kZeroBuilt && a.store_single && a.build_prefix[e + 1] - a.build_prefix[e] == 1) continue;
     if (a.tree_feature_masks) {
       // A forest tree reads only its own features' histograms (and feature 0's, for the
       // root statistics): the others are neither cleared nor subtracted nor scanned.
@@ -1473,13 +1475,13 @@ __device__ __forceinline__ bool pair_held(uint32_t s, uint32_t nb, bool hm, uint
 }
 
 // Words of the pair that starts at slot s (zeros where both slots are empty).
-template <bool FIXED, bool SUB>
+template <bool FIXED>
 __device__ __forceinline__ SlotWords load_slots(const TrainerDev& a, const ScanNode<FIXED>& node,
                                                 uint32_t f, uint32_t nb, bool hm, uint32_t S, uint32_t s) {
   SlotWords w{};
   if (pair_held(s, nb, hm, S)) {
     load_pair(w.own, a.hist + ((size_t(node.slot) * a.features + f) * S + s) * 3);
-    if (SUB && node.sub_from != 0)
+    if (node.sub_from != 0)
       load_pair(w.built, a.hist + ((size_t(node.sub_from - 1) * a.features + f) * S + s) * 3);
   }
   return w;
@@ -1487,22 +1489,23 @@ __device__ __forceinline__ SlotWords load_slots(const TrainerDev& a, const ScanN
 
 // One feature of one node, every thread of the CTA: calls visit(left, right, threshold,
 // default_left) for each candidate of the thread's slots. `first` holds page 0's words of
-// the thread's pair. SUB (the level's first launch): a sibling's histogram is formed as
-// parent minus built child on the way, with subtract_kernel's checks, and written back.
+// the thread's pair. A sibling's histogram (node.sub_from) is formed as parent minus built
+// child on the way, with subtract_kernel's checks, and written back where a later launch
+// reads it.
 // ROOT: the node's statistics are the feature's own totals (every feature of a root holds
 // all of its rows, so in fixed point they are the same), which it leaves in node.parent.
-template <bool FIXED, bool WIDE, bool SUB, bool ROOT, class Visit>
-__device__ __forceinline__ void scan_feature(const TrainerDev& a, ScanNode<FIXED>& node,
+template <bool FIXED, bool WIDE, bool ROOT, class Visit>
+__device__ __forceinline__ void scan_feature(const TrainerDev& a, ScanNode<FIXED>& node, bool write_back,
                                              uint32_t f, uint32_t nb, bool hm, const SlotWords& first,
                                              PageTotals<FIXED>* totals, uint32_t& buf, uint32_t& err,
                                              Visit&& visit) {
   const uint32_t S = WIDE ? a.slots : uint32_t(kSlots);
   const uint32_t pages = WIDE ? S / uint32_t(kSlots) : 1u;
-  const bool sub = SUB && node.sub_from != 0;
+  const bool sub = node.sub_from != 0;
   Stat<FIXED> miss = stat_zero<FIXED>(), carry = stat_zero<FIXED>();
   if (WIDE && hm) {  // the last page's last slot, needed from the first page on
     uint32_t ignored = 0;
-    SlotWords w = load_slots<FIXED, SUB>(a, node, f, nb, hm, S, S - 2);
+    SlotWords w = load_slots<FIXED>(a, node, f, nb, hm, S, S - 2);
 #pragma unroll
     for (uint32_t k = 3; k < 6; ++k)
       if (sub) w.own[k] = sibling_word<FIXED>(w.own[k], w.built[k], k - 3, ignored);
@@ -1511,15 +1514,17 @@ __device__ __forceinline__ void scan_feature(const TrainerDev& a, ScanNode<FIXED
   for (uint32_t p = 0; p < pages; ++p) {
     const uint32_t s = p * uint32_t(kSlots) + 2 * threadIdx.x;
     SlotWords w = first;
-    if (WIDE && p > 0) w = load_slots<FIXED, SUB>(a, node, f, nb, hm, S, s);
+    if (WIDE && p > 0) w = load_slots<FIXED>(a, node, f, nb, hm, S, s);
     if (sub && pair_held(s, nb, hm, S)) {
 #pragma unroll
       for (uint32_t k = 0; k < 6; ++k) w.own[k] = sibling_word<FIXED>(w.own[k], w.built[k], k % 3, err);
-      ulonglong2* out = reinterpret_cast<ulonglong2*>(
-          a.hist + ((size_t(node.slot) * a.features + f) * S + s) * 3);
-      out[0] = make_ulonglong2(w.own[0], w.own[1]);
-      out[1] = make_ulonglong2(w.own[2], w.own[3]);
-      out[2] = make_ulonglong2(w.own[4], w.own[5]);
+      if (write_back) {
+        ulonglong2* out = reinterpret_cast<ulonglong2*>(
+            a.hist + ((size_t(node.slot) * a.features + f) * S + s) * 3);
+        out[0] = make_ulonglong2(w.own[0], w.own[1]);
+        out[1] = make_ulonglong2(w.own[2], w.own[3]);
+        out[2] = make_ulonglong2(w.own[4], w.own[5]);
+      }
     }
     const Stat<FIXED> b0 = slot_stat<FIXED>(w.own[0], w.own[1], w.own[2], err);
     Stat<FIXED> b1 = slot_stat<FIXED>(w.own[3], w.own[4], w.own[5], err);
@@ -1573,7 +1578,7 @@ __device__ __forceinline__ void scan_feature(const TrainerDev& a, ScanNode<FIXED
 }
 
 template <bool FIXED, bool WIDE, bool ROOT>
-__global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(TrainerDev a, int parity) {
+__global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(TrainerDev a, int parity, bool last) {
   static_assert(!ROOT || (FIXED && !WIDE), "the features' totals are the same in fixed point only");
   __shared__ PageTotals<FIXED> s_totals[2];
   __shared__ uint32_t s_word[2][kScanFeaturesPerItem][kScanCtaWarps];
@@ -1607,7 +1612,7 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
     bool act = active(0);
     uint32_t nb = act ? a.bin_count[f0] : 0u;
     bool hm = act && a.has_missing[f0] != 0;
-    SlotWords w = !WIDE && act ? load_slots<FIXED, true>(a, node, f0, nb, hm, S, 2 * threadIdx.x) : SlotWords{};
+    SlotWords w = !WIDE && act ? load_slots<FIXED>(a, node, f0, nb, hm, S, 2 * threadIdx.x) : SlotWords{};
     for (uint32_t k = 0; k < nf; ++k) {
       // The next feature's words are in flight while this one is scanned (a wide feature's
       // pages are many and its registers fewer: its own words only).
@@ -1616,14 +1621,14 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
       const uint32_t nb_next = act_next ? a.bin_count[f + 1] : 0u;
       const bool hm_next = act_next && a.has_missing[f + 1] != 0;
       const SlotWords w_next = !WIDE && act_next
-                                   ? load_slots<FIXED, true>(a, node, f + 1, nb_next, hm_next, S, 2 * threadIdx.x)
+                                   ? load_slots<FIXED>(a, node, f + 1, nb_next, hm_next, S, 2 * threadIdx.x)
                                    : SlotWords{};
-      if (WIDE && act) w = load_slots<FIXED, true>(a, node, f, nb, hm, S, 2 * threadIdx.x);
+      if (WIDE && act) w = load_slots<FIXED>(a, node, f, nb, hm, S, 2 * threadIdx.x);
       uint32_t word = 0, exact = 0;
       if (act) {  // the same in every thread
         const ScreenScale scale = screen_scale<FIXED>(P, P.has_monotonic ? a.monotonic[f] : int8_t(0), kh);
-        scan_feature<FIXED, WIDE, true, ROOT>(
-            a, node, f, nb, hm, w, s_totals, buf, err,
+        scan_feature<FIXED, WIDE, ROOT>(
+            a, node, !last, f, nb, hm, w, s_totals, buf, err,
             [&](const Stat<FIXED>& cl, const Stat<FIXED>& cr, uint32_t, uint32_t) {
               if (!scale.on) {
                 exact = kFeatureExact;
@@ -1679,9 +1684,11 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
 }
 
 // One CTA per node. to_active: a leaf-wise step, whose nodes' splits go to their active
-// leaves.
+// leaves. last: the level's children are leaves, so no later level subtracts from a
+// sibling's histogram: the screen leaves it unwritten (a quarter of its bytes) and the few
+// features evaluated here form it again.
 template <bool FIXED, bool WIDE>
-__global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, int parity, bool to_active) {
+__global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, int parity, bool to_active, bool last) {
   __shared__ PageTotals<FIXED> s_totals[2];
   __shared__ uint32_t s_list[kScanCta], s_listed;
   __shared__ double s_gain[kScanCtaWarps];
@@ -1697,6 +1704,7 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
     const TreeState& tree = a.trees[rec.tree];
     const double inv_g = tree.inv_g, inv_h = tree.inv_h;
     ScanNode<FIXED> node = scan_node<FIXED>(rec, inv_h);
+    if (!last) node.sub_from = 0;
     const double lo = rec.lo, hi = rec.hi;
     const float m = __uint_as_float(a.node_screen[i]);
     const float cut = m >= 1e-30f ? m * (1.0f - 0x1p-18f) : -1.0f;
@@ -1719,9 +1727,9 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
         const bool hm = a.has_missing[f] != 0;
         const int8_t mono = P.has_monotonic ? a.monotonic[f] : int8_t(0);
         const ScreenScale scale = screen_scale<FIXED>(P, mono, tree.kh);
-        const SlotWords w = load_slots<FIXED, false>(a, node, f, nb, hm, S, 2 * threadIdx.x);
-        scan_feature<FIXED, WIDE, false, false>(
-            a, node, f, nb, hm, w, s_totals, buf, err,
+        const SlotWords w = load_slots<FIXED>(a, node, f, nb, hm, S, 2 * threadIdx.x);
+        scan_feature<FIXED, WIDE, false>(
+            a, node, false, f, nb, hm, w, s_totals, buf, err,
             [&](const Stat<FIXED>& l, const Stat<FIXED>& r, uint32_t t, uint32_t dl) {
               if (scale.on && cut > 0.0f) {
                 float score = 0.0f;
@@ -3496,36 +3504,36 @@ cudaError_t launch_scan_one(const TrainerDev& a, int parity, int grid, int threa
   return cudaGetLastError();
 }
 template <bool FIXED, bool WIDE>
-cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind,
+cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind, bool last,
                             cudaStream_t s) {
   const uint64_t resident = uint64_t(a.sm_count ? a.sm_count : 152) * 6;
   const uint32_t screen = uint32_t(std::min<uint64_t>(resident, uint64_t(max_nodes) * a.features));
   if constexpr (FIXED && !WIDE) {
     if (kind == ScanKind::kRoot && scan_forms_root(a))
-      split_screen_kernel<true, false, true><<<screen, kScanCta, 0, s>>>(a, parity);
+      split_screen_kernel<true, false, true><<<screen, kScanCta, 0, s>>>(a, parity, last);
     else
-      split_screen_kernel<true, false, false><<<screen, kScanCta, 0, s>>>(a, parity);
+      split_screen_kernel<true, false, false><<<screen, kScanCta, 0, s>>>(a, parity, last);
   } else {
-    split_screen_kernel<FIXED, WIDE, false><<<screen, kScanCta, 0, s>>>(a, parity);
+    split_screen_kernel<FIXED, WIDE, false><<<screen, kScanCta, 0, s>>>(a, parity, last);
   }
   const cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   const uint32_t exact = uint32_t(std::min<uint64_t>(resident, max_nodes));
-  split_exact_kernel<FIXED, WIDE><<<exact, kScanCta, 0, s>>>(a, parity, kind == ScanKind::kActive);
+  split_exact_kernel<FIXED, WIDE><<<exact, kScanCta, 0, s>>>(a, parity, kind == ScanKind::kActive, last);
   return cudaGetLastError();
 }
 
 
 cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind,
-                              int grid, cudaStream_t s) {
+                              bool last, int grid, cudaStream_t s) {
   const bool fixed = a.mode == kModeFixed, wide = a.slots != uint32_t(kSlots);
   if (a.slots < uint32_t(kSlots) || a.slots % uint32_t(kSlots) || max_nodes == 0) return cudaErrorInvalidValue;
   if (split_scan_kernels(a) == 2) {
     // node_screen was cleared by the level's zero_slots_kernel.
-    if (fixed) return wide ? launch_scan_two<true, true>(a, parity, max_nodes, kind, s)
-                           : launch_scan_two<true, false>(a, parity, max_nodes, kind, s);
-    return wide ? launch_scan_two<false, true>(a, parity, max_nodes, kind, s)
-                : launch_scan_two<false, false>(a, parity, max_nodes, kind, s);
+    if (fixed) return wide ? launch_scan_two<true, true>(a, parity, max_nodes, kind, last, s)
+                           : launch_scan_two<true, false>(a, parity, max_nodes, kind, last, s);
+    return wide ? launch_scan_two<false, true>(a, parity, max_nodes, kind, last, s)
+                : launch_scan_two<false, false>(a, parity, max_nodes, kind, last, s);
   }
   const int threads = int(a.scan_threads);
   if (threads < 32 || threads > kScanThreadsMax || threads % 32) return cudaErrorInvalidValue;
@@ -3558,25 +3566,29 @@ cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, uin
     finalize_kernel<<<1, 1024, 0, s>>>(a, parity, depth);
   return cudaGetLastError();
 }
-// CTAs per node of the cluster launch for a level of at most max_nodes split nodes over
-// `rows` rows in all (0: the three launches). As many as fit the GPU at once (one of these
-// CTAs per SM), up to the 16 of a non-portable cluster; not where that leaves a thread more
-// than 48 rows on average.
-static uint32_t partition_cluster_ctas(const TrainerDev& a, uint32_t max_nodes, uint64_t rows) {
+// CTAs per node of the cluster launch for a level of at most max_nodes split nodes (0: the
+// three launches). As many as fit the GPU at once (one of these CTAs per SM), up to the 16
+// of a non-portable cluster; not where a node that held every row (half of them from four
+// nodes on, a quarter in a leaf-wise step, whose nodes soon are small) would leave a thread
+// more than 16: at 1,000,000 rows the cluster launch takes 31-42 us a level, the three
+// launches 19; at 100,000 10 and 15; ten leaf-wise trees of 300,000 rows 15.1 and 15.9 ms.
+static uint32_t partition_cluster_ctas(const TrainerDev& a, uint32_t max_nodes) {
   const uint32_t sms = a.sm_count ? a.sm_count : 152;
   uint32_t ctas = 16;
   while (ctas > 1 && uint64_t(max_nodes) * ctas > sms) ctas >>= 1;
+  if (max_nodes > 2 * sms) return 0;  // each cluster would take several nodes in turn
   if (uint64_t(a.seg_stride) > uint64_t(ctas) * kClusterPartRows) return 0;  // the largest node possible
-  const uint64_t threads = std::min<uint64_t>(uint64_t(max_nodes) * ctas, sms) * kClusterThreads;
-  return rows <= 48 * threads ? ctas : 0;
+  const uint32_t largest =
+      a.lw_active ? a.seg_stride / 4 : (max_nodes / a.n_trees >= 4 ? a.seg_stride / 2 : a.seg_stride);
+  return largest <= 16u * ctas * kClusterThreads ? ctas : 0;
 }
 
 uint32_t partition_kernels(const TrainerDev& a, uint32_t max_nodes) {
-  return partition_cluster_ctas(a, max_nodes, uint64_t(a.n_trees) * a.seg_stride) ? 1u : 3u;
+  return partition_cluster_ctas(a, max_nodes) ? 1u : 3u;
 }
 
 cudaError_t launch_partition(const TrainerDev& a, uint32_t max_nodes, int grid, cudaStream_t s) {
-  if (const uint32_t ctas = partition_cluster_ctas(a, max_nodes, uint64_t(a.n_trees) * a.seg_stride)) {
+  if (const uint32_t ctas = partition_cluster_ctas(a, max_nodes)) {
     static std::atomic<unsigned long long> configured{0};  // one bit per device
     cudaError_t err = allow_large_clusters(configured, partition_cluster_kernel);
     if (err != cudaSuccess) return err;

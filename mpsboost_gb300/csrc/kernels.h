@@ -96,6 +96,8 @@ struct TrainerDev {
   Control* ctl;
   uint32_t* limb_votes;         // [nfb][2] of the launch's depth level: work items that passed
                                 // and failed the packed-limb check (null: split limbs only)
+  uint32_t store_single;        // below the roots: a node of one row chunk is stored by its work
+                                // items, so its slot is not cleared (register-direct kernel)
   uint32_t item_rows;           // rows per histogram work item (<= kItemRowsMax); 0: the
                                 // level's adaptive value ctl->item_rows
   uint32_t sm_count;
@@ -186,10 +188,11 @@ cudaError_t launch_subtract(const TrainerDev& a, int grid, cudaStream_t stream);
 // kRoot: level 0, whose statistics the scan forms where scan_forms_root (else
 // launch_root_stats has). kActive: a leaf-wise step; a two-launch scan writes its nodes'
 // splits to their active leaves (after a one-launch scan launch_leafwise_merge does).
+// last: the children of the scanned nodes are leaves.
 enum class ScanKind { kRoot, kLevel, kActive };
 bool scan_forms_root(const TrainerDev& a);
 cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind,
-                              int grid, cudaStream_t stream);
+                              bool last, int grid, cudaStream_t stream);
 uint32_t split_scan_kernels(const TrainerDev& a);  // launches per launch_split_scan
 // max_nodes: a bound on the level's nodes (ctl->n_nodes).
 cudaError_t launch_finalize(const TrainerDev& a, int parity, uint32_t depth, uint32_t max_nodes,

@@ -279,7 +279,7 @@ int mpsb_cuda_scan_splits(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     CK(launch_root_stats(a, s));
     const uint32_t one = 1;
     CK(cudaMemcpyAsync(&a.ctl->n_nodes, &one, sizeof one, cudaMemcpyHostToDevice, s));
-    CK(launch_split_scan(a, 0, 1, ScanKind::kRoot, b->sm_count * 8, s));
+    CK(launch_split_scan(a, 0, 1, ScanKind::kRoot, false, b->sm_count * 8, s));
     check_ctl(a, s);
     std::vector<SplitRec> rec(F);
     CK(cudaMemcpy(rec.data(), a.partial, F * sizeof(SplitRec), cudaMemcpyDeviceToHost));
