@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     // g/h in segment order (contiguous) or by row id (gathered).
     const float2* gh_seg = a.gh_ordered ? a.gh + seg : nullptr;
     const float2* gh_row = a.gh_ordered ? nullptr : a.gh + size_t(e.tree) * n;
-    const uint8_t* bins = a.bins + size_t(fb) * a.bins_block_stride;
+    const uint8_t* bins = a.bins + size_t(e.tree) * a.bins_tree_stride + size_t(fb) * a.bins_block_stride;
     const int kg = a.trees[e.tree].kg;
     const int kh = a.trees[e.tree].kh;
     // Unit-hessian builds: the quantized hessian of every row, round_half_even(2^kh).
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(THREADS, 1) hist_build_direct_kernel(TrainerDe
     const uint32_t* rows = a.rows + seg;
     const float2* gh_seg = a.gh_ordered ? a.gh + seg : nullptr;
     const float2* gh_row = a.gh_ordered ? nullptr : a.gh + size_t(e.tree) * n;
-    const uint8_t* bins = a.bins + size_t(fb) * a.bins_block_stride;
+    const uint8_t* bins = a.bins + size_t(e.tree) * a.bins_tree_stride + size_t(fb) * a.bins_block_stride;
     const uint64_t row_stride = a.bins_row_stride;
     const int kg = d.kg;
     const int kh = d.kh;

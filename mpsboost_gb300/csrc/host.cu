@@ -346,20 +346,34 @@ void parallel_trees(uint32_t count, F&& body) {
 // sample, without expanding it.
 double multiset_base_score(const mpsb_train_params& p, const double* y, const double* w,
                            const uint8_t* m, uint64_t n, int mode) {
+  // A piece of the expanded sample at a time: the terms are laid out without a branch per
+  // draw (four copies written, the count kept), then added in order.
   double total = 0.0, s = 0.0;
+  uint64_t drawn = 0;
   bool bad_w = false, bad_y = false;
-  for (uint64_t r = 0; r < n; ++r) {
-    for (uint32_t c = 0; c < m[r]; ++c) {
-      const double x = w ? w[r] : 1.0;
-      total += x;
-      s += y[r] * x;
+  constexpr uint32_t kPiece = 4096;
+  std::vector<double> ys(kPiece + 256 + 4), ws(w ? kPiece + 256 + 4 : 0);
+  for (uint64_t r = 0; r < n;) {
+    uint32_t pos = 0;
+    for (; r < n && pos < kPiece; ++r) {
+      const uint32_t c = m[r];
+      const double x = w ? w[r] : 1.0, v = y[r] * x;
+      bad_w |= (c != 0) & (!std::isfinite(x) | (x < 0.0));
+      bad_y |= (c != 0) & (!std::isfinite(y[r]) | ((mode == 2) & (y[r] < 0.0)));
+      for (uint32_t q = 0; q < 4; ++q) ys[pos + q] = v;
+      for (uint32_t q = 4; q < c; ++q) ys[pos + q] = v;
+      if (w) {
+        for (uint32_t q = 0; q < 4; ++q) ws[pos + q] = x;
+        for (uint32_t q = 4; q < c; ++q) ws[pos + q] = x;
+      }
+      pos += c;
     }
-    if (m[r]) {
-      const double x = w ? w[r] : 1.0;
-      bad_w |= !std::isfinite(x) || x < 0.0;
-      bad_y |= !std::isfinite(y[r]) || (mode == 2 && y[r] < 0.0);
-    }
+    for (uint32_t q = 0; q < pos; ++q) s += ys[q];
+    if (w)
+      for (uint32_t q = 0; q < pos; ++q) total += ws[q];
+    drawn += pos;
   }
+  if (!w) total = double(drawn);  // the sum of that many ones, exactly
   if (bad_w || bad_y || !std::isfinite(total) || !(total > 0.0) || !std::isfinite(s)) {
     // The exact error of the reference's sequential checks, over the expanded sample.
     std::vector<double> ys, ws;
@@ -933,7 +947,7 @@ struct mpsb_cuda_trainer {
     TrainerDev v = build_view();
     if (limb_votes) v.limb_votes = limb_votes + size_t(2) * dev.nfb * d;
     if (d == 0) v.store_single = 0;
-    if (d < blocked_levels) {
+    if (d < blocked_levels && !dev.feature_of) {
       v.bins = ds->bins_blocked.as<uint8_t>();
       v.bins_row_stride = kBlockFeatures;
       v.bins_block_stride = uint64_t(ds->n_rows) * kBlockFeatures;
@@ -1037,17 +1051,21 @@ struct mpsb_cuda_trainer {
 
 namespace {
 
-// A batch of forest trees: per tree its sample (a multiset of rows, ascending), feature
-// subset (as a mask and ranks), random-threshold seed and base score.
+// A batch of forest trees: per tree its sample (a multiset of rows, given as the number of
+// times each was drawn), feature subset, random-threshold seed and base score. Compact: the
+// trees train on their own features, numbered within their ascending subsets.
 struct ForestSpec {
   uint32_t n_trees = 0;
-  uint32_t cap = 0;                  // largest sample
-  std::vector<uint32_t> sample;      // [n_trees][cap]
-  std::vector<uint32_t> count;       // [n_trees]
-  std::vector<uint32_t> masks;       // [n_trees][path_words]
-  std::vector<uint32_t> ranks;       // [n_trees][features]
-  std::vector<uint32_t> seeds;       // [n_trees] or empty
-  std::vector<double> base_scores;   // [n_trees]
+  uint32_t cap = 0;                   // largest sample
+  const uint8_t* row_counts = nullptr;  // [n_trees][rows] (host)
+  std::vector<uint32_t> count;        // [n_trees]
+  bool compact = false;
+  uint32_t features = 0;              // the dataset's, or (compact) the largest subset
+  std::vector<uint32_t> feature_of;   // compact: [n_trees][features], 0xffffffff past a subset
+  std::vector<uint32_t> masks;        // [n_trees][path_words]
+  std::vector<uint32_t> ranks;        // [n_trees][features] (compact: empty, rank = number)
+  std::vector<uint32_t> seeds;        // [n_trees] or empty
+  std::vector<double> base_scores;    // [n_trees]
 };
 
 void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
@@ -1085,7 +1103,8 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   if (t->ovr && p->objective != MPSB_BINARY_LOGISTIC)
     throw TrainingError("one-vs-rest training uses the binary_logistic objective");
   const uint32_t T = t->n_trees;
-  const uint32_t F = ds->features;
+  const uint32_t F = forest ? forest->features : ds->features;  // a tree's feature numbers
+  const bool compact = forest && forest->compact;
   const uint32_t D = p->max_depth;
   if (D > 24) throw UnsupportedError("max_depth above 24 is not supported by the CUDA backend");
   const uint64_t max_leaves_eff = effective_max_leaves(*p);
@@ -1114,7 +1133,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.n_rows = ds->n_rows;
   a.seg_stride = uint32_t(seg_rows);
   a.features = F;
-  a.nfb = ds->nfb;
+  a.nfb = (F + kBlockFeatures - 1) / kBlockFeatures;
   a.n_trees = T;
   a.objective = p->objective;
   a.ovr = t->ovr ? 1 : 0;
@@ -1143,7 +1162,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
       a.scan_threads = tuned.scan_threads;
     }
   }
-  t->hcfg.bins_tmap = ds->has_bins_tmap ? &ds->bins_tmap : nullptr;
+  t->hcfg.bins_tmap = ds->has_bins_tmap && !compact ? &ds->bins_tmap : nullptr;
   // Launch-shape overrides (tuning sweeps): threads per CTA, pipeline stages, rows per work
   // item, split-scan CTA size.
   if (const char* v = std::getenv("MPSB_SCAN_THREADS"))
@@ -1244,18 +1263,23 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   }
   trace.mark("label/weight upload");
   if (!softmax_classes) t->base_scores.resize(T);
-  if (!softmax_classes) a.preds = t->alloc<double>(size_t(T) * n);
-  for (uint32_t k = 0; k < T && !softmax_classes; ++k) {
-    t->base_scores[k] = forest ? forest->base_scores[k]
-                        : !class_rows.empty()
+  if (forest) {  // single-round trees: every row's prediction is the base score
+    t->base_scores = forest->base_scores;
+    double* d_base = t->alloc<double>(T);
+    CK(cudaMemcpyAsync(d_base, t->base_scores.data(), size_t(T) * sizeof(double), cudaMemcpyHostToDevice, s));
+    a.tree_base = d_base;
+  }
+  if (!softmax_classes && !forest) a.preds = t->alloc<double>(size_t(T) * n);
+  for (uint32_t k = 0; k < T && !softmax_classes && !forest; ++k) {
+    t->base_scores[k] = !class_rows.empty()
                             ? logistic_base(double(class_rows[t->ovr ? k : 1u]), sums.total)
                             : base_score(*p, labels, weights, n, t->ovr ? int64_t(k) : -1, &sums);
     CK(launch_fill_f64(a.preds + size_t(k) * n, n, t->base_scores[k], s));
   }
   trace.mark("base scores, predictions");
   if (p->n_monotonic) {
-    int8_t* m = t->alloc<int8_t>(F);
-    CK(cudaMemcpyAsync(m, p->monotonic_constraints, F, cudaMemcpyHostToDevice, s));
+    int8_t* m = t->alloc<int8_t>(ds->features);
+    CK(cudaMemcpyAsync(m, p->monotonic_constraints, ds->features, cudaMemcpyHostToDevice, s));
     a.monotonic = m;
   }
   if (p->n_interaction_groups) {
@@ -1271,19 +1295,34 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
     a.group_masks = gm;
   }
   if (forest) {
-    const size_t cells = size_t(T) * forest->cap;
-    uint32_t* d_sample = t->alloc<uint32_t>(cells);
-    CK(cudaMemcpyAsync(d_sample, forest->sample.data(), cells * 4, cudaMemcpyHostToDevice, s));
+    uint32_t* d_sample = t->alloc<uint32_t>(size_t(T) * forest->cap);
+    DevBuf counts, chunk_sums;  // released once the samples are written
+    counts.alloc(size_t(T) * n);
+    chunk_sums.alloc(size_t(T) * ((n + kExpandChunk - 1) / kExpandChunk) * sizeof(uint32_t));
+    CK(cudaMemcpyAsync(counts.p, forest->row_counts, size_t(T) * n, cudaMemcpyHostToDevice, s));
+    CK(launch_expand_samples(counts.as<uint8_t>(), uint32_t(n), T, chunk_sums.as<uint32_t>(), forest->cap,
+                             d_sample, s));
     uint32_t* d_count = t->alloc<uint32_t>(T);
     CK(cudaMemcpyAsync(d_count, forest->count.data(), size_t(T) * 4, cudaMemcpyHostToDevice, s));
     uint32_t* d_masks = t->alloc<uint32_t>(size_t(T) * W);
     CK(cudaMemcpyAsync(d_masks, forest->masks.data(), size_t(T) * W * 4, cudaMemcpyHostToDevice, s));
-    uint32_t* d_ranks = t->alloc<uint32_t>(size_t(T) * F);
-    CK(cudaMemcpyAsync(d_ranks, forest->ranks.data(), size_t(T) * F * 4, cudaMemcpyHostToDevice, s));
+    if (compact) {
+      uint32_t* d_of = t->alloc<uint32_t>(size_t(T) * F);
+      CK(cudaMemcpyAsync(d_of, forest->feature_of.data(), size_t(T) * F * 4, cudaMemcpyHostToDevice, s));
+      uint8_t* d_bins = t->alloc<uint8_t>(size_t(T) * n * a.nfb * kBlockFeatures);
+      CK(launch_pack_tree_bins(ds->bins_fm.as<uint8_t>(), uint32_t(n), d_of, F, a.nfb, T, d_bins, s));
+      a.feature_of = d_of;
+      a.bins = d_bins;
+      a.bins_row_stride = uint64_t(a.nfb) * kBlockFeatures;
+      a.bins_tree_stride = uint64_t(n) * a.nfb * kBlockFeatures;
+    } else {
+      uint32_t* d_ranks = t->alloc<uint32_t>(size_t(T) * F);
+      CK(cudaMemcpyAsync(d_ranks, forest->ranks.data(), size_t(T) * F * 4, cudaMemcpyHostToDevice, s));
+      a.feature_rank = d_ranks;
+    }
     a.sample_rows = d_sample;
     a.sample_count = d_count;
     a.tree_feature_masks = d_masks;
-    a.feature_rank = d_ranks;
     if (!forest->seeds.empty()) {
       uint32_t* d_seeds = t->alloc<uint32_t>(T);
       CK(cudaMemcpyAsync(d_seeds, forest->seeds.data(), size_t(T) * 4, cudaMemcpyHostToDevice, s));
@@ -1715,11 +1754,12 @@ int mpsb_cuda_train_forest(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     validate_training_params(*p);
     validate_tree_params(*p, ds->features);
     validate_weights(weights, n);
-    const uint32_t F = ds->features, W = (F + 31) / 32;
+    const uint32_t F = ds->features;
     // Trees per trainer: the histogram slots of a tree's widest level dominate its device
     // memory, so batch as many trees as fit in half of the free memory.
     mpsb_train_params tp = *p;
     tp.n_estimators = 1;
+    PhaseTrace trace("forest");
     // Sample sizes of every tree (independent trees: worker threads).
     std::vector<uint64_t> sample_size(n_trees, 0);
     parallel_trees(n_trees, [&](uint32_t t) {
@@ -1728,7 +1768,9 @@ int mpsb_cuda_train_forest(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
       for (uint64_t r = 0; r < n; ++r) c += m[r];
       sample_size[t] = c;
     });
+    trace.mark("sample sizes");
     uint64_t cap_all = 1;
+    uint32_t widest = 1;  // the largest subset
     for (uint32_t t = 0; t < n_trees; ++t) {
       const uint64_t c = sample_size[t];
       if (c == 0) throw TrainingError("a forest tree's row sample must not be empty");
@@ -1736,6 +1778,7 @@ int mpsb_cuda_train_forest(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
       cap_all = std::max(cap_all, c);
       const uint32_t f0 = feature_offsets[t], f1 = feature_offsets[t + 1];
       if (f1 <= f0) throw TrainingError("a forest tree's feature subset must not be empty");
+      widest = std::max(widest, f1 - f0);
       std::vector<uint8_t> seen(F, 0);
       for (uint32_t i = f0; i < f1; ++i) {
         if (features[i] >= F) throw TrainingError("forest feature index out of range");
@@ -1745,8 +1788,12 @@ int mpsb_cuda_train_forest(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     const uint64_t leaves = std::min<uint64_t>(
         {uint64_t(1) << std::min<uint32_t>(p->max_depth, 30), std::max<uint64_t>(effective_max_leaves(*p), 2),
          std::max<uint64_t>(1, (cap_all + p->min_samples_leaf - 1) / p->min_samples_leaf)});
-    const uint64_t per_tree = leaves * uint64_t(F) * ds->slots * 24 + cap_all * (2 * 12 + 8) + n * 8 +
-                              uint64_t(2 * leaves + 1) * 64 * 8;
+    // Trees of few features train on a copy of their own (compact) where that is at most half
+    // of the dataset's: histograms, their slots and the scans then hold no other feature.
+    const bool compact = ds->slots == uint32_t(kSlots) && widest * 2 <= F;
+    const uint32_t FT = compact ? widest : F, W = (FT + 31) / 32;
+    const uint64_t per_tree = leaves * uint64_t(FT) * ds->slots * 24 + cap_all * (2 * 12 + 4) + n +
+                              (compact ? n * W * kBlockFeatures : 0) + uint64_t(2 * leaves + 1) * 64 * 8;
     size_t free_b = 0, total_b = 0;
     b->activate();
     CK(cudaMemGetInfo(&free_b, &total_b));
@@ -1762,44 +1809,52 @@ int mpsb_cuda_train_forest(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
         fs.count[k] = uint32_t(sample_size[t0 + k]);
         fs.cap = std::max<uint32_t>(fs.cap, fs.count[k]);
       }
-      fs.sample.assign(size_t(B) * fs.cap, 0);
+      fs.row_counts = row_counts + size_t(t0) * n;
+      fs.compact = compact;
+      fs.features = FT;
       fs.masks.assign(size_t(B) * W, 0);
-      fs.ranks.assign(size_t(B) * F, 0);
+      if (compact) fs.feature_of.assign(size_t(B) * FT, 0xffffffffu);
+      else fs.ranks.assign(size_t(B) * F, 0);
       fs.base_scores.resize(B);
       if (seeds) fs.seeds.assign(seeds + t0, seeds + t0 + B);
       const int mode = label_mode_of(tp.objective);
       parallel_trees(B, [&](uint32_t k) {
         const uint8_t* m = row_counts + size_t(t0 + k) * n;
-        uint32_t* dst = fs.sample.data() + size_t(k) * fs.cap;
-        uint32_t pos = 0;
-        for (uint64_t r = 0; r < n; ++r)
-          for (uint32_t c = 0; c < m[r]; ++c) dst[pos++] = uint32_t(r);
         // The reference fits the tree on its sample: base score over the sample's rows in
         // order (each row as often as it was drawn).
         if (mode) {
           fs.base_scores[k] = multiset_base_score(tp, labels, weights, m, n, mode);
         } else {
           std::vector<double> ys, ws;
-          ys.reserve(pos);
-          if (weights) ws.reserve(pos);
-          for (uint32_t i = 0; i < pos; ++i) {
-            ys.push_back(labels[dst[i]]);
-            if (weights) ws.push_back(weights[dst[i]]);
-          }
+          ys.reserve(fs.count[k]);
+          if (weights) ws.reserve(fs.count[k]);
+          for (uint64_t r = 0; r < n; ++r)
+            for (uint32_t c = 0; c < m[r]; ++c) {
+              ys.push_back(labels[r]);
+              if (weights) ws.push_back(weights[r]);
+            }
           fs.base_scores[k] = base_score(tp, ys.data(), weights ? ws.data() : nullptr, ys.size(), -1);
         }
         std::vector<uint32_t> sub(features + feature_offsets[t0 + k], features + feature_offsets[t0 + k + 1]);
         std::sort(sub.begin(), sub.end());
-        for (uint32_t i = 0; i < sub.size(); ++i) {
-          fs.masks[size_t(k) * W + sub[i] / 32] |= 1u << (sub[i] % 32);
-          fs.ranks[size_t(k) * F + sub[i]] = i;  // position in the tree's ascending subset
+        for (uint32_t i = 0; i < sub.size(); ++i) {  // i: position in the tree's ascending subset
+          const uint32_t f = compact ? i : sub[i];
+          fs.masks[size_t(k) * W + f / 32] |= 1u << (f % 32);
+          if (compact) fs.feature_of[size_t(k) * FT + i] = sub[i];
+          else fs.ranks[size_t(k) * F + f] = i;
         }
       });
+      trace.mark("base scores, subsets");
       std::unique_ptr<mpsb_cuda_trainer> t(new mpsb_cuda_trainer);
       setup_trainer(t.get(), b, ds, labels, weights, n, &tp, options | MPSB_OPT_NO_GRAPH, 0, &fs);
+      trace.mark("setup");
       t->run(1);
       t->synchronize();
+      trace.mark("growth");
       for (uint32_t k = 0; k < B; ++k) out[t0 + k] = export_model(t.get(), k, false);
+      trace.mark("export");
+      t.reset();
+      trace.mark("release");
     }
   });
 }

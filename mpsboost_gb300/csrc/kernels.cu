@@ -40,6 +40,11 @@ __device__ __forceinline__ void raise(Control* ctl, uint32_t bits) { atomicOr(&c
 
 __device__ __forceinline__ uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
+// The dataset's feature behind a tree's feature f (compact forests number a tree's own).
+__device__ __forceinline__ uint32_t dataset_feature(const TrainerDev& a, uint32_t tree, uint32_t f) {
+  return a.feature_of ? a.feature_of[size_t(tree) * a.features + f] : f;
+}
+
 // Rows per histogram work item for a level that builds `rows` rows: about per_sm (default
 // three) items per SM, a multiple of 512, within [1024, kItemRowsMax]. Where the
 // kItemRowsMax cap forces more items, their number is raised to the next multiple of the
@@ -334,7 +339,7 @@ __global__ void __launch_bounds__(256, SQ ? 8 : 4) gradients_kernel(const __grid
     if (SQ || (a.objective == 0 && !a.n_classes)) {
       // Squared error (the objective_pair case 0 then the weight products): g = w (p - y),
       // h = w; two FP64 operations per row on the narrow FP64 pipe.
-      const double pred = a.preds[tree_off + i];
+      const double pred = a.preds ? a.preds[tree_off + i] : a.tree_base[t];
       g = __dsub_rn(pred, y);  // p + (-y): negation is exact
       if (!f64_finite(y) || !f64_finite(pred) || !f64_finite(g)) bad = 1;
       h = 1.0;
@@ -348,7 +353,7 @@ __global__ void __launch_bounds__(256, SQ ? 8 : 4) gradients_kernel(const __grid
       if (a.n_classes) {
         if (!softmax_pair(a, y, i, *a.round_counter % a.n_classes, &g, &h)) bad = 1;
       } else {
-        const double pred = a.preds[tree_off + i];
+        const double pred = a.preds ? a.preds[tree_off + i] : a.tree_base[t];
         if (!objective_pair(a.objective, y, pred, a.params, &g, &h)) bad = 1;
       }
       if (a.weights != nullptr) {
@@ -1020,8 +1025,9 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
       active = (allowed >> (f & 31)) & 1u;
     }
     if (active) {  // warp-uniform
-      const uint32_t nb = a.bin_count[f];
-      const bool hm = a.has_missing[f] != 0;
+      const uint32_t df = dataset_feature(a, node.tree, f);
+      const uint32_t nb = a.bin_count[df];
+      const bool hm = a.has_missing[df] != 0;
       // At most 32 bins: one slot per lane (slot = lane), the missing slot apart.
       const bool few = !WIDE && nb <= 32u;
       const int kper = few ? 1 : 8;
@@ -1137,7 +1143,7 @@ __global__ void __launch_bounds__(kScanThreadsMax) split_scan_kernel(TrainerDev 
         }
         if (miss.count > parent.count || miss_h_above) err |= kErrMissing;
         const Stat<FIXED> nmp = stat_sub<FIXED>(parent, miss);
-        const int8_t mono = P.has_monotonic ? a.monotonic[f] : 0;
+        const int8_t mono = P.has_monotonic ? a.monotonic[df] : 0;
         const uint32_t rnd =
             P.split_strategy == 1
                 ? stable_random_threshold(
@@ -1610,23 +1616,25 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
       return k < nf && usable && ((allowed[(f0 + k) >> 5] >> ((f0 + k) & 31)) & 1u);
     };
     bool act = active(0);
-    uint32_t nb = act ? a.bin_count[f0] : 0u;
-    bool hm = act && a.has_missing[f0] != 0;
+    uint32_t df = act ? dataset_feature(a, rec.tree, f0) : 0u;
+    uint32_t nb = act ? a.bin_count[df] : 0u;
+    bool hm = act && a.has_missing[df] != 0;
     SlotWords w = !WIDE && act ? load_slots<FIXED>(a, node, f0, nb, hm, S, 2 * threadIdx.x) : SlotWords{};
     for (uint32_t k = 0; k < nf; ++k) {
       // The next feature's words are in flight while this one is scanned (a wide feature's
       // pages are many and its registers fewer: its own words only).
       const uint32_t f = f0 + k;
       const bool act_next = active(k + 1);
-      const uint32_t nb_next = act_next ? a.bin_count[f + 1] : 0u;
-      const bool hm_next = act_next && a.has_missing[f + 1] != 0;
+      const uint32_t df_next = act_next ? dataset_feature(a, rec.tree, f + 1) : 0u;
+      const uint32_t nb_next = act_next ? a.bin_count[df_next] : 0u;
+      const bool hm_next = act_next && a.has_missing[df_next] != 0;
       const SlotWords w_next = !WIDE && act_next
                                    ? load_slots<FIXED>(a, node, f + 1, nb_next, hm_next, S, 2 * threadIdx.x)
                                    : SlotWords{};
       if (WIDE && act) w = load_slots<FIXED>(a, node, f, nb, hm, S, 2 * threadIdx.x);
       uint32_t word = 0, exact = 0;
       if (act) {  // the same in every thread
-        const ScreenScale scale = screen_scale<FIXED>(P, P.has_monotonic ? a.monotonic[f] : int8_t(0), kh);
+        const ScreenScale scale = screen_scale<FIXED>(P, P.has_monotonic ? a.monotonic[df] : int8_t(0), kh);
         scan_feature<FIXED, WIDE, ROOT>(
             a, node, !last, f, nb, hm, w, s_totals, buf, err,
             [&](const Stat<FIXED>& cl, const Stat<FIXED>& cr, uint32_t, uint32_t) {
@@ -1660,6 +1668,7 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
       if (__any_sync(0xffffffffu, exact != 0)) word |= kFeatureExact;
       if (lane == 0) s_word[ib][k][warp] = word;
       act = act_next;
+      df = df_next;
       nb = nb_next;
       hm = hm_next;
       w = w_next;
@@ -1723,9 +1732,10 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
       const uint32_t listed = s_listed;
       for (uint32_t k = 0; k < listed; ++k) {
         const uint32_t f = s_list[k];
-        const uint32_t nb = a.bin_count[f];
-        const bool hm = a.has_missing[f] != 0;
-        const int8_t mono = P.has_monotonic ? a.monotonic[f] : int8_t(0);
+        const uint32_t df = dataset_feature(a, rec.tree, f);
+        const uint32_t nb = a.bin_count[df];
+        const bool hm = a.has_missing[df] != 0;
+        const int8_t mono = P.has_monotonic ? a.monotonic[df] : int8_t(0);
         const ScreenScale scale = screen_scale<FIXED>(P, mono, tree.kh);
         const SlotWords w = load_slots<FIXED>(a, node, f, nb, hm, S, 2 * threadIdx.x);
         scan_feature<FIXED, WIDE, false>(
@@ -1822,7 +1832,8 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
     if (bw < 0) {
       if (threadIdx.x == 0) *out = no_split();
     } else if (threadIdx.x == s_key[bw][4]) {
-      const int8_t mono = P.has_monotonic ? a.monotonic[feature] : int8_t(0);
+      const int8_t mono =
+          P.has_monotonic ? a.monotonic[dataset_feature(a, rec.tree, feature)] : int8_t(0);
       *out = split_record<FIXED>(P, cl, cr, inv_g, inv_h, mono, lo, hi, gain, feature, threshold,
                                  default_left);
     }
@@ -2058,7 +2069,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       write_leaf(&tn[li], lv);
       write_leaf(&tn[ri], rv);
       TreeNodeOut& pn = tn[node.node_index];
-      pn.feature_index = b.feature;
+      pn.feature_index = dataset_feature(a, t, b.feature);
       pn.threshold_bin = b.threshold;
       pn.left_child = li;
       pn.right_child = ri;
@@ -2129,7 +2140,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
         pe.parity = uint32_t(parity);
         pe.seg_off = node.seg_off;
         pe.seg_cnt = node.seg_cnt;
-        pe.feature = b.feature;
+        pe.feature = dataset_feature(a, t, b.feature);
         pe.threshold = b.threshold;
         pe.default_left = b.default_left;
         pe.lcount = uint32_t(b.lcount);
@@ -2144,7 +2155,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
         ls.seg_off = node.seg_off;
         ls.seg_cnt = node.seg_cnt;
         ls.split = 1;
-        ls.feature = b.feature;
+        ls.feature = dataset_feature(a, t, b.feature);
         ls.threshold = b.threshold;
         ls.default_left = b.default_left;
         ls.value = 0.0;
@@ -2308,7 +2319,7 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
       write_leaf(&tn[li], lv);
       write_leaf(&tn[ri], rv);
       TreeNodeOut& pn = tn[node.node_index];
-      pn.feature_index = b.feature;
+      pn.feature_index = dataset_feature(a, t, b.feature);
       pn.threshold_bin = b.threshold;
       pn.left_child = li;
       pn.right_child = ri;
@@ -2369,7 +2380,7 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
         pe.parity = uint32_t(parity);
         pe.seg_off = node.seg_off;
         pe.seg_cnt = node.seg_cnt;
-        pe.feature = b.feature;
+        pe.feature = dataset_feature(a, t, b.feature);
         pe.threshold = b.threshold;
         pe.default_left = b.default_left;
         pe.lcount = uint32_t(b.lcount);
@@ -2390,7 +2401,7 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
         }
       } else {
         ls.split = 1;
-        ls.feature = b.feature;
+        ls.feature = dataset_feature(a, t, b.feature);
         ls.threshold = b.threshold;
         ls.default_left = b.default_left;
         ls.left_value = lv;
@@ -3216,6 +3227,107 @@ __global__ void __launch_bounds__(256) apply_steps_kernel(TrainerDev a) {
   if (err) raise(a.ctl, err);
 }
 
+// ---- Forest trees ----------------------------------------------------------------------
+// A tree's sample is given as row multiplicities (u8 per row); its root segment is the
+// rows in ascending order, each as often as it was drawn. Rows in chunks of kExpandChunk:
+// chunk sums, a prefix per tree, then each chunk writes its part. HBM-bound: one byte read
+// twice and four written per row. Grid (chunks, trees).
+constexpr uint32_t kExpandThreads = 256, kExpandPer = 16;
+static_assert(kExpandChunk == kExpandThreads * kExpandPer, "a thread expands kExpandPer rows");
+
+__device__ __forceinline__ uint32_t expand_counts(const uint8_t* counts, uint32_t n, uint32_t row0,
+                                                  uint32_t (&c)[kExpandPer]) {
+  uint32_t sum = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kExpandPer; ++k) {
+    c[k] = row0 + k < n ? counts[row0 + k] : 0u;
+    sum += c[k];
+  }
+  return sum;
+}
+
+__global__ void __launch_bounds__(kExpandThreads) expand_sum_kernel(const uint8_t* counts, uint32_t n,
+                                                                    uint32_t* chunk_sum) {
+  __shared__ uint32_t sh[33];
+  uint32_t c[kExpandPer], v[1], tot[1];
+  const uint32_t row0 = blockIdx.x * kExpandChunk + threadIdx.x * kExpandPer;
+  v[0] = expand_counts(counts + size_t(blockIdx.y) * n, n, row0, c);
+  block_scan<1>(v, tot, sh);
+  if (threadIdx.x == 0) chunk_sum[size_t(blockIdx.y) * gridDim.x + blockIdx.x] = tot[0];
+}
+
+__global__ void __launch_bounds__(1024) expand_scan_kernel(uint32_t* chunk_sum, uint32_t chunks) {
+  __shared__ uint32_t sh[33];
+  uint32_t* c = chunk_sum + size_t(blockIdx.x) * chunks;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < chunks; base += blockDim.x) {
+    const uint32_t i = base + threadIdx.x;
+    uint32_t v[1] = {i < chunks ? c[i] : 0u}, tot[1];
+    block_scan<1>(v, tot, sh);
+    if (i < chunks) c[i] = carry + v[0];
+    carry += tot[0];
+  }
+}
+
+__global__ void __launch_bounds__(kExpandThreads) expand_write_kernel(const uint8_t* counts, uint32_t n,
+                                                                      const uint32_t* chunk_begin, uint32_t cap,
+                                                                      uint32_t* sample) {
+  __shared__ uint32_t sh[33];
+  uint32_t c[kExpandPer], v[1], tot[1];
+  const uint32_t row0 = blockIdx.x * kExpandChunk + threadIdx.x * kExpandPer;
+  v[0] = expand_counts(counts + size_t(blockIdx.y) * n, n, row0, c);
+  block_scan<1>(v, tot, sh);
+  uint32_t at = chunk_begin[size_t(blockIdx.y) * gridDim.x + blockIdx.x] + v[0];
+  uint32_t* out = sample + size_t(blockIdx.y) * cap;
+  for (uint32_t k = 0; k < kExpandPer; ++k)
+    for (uint32_t r = 0; r < c[k]; ++r, ++at)
+      if (at < cap) out[at] = row0 + k;  // always: cap is the largest sample
+}
+
+// Compact forests: each tree's own features, [trees][n][nfb * 32] u8 rows, from the
+// feature-major bins (a tree of 10 of 100 features then builds one feature block and 10
+// features' histograms instead of four and 100). A thread takes four rows: a 4-byte load
+// per feature, 4 x 4 byte transposes in registers, one 32-byte store per row. Grid (row
+// tiles of 512, feature blocks, trees); feature_of 0xffffffff: no feature.
+__global__ void __launch_bounds__(128) pack_tree_bins_kernel(const uint8_t* bins_fm, uint32_t n,
+                                                             const uint32_t* feature_of, uint32_t features,
+                                                             uint32_t nfb, uint8_t* out) {
+  const uint32_t tree = blockIdx.z, fb = blockIdx.y;
+  const uint32_t row = blockIdx.x * 512 + threadIdx.x * 4;
+  if (row >= n) return;
+  const bool words = n % 4 == 0;  // every feature's rows start on a word
+  uint32_t w[32];
+#pragma unroll
+  for (uint32_t c = 0; c < 32; ++c) {
+    const uint32_t f = fb * 32 + c;
+    const uint32_t df = f < features ? __ldg(feature_of + size_t(tree) * features + f) : 0xffffffffu;
+    w[c] = 0;
+    if (df != 0xffffffffu) {
+      const uint8_t* src = bins_fm + size_t(df) * n + row;
+      if (words) {
+        w[c] = __ldg(reinterpret_cast<const uint32_t*>(src));
+      } else {
+        for (uint32_t q = 0; q < 4 && row + q < n; ++q) w[c] |= uint32_t(__ldg(src + q)) << (8 * q);
+      }
+    }
+  }
+#pragma unroll
+  for (uint32_t r = 0; r < 4; ++r) {
+    uint32_t v[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      const uint32_t lo = __byte_perm(w[4 * q], w[4 * q + 1], r | ((4 + r) << 4));
+      const uint32_t hi = __byte_perm(w[4 * q + 2], w[4 * q + 3], r | ((4 + r) << 4));
+      v[q] = __byte_perm(lo, hi, 0x5410);
+    }
+    if (row + r < n)
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(
+                       out + ((size_t(tree) * n + row + r) * nfb + fb) * 32),
+                   "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                   : "memory");
+  }
+}
+
 // Rows of each class id 0..classes-1 (counts[classes]: rows whose label is none of them).
 // The class priors and the logistic base score of an unweighted fit are these whole
 // numbers, in any order of addition. HBM-bound (8 B per row); shared-memory counters per
@@ -3633,6 +3745,29 @@ cudaError_t launch_fill_f64(double* dst, uint64_t n, double value, cudaStream_t 
 cudaError_t launch_apply_leaves(const TrainerDev& a, int grid, cudaStream_t s) {
   apply_leaves_kernel<<<grid, 256, 0, s>>>(a);
   apply_steps_kernel<<<grid, 256, 0, s>>>(a);
+  return cudaGetLastError();
+}
+cudaError_t launch_expand_samples(const uint8_t* counts, uint32_t n, uint32_t trees, uint32_t* chunk_sum,
+                                  uint32_t cap, uint32_t* sample, cudaStream_t s) {
+  const uint32_t chunks = (n + kExpandChunk - 1) / kExpandChunk;
+  for (uint32_t t0 = 0; t0 < trees; t0 += 65535) {  // the grid's y limit
+    const uint32_t nt = std::min(65535u, trees - t0);
+    const uint8_t* c = counts + size_t(t0) * n;
+    uint32_t* sums = chunk_sum + size_t(t0) * chunks;
+    expand_sum_kernel<<<dim3(chunks, nt), kExpandThreads, 0, s>>>(c, n, sums);
+    expand_scan_kernel<<<nt, 1024, 0, s>>>(sums, chunks);
+    expand_write_kernel<<<dim3(chunks, nt), kExpandThreads, 0, s>>>(c, n, sums, cap, sample + size_t(t0) * cap);
+  }
+  return cudaGetLastError();
+}
+cudaError_t launch_pack_tree_bins(const uint8_t* bins_fm, uint32_t n, const uint32_t* feature_of,
+                                  uint32_t features, uint32_t nfb, uint32_t trees, uint8_t* out, cudaStream_t s) {
+  if (nfb > 65535) return cudaErrorInvalidValue;
+  for (uint32_t t0 = 0; t0 < trees; t0 += 65535) {
+    const uint32_t nt = std::min(65535u, trees - t0);
+    pack_tree_bins_kernel<<<dim3((n + 511) / 512, nfb, nt), 128, 0, s>>>(
+        bins_fm, n, feature_of + size_t(t0) * features, features, nfb, out + size_t(t0) * n * nfb * 32);
+  }
   return cudaGetLastError();
 }
 cudaError_t launch_label_counts(const double* labels, uint64_t n, uint32_t classes, unsigned long long* counts,

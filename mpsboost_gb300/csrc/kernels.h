@@ -16,6 +16,7 @@ struct TrainerDev {
   const uint8_t* bins;          // u8 bins for histograms: row r, feature f at
                                 //   r * bins_row_stride + (f/32) * bins_block_stride + f%32
   uint64_t bins_row_stride, bins_block_stride;
+  uint64_t bins_tree_stride;    // bytes between the trees' bins (0: all trees read the same)
   const uint8_t* bins_fm;       // [features][n_rows] feature-major u8 bins (routing rows)
   const uint32_t* bin_count;    // [features]
   const uint8_t* has_missing;   // [features]
@@ -32,7 +33,8 @@ struct TrainerDev {
   const double* weights;        // [n_rows], [n_trees][n_rows] or null (unit weights)
   uint32_t weights_per_tree;
   uint32_t objective;
-  double* preds;                // [n_trees][n_rows]
+  double* preds;                // [n_trees][n_rows]; null: every row's is tree_base[tree]
+  const double* tree_base;      // [n_trees] (single-round forest trees)
   float2* gh;                   // gh_ordered: [n_trees][2][seg_stride] in row-segment order
                                 // (moved along by the partition); else [n_trees][n_rows]
   uint32_t gh_ordered;
@@ -45,6 +47,10 @@ struct TrainerDev {
   const uint32_t* sample_rows;
   const uint32_t* sample_count;   // [n_trees]
   const uint32_t* feature_rank;   // [n_trees][features] or null (rank = feature)
+  // Compact forests: a tree's features are numbered within its own ascending subset
+  // (`features` is the largest subset; bins, histograms, masks and splits count that way)
+  // and feature_of [n_trees][features] names the dataset's. Null: the dataset's numbers.
+  const uint32_t* feature_of;
   const uint32_t* tree_seeds;     // [n_trees] or null (params.random_seed)
   uint32_t skip_apply;            // 1: no prediction update (forest trees are single-round)
   uint32_t unit_hess;             // every row's hessian is 1 (no weights; squared error or
@@ -203,6 +209,15 @@ uint32_t partition_kernels(const TrainerDev& a, uint32_t max_nodes);  // launche
 cudaError_t launch_partition_count(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_partition_finish(const TrainerDev& a, int grid, cudaStream_t stream);
 cudaError_t launch_apply_leaves(const TrainerDev& a, int grid, cudaStream_t stream);
+// Row samples of forest trees from their row multiplicities (counts [trees][n]) into sample
+// [trees][cap]; chunk_sum: scratch, [trees][ceil(n / kExpandChunk)].
+constexpr uint32_t kExpandChunk = 4096;
+cudaError_t launch_expand_samples(const uint8_t* counts, uint32_t n, uint32_t trees, uint32_t* chunk_sum,
+                                  uint32_t cap, uint32_t* sample, cudaStream_t stream);
+// Each tree's own features as rows [trees][n][nfb * 32] (feature_of: TrainerDev).
+cudaError_t launch_pack_tree_bins(const uint8_t* bins_fm, uint32_t n, const uint32_t* feature_of,
+                                  uint32_t features, uint32_t nfb, uint32_t trees, uint8_t* out,
+                                  cudaStream_t stream);
 // counts [classes + 1], zeroed by the caller: rows per class id, then rows of no class.
 constexpr uint32_t kLabelCountMax = 8192;  // classes (32 KB of shared counters)
 cudaError_t launch_label_counts(const double* labels, uint64_t n, uint32_t classes, unsigned long long* counts,

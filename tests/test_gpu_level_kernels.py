@@ -12,6 +12,7 @@ import pytest
 import mpsboost_gb300 as mb
 import oracle
 from conftest import seeded_matrix
+from test_gpu_forest import _oracle_tree
 
 pytestmark = pytest.mark.gpu
 
@@ -105,3 +106,33 @@ def test_class_counts_give_the_base_scores(backend, rows, classes):
             mb.train_regressor(backend, binned, y, objective="binary_logistic", **params)
         else:
             mb.train_softmax(backend, binned, y, classes, **params)
+
+
+# Forest trees on copies of their own features: subsets around a 32-feature block and the
+# half of the dataset's 70 from which the copy is made, ragged between trees; rows around
+# an expansion chunk's 4,096 and the pack's words; rows drawn 0, many and 255 times; random
+# thresholds and monotone constraints count the tree's and the dataset's features.
+@pytest.mark.parametrize("rows", [4095, 4097, 8192])
+@pytest.mark.parametrize("subset,extra", [(1, {}), (31, {}), (33, dict(split_strategy="random_threshold")),
+                                          (35, dict(monotonic_constraints=[1, 0, -1, 0, 0] * 14)), (36, {})])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_compact_forest_equals_replica(backend, port, rows, subset, extra, weighted):
+    x = seeded_matrix(rows + subset, rows, 70, 0.05, integer_columns=9)
+    y, w = targets(x, subset)
+    w = w if weighted else None
+    rng = np.random.default_rng(subset)
+    counts = rng.poisson(0.8, (3, rows)).astype(np.uint8)
+    counts[0, 5], counts[1, :2000] = 255, 0
+    subsets = [rng.choice(70, max(1, subset - 2 * t), replace=False) for t in range(3)]
+    seeds = np.arange(3, dtype=np.uint32)
+    params = dict(max_depth=5, min_samples_leaf=3, **extra)
+    binned = mb.quantize_dense(x, 64)
+    models = mb.train_forest(backend, binned, y, w, row_counts=counts, feature_subsets=subsets, seeds=seeds, **params)
+    ds = port.quantize_dense(x, 64)
+    for t, m in enumerate(models):
+        p = dict(params)
+        if "monotonic_constraints" in p:
+            p["monotonic_constraints"] = [p["monotonic_constraints"][f] for f in np.sort(subsets[t])]
+        base, nodes = _oracle_tree(port, ds, y, w, counts[t], subsets[t], p, seeds[t])
+        assert float(m.base_score).hex() == float(base).hex()
+        assert m.trees[0].tobytes() == nodes.tobytes()
