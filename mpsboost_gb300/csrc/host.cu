@@ -1909,6 +1909,54 @@ int mpsb_cuda_model_train_predictions(const mpsb_cuda_model* m, double* out) {
 
 namespace {
 
+// The trees in launch_predict_packed's node format; false where one does not fit it: too
+// many nodes or features, or a child that does not follow its parent (the general kernel
+// then walks the trees and reports a bad index or a cycle where a row meets it).
+struct HostForest {
+  std::vector<uint2> nodes;
+  std::vector<double> steps;
+  std::vector<uint4> trees;
+  std::vector<uint32_t> groups;
+};
+
+bool pack_forest(const std::vector<const std::vector<mpsb_tree_node>*>& trees, double lr,
+                 const mpsb_cuda_dataset* ds, HostForest& f) {
+  if (ds->features >= 32768) return false;
+  f.groups.push_back(0);
+  std::vector<uint32_t> ref;
+  for (size_t t = 0; t < trees.size(); ++t) {
+    const std::vector<mpsb_tree_node>& tree = *trees[t];
+    uint32_t inner = 0, leaves = 0;
+    ref.resize(tree.size());
+    for (size_t i = 0; i < tree.size(); ++i) ref[i] = (tree[i].flags & 1u) ? kPackedLeaf | leaves++ : inner++;
+    if (tree.empty() || inner > kPredictNodes || leaves > kPredictLeaves) return false;
+    const uint4 at = make_uint4(uint32_t(f.nodes.size()), uint32_t(f.steps.size()), ref[0], 0);
+    if (at.x + inner - (f.trees.empty() ? 0 : f.trees[f.groups.back()].x) > kPredictNodes ||
+        at.y + leaves - (f.trees.empty() ? 0 : f.trees[f.groups.back()].y) > kPredictLeaves)
+      f.groups.push_back(uint32_t(t));
+    f.trees.push_back(at);
+    for (size_t i = 0; i < tree.size(); ++i) {
+      const mpsb_tree_node& nd = tree[i];
+      if (nd.flags & 1u) {
+        f.steps.push_back(lr * nd.leaf_value);
+        continue;
+      }
+      if (nd.left_child <= i || nd.right_child <= i || nd.left_child >= tree.size() ||
+          nd.right_child >= tree.size() || nd.threshold_bin > 0xFFFFu)
+        return false;
+      const uint32_t missing_left = ds->h_has_missing[nd.feature_index] && nd.default_left ? 1u : 0u;
+      // A missing row's bin is above every threshold but the largest bin's, and goes by the
+      // node's direction there too.
+      if (ds->h_has_missing[nd.feature_index] && nd.threshold_bin >= ds->slots - 1) return false;
+      f.nodes.push_back(make_uint2(nd.feature_index << 17 | missing_left << 16 | nd.threshold_bin,
+                                   ref[nd.left_child] | ref[nd.right_child] << 16));
+    }
+  }
+  f.groups.push_back(uint32_t(trees.size()));
+  f.trees.push_back(make_uint4(uint32_t(f.nodes.size()), uint32_t(f.steps.size()), 0, 0));
+  return true;
+}
+
 // base + lr * sum of the given trees' leaves for every row, on the device.
 void predict_trees(mpsb_cuda_backend* b, const std::vector<const std::vector<mpsb_tree_node>*>& trees,
                    double base, double lr, const mpsb_cuda_dataset* ds, double* out) {
@@ -1919,6 +1967,34 @@ void predict_trees(mpsb_cuda_backend* b, const std::vector<const std::vector<mps
     for (const mpsb_tree_node& nd : *trees[t])
       if (!(nd.flags & 1u) && nd.feature_index >= ds->features)
         throw TrainingError("Prediction feature count does not match the tree model");
+  }
+  HostForest packed;
+  if (!trees.empty() && predict_rows(ds->n_rows, ds->features, ds->slots == uint32_t(kSlots) ? 1 : 2) != 0 &&
+      pack_forest(trees, lr, ds, packed)) {
+    // One upload and one buffer: nodes, leaf steps, tree and group tables, predictions.
+    const size_t nb = packed.nodes.size() * sizeof(uint2), sb = packed.steps.size() * sizeof(double),
+                 tb = packed.trees.size() * sizeof(uint4), gb = packed.groups.size() * sizeof(uint32_t);
+    const size_t at_s = (nb + 15) / 16 * 16, at_t = (at_s + sb + 15) / 16 * 16, at_g = at_t + tb,
+                 at_out = (at_g + gb + 15) / 16 * 16;
+    std::vector<unsigned char> host(at_out);
+    std::memcpy(host.data(), packed.nodes.data(), nb);
+    std::memcpy(host.data() + at_s, packed.steps.data(), sb);
+    std::memcpy(host.data() + at_t, packed.trees.data(), tb);
+    std::memcpy(host.data() + at_g, packed.groups.data(), gb);
+    DevBuf buf;
+    buf.alloc(at_out + size_t(ds->n_rows) * sizeof(double));
+    unsigned char* p = buf.as<unsigned char>();
+    double* d_out = reinterpret_cast<double*>(p + at_out);
+    cudaStream_t s = b->stream;
+    CK(cudaMemcpyAsync(p, host.data(), at_out, cudaMemcpyHostToDevice, s));
+    const PackedForest f{reinterpret_cast<const uint2*>(p), reinterpret_cast<const double*>(p + at_s),
+                         reinterpret_cast<const uint4*>(p + at_t), reinterpret_cast<const uint32_t*>(p + at_g),
+                         uint32_t(packed.groups.size() - 1)};
+    CK(launch_predict_packed(ds->bins_fm.as<uint8_t>(), ds->bins16_fm.as<uint16_t>(), ds->slots, ds->n_rows,
+                             ds->features, f, base, d_out, s));
+    CK(cudaMemcpyAsync(out, d_out, size_t(ds->n_rows) * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return;
   }
   std::vector<mpsb_tree_node> flat(offsets.back() ? offsets.back() : 1);
   for (size_t t = 0; t < trees.size(); ++t)

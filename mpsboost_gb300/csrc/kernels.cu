@@ -3401,6 +3401,59 @@ __global__ void predict_kernel(const BinT* bins_fm, uint32_t missing_slot, uint3
   if (bad) atomicOr(error, kErrCapacity);
 }
 
+// The same traversal from shared memory, for trees that fit its node format (PackedForest).
+// A CTA stages the bins of its rows ([feature][row], one row per thread) and walks the
+// trees in groups whose nodes and leaf steps it stages too, so a node visit is two
+// shared-memory loads where the general kernel above loads a 40-byte node and gathers a
+// byte from a 32-byte sector of the feature-major matrix. Bound by shared-memory load
+// latency and bank conflicts between lanes at different nodes.
+template <typename BinT>
+__global__ void __launch_bounds__(1024) predict_packed_kernel(const BinT* bins_fm, uint32_t missing_slot,
+                                                              uint32_t n_rows, uint32_t features,
+                                                              PackedForest f, double base, double* out) {
+  extern __shared__ __align__(16) unsigned char predict_smem[];
+  const uint32_t rows = blockDim.x;
+  const uint32_t pitch = predict_pitch<BinT>(rows);
+  double* s_steps = reinterpret_cast<double*>(predict_smem);                       // [kPredictLeaves]
+  uint2* s_nodes = reinterpret_cast<uint2*>(s_steps + kPredictLeaves);             // [kPredictNodes]
+  BinT* s_bins = reinterpret_cast<BinT*>(s_nodes + kPredictNodes);                 // [features][pitch]
+  const uint32_t row0 = blockIdx.x * rows, row = row0 + threadIdx.x;
+  if (size_t(n_rows) * sizeof(BinT) % 4 == 0 && row0 + rows <= n_rows) {  // whole words (rows is a multiple of 128)
+    const uint32_t words = rows * uint32_t(sizeof(BinT)) / 4, pitch4 = pitch * uint32_t(sizeof(BinT)) / 4;
+    const uint32_t per = rows / words;  // features per pass
+    const uint32_t w = threadIdx.x % words;
+    for (uint32_t c = threadIdx.x / words; c < features; c += per)
+      reinterpret_cast<uint32_t*>(s_bins)[size_t(c) * pitch4 + w] =
+          __ldg(reinterpret_cast<const uint32_t*>(bins_fm + size_t(c) * n_rows + row0) + w);
+  } else {
+    for (uint32_t c = 0; c < features; ++c)
+      s_bins[size_t(c) * pitch + threadIdx.x] = row < n_rows ? bins_fm[size_t(c) * n_rows + row] : BinT(0);
+  }
+  const BinT* mine = s_bins + threadIdx.x;
+  double acc = base;
+  for (uint32_t g = 0; g < f.n_groups; ++g) {
+    const uint32_t t0 = f.group_first[g], t1 = f.group_first[g + 1];
+    const uint4 first = f.trees[t0], end = f.trees[t1];  // {first node, first leaf, root, 0}
+    __syncthreads();  // the group before is done (and the bins are staged)
+    for (uint32_t i = threadIdx.x; i < end.x - first.x; i += rows) s_nodes[i] = f.nodes[first.x + i];
+    for (uint32_t i = threadIdx.x; i < end.y - first.y; i += rows) s_steps[i] = f.steps[first.y + i];
+    __syncthreads();
+    for (uint32_t t = t0; t < t1; ++t) {
+      const uint4 tree = f.trees[t];
+      const uint2* nodes = s_nodes + (tree.x - first.x);
+      uint32_t ref = tree.z;
+      while (!(ref & kPackedLeaf)) {  // children follow their parents
+        const uint2 nd = nodes[ref];
+        const uint32_t b = mine[size_t(nd.x >> 17) * pitch];
+        const bool left = b <= (nd.x & 0xFFFFu) || ((nd.x & 0x10000u) && b == missing_slot);
+        ref = left ? nd.y & 0xFFFFu : nd.y >> 16;
+      }
+      acc = __dadd_rn(acc, s_steps[tree.y - first.y + (ref & ~kPackedLeaf)]);
+    }
+  }
+  if (row < n_rows) out[row] = acc;
+}
+
 // Feature-major [features][rows] bins (u8 or u16) + optional missing mask -> three u8
 // layouts with missing rows at 255: rows padded to nfb * 32 bytes and column blocks
 // [nfb][rows][32] (histograms of sparse and dense levels), and a feature-major copy (row
@@ -3813,6 +3866,26 @@ cudaError_t launch_pack_bins16_block(const void* src_block, uint32_t width,
   pack_bins16_kernel<<<gx > 0 ? gx : 1, 256, 0, s>>>(src_block, width, missing_block, bin_count, n_rows,
                                                      features, fb, slots, out_blocked, out_fm, error);
   return cudaGetLastError();
+}
+template <typename BinT>
+static cudaError_t launch_predict_tile(const BinT* bins_fm, uint32_t missing_slot, uint32_t n_rows,
+                                       uint32_t features, const PackedForest& f, double base, double* out,
+                                       cudaStream_t s) {
+  const uint32_t rows = predict_rows(n_rows, features, sizeof(BinT));
+  if (rows == 0) return cudaErrorInvalidValue;
+  static std::atomic<unsigned long long> configured{0};  // one bit per device
+  const cudaError_t err = opt_in_dynamic_smem(configured, predict_packed_kernel<BinT>, kPredictSmemMax);
+  if (err != cudaSuccess) return err;
+  const size_t smem = kPredictTreeBytes + size_t(features) * predict_pitch<BinT>(rows) * sizeof(BinT);
+  predict_packed_kernel<BinT><<<(n_rows + rows - 1) / rows, rows, smem, s>>>(bins_fm, missing_slot, n_rows, features,
+                                                                            f, base, out);
+  return cudaGetLastError();
+}
+cudaError_t launch_predict_packed(const uint8_t* bins_fm, const uint16_t* bins16_fm, uint32_t slots,
+                                  uint32_t n_rows, uint32_t features, const PackedForest& f, double base,
+                                  double* out, cudaStream_t s) {
+  if (bins16_fm) return launch_predict_tile<uint16_t>(bins16_fm, slots - 1, n_rows, features, f, base, out, s);
+  return launch_predict_tile<uint8_t>(bins_fm, uint32_t(kMissingSlot), n_rows, features, f, base, out, s);
 }
 cudaError_t launch_predict(const uint8_t* bins_fm, const uint16_t* bins16_fm, uint32_t slots,
                            uint32_t n_rows, uint32_t nfb, const uint8_t* has_missing,

@@ -231,6 +231,38 @@ cudaError_t launch_predict(const uint8_t* bins_fm, const uint16_t* bins16_fm, ui
                            const TreeNodeOut* nodes, const uint32_t* tree_offsets,
                            uint32_t n_trees, double base, double learning_rate, double* out,
                            uint32_t* error, cudaStream_t stream);
+// Trees in the packed node format: 8 bytes per inner node, {feature << 17 | missing goes left
+// << 16 | threshold, left | right << 16}, a child reference being a node number in its tree
+// or kPackedLeaf | leaf number (16 bits: at most 32,768 of either, features below 32,768);
+// leaf steps lr x value; trees[t] = {first node, first leaf, root reference, 0} with one
+// more entry after the last; groups of trees whose nodes and leaves fit the staging.
+struct PackedForest {
+  const uint2* nodes;
+  const double* steps;
+  const uint4* trees;
+  const uint32_t* group_first;  // [n_groups + 1]
+  uint32_t n_groups;
+};
+constexpr uint32_t kPackedLeaf = 0x8000u;
+constexpr uint32_t kPredictNodes = 4096, kPredictLeaves = 4096;  // staged at a time: 64 KB
+constexpr size_t kPredictTreeBytes = size_t(kPredictNodes) * 8 + size_t(kPredictLeaves) * 8;
+constexpr size_t kPredictSmemMax = 227 * 1024;
+// Elements between two features' staged rows: a word more than the rows, so that lanes at
+// different features of neighbouring rows spread over the banks.
+template <typename BinT>
+constexpr __host__ __device__ uint32_t predict_pitch(uint32_t rows) { return rows + uint32_t(4 / sizeof(BinT)); }
+// Rows (threads) per CTA: as many as the staging takes, fewer where that leaves SMs idle
+// (128 at least; 0: the features' bins do not fit).
+inline uint32_t predict_rows(uint32_t n_rows, uint32_t features, size_t bin_bytes) {
+  uint32_t rows = 1024;
+  while (rows > 128 && (uint64_t(n_rows) < uint64_t(rows) * 152 ||
+                        kPredictTreeBytes + uint64_t(features) * (rows * bin_bytes + 4) > kPredictSmemMax))
+    rows >>= 1;
+  return kPredictTreeBytes + uint64_t(features) * (rows * bin_bytes + 4) <= kPredictSmemMax ? rows : 0u;
+}
+cudaError_t launch_predict_packed(const uint8_t* bins_fm, const uint16_t* bins16_fm, uint32_t slots,
+                                  uint32_t n_rows, uint32_t features, const PackedForest& f, double base,
+                                  double* out, cudaStream_t stream);
 // Wide datasets: one feature block fb of the u16 copies ([nfb][n_rows][32] column blocks
 // and [features][n_rows]) from a staged copy of its source features, missing rows at
 // slots - 1.

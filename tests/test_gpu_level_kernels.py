@@ -136,3 +136,65 @@ def test_compact_forest_equals_replica(backend, port, rows, subset, extra, weigh
         base, nodes = _oracle_tree(port, ds, y, w, counts[t], subsets[t], p, seeds[t])
         assert float(m.base_score).hex() == float(base).hex()
         assert m.trees[0].tobytes() == nodes.tobytes()
+
+
+def _traverse(trees, lr, base, bins, missing):
+    """Predictions tree by tree in FP64, as RegressionModel::Predict adds them."""
+    out = np.full(bins.shape[1], base)
+    rows = np.arange(bins.shape[1])
+    for t in trees:
+        at = np.zeros(rows.size, np.int64)
+        for _ in range(t.size):
+            f = t["feature_index"][at]
+            left = np.where(missing[f, rows], t["default_left"][at] != 0, bins[f, rows] <= t["threshold_bin"][at])
+            step = np.where(left, t["left_child"][at], t["right_child"][at]).astype(np.int64)
+            leaf = (t["flags"][at] & 1) != 0
+            if leaf.all():
+                break
+            at = np.where(leaf, at, step)
+        out = out + lr * t["leaf_value"][at]
+    return out
+
+
+def _grown(rng, features, bins, splits, shuffle):
+    """A tree grown by splitting a random leaf at a time; shuffled, children may precede
+    their parents."""
+    n = 2 * splits + 1
+    t = np.zeros(n, mb._lib.NODE_DTYPE)
+    t["flags"] = 1
+    t["leaf_value"] = rng.normal(size=n)
+    leaves, used = [0], 1
+    for _ in range(splits):
+        at = leaves.pop(rng.integers(len(leaves)))
+        t["flags"][at] = 0
+        t["feature_index"][at], t["threshold_bin"][at] = rng.integers(features), rng.integers(bins)
+        t["default_left"][at] = rng.integers(2)
+        t["left_child"][at], t["right_child"][at] = used, used + 1
+        leaves += [used, used + 1]
+        used += 2
+    if shuffle:
+        order = np.concatenate([[0], 1 + rng.permutation(n - 1)])  # new index of each node
+        u = np.empty_like(t)
+        u[order] = t
+        inner = (u["flags"] & 1) == 0
+        u["left_child"][inner], u["right_child"][inner] = order[u["left_child"][inner]], order[u["right_child"][inner]]
+        t = u
+    return t
+
+
+# Rows around a CTA's 128 and the staged words, features up to and past the staging, trees
+# of one leaf, of groups' size (4,096 nodes) and past it, u8 and u16 bins, missing rows; and
+# a tree whose children precede their parents, which the general kernel walks.
+@pytest.mark.parametrize("rows,features,bins,nan,splits,shuffle", [
+    (1, 1, 4, 0.0, [0, 1], False), (127, 5, 64, 0.2, [3, 0, 40], False), (129, 33, 255, 0.1, [63] * 70, False),
+    (1000, 64, 255, 0.1, [200] * 9, False), (2050, 12, 256, 0.1, [50] * 5, False),
+    (3001, 7, 900, 0.1, [500, 30], False), (400, 6, 128, 0.1, [4095, 10, 4096 - 10], False),
+    (400, 6, 128, 0.1, [4097], False), (300, 1300, 32, 0.0, [60], False), (500, 8, 64, 0.1, [30, 31], True),
+])
+def test_predict_edges(backend, rows, features, bins, nan, splits, shuffle):
+    rng = np.random.default_rng(rows)
+    binned = mb.quantize_dense(seeded_matrix(rows, max(rows, 2), features, nan), bins)
+    trees = [_grown(rng, features, max(2, bins - 2), s, shuffle) for s in splits]
+    model = mb.RegressionModel(0.25, 0.1, trees)
+    got = model.predict(backend, binned)
+    assert got.tobytes() == _traverse(trees, 0.1, 0.25, binned.bins, binned.missing).tobytes()
