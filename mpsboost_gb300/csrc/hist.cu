@@ -596,6 +596,7 @@ __device__ __forceinline__ void flush_cta_histogram_bulk(const TrainerDev& a, co
 // so the break-even is one failure in three to five; a block with a heavy cell (a feature
 // of few bins, many missing rows) fails its first items and stays on split limbs.
 constexpr uint32_t kPackFailCost = 8;
+constexpr uint32_t kWidePasses = kWideVotePasses;  // passes of a wide block, at most (8 features each)
 
 // A work item's description, prepared one item ahead by one warp.
 struct ItemDesc {
@@ -637,9 +638,13 @@ __device__ __forceinline__ void fetch_item_warp(const TrainerDev& a, uint32_t la
     d.kh = a.trees[d.e.tree].kh;
     d.single = a.store_single && a.build_prefix[lo + 1] - a.build_prefix[lo] == 1;
     if (a.limb_votes) {
-      const volatile uint32_t* votes = a.limb_votes + 2 * d.fb;  // other CTAs add to them
-      const uint32_t passed = votes[0], failed = votes[1];
-      d.packed = failed * kPackFailCost <= passed + 2 * kPackFailCost;
+      // Other CTAs add to the votes. A wide block's passes vote apart, a bit each.
+      const uint32_t passes = a.slots == uint32_t(kSlots) ? 1u : kWidePasses;
+      const volatile uint32_t* votes = a.limb_votes + size_t(2) * passes * d.fb;
+      for (uint32_t p = 0; p < passes; ++p) {
+        const uint32_t passed = votes[2 * p], failed = votes[2 * p + 1];
+        if (failed * kPackFailCost <= passed + 2 * kPackFailCost) d.packed |= 1u << p;
+      }
     }
   }
   if (lane == 0) *out = d;
@@ -918,10 +923,51 @@ namespace {
 // straight into the slot with 64-bit global atomics.
 constexpr uint32_t kWideBatch = 4;  // gathered words in flight per lane
 constexpr size_t kWideSmemBytes = 200 * 1024;  // the CTA histogram's limbs
-// Fixed-point flushes go through TMA bulk reductions of 8 cells of one feature (192
-// bytes), staged by kWideFlushWarps warps in rows after the histogram.
-constexpr int kWideFlushWarps = 4;
-constexpr size_t kWideStagingBytes = size_t(kWideFlushWarps) * 32 * kFlushRowWords * 8;
+constexpr size_t kSmemMax = 227 * 1024;
+// Fixed-point flushes go through TMA bulk reductions of 4 cells of one feature (96 bytes),
+// staged in rows after the histogram by as many warps as the shared memory has room for
+// (8-cell rows left 4 of 24 warps converting and storing while the others waited: 16 us a
+// pass of 16 features x 1,024 slots).
+constexpr int kWideFlushBins = 4;
+constexpr int kWideRowWords = kWideFlushBins * 3 + 2;  // padded: 16-byte aligned, conflict-free stores
+constexpr size_t kWideTileBytes = size_t(32) * kWideRowWords * 8;
+constexpr size_t kWideTail = 1024;  // kept at the end for the register-direct kernel
+
+// Adds the CTA histogram's cells ([slot][group], converted by cell(idx, count, g, h)) of gw
+// features into their slots at dst (feature-major). Every thread of the CTA; the staging
+// rows are free again when it returns.
+template <int THREADS, class Cell>
+__device__ __forceinline__ void wide_flush(uint32_t* wsm, size_t cell_bytes, uint32_t S, uint32_t group, uint32_t gw,
+                                           unsigned long long* dst, Cell&& cell) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t warps = min(uint32_t(THREADS / 32), uint32_t((kSmemMax - kWideTail - cell_bytes) / kWideTileBytes));
+  if (warp >= warps) return;
+  // Lane (bin group bg, feature fl) of a warp's tile: consecutive bins of its feature.
+  unsigned long long* row = reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(wsm) + cell_bytes) +
+                            (size_t(warp) * 32 + lane) * kWideRowWords;
+  const uint32_t row_addr = static_cast<uint32_t>(__cvta_generic_to_shared(row));
+  const uint32_t per_tile = 32u / group;  // bin groups per tile (group divides 32)
+  const uint32_t fl = lane % group, bg = lane / group;
+  for (uint32_t g0 = warp * per_tile; g0 < S / kWideFlushBins; g0 += warps * per_tile) {
+    const uint32_t b0 = (g0 + bg) * kWideFlushBins;  // S / 4 is a multiple of 64
+    unsigned long long out[kWideFlushBins * 3], any = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kWideFlushBins; ++j) {
+      cell((b0 + j) * group + fl, out[3 * j], out[3 * j + 1], out[3 * j + 2]);
+      any |= out[3 * j] | out[3 * j + 1] | out[3 * j + 2];
+    }
+    if (fl < gw && any != 0ull) {
+      bulk_wait_read();  // the row's previous bulk reduction has read it
+      ulonglong2* row2 = reinterpret_cast<ulonglong2*>(row);
+#pragma unroll
+      for (int q = 0; q < kWideFlushBins * 3 / 2; ++q) row2[q] = make_ulonglong2(out[2 * q], out[2 * q + 1]);
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the row's stores before the bulk read
+      bulk_reduce_add_u64(dst + (size_t(fl) * S + b0) * 3, row_addr, kWideFlushBins * 3 * 8);
+      bulk_commit();
+    }
+  }
+  bulk_wait_read();
+}
 
 template <int MODE>
 __host__ __device__ constexpr int wide_words() {  // 32-bit limbs per cell
@@ -930,7 +976,7 @@ __host__ __device__ constexpr int wide_words() {  // 32-bit limbs per cell
 
 // Features per shared-memory pass: the largest power of two <= 32 whose cells fit (0: none).
 template <int MODE>
-uint32_t wide_group(uint32_t slots) {
+__host__ __device__ uint32_t wide_group(uint32_t slots) {
   const size_t fit = kWideSmemBytes / (size_t(slots) * wide_words<MODE>() * sizeof(uint32_t));
   uint32_t g = kBlockFeatures;
   while (g > fit) g >>= 1;
@@ -943,15 +989,18 @@ __device__ __forceinline__ uint32_t ld_nc_u32(const void* p) {
   return v;
 }
 
+// A work item's rows for features [f_begin, f_end) of its block in split limbs, `group`
+// features per shared-memory pass, added to the node's slot. Every thread of the CTA.
 template <int MODE, int THREADS>
-__global__ void __launch_bounds__(THREADS) hist_build_wide_kernel(TrainerDev a, uint32_t group) {
+__device__ __noinline__ void wide_split_passes(const TrainerDev& a, const BuildEntry& e, uint32_t fb,
+                                               uint32_t row_begin, uint32_t row_count, int kg, int kh,
+                                               uint32_t group, uint32_t f_begin, uint32_t f_end,
+                                               uint32_t* wsm) {
   constexpr int WORDS = wide_words<MODE>();
   constexpr int WARPS = THREADS / 32;
-  extern __shared__ __align__(16) uint32_t wsm[];  // [WORDS][slots][group], then the staging rows
-  __shared__ uint32_t s_item, s_entry;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const uint32_t n = a.n_rows, nfb = a.nfb, S = a.slots;
+  const uint32_t n = a.n_rows, S = a.slots;
   const uint32_t cells = S * group;
   const uint32_t L = group >= 2 ? group / 2 : 1u;  // lanes per row
   const uint32_t R = 32u / L;                      // rows per step
@@ -959,44 +1008,18 @@ __global__ void __launch_bounds__(THREADS) hist_build_wide_kernel(TrainerDev a, 
   const uint32_t w = uint32_t(lane) % L;           // the lane's word of a row's group
   const uint32_t hist_base = static_cast<uint32_t>(__cvta_generic_to_shared(wsm));
   const uint32_t plane = cells * 4u;               // bytes per limb plane
-  for (;;) {
-    const uint32_t limit = a.item_end ? a.item_end : a.ctl->hist_items;
-    if (tid == 0) {
-      const uint32_t item = a.item_begin + atomicAdd(&a.ctl->hist_counter, 1u);
-      s_item = item;
-      if (item < limit) {
-        const uint32_t chunk = item / nfb;
-        uint32_t lo = 0, hi = a.ctl->n_build;  // last entry with prefix <= chunk
-        while (hi - lo > 1) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (a.build_prefix[mid] <= chunk) lo = mid; else hi = mid;
-        }
-        s_entry = lo;
-      }
-    }
-    __syncthreads();
-    const uint32_t item = s_item;
-    if (item >= limit) break;
-    const uint32_t fb = item % nfb;
-    const uint32_t chunk = item / nfb;
-    const BuildEntry e = a.build[s_entry];
-    const uint32_t item_rows = a.item_rows ? a.item_rows : a.ctl->item_rows;
-    const uint32_t row_begin = (chunk - a.build_prefix[s_entry]) * item_rows;
-    const uint32_t row_count = row_begin < e.seg_cnt ? min(item_rows, e.seg_cnt - row_begin) : 0u;
-    const size_t seg = (size_t(e.tree) * 2 + e.parity) * a.seg_stride + e.seg_off + row_begin;
-    const uint32_t* rows = a.rows + seg;
-    const float2* gh_seg = a.gh_ordered ? a.gh + seg : nullptr;
-    const float2* gh_row = a.gh_ordered ? nullptr : a.gh + size_t(e.tree) * n;
-    const uint16_t* bins = a.bins16 + size_t(fb) * n * kBlockFeatures;
-    const int kg = a.trees[e.tree].kg;
-    const int kh = a.trees[e.tree].kh;
-    const long long q_unit_h = MODE == kModeFixedCG ? quantize_f32(1.0f, kh) : 0ll;
-    const uint32_t width = min(uint32_t(kBlockFeatures), a.features - fb * kBlockFeatures);
-    unsigned long long* dst_base = a.hist + (size_t(e.slot) * a.features + size_t(fb) * kBlockFeatures) * S * 3;
-    const uint32_t ntiles = (row_count + 31u) / 32u;
-    const uint32_t step = group ? group : width;
-    for (uint32_t f0 = 0; f0 < width; f0 += step) {
-      const uint32_t gw = min(step, width - f0);
+  const size_t seg = (size_t(e.tree) * 2 + e.parity) * a.seg_stride + e.seg_off + row_begin;
+  const uint32_t* rows = a.rows + seg;
+  const float2* gh_seg = a.gh_ordered ? a.gh + seg : nullptr;
+  const float2* gh_row = a.gh_ordered ? nullptr : a.gh + size_t(e.tree) * n;
+  const uint16_t* bins = a.bins16 + size_t(fb) * n * kBlockFeatures;
+  const long long q_unit_h = MODE == kModeFixedCG ? quantize_f32(1.0f, kh) : 0ll;
+  unsigned long long* dst_base = a.hist + (size_t(e.slot) * a.features + size_t(fb) * kBlockFeatures) * S * 3;
+  const uint32_t ntiles = (row_count + 31u) / 32u;
+  const uint32_t step = group ? group : f_end - f_begin;
+  {
+    for (uint32_t f0 = f_begin; f0 < f_end; f0 += step) {
+      const uint32_t gw = min(step, f_end - f0);
       if (group) {
         uint4* z = reinterpret_cast<uint4*>(wsm);
         for (uint32_t i = tid; i < uint32_t(WORDS) * cells / 4u; i += THREADS) z[i] = make_uint4(0, 0, 0, 0);
@@ -1120,51 +1143,67 @@ __global__ void __launch_bounds__(THREADS) hist_build_wide_kernel(TrainerDev a, 
             atomicAdd(reinterpret_cast<double*>(dst + 1), double(__uint_as_float(wsm[cells + idx])));
             atomicAdd(reinterpret_cast<double*>(dst + 2), double(__uint_as_float(wsm[2 * cells + idx])));
           }
-        } else if (warp < kWideFlushWarps) {
-          // Lane (bin group bg, feature fl) of a warp's tile converts 8 consecutive bins of
-          // its feature into the slot's 24 words and hands them to one bulk reduction.
-          unsigned long long* row = reinterpret_cast<unsigned long long*>(
-              reinterpret_cast<unsigned char*>(wsm) + size_t(WORDS) * cells * 4) + (size_t(warp) * 32 + lane) * kFlushRowWords;
-          const uint32_t row_addr = static_cast<uint32_t>(__cvta_generic_to_shared(row));
-          const uint32_t per_tile = 32u / group;  // bin groups per tile (group divides 32)
-          const uint32_t fl = uint32_t(lane) % group, bg = uint32_t(lane) / group;
-          for (uint32_t g0 = uint32_t(warp) * per_tile; g0 < S / kFlushBins; g0 += kWideFlushWarps * per_tile) {
-            const uint32_t b0 = (g0 + bg) * kFlushBins;  // S / 8 is a multiple of 32
-            bulk_wait_read();  // the row's previous bulk reduction has read it
-            unsigned long long any = 0;
-#pragma unroll
-            for (uint32_t j = 0; j < kFlushBins; ++j) {
-              const uint32_t idx = (b0 + j) * group + fl;
-              unsigned long long c, g, h;
-              if constexpr (MODE == kModeFixed) {
-                c = wsm[idx];
-                g = (unsigned long long)((long long)int32_t(wsm[2 * cells + idx]) * 65536 + (long long)wsm[cells + idx]);
-                h = (unsigned long long)((long long)wsm[4 * cells + idx] * 65536 + (long long)wsm[3 * cells + idx]);
-              } else if constexpr (MODE == kModeFixedG) {
-                c = 0;  // the gradient-only root's count and hessian words are restored afterwards
-                g = (unsigned long long)((long long)int32_t(wsm[cells + idx]) * 65536 + (long long)wsm[idx]);
-                h = 0;
-              } else {
-                c = wsm[idx];
-                g = (unsigned long long)((long long)int32_t(wsm[2 * cells + idx]) * 65536 + (long long)wsm[cells + idx]);
-                h = (unsigned long long)((long long)c * q_unit_h);
-              }
-              row[3 * j + 0] = c;
-              row[3 * j + 1] = g;
-              row[3 * j + 2] = h;
-              any |= c | g | h;
-            }
-            if (fl < gw && any != 0ull) {
-              asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the row's stores before the bulk read
-              bulk_reduce_add_u64(dst_base + (size_t(f0 + fl) * S + b0) * 3, row_addr, kFlushBins * 3 * 8);
-              bulk_commit();
-            }
-          }
-          bulk_wait_read();  // the staging rows are free again
+        } else {
+          wide_flush<THREADS>(wsm, size_t(WORDS) * cells * 4, S, group, gw, dst_base + size_t(f0) * S * 3,
+                              [&](uint32_t idx, unsigned long long& c, unsigned long long& g, unsigned long long& h) {
+                                if constexpr (MODE == kModeFixed) {
+                                  c = wsm[idx];
+                                  g = (unsigned long long)((long long)int32_t(wsm[2 * cells + idx]) * 65536 +
+                                                           (long long)wsm[cells + idx]);
+                                  h = (unsigned long long)((long long)wsm[4 * cells + idx] * 65536 +
+                                                           (long long)wsm[3 * cells + idx]);
+                                } else if constexpr (MODE == kModeFixedG) {
+                                  c = 0;  // the gradient-only root's count and hessian words are restored
+                                  g = (unsigned long long)((long long)int32_t(wsm[cells + idx]) * 65536 +
+                                                           (long long)wsm[idx]);
+                                  h = 0;
+                                } else {
+                                  c = wsm[idx];
+                                  g = (unsigned long long)((long long)int32_t(wsm[2 * cells + idx]) * 65536 +
+                                                           (long long)wsm[cells + idx]);
+                                  h = (unsigned long long)((long long)c * q_unit_h);
+                                }
+                              });
         }
         __syncthreads();
       }
     }
+  }
+}
+
+template <int MODE, int THREADS>
+__global__ void __launch_bounds__(THREADS) hist_build_wide_kernel(const __grid_constant__ TrainerDev a, uint32_t group) {
+  extern __shared__ __align__(16) uint32_t wsm[];  // [limb][slots][group], then the staging rows
+  __shared__ uint32_t s_item, s_entry;
+  const int tid = threadIdx.x;
+  const uint32_t nfb = a.nfb;
+  for (;;) {
+    const uint32_t limit = a.item_end ? a.item_end : a.ctl->hist_items;
+    if (tid == 0) {
+      const uint32_t item = a.item_begin + atomicAdd(&a.ctl->hist_counter, 1u);
+      s_item = item;
+      if (item < limit) {
+        const uint32_t chunk = item / nfb;
+        uint32_t lo = 0, hi = a.ctl->n_build;  // last entry with prefix <= chunk
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (a.build_prefix[mid] <= chunk) lo = mid; else hi = mid;
+        }
+        s_entry = lo;
+      }
+    }
+    __syncthreads();
+    const uint32_t item = s_item;
+    if (item >= limit) break;
+    const uint32_t fb = item % nfb;
+    const uint32_t chunk = item / nfb;
+    const BuildEntry e = a.build[s_entry];
+    const uint32_t item_rows = a.item_rows ? a.item_rows : a.ctl->item_rows;
+    const uint32_t row_begin = (chunk - a.build_prefix[s_entry]) * item_rows;
+    const uint32_t row_count = row_begin < e.seg_cnt ? min(item_rows, e.seg_cnt - row_begin) : 0u;
+    const uint32_t width = min(uint32_t(kBlockFeatures), a.features - fb * kBlockFeatures);
+    wide_split_passes<MODE, THREADS>(a, e, fb, row_begin, row_count, a.trees[e.tree].kg, a.trees[e.tree].kh, group, 0,
+                                     width, wsm);
     if (tid == 0) {
       atomicAdd(&a.ctl->cells, (unsigned long long)row_count * width);
       if (fb == 0) atomicAdd(&a.ctl->rows_built, (unsigned long long)row_count);
@@ -1174,21 +1213,303 @@ __global__ void __launch_bounds__(THREADS) hist_build_wide_kernel(TrainerDev a, 
   bulk_wait_all();  // this thread's bulk reductions have reached the slots
 }
 
+// ---- Register-direct wide builds ---------------------------------------------------------
+// As hist_build_direct_kernel: a lane owns a row and loads the GROUP u16 bins of a pass with
+// one or two 256-bit loads (GROUP 8: one 128-bit), quantizes its pair once, and in round i
+// updates feature i ^ (lane % GROUP), so that a round's reductions spread over the group.
+// The limbs are packed:
+//  kModeFixed    three words: sums of q_g and q_h mod 2^32, and the sums of their high parts
+//                floor(q / 2^25) (13 and 12 bits) above a 7-bit row count: exact while a cell
+//                holds at most 127 rows of the item (2^25 * 127 < 2^32);
+//  kModeFixedCG  two words, as the u8 kernel's: at most 2,047 rows;
+//  kModeFixedG   the two split limbs of the gradient: always exact.
+// Three words instead of five double the features of a pass (16 instead of 8 at 1,024
+// slots), so a block's rows are read half as often and zeroed, flushed and waited for in
+// half as many passes. Missing rows, which may be many, only count in a per-feature
+// counter; their sums are the item's totals less the other cells'. A feature's count
+// fields and missing rows add up to the item's rows exactly when no cell passed its limit;
+// a pass that fails is built again in split limbs, and its feature group votes (a few-valued
+// feature fails every item; with one vote per block the whole block went back to split limbs,
+// or paid for the failing passes: 20.7 ms instead of 19.2 ms in the last line below).
+// Bound by the shared-memory reductions (three an update) and by what a pass costs apart from
+// its rows: zeroing 196 KB, counting, flushing. GB300, 1,000,000 x 64, depth 8, 5 trees, the
+// whole fit, split limbs -> here: 1,024 bins weighted 15.9 -> 13.4 ms (a level's build
+// 228 -> 166 us), 300 bins 10.4 -> 9.5, 2,000 bins with 10% missing 24.9 -> 20.0, 1,024 bins
+// unweighted with 16 few-valued features 13.3 -> 11.5, the same logistic with missing rows
+// 19.9 -> 19.2.
+template <int MODE>
+__host__ __device__ constexpr int wide_direct_words() { return MODE == kModeFixed ? 3 : 2; }
+constexpr int kWidePackShift = 25, kWidePackCount = 7, kWidePackH = 12;
+
+struct WideTail {  // after the cells and the flush staging
+  ItemDesc desc;
+  uint32_t counted[kBlockFeatures], missing[kBlockFeatures];
+  unsigned long long sum_g[kBlockFeatures], sum_h[kBlockFeatures], total_g, total_h;
+};
+static_assert(sizeof(WideTail) <= kWideTail, "the wide kernel's shared memory");
+
+template <int MODE, int GROUP, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) hist_build_wide_direct_kernel(const __grid_constant__ TrainerDev a) {
+  constexpr int WORDS = wide_direct_words<MODE>();
+  constexpr int WARPS = THREADS / 32;
+  constexpr bool PACKED = MODE != kModeFixedG;
+  constexpr int QUADS = GROUP / 8;  // 16-byte pieces of a row's pass
+  constexpr uint32_t kCountBits = MODE == kModeFixed ? uint32_t(kWidePackCount) : kPackCountBits;
+  constexpr uint32_t kCountMask = (1u << kCountBits) - 1u;
+  extern __shared__ __align__(16) uint32_t wsm[];  // [word][slot][GROUP], the staging rows, the tail
+  WideTail& tail = *reinterpret_cast<WideTail*>(reinterpret_cast<unsigned char*>(wsm) + kSmemMax - kWideTail);
+  const int tid = threadIdx.x;
+  const uint32_t lane = uint32_t(tid & 31);
+  const int warp = tid >> 5;
+  const uint32_t n = a.n_rows, S = a.slots;
+  const uint32_t cells = S * GROUP;
+  const uint32_t plane = cells * 4u;
+  const uint32_t hist_base = static_cast<uint32_t>(__cvta_generic_to_shared(wsm));
+  const uint32_t miss_base = static_cast<uint32_t>(__cvta_generic_to_shared(tail.missing));
+  if (warp == 0) fetch_item_warp(a, lane, &tail.desc);
+  __syncthreads();
+  for (;;) {
+    const ItemDesc d = tail.desc;
+    if (d.item >= d.limit) break;
+    const uint32_t fb = d.fb, row_count = d.row_count;
+    const BuildEntry e = d.e;
+    const size_t seg = (size_t(e.tree) * 2 + e.parity) * a.seg_stride + e.seg_off + d.row_begin;
+    const uint32_t* rows = a.rows + seg;
+    const float2* gh_seg = a.gh_ordered ? a.gh + seg : nullptr;
+    const float2* gh_row = a.gh_ordered ? nullptr : a.gh + size_t(e.tree) * n;
+    const uint16_t* bins = a.bins16 + size_t(fb) * n * kBlockFeatures;
+    const int kg = d.kg, kh = d.kh;
+    const long long q_unit_h = MODE == kModeFixedCG ? quantize_f32(1.0f, kh) : 0ll;
+    const uint32_t width = min(uint32_t(kBlockFeatures), a.features - fb * kBlockFeatures);
+    unsigned long long* dst_base = a.hist + (size_t(e.slot) * a.features + size_t(fb) * kBlockFeatures) * S * 3;
+    const uint32_t ngroups = (row_count + 31u) / 32u;
+    const uint32_t my = uint32_t(warp) < ngroups ? (ngroups - uint32_t(warp) + WARPS - 1) / WARPS : 0u;
+    for (uint32_t f0 = 0; f0 < width; f0 += GROUP) {
+      const uint32_t gw = min(uint32_t(GROUP), width - f0);
+      const bool packed = !PACKED || ((d.packed >> (f0 / GROUP)) & 1u);
+      bool good = packed;
+      if (packed) {
+        {
+          uint4* z = reinterpret_cast<uint4*>(wsm);
+          for (uint32_t i = tid; i < uint32_t(WORDS) * cells / 4u; i += THREADS) z[i] = make_uint4(0, 0, 0, 0);
+        }
+        if (tid < kBlockFeatures) {
+          tail.counted[tid] = tail.missing[tid] = 0;
+          tail.sum_g[tid] = tail.sum_h[tid] = 0;
+          if (tid == 0) tail.total_g = tail.total_h = 0;
+        }
+        // Features of the pass with missing rows, one bit each (the same in every thread).
+        const uint32_t hm_mask = __ballot_sync(
+            0xffffffffu, PACKED && lane < gw && a.has_missing[fb * kBlockFeatures + f0 + lane] != 0);
+        __syncthreads();
+        auto row_at = [&](uint32_t k) -> uint32_t {
+          const uint32_t pos = (uint32_t(warp) + k * WARPS) * 32u + lane;
+          if (k >= my || pos >= row_count) return 0u;
+          const uint32_t r = __ldg(rows + pos);
+          return r < n ? r : 0u;  // row ids are < n by construction
+        };
+        struct RowBins {
+          uint32_t w[GROUP / 2];
+        };
+        auto bins_at = [&](uint32_t k, uint32_t r) -> RowBins {
+          RowBins v{};
+          if (k >= my) return v;
+          const uint16_t* src = bins + size_t(r) * kBlockFeatures + f0;
+          if constexpr (GROUP == 8) {
+            const uint4 x = __ldg(reinterpret_cast<const uint4*>(src));
+            v.w[0] = x.x; v.w[1] = x.y; v.w[2] = x.z; v.w[3] = x.w;
+          } else {
+#pragma unroll
+            for (int q = 0; q < QUADS / 2; ++q) {
+              const Bins32 x = ld_nc_na_v8(src + 16 * q);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) v.w[8 * q + j] = x.w[j];
+            }
+          }
+          return v;
+        };
+        auto gh_at = [&](uint32_t k, uint32_t r) -> float2 {
+          const uint32_t pos = (uint32_t(warp) + k * WARPS) * 32u + lane;
+          if (k >= my || pos >= row_count) return make_float2(0.f, 0.f);
+          return gh_seg ? __ldg(gh_seg + pos) : __ldg(gh_row + r);
+        };
+        long long total_g = 0, total_h = 0;
+        uint32_t r_ahead = row_at(0);
+        RowBins b_next = bins_at(0, r_ahead);
+        float2 g_next = gh_at(0, r_ahead);
+        r_ahead = row_at(1);
+        for (uint32_t k = 0; k < my; ++k) {
+          const RowBins b = b_next;
+          const float2 p = g_next;
+          b_next = bins_at(k + 1, r_ahead);  // the next group's, in flight meanwhile
+          g_next = gh_at(k + 1, r_ahead);
+          r_ahead = row_at(k + 2);
+          if ((uint32_t(warp) + k * WARPS) * 32u + lane >= row_count) continue;
+          const long long qg = quantize_f32(p.x, kg);
+          uint32_t v0 = uint32_t(qg), v1, v2 = 0;
+          if constexpr (MODE == kModeFixed) {
+            const long long qh = quantize_f32(p.y, kh);
+            v1 = uint32_t(qh);
+            v2 = (uint32_t(int32_t(qg >> kWidePackShift)) << (kWidePackCount + kWidePackH)) |
+                 (uint32_t(qh >> kWidePackShift) << kWidePackCount) | 1u;
+            if (hm_mask) total_h += qh;
+          } else if constexpr (MODE == kModeFixedCG) {
+            v1 = (uint32_t(int32_t(qg >> kPackShift)) << kPackCountBits) | 1u;
+          } else {
+            v0 = uint32_t(qg) & 0xFFFFu;
+            v1 = uint32_t(int32_t(qg >> 16));
+          }
+          if (hm_mask) total_g += qg;
+          // Round i: feature i ^ (lane % GROUP). Word j of w holds features (2 j, 2 j + 1) ^
+          // (lane % GROUP): words permuted by the upper bits of the lane, halves by the last.
+          const uint32_t lg = lane % GROUP;
+          uint32_t w[GROUP / 2];
+#pragma unroll
+          for (int j = 0; j < GROUP / 2; ++j) w[j] = b.w[j];
+#pragma unroll
+          for (uint32_t bit = 1; bit < GROUP / 2; bit <<= 1) {
+            const bool swap = ((lg >> 1) & bit) != 0;  // per lane: selects, no divergence
+#pragma unroll
+            for (uint32_t j = 0; j < GROUP / 2; ++j)
+              if ((j & bit) == 0) {
+                const uint32_t x = w[j], y = w[j | bit];
+                w[j] = swap ? y : x;
+                w[j | bit] = swap ? x : y;
+              }
+          }
+          const uint32_t sel = (lg & 1u) ? 0x1032u : 0x3210u;
+#pragma unroll
+          for (int j = 0; j < GROUP / 2; ++j) w[j] = __byte_perm(w[j], 0u, sel);
+#pragma unroll
+          for (uint32_t i = 0; i < GROUP; ++i) {
+            const uint32_t f = i ^ lg;
+            const uint32_t bin = min((i & 1u) ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu, S - 1u);
+            const uint32_t addr = hist_base + (bin * GROUP + f) * 4u;
+            if (PACKED && bin == S - 1u && ((hm_mask >> f) & 1u)) {
+              red_shared_u32(miss_base + f * 4u, 1u);
+            } else {
+              red_shared_u32(addr, v0);
+              red_shared_u32(addr + plane, v1);
+              if constexpr (WORDS > 2) red_shared_u32(addr + 2u * plane, v2);
+            }
+          }
+        }
+        if (hm_mask) {  // the item's totals, for the missing rows' sums
+          for (int off = 16; off > 0; off >>= 1) {
+            total_g += __shfl_xor_sync(0xffffffffu, total_g, off);
+            total_h += __shfl_xor_sync(0xffffffffu, total_h, off);
+          }
+          if (lane == 0) {
+            atomicAdd(&tail.total_g, (unsigned long long)total_g);
+            atomicAdd(&tail.total_h, (unsigned long long)total_h);
+          }
+        }
+        __syncthreads();
+        const uint32_t fl = lane % GROUP;
+        if (PACKED) {
+          const uint32_t* counts = wsm + (WORDS - 1) * cells;
+          uint32_t sum = 0;
+          for (uint32_t idx = tid; idx < cells; idx += THREADS) sum += counts[idx] & kCountMask;
+          atomicAdd(tail.counted + fl, sum);  // THREADS is a multiple of GROUP: the thread's feature
+          __syncthreads();
+          const bool mine = lane >= gw || tail.counted[lane] + tail.missing[lane] == row_count;
+          good = __all_sync(0xffffffffu, mine);  // the same in every warp
+          if (tid == 0) atomicAdd(a.limb_votes + 2 * (kWidePasses * fb + f0 / GROUP) + (good ? 0 : 1), 1u);
+        }
+        if (good) {
+          unsigned long long fg = 0, fh = 0;  // the lane's cells' sums
+          wide_flush<THREADS>(
+              wsm, size_t(WORDS) * cells * 4, S, GROUP, gw, dst_base + size_t(f0) * S * 3,
+              [&](uint32_t idx, unsigned long long& c, unsigned long long& g, unsigned long long& h) {
+                if constexpr (MODE == kModeFixed) {
+                  const uint32_t hc = wsm[2 * cells + idx];
+                  c = hc & kCountMask;
+                  const long long near_g = (long long)(int32_t(hc) >> (kWidePackCount + kWidePackH)) * (1ll << kWidePackShift);
+                  const long long near_h =
+                      (long long)((hc >> kWidePackCount) & ((1u << kWidePackH) - 1u)) * (1ll << kWidePackShift);
+                  g = (unsigned long long)(near_g + (long long)(wsm[idx] - uint32_t(near_g)));
+                  h = (unsigned long long)(near_h + (long long)(wsm[cells + idx] - uint32_t(near_h)));
+                } else if constexpr (MODE == kModeFixedCG) {
+                  const uint32_t gc = wsm[cells + idx];
+                  c = gc & kCountMask;
+                  g = packed_sum(wsm[idx], int32_t(gc) >> kPackCountBits);
+                  h = (unsigned long long)((long long)c * q_unit_h);
+                } else {
+                  c = 0;  // the gradient-only root's count and hessian words are restored
+                  g = (unsigned long long)((long long)int32_t(wsm[cells + idx]) * 65536 + (long long)wsm[idx]);
+                  h = 0;
+                }
+                fg += g;
+                fh += h;
+              });
+          if (PACKED && hm_mask) {
+            atomicAdd(tail.sum_g + fl, fg);
+            atomicAdd(tail.sum_h + fl, fh);
+          }
+        }
+        if (PACKED && hm_mask) {
+          __syncthreads();
+          if (good && tid < int(gw) && ((hm_mask >> tid) & 1u) && tail.missing[tid]) {
+            unsigned long long* dst = dst_base + (size_t(f0 + tid) * S + S - 1) * 3;
+            const unsigned long long c = tail.missing[tid];
+            atomicAdd(dst + 0, c);
+            atomicAdd(dst + 1, tail.total_g - tail.sum_g[tid]);
+            atomicAdd(dst + 2, MODE == kModeFixedCG ? (unsigned long long)((long long)c * q_unit_h)
+                                                    : tail.total_h - tail.sum_h[tid]);
+          }
+        }
+        __syncthreads();
+      }
+      if (!good)
+        wide_split_passes<MODE, THREADS>(a, e, fb, d.row_begin, row_count, kg, kh, wide_group<MODE>(S), f0, f0 + gw, wsm);
+    }
+    if (tid == 0) {
+      atomicAdd(&a.ctl->cells, (unsigned long long)row_count * width);
+      if (fb == 0) atomicAdd(&a.ctl->rows_built, (unsigned long long)row_count);
+    }
+    if (warp == 0) fetch_item_warp(a, lane, &tail.desc);
+    __syncthreads();
+  }
+  bulk_wait_all();  // this thread's bulk reductions have reached the slots
+}
+
+template <int MODE, int GROUP>
+cudaError_t launch_wide_direct(const TrainerDev& a, int grid, cudaStream_t stream) {
+  constexpr int kThreads = 768;
+  constexpr size_t smem = kSmemMax;
+  static std::atomic<unsigned long long> configured{0};  // one bit per device
+  const cudaError_t err = opt_in_dynamic_smem(configured, hist_build_wide_direct_kernel<MODE, GROUP, kThreads>, smem);
+  if (err != cudaSuccess) return err;
+  hist_build_wide_direct_kernel<MODE, GROUP, kThreads><<<grid, kThreads, smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
 template <int MODE, int THREADS>
 cudaError_t launch_wide(const TrainerDev& a, int grid, cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};  // one bit per device
   const cudaError_t err = opt_in_dynamic_smem(configured, hist_build_wide_kernel<MODE, THREADS>,
-                                              kWideSmemBytes + kWideStagingBytes);
+                                              kSmemMax - kWideTail);
   if (err != cudaSuccess) return err;
   const uint32_t group = wide_group<MODE>(a.slots);
-  const size_t smem = group ? size_t(group) * a.slots * wide_words<MODE>() * sizeof(uint32_t) + kWideStagingBytes : 0;
+  const size_t smem = group ? kSmemMax - kWideTail : 0;
   hist_build_wide_kernel<MODE, THREADS><<<grid, THREADS, smem, stream>>>(a, group);
   return cudaGetLastError();
 }
 
-// Wide launches: 1024 threads, or 512.
+// Wide launches: register-direct where a pass holds at least 8 features' cells (2,133 slots
+// weighted: the longest load of a row's bins that is still 16 bytes; a pass of four would read
+// each 32-byte sector four times), measured from 512 to 2,048 slots above. Else, and for
+// float sums, split limbs by 1024 threads, or 512.
 template <int MODE>
 cudaError_t launch_wide_shape(const TrainerDev& a, int threads, int grid, cudaStream_t stream) {
+  if constexpr (MODE != kModeFloat) {
+    if (a.limb_votes) {
+      const size_t fit = kWideSmemBytes / (size_t(a.slots) * wide_direct_words<MODE>() * sizeof(uint32_t));
+      if (fit >= 32) return launch_wide_direct<MODE, 32>(a, grid, stream);
+      if (fit >= 16) return launch_wide_direct<MODE, 16>(a, grid, stream);
+      if (fit >= 8) return launch_wide_direct<MODE, 8>(a, grid, stream);
+    }
+  }
   if (threads == 512) return launch_wide<MODE, 512>(a, grid, stream);
   return launch_wide<MODE, 1024>(a, grid, stream);
 }

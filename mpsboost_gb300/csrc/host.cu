@@ -766,7 +766,8 @@ struct mpsb_cuda_trainer {
   std::vector<uint64_t> level_cells_total;
   uint32_t rounds_enqueued = 0;
   uint32_t blocked_levels = 2;  // levels built from the column-blocked bins
-  uint32_t* limb_votes = nullptr;  // [levels][nfb][2] (device): TrainerDev::limb_votes by level
+  uint32_t* limb_votes = nullptr;  // (device) TrainerDev::limb_votes, level by level
+  size_t limb_vote_words = 0;      // per level
   mpsb_cuda_stats stats{};
   uint64_t kernels_per_round[2] = {0, 0};
   uint64_t cells_base = 0, rows_base = 0, part_base = 0;
@@ -936,7 +937,7 @@ struct mpsb_cuda_trainer {
   // A leaf-wise step's view: the packed-limb votes of level 1 stand for every step.
   TrainerDev step_view() const {
     TrainerDev v = build_view();
-    if (limb_votes) v.limb_votes = limb_votes + size_t(2) * dev.nfb;
+    if (limb_votes) v.limb_votes = limb_votes + limb_vote_words;
     return v;
   }
 
@@ -945,7 +946,7 @@ struct mpsb_cuda_trainer {
   // row-major copy, whose 128-byte row line serves all feature blocks through L2.
   TrainerDev level_view(uint32_t d) const {
     TrainerDev v = build_view();
-    if (limb_votes) v.limb_votes = limb_votes + size_t(2) * dev.nfb * d;
+    if (limb_votes) v.limb_votes = limb_votes + limb_vote_words * d;
     if (d == 0) v.store_single = 0;
     if (d < blocked_levels && !dev.feature_of) {
       v.bins = ds->bins_blocked.as<uint8_t>();
@@ -1394,10 +1395,14 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.tree_nodes = t->alloc<TreeNodeOut>(size_t(T) * tree_nodes);
   a.ctl = t->alloc<Control>(1);
   CK(cudaMemsetAsync(a.ctl, 0, sizeof(Control), s));
-  // Packed histogram limbs (MPSB_PACKED=0: split limbs only).
+  // Packed histogram limbs (MPSB_PACKED=0: split limbs only). A wide fixed-point cell packs
+  // at most 127 rows of an item: items are kept to about 32 rows a bin.
   const char* packed = std::getenv("MPSB_PACKED");
-  if (a.mode == kModeFixed && ds->slots == uint32_t(kSlots) && !(packed && std::atoi(packed) == 0)) {
-    const size_t votes = size_t(std::max<uint32_t>(D, 2)) * ds->nfb * 2;
+  if (a.mode == kModeFixed && !(packed && std::atoi(packed) == 0)) {
+    if (ds->slots != uint32_t(kSlots))
+      a.item_rows_max = std::min<uint32_t>(kItemRowsMax, std::max<uint32_t>(4096u, 32u * ds->slots));
+    t->limb_vote_words = size_t(a.nfb) * 2 * (ds->slots == uint32_t(kSlots) ? 1 : kWideVotePasses);
+    const size_t votes = size_t(std::max<uint32_t>(D, 2)) * t->limb_vote_words;
     t->limb_votes = t->alloc<uint32_t>(votes);
     CK(cudaMemsetAsync(t->limb_votes, 0, votes * sizeof(uint32_t), s));
   }

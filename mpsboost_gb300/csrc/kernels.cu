@@ -46,21 +46,22 @@ __device__ __forceinline__ uint32_t dataset_feature(const TrainerDev& a, uint32_
 }
 
 // Rows per histogram work item for a level that builds `rows` rows: about per_sm (default
-// three) items per SM, a multiple of 512, within [1024, kItemRowsMax]. Where the
-// kItemRowsMax cap forces more items, their number is raised to the next multiple of the
+// three) items per SM, a multiple of 512, within [1024, item_rows_max]. Where the
+// upper end forces more items, their number is raised to the next multiple of the
 // SM count, so that the persistent CTAs end the level together. At the lower end an item's
 // reductions (about 1.5 us) weigh as much as its flush: 100,000 x 32, depth 6, 50 trees
 // take 17.5, 17.3, 17.7 and 18.7 ms with items of 512, 1,024, 2,048 and 4,096 rows.
-__device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, uint32_t nfb, uint32_t sms,
-                                                      uint32_t per_sm) {
-  const uint64_t n_sm = sms ? sms : 152;
+__device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, const TrainerDev& a, uint32_t per_sm) {
+  const uint64_t n_sm = a.sm_count ? a.sm_count : 152;
+  const uint32_t nfb = a.nfb;
+  const uint32_t most = a.item_rows_max ? a.item_rows_max : kItemRowsMax;
   uint64_t target = n_sm * (per_sm ? per_sm : 3);
-  const uint64_t min_items = (rows * nfb + kItemRowsMax - 1) / kItemRowsMax;
+  const uint64_t min_items = (rows * nfb + most - 1) / most;
   if (target < min_items) target = (min_items + n_sm - 1) / n_sm * n_sm;
   uint64_t per = (rows * nfb + target - 1) / target;
   per = (per + 511) / 512 * 512;
   if (per < 1024) per = 1024;
-  if (per > kItemRowsMax) per = kItemRowsMax;
+  if (per > most) per = most;
   return uint32_t(per);
 }
 
@@ -233,7 +234,7 @@ __device__ __noinline__ void round_setup(const TrainerDev& a, bool g_only) {
     uint64_t total = 0;
     for (uint32_t t = 0; t < a.n_trees; ++t) total += root_rows(a, t);
     const uint32_t item_rows =
-        a.item_rows ? a.item_rows : adaptive_item_rows(total, a.nfb, a.sm_count, a.items_per_sm);
+        a.item_rows ? a.item_rows : adaptive_item_rows(total, a, a.items_per_sm);
     uint32_t acc = 0;
     for (uint32_t t = 0; t < a.n_trees; ++t) {
       a.build_prefix[t] = acc;
@@ -1987,7 +1988,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
   const uint32_t base_per_sm = a.items_per_sm ? a.items_per_sm : 3u;
   const uint32_t level_per_sm = n >= 8 ? base_per_sm + 1 : (base_per_sm > 2 ? base_per_sm - 1 : base_per_sm);
   const uint32_t item_rows =
-      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(built_units) * 256, a.nfb, a.sm_count, level_per_sm);
+      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(built_units) * 256, a, level_per_sm);
 
   // Phase B1: acceptance under max_leaves, accepted prefix, chunk prefixes.
   // Scanned values: 0 accepted, 1 build chunks, 2 partition chunks, 3 leaf segments,
@@ -2279,7 +2280,7 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
   const uint32_t base_per_sm = a.items_per_sm ? a.items_per_sm : 3u;
   const uint32_t level_per_sm = n >= 8 ? base_per_sm + 1 : (base_per_sm > 2 ? base_per_sm - 1 : base_per_sm);
   const uint32_t item_rows =
-      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(tot3[1]) * 256, a.nfb, a.sm_count, level_per_sm);
+      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(tot3[1]) * 256, a, level_per_sm);
   const bool acc = i < n && b.valid && (leaf_count + (v3[0] - s_valid_base[ord]) < P.max_leaves);
   const bool leafseg = i < n && (!acc || last);
   // 0 accepted, 1 build chunks, 2 partition chunks, 3 leaf segments, 4 leaf chunks, 5 freed.
@@ -3027,7 +3028,7 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
   if (warp == 0) {  // work lists of the step, 32 entries at a time
     Control* ctl = a.ctl;
     const uint32_t item_rows =
-        a.item_rows ? a.item_rows : adaptive_item_rows(built_rows, a.nfb, a.sm_count, a.items_per_sm);
+        a.item_rows ? a.item_rows : adaptive_item_rows(built_rows, a, a.items_per_sm);
     auto prefix = [&](uint32_t n, uint32_t* out, auto&& chunks_of) -> uint32_t {
       uint32_t acc = 0;
       for (uint32_t e0 = 0; e0 < n; e0 += 32) {

@@ -10,6 +10,8 @@
 
 namespace mpsb {
 
+constexpr uint32_t kWideVotePasses = 4;  // passes of a wide block of 32 features, at most
+
 // Device pointers and sizes of one training session, passed by value to every kernel.
 struct TrainerDev {
   // dataset
@@ -100,8 +102,10 @@ struct TrainerDev {
   TreeNodeOut* tree_nodes;      // [n_trees][max_tree_nodes]
   uint32_t max_tree_nodes;
   Control* ctl;
-  uint32_t* limb_votes;         // [nfb][2] of the launch's depth level: work items that passed
-                                // and failed the packed-limb check (null: split limbs only)
+  uint32_t* limb_votes;         // [nfb][2], wide [nfb][kWideVotePasses][2], of the launch's depth
+                                // level: work items (a wide block's passes) that passed and
+                                // failed the packed-limb check (null: split limbs only)
+  uint32_t item_rows_max;       // the adaptive item size's upper end (0: kItemRowsMax)
   uint32_t store_single;        // below the roots: a node of one row chunk is stored by its work
                                 // items, so its slot is not cleared (register-direct kernel)
   uint32_t item_rows;           // rows per histogram work item (<= kItemRowsMax); 0: the

@@ -73,6 +73,23 @@ def test_packed_limb_overflow(backend, port, heavy, weighted):
                           max_depth=4, min_samples_leaf=2)
 
 
+# Wide pages: the packed limbs' largest cells (127 rows weighted, 2,047 unweighted) and one past
+# them, missing rows in most and in few cells, few-valued features whose passes fall back to split
+# limbs, and passes of 32, 16 and 8 features (weighted, 512 / 1,024 / 2,048 slots) at feature
+# counts around a pass and a block; past 2,133 slots the split limbs alone.
+@pytest.mark.parametrize("bins,features", [(300, 33), (511, 7), (700, 17), (1000, 40), (2000, 9), (2200, 5)])
+@pytest.mark.parametrize("heavy,nan", [(127, 0.0), (128, 0.3), (2047, 0.0), (2048, 0.02)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_wide_packed_limbs(backend, port, bins, features, heavy, nan, weighted):
+    x = seeded_matrix(bins + heavy, 9_000, features, nan)
+    x[:, 1] = np.arange(9_000)
+    x[:heavy, 1] = -1.0
+    x[:, features - 1] = np.arange(9_000) % 3
+    y, w = targets(x, heavy)
+    assert_equals_replica(backend, port, x, y, w if weighted else None, bins, n_estimators=2, learning_rate=0.3,
+                          max_depth=4, min_samples_leaf=2)
+
+
 def test_integer_pipe_logistic_within_half_an_ulp(tmp_path):
     """e^-t and the logistic function's pieces on the integer pipe against long double."""
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
