@@ -480,6 +480,13 @@ int mpsb_cuda_autotune(mpsb_cuda_backend* backend, const mpsb_cuda_dataset* data
                        uint32_t rounds_per_trial, mpsb_cuda_tuning* out);
 /* Forget every tuned shape. */
 void mpsb_cuda_autotune_clear(void);
+
+/* Host helpers of the bindings. class_ids: 1 when every label is a whole number in
+ * [0, limit) (2: some are -0.0), with seen[c] = 1 at each c that occurs; else 0.
+ * touch_pages: writes a zero byte to each page of an uninitialised result buffer, so that
+ * the copy that fills it does not wait for the page faults. */
+int mpsb_cuda_class_ids(const double* labels, uint64_t n, uint32_t limit, uint8_t* seen);
+void mpsb_cuda_touch_pages(void* p, uint64_t bytes);
 void mpsb_cuda_trainer_destroy(mpsb_cuda_trainer* trainer);
 
 #ifdef __cplusplus

@@ -203,6 +203,8 @@ SIGNATURES = {
     "mpsb_cuda_trainer_export": (_I32, [_VP, C.POINTER(_VP)]),
     "mpsb_cuda_autotune": (_I32, [_VP, _VP, _VP, _VP, _U64, _VP, _U32, _U32, C.POINTER(Tuning)]),
     "mpsb_cuda_autotune_clear": (None, []),
+    "mpsb_cuda_class_ids": (_I32, [_VP, _U64, _U32, _VP]),
+    "mpsb_cuda_touch_pages": (None, [_VP, _U64]),
     "mpsb_cuda_trainer_destroy": (None, [_VP]),
 }
 

@@ -22,6 +22,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -744,6 +745,31 @@ def train_softmax(backend: CudaBackend, dataset, labels, n_classes: int, weights
     return m
 
 
+class _ResultBuffers:
+    """The FP64 results of a fit, one array per model. From 4 MB on a thread maps their pages
+    while the device trains: the copy of ten 8 MB results into fresh pages takes 3.5 ms, 2.6 of
+    them page faults. (Past 4 GB, or smaller, they are allocated when asked for.)"""
+
+    def __init__(self, count: int, rows: int):
+        self.rows, self.arrays, self.thread = rows, [], None
+        if 4 << 20 <= 8 * count * rows <= 4 << 30:
+            self.arrays = [np.empty(rows, np.float64) for _ in range(count)]
+            self.thread = threading.Thread(target=self._map, daemon=True)
+            self.thread.start()
+
+    def _map(self) -> None:
+        lib = _lib.load()
+        for a in self.arrays:
+            lib.mpsb_cuda_touch_pages(ptr(a), a.nbytes)
+
+    def join(self) -> None:
+        if self.thread is not None:
+            self.thread.join()
+
+    def __getitem__(self, k: int) -> np.ndarray:
+        return self.arrays[k] if self.arrays else np.empty(self.rows, np.float64)
+
+
 def _train(backend, dataset, labels, weights, options, n_classes, **params):
     dev = backend.dataset(dataset)
     y = np.ascontiguousarray(labels, dtype=np.float64)
@@ -751,21 +777,25 @@ def _train(backend, dataset, labels, weights, options, n_classes, **params):
     params.setdefault("max_bins", dataset.max_bins)
     p, keep = make_params(**params)
     lib = _lib.load()
-    if n_classes:
-        handles = (C.c_void_p * n_classes)()
-        check(lib.mpsb_cuda_train_ovr(backend.handle, dev.handle, ptr(y), ptr(w), y.size, n_classes,
-                                      C.byref(p), options, handles))
-        raw = list(handles)
-    else:
-        h = C.c_void_p()
-        check(lib.mpsb_cuda_train_regressor(backend.handle, dev.handle, ptr(y), ptr(w), y.size,
-                                            C.byref(p), options, C.byref(h)))
-        raw = [h.value]
+    results = _ResultBuffers(max(n_classes, 1), dataset.rows)
+    try:
+        if n_classes:
+            handles = (C.c_void_p * n_classes)()
+            check(lib.mpsb_cuda_train_ovr(backend.handle, dev.handle, ptr(y), ptr(w), y.size, n_classes,
+                                          C.byref(p), options, handles))
+            raw = list(handles)
+        else:
+            h = C.c_void_p()
+            check(lib.mpsb_cuda_train_regressor(backend.handle, dev.handle, ptr(y), ptr(w), y.size,
+                                                C.byref(p), options, C.byref(h)))
+            raw = [h.value]
+    finally:
+        results.join()
     del keep
     models = []
-    for h in raw:
+    for k, h in enumerate(raw):
         m = RegressionModel._from_handle(h)
-        m.train_predictions = np.empty(dataset.rows, np.float64)
+        m.train_predictions = results[k]
         check(lib.mpsb_cuda_model_train_predictions(h, ptr(m.train_predictions)))
         lib.mpsb_cuda_model_destroy(h)
         if m.schema is None:

@@ -363,12 +363,11 @@ __global__ void transform_kernel(const uint32_t* keys, const uint8_t* missing, u
 }
 
 struct Scratch {
-  std::vector<std::unique_ptr<DevBuf>> bufs;
+  DevArena mem;
+  explicit Scratch(const mpsb_cuda_backend* b) { mem.pool = b->pool; }
   template <class T>
   T* alloc(size_t count) {
-    bufs.emplace_back(new DevBuf);
-    bufs.back()->alloc(count * sizeof(T));
-    return bufs.back()->as<T>();
+    return static_cast<T*>(mem.alloc(count * sizeof(T)));
   }
 };
 
@@ -741,7 +740,7 @@ int mpsb_cuda_dataset_quantize(mpsb_cuda_backend* b, const void* data, int scala
     if (features > 65535) throw UnsupportedError("device binning takes at most 65535 features");
     b->activate();
     cudaStream_t s = b->stream;
-    Scratch ss;
+    Scratch ss(b);
     uint32_t* keys = nullptr;
     uint8_t* missing = nullptr;
     std::vector<uint64_t> missing_count;
@@ -848,7 +847,7 @@ int mpsb_cuda_dataset_transform(mpsb_cuda_backend* b, const mpsb_cuda_dataset* s
       throw DataError("Prediction input feature count does not match the binned schema");
     b->activate();
     cudaStream_t s = b->stream;
-    Scratch ss;
+    Scratch ss(b);
     uint32_t* keys = nullptr;
     uint8_t* missing = nullptr;
     std::vector<uint64_t> missing_count;

@@ -9,6 +9,7 @@
 // replayed per round. No row ever returns to the host inside a round; the host reads
 // back only the finished trees.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -25,6 +26,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -97,6 +99,130 @@ uint32_t dataset_slots(const uint32_t* bin_count, const uint8_t* has_missing, ui
   }
   if (need <= uint64_t(kSlots)) return uint32_t(kSlots);
   return uint32_t((need + kSlots - 1) / kSlots * kSlots);
+}
+
+// ---- device memory kept between calls -------------------------------------------------
+namespace {
+std::mutex g_pools_mutex;
+std::vector<DevicePool*> g_pools;
+}  // namespace
+
+DevicePool::DevicePool(int dev, cudaStream_t backend_stream) : device(dev), stream_(backend_stream) {
+  std::lock_guard<std::mutex> lock(g_pools_mutex);
+  g_pools.push_back(this);
+}
+
+DevicePool::~DevicePool() {
+  {
+    std::lock_guard<std::mutex> lock(g_pools_mutex);
+    g_pools.erase(std::find(g_pools.begin(), g_pools.end(), this));
+  }
+  trim();
+}
+
+// A kept block of at most an eighth more than the size wanted, or a new one.
+void* DevicePool::take(size_t* bytes) {
+  const size_t want = (*bytes + kBlock - 1) / kBlock * kBlock;
+  {
+    std::lock_guard<std::mutex> lock(mutex_);
+    auto best = free_.end();
+    for (auto it = free_.begin(); it != free_.end(); ++it)
+      if (it->second >= want && it->second <= want + want / 8 && (best == free_.end() || it->second < best->second))
+        best = it;
+    if (best != free_.end()) {
+      void* p = best->first;
+      *bytes = best->second;
+      kept_ -= best->second;
+      free_.erase(best);
+      return p;
+    }
+  }
+  DevBuf fresh;
+  fresh.alloc(want);
+  *bytes = want;
+  return std::exchange(fresh.p, nullptr);
+}
+
+void DevicePool::give(void* p, size_t bytes) {
+  std::lock_guard<std::mutex> lock(mutex_);
+  if (!stream_ || bytes > kMost) {
+    cudaFree(p);
+    return;
+  }
+  try {
+    free_.emplace_back(p, bytes);
+  } catch (const std::bad_alloc&) {
+    cudaFree(p);
+    return;
+  }
+  kept_ += bytes;
+  while (kept_ > kMost) {
+    cudaFree(free_.front().first);
+    kept_ -= free_.front().second;
+    free_.pop_front();
+  }
+}
+
+void DevicePool::trim() {
+  std::lock_guard<std::mutex> lock(mutex_);
+  for (auto& f : free_) cudaFree(f.first);
+  free_.clear();
+  kept_ = 0;
+}
+
+void DevicePool::close() {
+  {
+    std::lock_guard<std::mutex> lock(mutex_);
+    stream_ = nullptr;
+  }
+  trim();
+}
+
+bool DevicePool::idle() {
+  cudaStream_t s;
+  {
+    std::lock_guard<std::mutex> lock(mutex_);
+    s = stream_;
+  }
+  return s && cudaStreamSynchronize(s) == cudaSuccess;
+}
+
+size_t DevicePool::kept() const {
+  std::lock_guard<std::mutex> lock(mutex_);
+  return kept_;
+}
+
+void DevicePool::trim_all() {
+  std::lock_guard<std::mutex> lock(g_pools_mutex);
+  for (DevicePool* p : g_pools) p->trim();
+}
+
+void* DevArena::alloc(size_t bytes) {
+  bytes = (std::max<size_t>(bytes, 16) + 255) / 256 * 256;  // cudaMalloc's alignment
+  if (bytes <= left_) {
+    void* p = slab_;
+    slab_ += bytes;
+    left_ -= bytes;
+    return p;
+  }
+  size_t block = bytes;
+  void* p = pool->take(&block);
+  blocks_.emplace_back(p, block);
+  if (block - bytes > left_) {  // the rest serves the next small ones
+    slab_ = static_cast<char*>(p) + bytes;
+    left_ = block - bytes;
+  }
+  return p;
+}
+
+DevArena::~DevArena() {
+  if (blocks_.empty()) return;
+  // After an error of the device nothing is kept; cudaFree then waits by itself.
+  const bool idle = pool->idle();
+  for (auto& b : blocks_) {
+    if (idle) pool->give(b.first, b.second);
+    else cudaFree(b.first);
+  }
 }
 
 // ---- reference semantics evaluated on the host --------------------------------------
@@ -250,6 +376,43 @@ RowSums row_sums(const double* w, const double* y, uint64_t n, int label_mode, c
 
 double validate_weights(const double* w, uint64_t n) {  // trainer.cpp:44-66
   return row_sums(w, nullptr, n, 0, nullptr).total;
+}
+
+// Whether every label is a whole number in [0, limit); `seen` (or null) gets a 1 at each
+// that occurs. 2: some are -0.0. A thread per 2^17 rows, at most 16; nothing is thrown.
+int class_ids(const double* y, uint64_t n, uint32_t limit, uint8_t* seen) {
+  std::atomic<bool> bad{false}, minus{false};
+  auto check = [&](uint64_t lo, uint64_t hi) {
+    bool ok = true, neg = false;
+    for (uint64_t i = lo; i < hi && ok; i += 4096) {
+      const uint64_t end = std::min(hi, i + 4096);
+      for (uint64_t k = i; k < end; ++k) {
+        ok &= (y[k] >= 0.0) & (y[k] < double(limit)) & (std::trunc(y[k]) == y[k]);
+        neg |= std::signbit(y[k]);
+      }
+      for (uint64_t k = i; seen && ok && k < end; ++k) {
+        uint8_t* s = seen + uint32_t(y[k]);  // written once: its line stays shared by the threads
+        if (!__atomic_load_n(s, __ATOMIC_RELAXED)) __atomic_store_n(s, uint8_t(1), __ATOMIC_RELAXED);
+      }
+    }
+    if (!ok) bad.store(true, std::memory_order_relaxed);
+    if (neg) minus.store(true, std::memory_order_relaxed);
+  };
+  const uint64_t workers = std::max<uint64_t>(
+      1, std::min<uint64_t>(std::max(1u, std::min(16u, std::thread::hardware_concurrency())), n >> 17));
+  std::thread pool[16];
+  for (uint64_t k = 1; k < workers; ++k) {
+    const uint64_t lo = n * k / workers, hi = n * (k + 1) / workers;
+    try {
+      pool[k] = std::thread(check, lo, hi);
+    } catch (const std::system_error&) {
+      check(lo, hi);
+    }
+  }
+  check(0, n / workers);
+  for (auto& t : pool)
+    if (t.joinable()) t.join();
+  return bad.load() ? 0 : (minus.load() ? 2 : 1);
 }
 
 const char* count_objective_name(uint32_t objective) {
@@ -461,6 +624,7 @@ int mpsb_cuda_backend_create(int device, mpsb_cuda_backend** out) {
     CK(cudaEventCreate(&b->t1));
     b->error.alloc(sizeof(uint32_t));
     CK(cudaMemset(b->error.p, 0, sizeof(uint32_t)));
+    b->pool = std::make_shared<DevicePool>(device, b->stream);
     *out = b.release();
   });
 }
@@ -749,7 +913,7 @@ struct mpsb_cuda_trainer {
   bool ovr = false;
   TrainerDev dev{};
   HistConfig hcfg;
-  std::vector<std::unique_ptr<DevBuf>> bufs;
+  DevArena mem;
   std::vector<double> base_scores;
   // One graph for a full round and one for a round that reuses the roots' count and
   // hessian histograms.
@@ -775,9 +939,7 @@ struct mpsb_cuda_trainer {
 
   template <class T>
   T* alloc(size_t count) {
-    bufs.emplace_back(new DevBuf);
-    bufs.back()->alloc(count * sizeof(T));
-    return bufs.back()->as<T>();
+    return static_cast<T*>(mem.alloc(count * sizeof(T)));
   }
 
   cudaStream_t side = nullptr;                      // work beside the main stream
@@ -786,7 +948,10 @@ struct mpsb_cuda_trainer {
   ~mpsb_cuda_trainer() {
     if (fork_ev) cudaEventDestroy(fork_ev);
     if (zero_ev) cudaEventDestroy(zero_ev);
-    if (side) cudaStreamDestroy(side);
+    if (side) {
+      cudaStreamSynchronize(side);  // `mem` is reused once the backend's stream is idle
+      cudaStreamDestroy(side);
+    }
     for (int i = 0; i < 2; ++i) {
       if (graph_exec[i]) cudaGraphExecDestroy(graph_exec[i]);
       if (graph[i]) cudaGraphDestroy(graph[i]);
@@ -1089,6 +1254,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   trace.mark("dataset upload complete");
   b->activate();
   t->b = b;
+  t->mem.pool = b->pool;
   t->ds = ds;
   CK(cudaStreamCreateWithFlags(&t->side, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&t->fork_ev, cudaEventDisableTiming));
@@ -1297,12 +1463,13 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   }
   if (forest) {
     uint32_t* d_sample = t->alloc<uint32_t>(size_t(T) * forest->cap);
-    DevBuf counts, chunk_sums;  // released once the samples are written
-    counts.alloc(size_t(T) * n);
-    chunk_sums.alloc(size_t(T) * ((n + kExpandChunk - 1) / kExpandChunk) * sizeof(uint32_t));
-    CK(cudaMemcpyAsync(counts.p, forest->row_counts, size_t(T) * n, cudaMemcpyHostToDevice, s));
-    CK(launch_expand_samples(counts.as<uint8_t>(), uint32_t(n), T, chunk_sums.as<uint32_t>(), forest->cap,
-                             d_sample, s));
+    DevArena samples;  // released once the samples are written
+    samples.pool = b->pool;
+    uint8_t* counts = static_cast<uint8_t*>(samples.alloc(size_t(T) * n));
+    uint32_t* chunk_sums = static_cast<uint32_t*>(
+        samples.alloc(size_t(T) * ((n + kExpandChunk - 1) / kExpandChunk) * sizeof(uint32_t)));
+    CK(cudaMemcpyAsync(counts, forest->row_counts, size_t(T) * n, cudaMemcpyHostToDevice, s));
+    CK(launch_expand_samples(counts, uint32_t(n), T, chunk_sums, forest->cap, d_sample, s));
     uint32_t* d_count = t->alloc<uint32_t>(T);
     CK(cudaMemcpyAsync(d_count, forest->count.data(), size_t(T) * 4, cudaMemcpyHostToDevice, s));
     uint32_t* d_masks = t->alloc<uint32_t>(size_t(T) * W);
@@ -1425,15 +1592,31 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   trace.mark("working state");
 }
 
-mpsb_cuda_model* export_model(mpsb_cuda_trainer* t, uint32_t tree_index,
+// A trainer's finished trees on the host: their sizes and, where all of them with the room
+// between them are at most 1 MB, their nodes. One copy of 490 KB takes 20 us; 20 trees copied
+// one by one take 220.
+struct TreeDownload {
+  uint32_t rounds = 0;
+  std::vector<uint32_t> counts;          // [rounds][n_trees]
+  std::vector<mpsb_tree_node> nodes;     // [rounds][n_trees][max_tree_nodes], or empty
+
+  explicit TreeDownload(const TrainerDev& a) {
+    CK(cudaMemcpy(&rounds, a.round_counter, sizeof rounds, cudaMemcpyDeviceToHost));
+    counts.resize(size_t(rounds) * a.n_trees);
+    if (counts.empty()) return;
+    CK(cudaMemcpy(counts.data(), a.model_counts, counts.size() * 4, cudaMemcpyDeviceToHost));
+    const uint64_t all = uint64_t(counts.size()) * a.max_tree_nodes;
+    if (all * sizeof(mpsb_tree_node) > (1u << 20)) return;
+    nodes.resize(all);
+    CK(cudaMemcpy(nodes.data(), a.model_nodes, all * sizeof(mpsb_tree_node), cudaMemcpyDeviceToHost));
+  }
+};
+
+mpsb_cuda_model* export_model(mpsb_cuda_trainer* t, uint32_t tree_index, const TreeDownload& down,
                               bool with_predictions = true) {
   const TrainerDev& a = t->dev;
   PhaseTrace trace("export");
-  uint32_t rounds = 0;
-  CK(cudaMemcpy(&rounds, a.round_counter, sizeof rounds, cudaMemcpyDeviceToHost));
-  std::vector<uint32_t> counts(size_t(rounds) * a.n_trees);
-  if (!counts.empty())
-    CK(cudaMemcpy(counts.data(), a.model_counts, counts.size() * 4, cudaMemcpyDeviceToHost));
+  const uint32_t rounds = down.rounds;
   std::unique_ptr<mpsb_cuda_model> m(new mpsb_cuda_model);
   m->base = t->base_scores[tree_index];
   m->learning_rate = t->params.learning_rate;
@@ -1454,11 +1637,16 @@ mpsb_cuda_model* export_model(mpsb_cuda_trainer* t, uint32_t tree_index,
   m->n_trees = rounds;
   m->trees.resize(rounds);
   for (uint32_t r = 0; r < rounds; ++r) {
-    const uint32_t c = counts[size_t(r) * a.n_trees + tree_index];
+    const size_t k = size_t(r) * a.n_trees + tree_index;
+    const uint32_t c = down.counts[k];
+    if (!down.nodes.empty()) {
+      const mpsb_tree_node* nodes = down.nodes.data() + k * a.max_tree_nodes;
+      m->trees[r].assign(nodes, nodes + c);
+      continue;
+    }
     m->trees[r].resize(c);
-    CK(cudaMemcpy(m->trees[r].data(),
-                  a.model_nodes + (size_t(r) * a.n_trees + tree_index) * a.max_tree_nodes,
-                  size_t(c) * sizeof(mpsb_tree_node), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(m->trees[r].data(), a.model_nodes + k * a.max_tree_nodes, size_t(c) * sizeof(mpsb_tree_node),
+                  cudaMemcpyDeviceToHost));
   }
   trace.mark("trees");
   if (with_predictions) {
@@ -1477,7 +1665,7 @@ mpsb_cuda_model* export_model(mpsb_cuda_trainer* t, uint32_t tree_index,
 // A softmax model: K base scores, the trees of every (round, class) in that order, and
 // the training margins [rows][K].
 mpsb_cuda_model* export_softmax(mpsb_cuda_trainer* t) {
-  mpsb_cuda_model* m = export_model(t, 0, false);
+  mpsb_cuda_model* m = export_model(t, 0, TreeDownload(t->dev), false);
   const uint32_t K = t->softmax_classes;
   const TrainerDev& a = t->dev;
   m->class_count = K;
@@ -1551,7 +1739,7 @@ int mpsb_cuda_trainer_level_stats(const mpsb_cuda_trainer* t, uint32_t n_levels,
 int mpsb_cuda_trainer_export(mpsb_cuda_trainer* t, mpsb_cuda_model** out) {
   return guard([&] {
     t->synchronize();
-    *out = export_model(t, 0);
+    *out = export_model(t, 0, TreeDownload(t->dev));
   });
 }
 
@@ -1690,6 +1878,17 @@ int mpsb_cuda_autotune(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds, const 
   });
 }
 
+int mpsb_cuda_class_ids(const double* labels, uint64_t n, uint32_t limit, uint8_t* seen) {
+  if (!labels || !seen) return 0;
+  return class_ids(labels, n, limit, seen);
+}
+
+void mpsb_cuda_touch_pages(void* p, uint64_t bytes) {
+  const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE)), end = uintptr_t(p) + bytes;
+  for (uintptr_t at = uintptr_t(p); at < end; at = (at / page + 1) * page)
+    *reinterpret_cast<volatile unsigned char*>(at) = 0;
+}
+
 void mpsb_cuda_autotune_clear(void) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   g_tune_table.clear();
@@ -1704,7 +1903,7 @@ int mpsb_cuda_train_regressor(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     setup_trainer(t.get(), b, ds, labels, weights, n, p, options, 0);
     t->run(p->n_estimators);
     t->synchronize();
-    *out = export_model(t.get(), 0);
+    *out = export_model(t.get(), 0, TreeDownload(t->dev));
   });
 }
 
@@ -1714,17 +1913,13 @@ int mpsb_cuda_train_ovr(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
                         mpsb_cuda_model** out) {
   return guard([&] {
     if (n_classes < 2) throw TrainingError("one-vs-rest needs at least two classes");
-    bool ids = true;
-    for (uint64_t i = 0; i < n; ++i) {
-      const double y = labels[i];
-      ids &= (y >= 0.0) & (y < double(n_classes)) & (std::floor(y) == y);
-    }
-    if (!ids) throw TrainingError("one-vs-rest labels must be class ids in [0, n_classes)");
+    if (labels && !class_ids(labels, n, n_classes, nullptr)) throw TrainingError("one-vs-rest labels must be class ids in [0, n_classes)");
     std::unique_ptr<mpsb_cuda_trainer> t(new mpsb_cuda_trainer);
     setup_trainer(t.get(), b, ds, labels, weights, n, p, options, n_classes);
     t->run(p->n_estimators);
     t->synchronize();
-    for (uint32_t k = 0; k < n_classes; ++k) out[k] = export_model(t.get(), k);
+    const TreeDownload down(t->dev);
+    for (uint32_t k = 0; k < n_classes; ++k) out[k] = export_model(t.get(), k, down);
   });
 }
 
@@ -1802,6 +1997,7 @@ int mpsb_cuda_train_forest(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     size_t free_b = 0, total_b = 0;
     b->activate();
     CK(cudaMemGetInfo(&free_b, &total_b));
+    free_b += b->pool->kept();
     uint64_t batch = std::max<uint64_t>(1, (free_b / 2) / std::max<uint64_t>(per_tree, 1));
     if (const char* v = std::getenv("MPSB_FOREST_BATCH")) batch = std::max(1, std::atoi(v));
     batch = std::min<uint64_t>(batch, n_trees);
@@ -1856,7 +2052,8 @@ int mpsb_cuda_train_forest(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
       t->run(1);
       t->synchronize();
       trace.mark("growth");
-      for (uint32_t k = 0; k < B; ++k) out[t0 + k] = export_model(t.get(), k, false);
+      const TreeDownload down(t->dev);
+      for (uint32_t k = 0; k < B; ++k) out[t0 + k] = export_model(t.get(), k, down, false);
       trace.mark("export");
       t.reset();
       trace.mark("release");
@@ -1986,9 +2183,9 @@ void predict_trees(mpsb_cuda_backend* b, const std::vector<const std::vector<mps
     std::memcpy(host.data() + at_s, packed.steps.data(), sb);
     std::memcpy(host.data() + at_t, packed.trees.data(), tb);
     std::memcpy(host.data() + at_g, packed.groups.data(), gb);
-    DevBuf buf;
-    buf.alloc(at_out + size_t(ds->n_rows) * sizeof(double));
-    unsigned char* p = buf.as<unsigned char>();
+    DevArena mem;
+    mem.pool = b->pool;
+    unsigned char* p = static_cast<unsigned char*>(mem.alloc(at_out + size_t(ds->n_rows) * sizeof(double)));
     double* d_out = reinterpret_cast<double*>(p + at_out);
     cudaStream_t s = b->stream;
     CK(cudaMemcpyAsync(p, host.data(), at_out, cudaMemcpyHostToDevice, s));

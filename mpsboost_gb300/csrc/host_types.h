@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <list>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -63,6 +64,55 @@ inline void cuda_check(cudaError_t e, const char* what) {
 }
 #define CK(expr) ::mpsb::cuda_check((expr), #expr)
 
+// Device memory kept between a backend's calls, so that a fit does not map and unmap its
+// working state each time (cudaMalloc + cudaFree: 0.09 ms for 64 MB, 2 ms for 4 GB; a
+// 32-tree forest's release took 4.2 ms). At most 8 GiB stay, the oldest go first; all of it
+// is given back when an allocation fails and when the backend is gone. A block enters the
+// pool only after the backend's stream has finished with it (DevArena), so the next owner may
+// be any thread and stream.
+class DevicePool {
+ public:
+  static constexpr size_t kBlock = size_t(2) << 20;
+  static constexpr size_t kMost = size_t(8) << 30;
+  const int device;
+
+  DevicePool(int dev, cudaStream_t backend_stream);
+  ~DevicePool();
+  DevicePool(const DevicePool&) = delete;
+  DevicePool& operator=(const DevicePool&) = delete;
+  void* take(size_t* bytes);  // *bytes: the size wanted, then the block's
+  void give(void* p, size_t bytes);
+  void trim();
+  void close();  // the backend is going: nothing is kept from here on
+  bool idle();   // waits for the backend's stream
+  size_t kept() const;
+  static void trim_all();
+
+ private:
+  mutable std::mutex mutex_;
+  cudaStream_t stream_;  // null: closed
+  std::list<std::pair<void*, size_t>> free_;  // oldest first
+  size_t kept_ = 0;
+};
+
+// The device allocations of one session or call, released together once the backend's stream
+// is idle (work on any other stream must have been waited for). Small ones share blocks of 2 MB.
+class DevArena {
+ public:
+  std::shared_ptr<DevicePool> pool;
+
+  DevArena() = default;
+  ~DevArena();
+  DevArena(const DevArena&) = delete;
+  DevArena& operator=(const DevArena&) = delete;
+  void* alloc(size_t bytes);
+
+ private:
+  std::vector<std::pair<void*, size_t>> blocks_;
+  char* slab_ = nullptr;
+  size_t left_ = 0;
+};
+
 // Owning device allocation.
 struct DevBuf {
   void* p = nullptr;
@@ -79,7 +129,12 @@ struct DevBuf {
   void alloc(size_t n) {
     reset();
     if (n == 0) n = 16;
-    const cudaError_t e = cudaMalloc(&p, n);
+    cudaError_t e = cudaMalloc(&p, n);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      DevicePool::trim_all();
+      e = cudaMalloc(&p, n);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       throw BackendError("cudaMalloc of " + std::to_string(n) + " bytes failed: " +
@@ -111,6 +166,7 @@ struct mpsb_cuda_backend {
   int sm_count = 0;
   cudaDeviceProp prop{};
   mpsb::DevBuf error;  // one uint32 status word for standalone kernels
+  std::shared_ptr<mpsb::DevicePool> pool;  // working memory kept between calls
 
   void activate() const { CK(cudaSetDevice(device)); }
   uint32_t take_error() {
@@ -121,6 +177,7 @@ struct mpsb_cuda_backend {
     return e;
   }
   ~mpsb_cuda_backend() {
+    if (pool) pool->close();
     if (t0) cudaEventDestroy(t0);
     if (t1) cudaEventDestroy(t1);
     if (copy_stream) cudaStreamDestroy(copy_stream);

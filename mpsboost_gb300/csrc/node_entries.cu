@@ -22,13 +22,12 @@ namespace {
 
 // Device buffers and kernel arguments of one node-level call.
 struct Session {
-  std::vector<std::unique_ptr<DevBuf>> bufs;
+  DevArena mem;
   TrainerDev a{};
+  explicit Session(const mpsb_cuda_backend* b) { mem.pool = b->pool; }
   template <class T>
   T* alloc(size_t count) {
-    bufs.emplace_back(new DevBuf);
-    bufs.back()->alloc(count * sizeof(T));
-    return bufs.back()->as<T>();
+    return static_cast<T*>(mem.alloc(count * sizeof(T)));
   }
   template <class T>
   T* upload(const T* host, size_t count, cudaStream_t s) {
@@ -196,7 +195,7 @@ int mpsb_cuda_squared_error(mpsb_cuda_backend* b, const double* labels, const do
   return guard([&] {
     if (n == 0) throw TrainingError("Labels must not be empty");
     b->activate();
-    Session ss;
+    Session ss(b);
     cudaStream_t s = b->stream;
     const double* dl = ss.upload(labels, n, s);
     const double* dp = ss.upload(preds, n, s);
@@ -214,7 +213,7 @@ int mpsb_cuda_build_layer_histograms(mpsb_cuda_backend* b, const mpsb_cuda_datas
   return guard([&] {
     if (n_nodes == 0) return;
     b->activate();
-    Session ss;
+    Session ss(b);
     TreeState st;
     build_slots(ss, b, ds, rows, node_offsets, n_nodes, pairs, n_pairs, &st);
     check_ctl(ss.a, b->stream);
@@ -240,7 +239,7 @@ int mpsb_cuda_scan_splits(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     validate_tree_params(*p, ds->features);
     b->activate();
     cudaStream_t s = b->stream;
-    Session ss;
+    Session ss(b);
     TreeState st;
     const uint64_t offsets[2] = {0, n_rows};
     build_slots(ss, b, ds, rows, offsets, 1, pairs, n_pairs, &st);
@@ -313,7 +312,7 @@ int mpsb_cuda_partition_rows(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds,
     if (n_rows >= 0xFFFFFFFFull - ds->n_rows) throw UnsupportedError("too many rows in one call");
     b->activate();
     cudaStream_t s = b->stream;
-    Session ss;
+    Session ss(b);
     base_session(ss, b, ds);
     TrainerDev& a = ss.a;
     const std::vector<uint32_t> r32 = rows_u32(rows, n_rows, ds->n_rows, "Partition row index is out of bounds");

@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import os
 import subprocess
+import threading
 
 import numpy as np
 import pytest
@@ -215,3 +216,36 @@ def test_predict_edges(backend, rows, features, bins, nan, splits, shuffle):
     model = mb.RegressionModel(0.25, 0.1, trees)
     got = model.predict(backend, binned)
     assert got.tobytes() == _traverse(trees, 0.1, 0.25, binned.bins, binned.missing).tobytes()
+
+
+# Working memory kept between calls: fits of sizes that share, outgrow and split the kept blocks
+# give the same bytes again, on one backend and on two threads with one each; 600,000 rows also
+# take the result buffers mapped beside the training.
+@pytest.mark.parametrize("threads", [1, 2])
+def test_kept_memory_changes_nothing(threads):
+    shapes = [(600_000, 5, 255), (3_000, 70, 255), (40_000, 9, 700), (1_000, 3, 16), (45_000, 9, 700)]
+    data = []
+    for rows, features, bins in shapes:
+        x = seeded_matrix(rows, rows, features, 0.05)
+        data.append((x, *targets(x, rows), bins))
+
+    def fits(out):
+        b = mb.CudaBackend(0)
+        for _ in range(2):
+            for x, y, w, bins in data:
+                binned = mb.quantize_device(b, x, bins)
+                m = mb.train_regressor(b, binned, y, w, n_estimators=2, max_depth=4)
+                forest = mb.train_forest(b, binned, y, row_counts=np.ones((3, y.size), np.uint8),
+                                         feature_subsets=[np.array([0]), np.array([1, 2]), np.array([0, 2])], max_depth=3)
+                np.testing.assert_array_equal(m.train_predictions, m.predict(b, binned))
+                out.append((m.train_predictions.tobytes(), [t.tobytes() for f in [m, *forest] for t in f.trees]))
+                binned.close()
+
+    outs = [[] for _ in range(threads)]
+    pool = [threading.Thread(target=fits, args=(o,)) for o in outs]
+    for t in pool:
+        t.start()
+    for t in pool:
+        t.join()
+    for o in outs:
+        assert len(o) == 2 * len(data) and o == outs[0] and o[: len(data)] == o[len(data):]
