@@ -1562,6 +1562,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.tree_nodes = t->alloc<TreeNodeOut>(size_t(T) * tree_nodes);
   a.ctl = t->alloc<Control>(1);
   CK(cudaMemsetAsync(a.ctl, 0, sizeof(Control), s));
+  a.early_launch = 1;
   // Packed histogram limbs (MPSB_PACKED=0: split limbs only). A wide fixed-point cell packs
   // at most 127 rows of an item: items are kept to about 32 rows a bin.
   const char* packed = std::getenv("MPSB_PACKED");

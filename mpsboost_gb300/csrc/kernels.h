@@ -106,6 +106,7 @@ struct TrainerDev {
                                 // level: work items (a wide block's passes) that passed and
                                 // failed the packed-limb check (null: split limbs only)
   uint32_t item_rows_max;       // the adaptive item size's upper end (0: kItemRowsMax)
+  uint32_t early_launch;        // a round's kernels wait for one another on the device (launch_chained)
   uint32_t store_single;        // below the roots: a node of one row chunk is stored by its work
                                 // items, so its slot is not cleared (register-direct kernel)
   uint32_t item_rows;           // rows per histogram work item (<= kItemRowsMax); 0: the
