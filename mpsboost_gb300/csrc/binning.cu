@@ -9,11 +9,13 @@
 // number of boundaries below it (lower_bound).
 //
 // No sort: the order statistics come from a three-round radix selection over the 32-bit
-// order-preserving image of each float (11 + 11 + 10 bits). Round one histograms the top
-// 11 bits of every value of a feature; each target rank then names its bucket, and the
-// next round histograms the middle 11 bits of the values in those buckets only (at most
-// 256 target buckets per feature), and so on. Three passes over the column, shared- and
-// global-memory counters, and a per-feature selection block between passes.
+// order-preserving image of each float (16 + 8 + 8 bits; missing rows and the padding of a
+// column to 32 rows hold the largest key, which no value has). Round one counts the top 16
+// bits of every value of a feature; each target rank then names its bucket, and the next
+// round counts the next 8 bits of the values in those buckets only (at most 256 target
+// buckets per feature), and so on. Each round's 65,536 counters fit a CTA's shared memory as
+// 16-bit halves, and a CTA takes at most 65,535 rows of one feature, so a half cannot
+// overflow; a membership bitmap with prefix counts names a value's bucket.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,7 +30,8 @@ using namespace mpsb;
 namespace {
 
 constexpr int kTargets = 256;        // at most max_bins order statistics per feature
-constexpr uint32_t kNoSlot = 0xFFFFu;
+constexpr uint32_t kMissingKey = 0xFFFFFFFFu;
+constexpr uint32_t kDigits = 65536;  // counters of a round: 2^16 buckets, or 256 slots x 2^8
 constexpr uint32_t kErrInf = 1u;      // an Inf in the input
 constexpr uint32_t kErrRange = 2u;    // a float64 value outside the float32 range
 
@@ -50,76 +53,182 @@ __device__ __forceinline__ uint64_t quantile_rank(uint64_t part, uint64_t total,
 
 // Input element (row, feature) at byte offset row * rs + feature * cs; returns false with
 // an error bit for values the reference rejects.
-__device__ __forceinline__ float load_value(const uint8_t* data, int scalar_type, uint64_t rs,
-                                            uint64_t cs, uint64_t r, uint32_t f, uint32_t* err) {
+template <class T, bool ALIGNED>
+__device__ __forceinline__ T load_raw(const uint8_t* data, uint64_t rs, uint64_t cs, uint64_t r, uint32_t f) {
   const uint8_t* p = data + r * rs + uint64_t(f) * cs;
-  if (scalar_type == 1) {
-    float x;
-    memcpy(&x, p, sizeof x);
-    if (isinf(x)) *err |= kErrInf;
-    return x;
-  }
-  double x;
-  memcpy(&x, p, sizeof x);
+  T x;
+  if constexpr (ALIGNED) x = __ldg(reinterpret_cast<const T*>(p));
+  else memcpy(&x, p, sizeof x);  // a byte at a time
+  return x;
+}
+template <class T>
+__device__ __forceinline__ float checked_value(T x, uint32_t* err) {
   if (isnan(x)) return __uint_as_float(0x7FC00000u);
-  if (isinf(x)) {
-    *err |= kErrInf;
-    return 0.0f;
-  }
-  if (x > 3.4028234663852886e38 || x < -3.4028234663852886e38) *err |= kErrRange;
+  if (isinf(x)) *err |= kErrInf;
+  else if (fabs(x) > T(3.4028234663852886e38)) *err |= kErrRange;
   return float(x);  // correctly rounded, as the host's static_cast
 }
 
-// Input matrix -> feature-major order keys and missing flags, through a 32 x 32 tile so
-// both the row-major reads and the feature-major writes are coalesced.
-__global__ void keys_kernel(const uint8_t* data, int scalar_type, uint64_t rs, uint64_t cs,
-                            uint32_t n, uint32_t features, uint32_t* keys, uint8_t* missing,
-                            unsigned long long* miss_count, uint32_t* error) {
-  __shared__ float tile[32][33];
-  __shared__ uint32_t miss[32];
-  if (threadIdx.y == 0) miss[threadIdx.x] = 0;
-  const uint32_t r0 = blockIdx.x * 32, f0 = blockIdx.y * 32;
-  uint32_t err = 0;
+// Input matrix -> feature-major order keys (columns of `stride` >= n keys, the rest missing)
+// and, where `missing` is given, flags of stride n; through a tile of 128 rows x 32 features,
+// so both the row-major reads and the feature-major writes are coalesced. Sixteen loads in
+// flight per thread; a CTA takes tiles in turn and adds its missing counts once (added per
+// tile, the features' counters, sixteen to a cache line, set the time: 700 us for
+// 1,000,000 x 100 with 5 % missing, 338 now; 577 in 32 x 32 tiles).
+constexpr uint32_t kKeyRows = 128;
+template <class T, bool ALIGNED>
+__global__ void __launch_bounds__(256) keys_kernel(const uint8_t* data, uint64_t rs, uint64_t cs, uint32_t n, uint32_t features, size_t stride, uint32_t* keys,
+                                                   uint8_t* missing, unsigned long long* miss_count,
+                                                   uint32_t* error) {
+  __shared__ float tile[kKeyRows][33];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t f0 = blockIdx.y * 32;
+  uint32_t err = 0, gone[4] = {};
   // Lanes walk the matrix's contiguous direction: features for row-major input, rows for
   // column-major input (the tile is indexed [row][feature] either way).
   const bool row_major = cs < rs;
-  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
-    const uint32_t r = row_major ? r0 + i : r0 + threadIdx.x;
-    const uint32_t f = row_major ? f0 + threadIdx.x : f0 + i;
-    const float v = (r < n && f < features) ? load_value(data, scalar_type, rs, cs, r, f, &err) : 0.0f;
-    if (row_major) tile[i][threadIdx.x] = v;
-    else tile[threadIdx.x][i] = v;
-  }
-  __syncthreads();
-  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
-    const uint32_t f = f0 + i, r = r0 + threadIdx.x;
-    if (f < features && r < n) {
-      const float x = tile[threadIdx.x][i];
-      const size_t o = size_t(f) * n + r;
-      keys[o] = order_key(x);
-      missing[o] = isnan(x) ? 1 : 0;
-      if (isnan(x)) atomicAdd(&miss[i], 1u);
+  for (uint32_t r0 = blockIdx.x * kKeyRows; r0 < n; r0 += gridDim.x * kKeyRows) {
+    T v[16];
+#pragma unroll
+    for (uint32_t k = 0; k < 16; ++k) {  // past an edge: the last row or feature again, unused
+      const uint32_t i = warp * 16 + k;  // row, or (column-major) feature i / 4 and 32 rows
+      const uint32_t r = row_major ? i : (i & 3u) * 32 + lane, f = row_major ? lane : i >> 2;
+      v[k] = load_raw<T, ALIGNED>(data, rs, cs, min(r0 + r, n - 1), min(f0 + f, features - 1));
     }
+#pragma unroll
+    for (uint32_t k = 0; k < 16; ++k) {
+      const uint32_t i = warp * 16 + k;
+      const uint32_t r = row_major ? i : (i & 3u) * 32 + lane, f = row_major ? lane : i >> 2;
+      const float x = checked_value<T>(v[k], &err);
+      tile[r][f] = r0 + r < n ? x : __uint_as_float(0x7FC00000u);
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint32_t f = f0 + warp * 4 + q;
+      if (f >= features) break;
+#pragma unroll
+      for (uint32_t k = 0; k < kKeyRows / 32; ++k) {
+        const uint32_t r = r0 + k * 32 + lane;
+        if (r >= stride) break;
+        const float x = tile[k * 32 + lane][warp * 4 + q];
+        const bool nan = isnan(x);
+        keys[size_t(f) * stride + r] = nan ? kMissingKey : order_key(x);
+        if (r < n) {
+          if (missing != nullptr) missing[size_t(f) * n + r] = nan ? 1 : 0;
+          gone[q] += nan ? 1u : 0u;
+        }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    const uint32_t f = f0 + warp * 4 + q, sum = __reduce_add_sync(0xffffffffu, gone[q]);
+    if (lane == 0 && sum) atomicAdd(&miss_count[f], (unsigned long long)sum);
   }
   if (err) atomicOr(error, err);
-  __syncthreads();
-  if (threadIdx.y == 0 && miss[threadIdx.x] && f0 + threadIdx.x < features)
-    atomicAdd(&miss_count[f0 + threadIdx.x], (unsigned long long)miss[threadIdx.x]);
 }
 
-// Round one: per-feature histogram of the top 11 key bits of the non-missing values.
-__global__ void hist_top_kernel(const uint32_t* keys, const uint8_t* missing, uint32_t n,
-                                uint32_t* hist1) {
-  __shared__ uint32_t sh[2048];
-  const uint32_t f = blockIdx.y;
-  for (uint32_t i = threadIdx.x; i < 2048; i += blockDim.x) sh[i] = 0;
+// Rounds of the selection: counts of a digit of one feature's keys over a chunk of its rows
+// (at most 65,535: the counters are 16-bit halves). LEVEL 0: the top 16 bits. LEVEL 1 and 2:
+// the next 8 bits of the keys whose higher bits are a target's, counted per target bucket
+// (slot): the bucket's bit in bits1 (top 16 bits) or bits2 (slot, next 8 bits), its slot the
+// set bits before it. hist: [features][kDigits].
+// Reads each key once, 64 bytes in flight per thread; 1,000,000 x 100 takes 102, 218 and 205
+// us for the three rounds (11 + 11 + 10 bits with global counters and 4-byte loads: 502, 600,
+// 680).
+constexpr uint32_t kDigitThreads = 1024;
+constexpr uint32_t kBitWords = kDigits / 32;
+constexpr size_t digit_smem(int level) { return kDigits * 2 + size_t(level) * kBitWords * 6; }
+
+struct BucketSlots {  // in shared memory: membership bits, and the bits set before each word
+  uint32_t* bits;
+  uint16_t* before;
+
+  // Every thread of the CTA; `warp_sum` holds 33 words.
+  __device__ void load(const uint32_t* src, uint32_t* warp_sum) {
+    static_assert(kBitWords == 2 * kDigitThreads, "two words per thread");
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint2 w = reinterpret_cast<const uint2*>(src)[threadIdx.x];
+    const uint32_t own = __popc(w.x) + __popc(w.y);
+    uint32_t incl = own;
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= uint32_t(off)) incl += y;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    uint32_t base = incl - own;
+    for (uint32_t q = 0; q < warp; ++q) base += warp_sum[q];
+    reinterpret_cast<uint2*>(bits)[threadIdx.x] = w;
+    before[2 * threadIdx.x] = uint16_t(base);
+    before[2 * threadIdx.x + 1] = uint16_t(base + __popc(w.x));
+    __syncthreads();
+  }
+  __device__ bool find(uint32_t bucket, uint32_t* slot) const {
+    const uint32_t w = bits[bucket >> 5], bit = bucket & 31u;
+    if (!((w >> bit) & 1u)) return false;
+    *slot = before[bucket >> 5] + __popc(w & ((1u << bit) - 1u));
+    return true;
+  }
+};
+
+template <int LEVEL>
+__global__ void __launch_bounds__(kDigitThreads, 1) count_digits_kernel(const uint32_t* keys, size_t stride,
+                                                                        uint32_t chunk, const uint32_t* bits1,
+                                                                        const uint32_t* bits2, uint32_t* hist) {
+  extern __shared__ __align__(16) uint32_t cnt[];  // [kDigits / 2], then the bucket tables
+  __shared__ uint32_t warp_sum[33];
+  const uint32_t f = blockIdx.y, tid = threadIdx.x;
+  BucketSlots one, two;
+  one.bits = cnt + kDigits / 2;
+  one.before = reinterpret_cast<uint16_t*>(one.bits + kBitWords);
+  two.bits = reinterpret_cast<uint32_t*>(one.before + kBitWords);
+  two.before = reinterpret_cast<uint16_t*>(two.bits + kBitWords);
+  for (uint32_t i = tid; i < kDigits / 8; i += kDigitThreads) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0, 0, 0, 0);
+  if (LEVEL >= 1) one.load(bits1 + size_t(f) * kBitWords, warp_sum);
+  if (LEVEL >= 2) two.load(bits2 + size_t(f) * kBitWords, warp_sum);
   __syncthreads();
-  const size_t base = size_t(f) * n;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
-    if (!missing[base + r]) atomicAdd(&sh[keys[base + r] >> 21], 1u);
+  auto tally = [&](uint32_t k) {
+    uint32_t at = k >> 16;
+    if (LEVEL >= 1) {
+      uint32_t slot;
+      if (!one.find(at, &slot)) return;
+      at = slot * 256 + ((k >> 8) & 255u);
+      if (LEVEL >= 2) {
+        if (!two.find(at, &slot)) return;
+        at = slot * 256 + (k & 255u);
+      }
+    }
+    atomicAdd(&cnt[at >> 1], 1u << ((at & 1u) * 16));
+  };
+  const size_t r0 = size_t(blockIdx.x) * chunk;
+  const uint32_t quads = r0 < stride ? uint32_t(min(size_t(chunk), stride - r0) / 4) : 0u;
+  const uint4* src = reinterpret_cast<const uint4*>(keys + size_t(f) * stride + r0);
+  for (uint32_t q0 = tid; q0 < quads; q0 += 4 * kDigitThreads) {
+    uint4 v[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+      const uint32_t q = q0 + u * kDigitThreads;
+      v[u] = q < quads ? __ldg(src + q) : make_uint4(kMissingKey, kMissingKey, kMissingKey, kMissingKey);
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+      if (q0 + u * kDigitThreads >= quads) break;
+      tally(v[u].x);
+      tally(v[u].y);
+      tally(v[u].z);
+      tally(v[u].w);
+    }
+  }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < 2048; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist1[size_t(f) * 2048 + i], sh[i]);
+  uint32_t* out = hist + size_t(f) * kDigits;
+  for (uint32_t i = tid; i < kDigits / 2; i += kDigitThreads) {
+    const uint32_t w = cnt[i];
+    if (w & 0xFFFFu) atomicAdd(out + 2 * i, w & 0xFFFFu);
+    if (w >> 16) atomicAdd(out + 2 * i + 1, w >> 16);
+  }
 }
 
 // Per feature selection state between rounds.
@@ -129,107 +238,14 @@ struct Select {
   uint32_t rank[kTargets];     // residual rank inside the current bucket
   uint32_t prefix[kTargets];   // key bits chosen so far
   uint16_t slot[kTargets];     // bucket slot of the current round
-  uint16_t n_slots;
 };
 
-// Block scan of 2048 counters held 8 per thread (256 threads): exclusive prefix in place.
-__device__ void scan2048(uint32_t* c, uint32_t* total) {
-  __shared__ uint32_t part[256];
-  const int t = threadIdx.x;
-  uint32_t v[8], s = 0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    v[k] = c[t * 8 + k];
-    s += v[k];
-  }
-  part[t] = s;
-  __syncthreads();
-  for (int off = 1; off < 256; off <<= 1) {
-    const uint32_t y = t >= off ? part[t - off] : 0u;
-    __syncthreads();
-    part[t] += y;
-    __syncthreads();
-  }
-  uint32_t run = part[t] - s;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    c[t * 8 + k] = run;
-    run += v[k];
-  }
-  if (t == 255) *total = part[255];
-  __syncthreads();
-}
-
-// After round one: targets, their top-11-bit buckets and residual ranks, slots of the
-// distinct buckets (ranks are non-decreasing, so equal buckets are adjacent).
-__global__ void __launch_bounds__(256) select_top_kernel(const uint32_t* hist1, uint32_t max_bins,
-                                                         Select* sel, uint16_t* slot1) {
-  __shared__ uint32_t c[2048];
-  __shared__ uint32_t total;
-  __shared__ uint32_t bucket[kTargets];
-  const uint32_t f = blockIdx.x;
-  for (int i = threadIdx.x; i < 2048; i += blockDim.x) c[i] = hist1[size_t(f) * 2048 + i];
-  __syncthreads();
-  scan2048(c, &total);
-  Select& S = sel[f];
-  const uint32_t m = total;
-  const uint32_t desired = m < max_bins ? m : max_bins;
-  if (threadIdx.x == 0) {
-    S.m = m;
-    S.n_targets = desired;
-  }
-  const uint32_t j = threadIdx.x;
-  if (j < desired) {
-    const uint32_t rank = j + 1 < desired ? uint32_t(quantile_rank(j + 1, m, desired)) : m - 1;
-    uint32_t lo = 0, hi = 2048;  // last bucket whose prefix <= rank
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (c[mid] <= rank) lo = mid; else hi = mid;
-    }
-    bucket[j] = lo;
-    S.rank[j] = rank - c[lo];
-    S.prefix[j] = lo;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint16_t s = 0;
-    for (uint32_t k = 0; k < desired; ++k) {
-      if (k > 0 && bucket[k] != bucket[k - 1]) ++s;
-      S.slot[k] = s;
-      slot1[size_t(f) * 2048 + bucket[k]] = s;
-    }
-    S.n_slots = desired ? uint16_t(s + 1) : 0;
-  }
-}
-
-// Rounds two and three: histogram of the next digit of the values whose higher digits
-// select a target slot. level 1: middle 11 bits under slot1; level 2: low 10 bits under
-// (slot1, slot2).
-template <int LEVEL>
-__global__ void hist_next_kernel(const uint32_t* keys, const uint8_t* missing, uint32_t n,
-                                 const uint16_t* slot1, const uint16_t* slot2, uint32_t* hist) {
-  const uint32_t f = blockIdx.y;
-  const size_t base = size_t(f) * n;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    if (missing[base + r]) continue;
-    const uint32_t k = keys[base + r];
-    const uint32_t s1 = slot1[size_t(f) * 2048 + (k >> 21)];
-    if (s1 == kNoSlot) continue;
-    if (LEVEL == 1) {
-      atomicAdd(&hist[(size_t(f) * kTargets + s1) * 2048 + ((k >> 10) & 0x7FFu)], 1u);
-    } else {
-      const uint32_t s2 = slot2[(size_t(f) * kTargets + s1) * 2048 + ((k >> 10) & 0x7FFu)];
-      if (s2 == kNoSlot) continue;
-      atomicAdd(&hist[(size_t(f) * kTargets + s2) * 1024 + (k & 0x3FFu)], 1u);
-    }
-  }
-}
-
-// Exclusive count of the block's flags before the thread (kTargets threads), and the total.
+// Exclusive count of the block's flags before the thread, and the total (flags in the first
+// kTargets threads only).
 __device__ __forceinline__ uint32_t flags_before(bool flag, uint32_t* warp_sum, uint32_t* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t ballot = __ballot_sync(0xffffffffu, flag);
-  if (lane == 0) warp_sum[warp] = uint32_t(__popc(ballot));
+  if (lane == 0 && warp < kTargets / 32) warp_sum[warp] = uint32_t(__popc(ballot));
   __syncthreads();
   uint32_t before = uint32_t(__popc(ballot & ((1u << lane) - 1u))), all = 0;
 #pragma unroll
@@ -242,31 +258,21 @@ __device__ __forceinline__ uint32_t flags_before(bool flag, uint32_t* warp_sum, 
   return before;
 }
 
-// Selection of rounds two and three, a warp per target: the digit of its slot's histogram
-// that holds the residual rank, and the rank inside it. Lane l sums the counters of its
-// 1/32 of the digits, a warp prefix finds the lane that holds the rank, and the warp then
-// scans that lane's counters. (One thread per target walked up to 2,047 counters one load
-// after another: 190 us whatever the row count.)
-template <int LEVEL>
-__global__ void __launch_bounds__(256) select_digit_kernel(const uint32_t* hist, Select* sel) {
-  constexpr uint32_t D = LEVEL == 1 ? 2048 : 1024;
-  constexpr int SHIFT = LEVEL == 1 ? 11 : 10;
-  constexpr uint32_t PER = D / 32;  // counters per lane
-  const uint32_t f = blockIdx.x;
-  Select& S = sel[f];
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t j = blockIdx.y * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (j >= S.n_targets) return;
-  const uint32_t* h = hist + (size_t(f) * kTargets + S.slot[j]) * D;
-  const uint32_t rank = S.rank[j];
-  uint32_t own = 0;
-  const uint4* h4 = reinterpret_cast<const uint4*>(h + lane * PER);
-#pragma unroll
-  for (uint32_t q = 0; q < PER / 4; ++q) {
-    const uint4 v = __ldg(h4 + q);
-    own += v.x + v.y + v.z + v.w;
-  }
-  auto inclusive = [&](uint32_t x) -> uint32_t {
+// After round one: targets, their top-16-bit buckets and residual ranks, slots of the
+// distinct buckets (ranks are non-decreasing, so equal buckets are adjacent) and the
+// buckets' membership bits. A block per feature: 64 counters at a time are summed by a warp,
+// the 1,024 sums scanned, and a warp per target searches them and then its 64 counters.
+__global__ void __launch_bounds__(1024) select_top_kernel(const uint32_t* hist, uint32_t max_bins, Select* sel,
+                                                          uint32_t* bits) {
+  __shared__ uint32_t s_incl[1024], s_warp[32], s_bucket[kTargets], warp_sum[kTargets / 32];
+  const uint32_t f = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint2* h = reinterpret_cast<const uint2*>(hist + size_t(f) * kDigits);
+  auto pair_of = [&](uint32_t group) {
+    uint2 v = __ldg(h + group * 32 + lane);
+    if (group == 1023 && lane == 31) v.y = 0;  // the missing keys' bucket
+    return v;
+  };
+  auto inclusive = [&](uint32_t x) {
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
@@ -274,34 +280,100 @@ __global__ void __launch_bounds__(256) select_digit_kernel(const uint32_t* hist,
     }
     return x;
   };
-  // The first lane whose prefix passes the rank (the last lane where none does: the
-  // counters of a slot hold more values than its ranks).
-  const uint32_t incl = inclusive(own);
-  const uint32_t over = __ballot_sync(0xffffffffu, incl > rank);
-  const uint32_t who = over ? uint32_t(__ffs(over)) - 1u : 31u;
-  uint32_t rest = rank - __shfl_sync(0xffffffffu, incl - own, int(who));
-  uint32_t digit = who * PER;
-  for (uint32_t q = 0; q < PER; q += 32) {
-    const uint32_t c = __ldg(h + who * PER + q + lane);
-    const uint32_t x = inclusive(c);
-    const uint32_t past = __ballot_sync(0xffffffffu, x > rest);
-    if (past || q + 32 >= PER) {
-      const uint32_t at = past ? uint32_t(__ffs(past)) - 1u : 31u;
-      digit += q + at;
-      rest -= __shfl_sync(0xffffffffu, x - c, int(at));
-      break;
-    }
-    rest -= __shfl_sync(0xffffffffu, x, 31);
+  uint32_t own = 0;
+#pragma unroll 8
+  for (uint32_t g = 0; g < 32; ++g) {
+    const uint2 v = pair_of(warp * 32 + g);
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, v.x + v.y);
+    if (lane == g) own = sum;
   }
-  if (lane == 0) {
-    S.rank[j] = rest;
-    S.prefix[j] = (S.prefix[j] << SHIFT) | digit;
+  uint32_t incl = inclusive(own);
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  uint32_t m = 0;
+  for (uint32_t q = 0; q < 32; ++q) {
+    if (q == warp) incl += m;
+    m += s_warp[q];
+  }
+  s_incl[threadIdx.x] = incl;
+  __syncthreads();
+  Select& S = sel[f];
+  const uint32_t desired = m < max_bins ? m : max_bins;
+  if (threadIdx.x == 0) {
+    S.m = m;
+    S.n_targets = desired;
+  }
+  for (uint32_t j = warp; j < desired; j += 32) {
+    const uint32_t rank = j + 1 < desired ? uint32_t(quantile_rank(j + 1, m, desired)) : m - 1;
+    uint32_t lo = 0, hi = 1023;  // first group whose counts pass the rank
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (s_incl[mid] > rank) hi = mid; else lo = mid + 1;
+    }
+    uint32_t rest = rank - (lo ? s_incl[lo - 1] : 0u);
+    const uint2 v = pair_of(lo);
+    const uint32_t x = inclusive(v.x + v.y);
+    const uint32_t who = uint32_t(__ffs(__ballot_sync(0xffffffffu, x > rest))) - 1u;
+    if (lane == who) {
+      rest -= x - (v.x + v.y);
+      const uint32_t odd = rest >= v.x ? 1u : 0u;
+      S.rank[j] = rest - (odd ? v.x : 0u);
+      S.prefix[j] = s_bucket[j] = lo * 64 + 2 * lane + odd;
+    }
+  }
+  __syncthreads();
+  const uint32_t k = threadIdx.x;
+  const bool live = k < desired;
+  const bool starts = live && k > 0 && s_bucket[k] != s_bucket[k - 1];
+  uint32_t total;
+  const uint32_t s = flags_before(starts, warp_sum, &total) + (starts ? 1u : 0u);
+  if (live) {
+    S.slot[k] = uint16_t(s);
+    if (k == 0 || starts) atomicOr(bits + size_t(f) * kBitWords + (s_bucket[k] >> 5), 1u << (s_bucket[k] & 31u));
   }
 }
 
-// Slots of the distinct (top, middle) prefixes after round two (equal prefixes are
-// adjacent): a thread per target, block per feature.
-__global__ void __launch_bounds__(kTargets) assign_slots_kernel(Select* sel, uint16_t* slot2) {
+// Selection of rounds two and three, a warp per target: the digit of its slot's 256 counters
+// that holds the residual rank, and the rank inside it.
+__global__ void __launch_bounds__(256) select_digit_kernel(const uint32_t* hist, Select* sel) {
+  const uint32_t f = blockIdx.x;
+  Select& S = sel[f];
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t j = blockIdx.y * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (j >= S.n_targets) return;
+  const uint4* h = reinterpret_cast<const uint4*>(hist + size_t(f) * kDigits + size_t(S.slot[j]) * 256);
+  const uint4 p = __ldg(h + 2 * lane), q = __ldg(h + 2 * lane + 1);
+  const uint32_t c[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+  uint32_t own = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) own += c[k];
+  uint32_t incl = own;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= uint32_t(off)) incl += y;
+  }
+  // The lane whose counters hold the rank (a slot's counters hold more values than its ranks).
+  uint32_t rest = S.rank[j];
+  const uint32_t over = __ballot_sync(0xffffffffu, incl > rest);
+  const uint32_t who = over ? uint32_t(__ffs(over)) - 1u : 31u;
+  if (lane != who) return;
+  rest -= incl - own;
+  uint32_t digit = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 7; ++k) {
+    if (digit == k && rest >= c[k]) {
+      rest -= c[k];
+      digit = k + 1;
+    }
+  }
+  S.rank[j] = rest;
+  S.prefix[j] = (S.prefix[j] << 8) | (who * 8 + digit);
+}
+
+// Slots of the distinct 24-bit prefixes after round two (equal prefixes are adjacent) and
+// their membership bits: a thread per target, block per feature.
+__global__ void __launch_bounds__(kTargets) assign_slots_kernel(Select* sel, uint32_t* bits) {
   __shared__ uint32_t warp_sum[kTargets / 32];
   const uint32_t f = blockIdx.x, k = threadIdx.x;
   Select& S = sel[f];
@@ -311,7 +383,8 @@ __global__ void __launch_bounds__(kTargets) assign_slots_kernel(Select* sel, uin
   uint32_t total;
   const uint32_t s = flags_before(starts, warp_sum, &total) + (starts ? 1u : 0u);
   if (live) {
-    slot2[(size_t(f) * kTargets + S.slot[k]) * 2048 + (prefix & 0x7FFu)] = uint16_t(s);
+    const uint32_t bucket = uint32_t(S.slot[k]) * 256 + (prefix & 255u);
+    if (k == 0 || starts) atomicOr(bits + size_t(f) * kBitWords + (bucket >> 5), 1u << (bucket & 31u));
     S.slot[k] = uint16_t(s);
   }
 }
@@ -337,28 +410,98 @@ __global__ void __launch_bounds__(kTargets) finish_kernel(const Select* sel, flo
   if (k == 0) counts[f] = total;
 }
 
-// bin = lower_bound(boundaries, value) in float order (so -0 and +0 bin alike); missing
-// rows get bin 0 (their flag marks them).
-__global__ void transform_kernel(const uint32_t* keys, const uint8_t* missing, uint32_t n,
-                                 const float* bounds, const uint32_t* counts, uint8_t* bins) {
-  __shared__ float b[kTargets];
-  const uint32_t f = blockIdx.y;
-  const uint32_t nb = counts[f];
-  for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) b[i] = bounds[size_t(f) * kTargets + i];
+// bin = lower_bound(boundaries, value) in float order (so -0 and +0 bin alike): the 255
+// boundaries as a search tree in level order (+inf past the last), whose upper levels' few
+// nodes lie side by side in different shared-memory banks; the leaf reached is the count of
+// boundaries below the value.
+constexpr uint32_t kTreeNodes = 256;  // node 0 unused
+__device__ __forceinline__ void load_tree(const float* bounds, uint32_t nb, float* tree, uint32_t first,
+                                          uint32_t step) {
+  for (uint32_t k = first; k < kTreeNodes; k += step) {
+    if (k == 0) continue;
+    const uint32_t level = 31u - uint32_t(__clz(k));
+    const uint32_t at = ((2 * (k - (1u << level)) + 1) << (7 - level)) - 1;  // in order
+    tree[k] = at < nb ? bounds[at] : INFINITY;
+  }
+}
+__device__ __forceinline__ uint32_t tree_bin(const float* tree, float x) {
+  uint32_t k = 1;
+#pragma unroll
+  for (int level = 0; level < 8; ++level) k = 2 * k + (tree[k] < x ? 1u : 0u);
+  return k - kTreeNodes;
+}
+
+// Keys -> the u8 dataset's three copies of the bins (row-major rows of nfb * 32 bytes, column
+// blocks, feature-major), missing rows at kMissingSlot: 128 rows of a feature block at a time.
+// Each warp bins four features of the tile, 16 keys in flight per lane; the two row layouts
+// leave through shared memory in 16-byte pieces. 1,000,000 x 100: 357 us; binning to an
+// intermediate copy (750 us) and packing it (327 us) before.
+__global__ void __launch_bounds__(256) bin_pack_kernel(const uint32_t* keys, size_t stride, uint32_t n,
+                                                       uint32_t features, const float* bounds,
+                                                       const uint32_t* counts, uint8_t* out, uint8_t* out_blocked,
+                                                       uint8_t* out_fm) {
+  constexpr uint32_t kPitch = 36;  // bytes per tile row: nine words, no bank conflicts
+  __shared__ float tree[kBlockFeatures][kTreeNodes];
+  __shared__ __align__(16) uint8_t tile[128 * kPitch];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t fb = blockIdx.y, nfb = gridDim.y;
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    const uint32_t f = fb * kBlockFeatures + warp * 4 + q;
+    if (f < features) load_tree(bounds + size_t(f) * kTargets, counts[f], tree[warp * 4 + q], lane, 32);
+  }
   __syncthreads();
-  const size_t base = size_t(f) * n;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    uint32_t bin = 0;
-    if (!missing[base + r]) {
-      const float x = key_value(keys[base + r]);
-      uint32_t lo = 0, hi = nb;  // first boundary not less than x
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (b[mid] < x) lo = mid + 1; else hi = mid;
+  for (uint32_t r0 = blockIdx.x * 128; r0 < n; r0 += gridDim.x * 128) {
+    uint32_t key[4][4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint32_t f = fb * kBlockFeatures + warp * 4 + q;
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t r = r0 + k * 32 + lane;
+        key[q][k] = f < features && r < n ? __ldg(keys + size_t(f) * stride + r) : kMissingKey;
       }
-      bin = lo;
     }
-    bins[base + r] = uint8_t(bin);
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint32_t c = warp * 4 + q, f = fb * kBlockFeatures + c;
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t r = k * 32 + lane;
+        uint32_t bin = 0;
+        if (f < features) {
+          bin = key[q][k] == kMissingKey ? uint32_t(kMissingSlot) : tree_bin(tree[c], key_value(key[q][k]));
+          if (r0 + r < n) out_fm[size_t(f) * n + r0 + r] = uint8_t(bin);
+        }
+        tile[r * kPitch + c] = uint8_t(bin);
+      }
+    }
+    __syncthreads();
+    const uint32_t r = threadIdx.x >> 1, half = (threadIdx.x & 1u) * 16, row = r0 + r;
+    if (row < n) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(tile + r * kPitch + half);
+      const uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(out + (size_t(row) * nfb + fb) * kBlockFeatures + half) = v;
+      *reinterpret_cast<uint4*>(out_blocked + (size_t(fb) * n + row) * kBlockFeatures + half) = v;
+    }
+    __syncthreads();
+  }
+}
+
+// Feature-major bins (missing rows 0) and missing flags of stride n, for the datasets whose
+// bins fit u8 but whose missing slot does not (256 bins and missing values).
+__global__ void __launch_bounds__(256) transform_kernel(const uint32_t* keys, size_t stride, uint32_t n,
+                                                        const float* bounds, const uint32_t* counts,
+                                                        uint8_t* bins, uint8_t* missing) {
+  __shared__ float tree[kTreeNodes];
+  const uint32_t f = blockIdx.y;
+  load_tree(bounds + size_t(f) * kTargets, counts[f], tree, threadIdx.x, blockDim.x);
+  __syncthreads();
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    const uint32_t key = __ldg(keys + size_t(f) * stride + r);
+    const bool gone = key == kMissingKey;
+    bins[size_t(f) * n + r] = gone ? 0 : uint8_t(tree_bin(tree, key_value(key)));
+    missing[size_t(f) * n + r] = gone ? 1 : 0;
   }
 }
 
@@ -386,37 +529,68 @@ void check_view(const void* data, int scalar_type, uint64_t rows, uint32_t featu
   *extent = c;
 }
 
-// Upload the matrix and turn it into keys + missing flags.
-void make_keys(mpsb_cuda_backend* b, Scratch& ss, const void* data, int scalar_type, uint64_t rows,
-               uint32_t features, uint64_t rs, uint64_t cs, uint32_t** keys, uint8_t** missing,
-               std::vector<uint64_t>* missing_count) {
+// Order keys of an uploaded matrix: columns of `stride` keys and, for more than 256 bins,
+// missing flags.
+struct Keys {
+  uint32_t* keys = nullptr;
+  uint8_t* missing = nullptr;
+  size_t stride = 0;
+  uint32_t n = 0, features = 0;
+  std::vector<uint64_t> missing_count;
+};
+
+// Upload the matrix and turn it into keys. wide: unpadded columns, with missing flags.
+Keys make_keys(mpsb_cuda_backend* b, Scratch& ss, const void* data, int scalar_type, uint64_t rows,
+               uint32_t features, uint64_t rs, uint64_t cs, bool wide) {
   uint64_t extent = 0;
   check_view(data, scalar_type, rows, features, rs, cs, &extent);
   cudaStream_t s = b->stream;
   uint8_t* raw = ss.alloc<uint8_t>(extent);
   CK(cudaMemcpyAsync(raw, data, extent, cudaMemcpyHostToDevice, s));
-  const size_t cells = size_t(rows) * features;
-  *keys = ss.alloc<uint32_t>(cells);
-  *missing = ss.alloc<uint8_t>(cells);
+  Keys k;
+  k.n = uint32_t(rows);
+  k.features = features;
+  k.stride = wide ? rows : (rows + 31) / 32 * 32;
+  k.keys = ss.alloc<uint32_t>(k.stride * features);
+  if (wide) k.missing = ss.alloc<uint8_t>(size_t(rows) * features);
   unsigned long long* miss = ss.alloc<unsigned long long>(features);
   CK(cudaMemsetAsync(miss, 0, features * sizeof(unsigned long long), s));
   CK(cudaMemsetAsync(b->error.p, 0, sizeof(uint32_t), s));
-  const dim3 grid(uint32_t((rows + 31) / 32), (features + 31) / 32);
-  keys_kernel<<<grid, dim3(32, 8), 0, s>>>(raw, scalar_type, rs, cs, uint32_t(rows), features, *keys,
-                                             *missing, miss, b->error.as<uint32_t>());
+  const uint32_t blocks = (features + 31) / 32;
+  const dim3 grid(std::max(1u, std::min(uint32_t((rows + kKeyRows - 1) / kKeyRows), uint32_t(b->sm_count) * 8 / blocks + 1)),
+                  blocks);
+  // Strides of whole elements (the upload starts aligned): one load per value.
+  const uint64_t size = scalar_type == 1 ? 4 : 8;
+  const bool aligned = rs % size == 0 && cs % size == 0;
+  auto kernel = scalar_type == 1 ? (aligned ? keys_kernel<float, true> : keys_kernel<float, false>)
+                                 : (aligned ? keys_kernel<double, true> : keys_kernel<double, false>);
+  kernel<<<grid, 256, 0, s>>>(raw, rs, cs, k.n, features, k.stride, k.keys, k.missing, miss, b->error.as<uint32_t>());
   CK(cudaGetLastError());
-  missing_count->assign(features, 0);
-  CK(cudaMemcpyAsync(missing_count->data(), miss, features * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  k.missing_count.assign(features, 0);
+  CK(cudaMemcpyAsync(k.missing_count.data(), miss, features * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   const uint32_t e = b->take_error();  // synchronizes the stream
   if (e & kErrInf) throw DataError("Input matrix contains Inf");
   if (e & kErrRange) throw DataError("float64 input value exceeds the finite float32 range");
+  return k;
 }
 
-// Build the resident dataset from feature-major bins (u8 or u16: `width` bytes) and
-// missing flags on the device.
-mpsb_cuda_dataset* finish_dataset(mpsb_cuda_backend* b, const void* bins_fm, uint32_t width,
-                                  const uint8_t* missing, uint32_t rows, uint32_t features,
-                                  std::vector<uint32_t> bin_count, std::vector<uint64_t> missing_count) {
+// The counting passes of a selection over u8 bins: chunks of one feature, enough for two CTAs
+// per SM where the rows allow, at most 65,535 rows each.
+template <int LEVEL>
+void count_digits(mpsb_cuda_backend* b, const Keys& k, const uint32_t* bits1, const uint32_t* bits2, uint32_t* hist) {
+  static std::atomic<unsigned long long> configured{0};  // one bit per device
+  CK(opt_in_dynamic_smem(configured, count_digits_kernel<LEVEL>, digit_smem(LEVEL)));
+  const size_t want = (k.stride * k.features + 2 * size_t(b->sm_count) - 1) / (2 * size_t(b->sm_count));
+  const uint32_t chunk = uint32_t(std::min<size_t>(65504, std::max<size_t>(4096, (want + 31) / 32 * 32)));
+  const dim3 grid(uint32_t((k.stride + chunk - 1) / chunk), k.features);
+  count_digits_kernel<LEVEL><<<grid, kDigitThreads, digit_smem(LEVEL), b->stream>>>(k.keys, k.stride, chunk, bits1,
+                                                                                 bits2, hist);
+  CK(cudaGetLastError());
+}
+
+// A resident dataset's host tables and its per-feature device arrays, without bins.
+mpsb_cuda_dataset* start_dataset(mpsb_cuda_backend* b, uint32_t rows, uint32_t features,
+                                 std::vector<uint32_t> bin_count, std::vector<uint64_t> missing_count) {
   cudaStream_t s = b->stream;
   std::unique_ptr<mpsb_cuda_dataset> d(new mpsb_cuda_dataset);
   d->backend = b;
@@ -433,26 +607,59 @@ mpsb_cuda_dataset* finish_dataset(mpsb_cuda_backend* b, const void* bins_fm, uin
   d->has_missing.alloc(features);
   CK(cudaMemcpyAsync(d->bin_count.p, d->h_bin_count.data(), features * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d->has_missing.p, d->h_has_missing.data(), features, cudaMemcpyHostToDevice, s));
-  if (d->slots != uint32_t(kSlots)) {
-    d->bins16.alloc(size_t(d->nfb) * rows * kBlockFeatures * sizeof(uint16_t));
-    d->bins16_fm.alloc(size_t(features) * rows * sizeof(uint16_t));
-    for (uint32_t fb = 0; fb < d->nfb; ++fb) {
-      const size_t first = size_t(fb) * kBlockFeatures * rows;
-      CK(launch_pack_bins16_block(static_cast<const uint8_t*>(bins_fm) + first * width, width,
-                                  missing ? missing + first : nullptr,
-                                  d->bin_count.as<uint32_t>(), rows,
-                                  features, fb, d->slots, d->bins16.as<uint16_t>(),
-                                  d->bins16_fm.as<uint16_t>(), b->error.as<uint32_t>(), s));
-    }
-  } else {
+  return d.release();
+}
+
+// The dataset of feature-major bins (u8 or u16: `width` bytes) and missing flags.
+mpsb_cuda_dataset* finish_packed(mpsb_cuda_backend* b, std::unique_ptr<mpsb_cuda_dataset> d, const void* bins_fm,
+                               uint32_t width, const uint8_t* missing) {
+  const uint32_t rows = d->n_rows, features = d->features;
+  if (d->slots == uint32_t(kSlots)) {  // more than 256 bins asked for, no feature has them
     d->bins.alloc(size_t(d->nfb) * rows * kBlockFeatures);
     d->bins_blocked.alloc(size_t(d->nfb) * rows * kBlockFeatures);
     d->bins_fm.alloc(size_t(features) * rows);
     CK(launch_pack_bins(bins_fm, width, missing, d->bin_count.as<uint32_t>(), rows, features, d->nfb,
                         d->bins.as<uint8_t>(), d->bins_blocked.as<uint8_t>(), d->bins_fm.as<uint8_t>(),
-                        b->error.as<uint32_t>(), s));
+                        b->error.as<uint32_t>(), b->stream));
+    if (b->take_error()) throw DataError("Binned value exceeds the feature histogram range");
+    attach_bins_tmap(d.get());
+    return d.release();
+  }
+  d->bins16.alloc(size_t(d->nfb) * rows * kBlockFeatures * sizeof(uint16_t));
+  d->bins16_fm.alloc(size_t(features) * rows * sizeof(uint16_t));
+  for (uint32_t fb = 0; fb < d->nfb; ++fb) {
+    const size_t first = size_t(fb) * kBlockFeatures * rows;
+    CK(launch_pack_bins16_block(static_cast<const uint8_t*>(bins_fm) + first * width, width, missing + first,
+                                d->bin_count.as<uint32_t>(), rows, features, fb, d->slots, d->bins16.as<uint16_t>(),
+                                d->bins16_fm.as<uint16_t>(), b->error.as<uint32_t>(), b->stream));
   }
   if (b->take_error()) throw DataError("Binned value exceeds the feature histogram range");
+  return d.release();
+}
+
+// The dataset of at most 256 bins a feature from its keys and boundaries ([features][kTargets]
+// with their counts, on the device).
+mpsb_cuda_dataset* finish_narrow(mpsb_cuda_backend* b, Scratch& ss, const Keys& k, const float* bounds,
+                                 const uint32_t* counts, std::vector<uint32_t> bin_count) {
+  std::unique_ptr<mpsb_cuda_dataset> d(start_dataset(b, k.n, k.features, std::move(bin_count), k.missing_count));
+  cudaStream_t s = b->stream;
+  const uint32_t n = k.n;
+  if (d->slots != uint32_t(kSlots)) {
+    uint8_t* bins_fm = ss.alloc<uint8_t>(size_t(k.features) * n);
+    uint8_t* missing = ss.alloc<uint8_t>(size_t(k.features) * n);
+    const dim3 grid(std::max(1u, std::min((n + 255) / 256, uint32_t(b->sm_count) * 8 / k.features + 1)), k.features);
+    transform_kernel<<<grid, 256, 0, s>>>(k.keys, k.stride, n, bounds, counts, bins_fm, missing);
+    CK(cudaGetLastError());
+    return finish_packed(b, std::move(d), bins_fm, 1, missing);
+  }
+  d->bins.alloc(size_t(d->nfb) * n * kBlockFeatures);
+  d->bins_blocked.alloc(size_t(d->nfb) * n * kBlockFeatures);
+  d->bins_fm.alloc(size_t(k.features) * n);
+  const dim3 grid(std::max(1u, std::min((n + 127) / 128, uint32_t(b->sm_count) * 6 / d->nfb + 1)), d->nfb);
+  bin_pack_kernel<<<grid, 256, 0, s>>>(k.keys, k.stride, n, k.features, bounds, counts, d->bins.as<uint8_t>(),
+                                       d->bins_blocked.as<uint8_t>(), d->bins_fm.as<uint8_t>());
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(s));
   attach_bins_tmap(d.get());
   return d.release();
 }
@@ -465,7 +672,6 @@ mpsb_cuda_dataset* finish_dataset(mpsb_cuda_backend* b, const void* bins_fm, uin
 // last and the first m keys of a feature are its non-missing values in order.
 constexpr int kSortThreads = 256;
 constexpr uint32_t kSortTile = 4096;  // keys per (feature, tile) block
-constexpr uint32_t kMissingKey = 0xFFFFFFFFu;
 
 __global__ void sort_keys_init_kernel(const uint32_t* keys, const uint8_t* missing, size_t cells,
                                       uint32_t* out) {
@@ -741,26 +947,23 @@ int mpsb_cuda_dataset_quantize(mpsb_cuda_backend* b, const void* data, int scala
     b->activate();
     cudaStream_t s = b->stream;
     Scratch ss(b);
-    uint32_t* keys = nullptr;
-    uint8_t* missing = nullptr;
-    std::vector<uint64_t> missing_count;
-    make_keys(b, ss, data, scalar_type, rows, features, row_stride, col_stride, &keys, &missing,
-              &missing_count);
-    const uint32_t n = uint32_t(rows);
+    const bool wide = max_bins > uint32_t(kTargets);
+    Keys k = make_keys(b, ss, data, scalar_type, rows, features, row_stride, col_stride, wide);
+    const uint32_t n = k.n;
     // Schema on the host: per feature the boundary count and `stride` boundary slots.
     std::vector<uint32_t> h_counts(features);
     std::vector<float> h_bounds;
     size_t stride = 0;
     std::unique_ptr<mpsb_cuda_dataset> d;
-    if (max_bins > uint32_t(kTargets)) {
+    if (wide) {
       stride = max_bins - 1;
       float* bounds = ss.alloc<float>(size_t(features) * stride);
       uint32_t* counts = ss.alloc<uint32_t>(features);
       uint16_t* bins16 = ss.alloc<uint16_t>(size_t(features) * n);
-      quantize_wide(s, ss, keys, missing, missing_count, n, features, max_bins, bounds, counts, bins16);
+      quantize_wide(s, ss, k.keys, k.missing, k.missing_count, n, features, max_bins, bounds, counts, bins16);
       const dim3 grid(std::max(1u, std::min((n + 255) / 256, uint32_t(b->sm_count) * 4 / std::max(1u, features) + 1)),
                       features);
-      transform_wide_kernel<<<grid, 256, 0, s>>>(keys, missing, n, bounds, stride, counts, bins16);
+      transform_wide_kernel<<<grid, 256, 0, s>>>(k.keys, k.missing, n, bounds, stride, counts, bins16);
       CK(cudaGetLastError());
       h_bounds.resize(size_t(features) * stride);
       CK(cudaMemcpyAsync(h_counts.data(), counts, features * 4, cudaMemcpyDeviceToHost, s));
@@ -768,42 +971,30 @@ int mpsb_cuda_dataset_quantize(mpsb_cuda_backend* b, const void* data, int scala
       CK(cudaStreamSynchronize(s));
       std::vector<uint32_t> bin_count(features);
       for (uint32_t f = 0; f < features; ++f) bin_count[f] = h_counts[f] + 1;
-      d.reset(finish_dataset(b, bins16, 2, missing, n, features, bin_count, missing_count));
+      d.reset(start_dataset(b, n, features, bin_count, k.missing_count));
+      d.reset(finish_packed(b, std::move(d), bins16, 2, k.missing));
     } else {
-      uint32_t* hist1 = ss.alloc<uint32_t>(size_t(features) * 2048);
-      uint32_t* hist2 = ss.alloc<uint32_t>(size_t(features) * kTargets * 2048);
-      uint32_t* hist3 = ss.alloc<uint32_t>(size_t(features) * kTargets * 1024);
-      uint16_t* slot1 = ss.alloc<uint16_t>(size_t(features) * 2048);
-      uint16_t* slot2 = ss.alloc<uint16_t>(size_t(features) * kTargets * 2048);
+      // Three rounds' counters and two rounds' membership bits, cleared together.
+      const size_t digits = size_t(features) * kDigits, words = size_t(features) * kBitWords;
+      uint32_t* hist = ss.alloc<uint32_t>(3 * digits + 2 * words);
+      uint32_t *bits1 = hist + 3 * digits, *bits2 = bits1 + words;
       Select* sel = ss.alloc<Select>(features);
       float* bounds = ss.alloc<float>(size_t(features) * kTargets);
       uint32_t* counts = ss.alloc<uint32_t>(features);
-      uint8_t* bins_fm = ss.alloc<uint8_t>(size_t(features) * n);
-      CK(cudaMemsetAsync(hist1, 0, size_t(features) * 2048 * 4, s));
-      CK(cudaMemsetAsync(hist2, 0, size_t(features) * kTargets * 2048 * 4, s));
-      CK(cudaMemsetAsync(hist3, 0, size_t(features) * kTargets * 1024 * 4, s));
-      CK(cudaMemsetAsync(slot1, 0xFF, size_t(features) * 2048 * 2, s));
-      CK(cudaMemsetAsync(slot2, 0xFF, size_t(features) * kTargets * 2048 * 2, s));
-      const dim3 grid(std::max(1u, std::min((n + 255) / 256, uint32_t(b->sm_count) * 4 / std::max(1u, features) + 1)),
-                      features);
-      hist_top_kernel<<<grid, 256, 0, s>>>(keys, missing, n, hist1);
-      CK(cudaGetLastError());
-      select_top_kernel<<<features, 256, 0, s>>>(hist1, max_bins, sel, slot1);
-      CK(cudaGetLastError());
-      hist_next_kernel<1><<<grid, 256, 0, s>>>(keys, missing, n, slot1, slot2, hist2);
-      CK(cudaGetLastError());
+      CK(cudaMemsetAsync(hist, 0, (3 * digits + 2 * words) * sizeof(uint32_t), s));
       const dim3 targets(features, kTargets / 8);  // eight targets (warps) per block
-      select_digit_kernel<1><<<targets, 256, 0, s>>>(hist2, sel);
+      count_digits<0>(b, k, nullptr, nullptr, hist);
+      select_top_kernel<<<features, 1024, 0, s>>>(hist, max_bins, sel, bits1);
       CK(cudaGetLastError());
-      assign_slots_kernel<<<features, kTargets, 0, s>>>(sel, slot2);
+      count_digits<1>(b, k, bits1, nullptr, hist + digits);
+      select_digit_kernel<<<targets, 256, 0, s>>>(hist + digits, sel);
       CK(cudaGetLastError());
-      hist_next_kernel<2><<<grid, 256, 0, s>>>(keys, missing, n, slot1, slot2, hist3);
+      assign_slots_kernel<<<features, kTargets, 0, s>>>(sel, bits2);
       CK(cudaGetLastError());
-      select_digit_kernel<2><<<targets, 256, 0, s>>>(hist3, sel);
+      count_digits<2>(b, k, bits1, bits2, hist + 2 * digits);
+      select_digit_kernel<<<targets, 256, 0, s>>>(hist + 2 * digits, sel);
       CK(cudaGetLastError());
       finish_kernel<<<features, kTargets, 0, s>>>(sel, bounds, counts);
-      CK(cudaGetLastError());
-      transform_kernel<<<grid, 256, 0, s>>>(keys, missing, n, bounds, counts, bins_fm);
       CK(cudaGetLastError());
       // Schema back to the host.
       stride = kTargets;
@@ -816,9 +1007,9 @@ int mpsb_cuda_dataset_quantize(mpsb_cuda_backend* b, const void* data, int scala
       std::vector<uint32_t> bin_count(features);
       for (uint32_t f = 0; f < features; ++f) {
         bin_count[f] = h_counts[f] + 1;
-        if (missing_count[f] + h_sel[f].m != rows) throw BackendError("device binning lost rows");
+        if (k.missing_count[f] + h_sel[f].m != rows) throw BackendError("device binning lost rows");
       }
-      d.reset(finish_dataset(b, bins_fm, 1, missing, n, features, bin_count, missing_count));
+      d.reset(finish_narrow(b, ss, k, bounds, counts, bin_count));
     }
     d->max_bins = max_bins;
     d->boundary_offset.resize(features);
@@ -848,13 +1039,9 @@ int mpsb_cuda_dataset_transform(mpsb_cuda_backend* b, const mpsb_cuda_dataset* s
     b->activate();
     cudaStream_t s = b->stream;
     Scratch ss(b);
-    uint32_t* keys = nullptr;
-    uint8_t* missing = nullptr;
-    std::vector<uint64_t> missing_count;
-    make_keys(b, ss, data, scalar_type, rows, features, row_stride, col_stride, &keys, &missing,
-              &missing_count);
-    const uint32_t n = uint32_t(rows);
     const bool wide = schema->max_bins > uint32_t(kTargets);
+    Keys k = make_keys(b, ss, data, scalar_type, rows, features, row_stride, col_stride, wide);
+    const uint32_t n = k.n;
     const size_t stride = wide ? schema->max_bins - 1 : size_t(kTargets);
     std::vector<float> h_bounds(size_t(features) * stride, 0.0f);
     for (uint32_t f = 0; f < features; ++f)
@@ -870,14 +1057,12 @@ int mpsb_cuda_dataset_transform(mpsb_cuda_backend* b, const mpsb_cuda_dataset* s
     std::unique_ptr<mpsb_cuda_dataset> d;
     if (wide) {
       uint16_t* bins16 = ss.alloc<uint16_t>(size_t(features) * n);
-      transform_wide_kernel<<<grid, 256, 0, s>>>(keys, missing, n, bounds, stride, counts, bins16);
+      transform_wide_kernel<<<grid, 256, 0, s>>>(k.keys, k.missing, n, bounds, stride, counts, bins16);
       CK(cudaGetLastError());
-      d.reset(finish_dataset(b, bins16, 2, missing, n, features, schema->h_bin_count, missing_count));
+      d.reset(start_dataset(b, n, features, schema->h_bin_count, k.missing_count));
+      d.reset(finish_packed(b, std::move(d), bins16, 2, k.missing));
     } else {
-      uint8_t* bins_fm = ss.alloc<uint8_t>(size_t(features) * n);
-      transform_kernel<<<grid, 256, 0, s>>>(keys, missing, n, bounds, counts, bins_fm);
-      CK(cudaGetLastError());
-      d.reset(finish_dataset(b, bins_fm, 1, missing, n, features, schema->h_bin_count, missing_count));
+      d.reset(finish_narrow(b, ss, k, bounds, counts, schema->h_bin_count));
     }
     d->max_bins = schema->max_bins;
     d->boundaries = schema->boundaries;

@@ -55,6 +55,29 @@ def test_quantize_matches_host(backend, rows, cols, max_bins):
     _same(mb.quantize_device(backend, x, max_bins), mb.quantize_dense(x, max_bins))
 
 
+# Rows around a column's padding, a tile of 128 rows and a counting pass's 65,504; features
+# around a block of 32; values that share their top 16 or 24 key bits, NaNs of either sign,
+# columns of few values; 255 boundaries, and 256 bins with missing cells (the wide layout).
+@pytest.mark.parametrize("rows", [31, 33, 129, 4097, 65_504, 65_537, 200_003])
+@pytest.mark.parametrize("features,max_bins", [(5, 255), (33, 256), (32, 17)])
+@pytest.mark.parametrize("missing", [False, True])
+def test_selection_edges(backend, rows, features, max_bins, missing):
+    rng = np.random.default_rng(rows)
+    x = rng.normal(size=(rows, features)).astype(np.float32)
+    near = (1.0 + rng.integers(0, 1 << 12, rows) * 2.0**-23).astype(np.float32)
+    x[:, 0] = near * np.where(rng.random(rows) < 0.3, -1, 1)          # one bucket of top bits a sign
+    x[:, 1] = (1.0 + rng.integers(0, 200, rows) * 2.0**-23).astype(np.float32)  # one 24-bit prefix
+    x[:, 2] = rng.integers(0, 3, rows) - 1
+    x[:, 3] = np.ldexp(1.0, rng.integers(-140, 127, rows)).astype(np.float32)
+    if missing:
+        gone = rng.random((rows, features)) < 0.1
+        x[gone] = np.where(rng.random(gone.sum()) < 0.5, np.nan, -np.nan)
+    dev, host = mb.quantize_device(backend, x, max_bins), mb.quantize_dense(x, max_bins)
+    _same(dev, host)
+    y = x[::-1] * np.float32(1.01)
+    _same(dev.transform(y), host.transform(y))
+
+
 def test_layouts_and_dtypes(backend):
     x = _matrix(3, 5000, 9)
     host = mb.quantize_dense(x, 128)
