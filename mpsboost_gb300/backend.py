@@ -430,8 +430,9 @@ class CudaBackend:
                 self.handle, dev.handle, ptr(rows), ptr(offsets), len(parts), ptr(g), g.shape[0], ptr(out)
             )
         )
-        splits = np.cumsum(dataset.bin_counts)[:-1]
-        return [np.split(out[i * per_node : (i + 1) * per_node], splits) for i in range(len(parts))]
+        ends = np.cumsum(dataset.bin_counts, dtype=np.int64).tolist()
+        spans = list(zip([0] + ends[:-1], ends))
+        return [[out[i * per_node + a : i * per_node + b] for a, b in spans] for i in range(len(parts))]
 
     def histograms(self, dataset: BinnedDataset, labels, predictions, rows) -> dict:
         """The reference hook's shape: squared-error pairs, then one node's histograms."""

@@ -249,3 +249,43 @@ def test_kept_memory_changes_nothing(threads):
         t.join()
     for o in outs:
         assert len(o) == 2 * len(data) and o == outs[0] and o[: len(data)] == o[len(data):]
+
+
+# Node-level calls convert their inputs and results on the device: row sets around a warp and a
+# CTA, few-valued and missing features on u8 and u16 pages, bit-exact to the replica; the first
+# error in the checks' order, rows before pairs, and scales of tiny and of zero pairs.
+@pytest.mark.parametrize("bins", [5, 255, 700])
+@pytest.mark.parametrize("rows", [1, 31, 257, 70_001])
+@pytest.mark.parametrize("scale", [1.0, 1e-30, 0.0])
+def test_node_histograms_edges(backend, port, bins, rows, scale):
+    n = 70_001
+    x = seeded_matrix(bins, n, 35, 0.1, 6)
+    binned, ds = mb.quantize_dense(x, bins), port.quantize_dense(x, bins)
+    rng = np.random.default_rng(rows)
+    pairs = np.column_stack([rng.normal(size=n), rng.uniform(0.0, 2.0, n)]) * scale
+    sel = rng.permutation(n)[:rows]
+    p32 = pairs.astype(np.float32)
+    kg, kh = port.fixed_scales(p32)
+    want, miss = port.fixed_histograms(ds, p32, kg, kh, sel)
+    for got in backend.layer_histograms(binned, pairs, [sel, sel]):
+        for f, (gf, wf) in enumerate(zip(got, want)):
+            total = {k: wf[k].copy() for k in ("count", "gradient_q", "hessian_q")}
+            for k in total:
+                total[k][0] += miss[f][k]
+            np.testing.assert_array_equal(gf["count"], total["count"])
+            np.testing.assert_array_equal(gf["gradient_sum"], total["gradient_q"].astype(np.float64) * 2.0 ** -kg)
+            np.testing.assert_array_equal(gf["hessian_sum"], total["hessian_q"].astype(np.float64) * 2.0 ** -kh)
+
+
+def test_node_histogram_errors_keep_their_order(backend):
+    binned = mb.quantize_dense(seeded_matrix(1, 300, 3), 16)
+    pairs = np.ones((300, 2))
+    def bad(at, value):
+        p = pairs.copy()
+        p[at] = value
+        return p
+    for p, rows, match in [(bad((7, 1), -1.0), [1, 300], "out of bounds"), (bad((7, 1), -1.0), [1], "non-negative"),
+                           (bad((299, 0), np.nan), [1], "finite"), (bad((0, 0), 1e39), [1], "float32 range"),
+                           (bad((0, 0), 1e39), [1, 2**40], "out of bounds")]:
+        with pytest.raises(mb.TrainingError, match=match):
+            backend.layer_histograms(binned, p, [rows])
