@@ -1311,7 +1311,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   // SMs; MPSB_SCAN_THREADS overrides (a multiple of 32, at most 512).
   a.scan_threads = 128;
   // rows per histogram work item: chosen per level on the device (about three items per
-  // SM, within the 2^16-row limb bound)
+  // SM, one for wide datasets, within the 2^16-row limb bound)
   a.item_rows = 0;
   // Squared error and quantile have h = 1 per row; without weights every row's quantized
   // hessian is the same unit (MPSB_UNIT_HESS=0 builds the hessian limbs anyway).
@@ -1770,7 +1770,7 @@ int mpsb_cuda_autotune(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds, const 
     cur.hist_threads = uint32_t(t->hcfg.threads);
     cur.hist_stages = uint32_t(t->hcfg.stages);
     cur.root_threads = uint32_t(t->hcfg.root_threads);
-    cur.items_per_sm = t->dev.items_per_sm ? t->dev.items_per_sm : 3u;
+    cur.items_per_sm = t->dev.items_per_sm ? t->dev.items_per_sm : default_items_per_sm(ds->slots);
     cur.blocked_levels = t->blocked_levels;
     cur.scan_threads = t->dev.scan_threads;
     const uint32_t min_scan = t->dev.scan_threads;  // the chunk tables are sized for it

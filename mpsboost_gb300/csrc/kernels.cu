@@ -45,17 +45,37 @@ __device__ __forceinline__ uint32_t dataset_feature(const TrainerDev& a, uint32_
   return a.feature_of ? a.feature_of[size_t(tree) * a.features + f] : f;
 }
 
-// Rows per histogram work item for a level that builds `rows` rows: about per_sm (default
-// three) items per SM, a multiple of 512, within [1024, item_rows_max]. Where the
-// upper end forces more items, their number is raised to the next multiple of the
+constexpr uint64_t kLongItemRows = 12288;
+
+// Work items per SM a level is cut into. u8 datasets: three, two while the level has fewer
+// than eight nodes. Wide ones: one, because each of an item's passes zeroes and flushes
+// 200 KB whatever its rows (three items: 12.5 -> 10.2 ms for 1,000,000 x 64 at 1,024 bins
+// with one, 18.7 -> 15.7 at 2,000, 8.3 -> 7.7 at 300).
+__device__ __forceinline__ uint32_t level_items_per_sm(const TrainerDev& a, uint32_t nodes) {
+  const uint32_t base = a.items_per_sm ? a.items_per_sm : default_items_per_sm(a.slots);
+  return nodes < 8 && base > 2 ? base - 1 : base;
+}
+
+// Rows per histogram work item for a level that builds `rows` rows of `nodes` nodes: about
+// per_sm items per SM, a multiple of 512, within [1024, item_rows_max]. Every node's last item
+// is cut short, by half on average, so that many items fewer are aimed at: without that a
+// level overshoots its multiple of the SM count and ends in a wave of a few items
+// (one-vs-rest of ten classes 15.1 -> 14.5 ms, 1,024 bins 9.9 -> 9.4). One more per SM from
+// eight nodes on where the items still hold kLongItemRows rows: a large level ends more evenly
+// with more of them, and their flushes hardly count (10,000,000 x 128: 76.4 ms without, 75.8
+// with; the same from 8,192 rows, 76.4 from 16,384). Where the upper end
+// forces more items, their number is raised to the next multiple of the
 // SM count, so that the persistent CTAs end the level together. At the lower end an item's
 // reductions (about 1.5 us) weigh as much as its flush: 100,000 x 32, depth 6, 50 trees
 // take 17.5, 17.3, 17.7 and 18.7 ms with items of 512, 1,024, 2,048 and 4,096 rows.
-__device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, const TrainerDev& a, uint32_t per_sm) {
+__device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, const TrainerDev& a, uint32_t per_sm,
+                                                      uint32_t nodes) {
   const uint64_t n_sm = a.sm_count ? a.sm_count : 152;
   const uint32_t nfb = a.nfb;
   const uint32_t most = a.item_rows_max ? a.item_rows_max : kItemRowsMax;
-  uint64_t target = n_sm * (per_sm ? per_sm : 3);
+  if (a.slots == uint32_t(kSlots) && nodes >= 8 && rows * nfb >= kLongItemRows * n_sm * (per_sm + 1)) ++per_sm;
+  uint64_t target = n_sm * per_sm;
+  if (uint64_t(nodes) * nfb <= target) target -= uint64_t(nodes) * nfb / 2;
   const uint64_t min_items = (rows * nfb + most - 1) / most;
   if (target < min_items) target = (min_items + n_sm - 1) / n_sm * n_sm;
   uint64_t per = (rows * nfb + target - 1) / target;
@@ -234,7 +254,7 @@ __device__ __noinline__ void round_setup(const TrainerDev& a, bool g_only) {
     uint64_t total = 0;
     for (uint32_t t = 0; t < a.n_trees; ++t) total += root_rows(a, t);
     const uint32_t item_rows =
-        a.item_rows ? a.item_rows : adaptive_item_rows(total, a, a.items_per_sm);
+        a.item_rows ? a.item_rows : adaptive_item_rows(total, a, a.items_per_sm ? a.items_per_sm : default_items_per_sm(a.slots), a.n_trees);
     uint32_t acc = 0;
     for (uint32_t t = 0; t < a.n_trees; ++t) {
       a.build_prefix[t] = acc;
@@ -1988,10 +2008,9 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
   // with a partial last chunk) the other way round: one item fewer below 8 nodes here,
   // one more from 8 (measured on the 10M x 128 workload: 2 best for depths 1-3, 4 for
   // depths 4-7).
-  const uint32_t base_per_sm = a.items_per_sm ? a.items_per_sm : 3u;
-  const uint32_t level_per_sm = n >= 8 ? base_per_sm + 1 : (base_per_sm > 2 ? base_per_sm - 1 : base_per_sm);
+  const uint32_t level_per_sm = level_items_per_sm(a, n);
   const uint32_t item_rows =
-      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(built_units) * 256, a, level_per_sm);
+      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(built_units) * 256, a, level_per_sm, n);
 
   // Phase B1: acceptance under max_leaves, accepted prefix, chunk prefixes.
   // Scanned values: 0 accepted, 1 build chunks, 2 partition chunks, 3 leaf segments,
@@ -2281,10 +2300,9 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
   const uint32_t ord = first ? v3[2] : (i < n ? v3[2] - 1 : 0u);
   if (first) s_valid_base[ord] = v3[0];
   __syncthreads();
-  const uint32_t base_per_sm = a.items_per_sm ? a.items_per_sm : 3u;
-  const uint32_t level_per_sm = n >= 8 ? base_per_sm + 1 : (base_per_sm > 2 ? base_per_sm - 1 : base_per_sm);
+  const uint32_t level_per_sm = level_items_per_sm(a, n);
   const uint32_t item_rows =
-      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(tot3[1]) * 256, a, level_per_sm);
+      a.item_rows ? a.item_rows : adaptive_item_rows(uint64_t(tot3[1]) * 256, a, level_per_sm, tot3[0]);
   const bool acc = i < n && b.valid && (leaf_count + (v3[0] - s_valid_base[ord]) < P.max_leaves);
   const bool leafseg = i < n && (!acc || last);
   // 0 accepted, 1 build chunks, 2 partition chunks, 3 leaf segments, 4 leaf chunks, 5 freed.
@@ -3038,7 +3056,7 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
   if (warp == 0) {  // work lists of the step, 32 entries at a time
     Control* ctl = a.ctl;
     const uint32_t item_rows =
-        a.item_rows ? a.item_rows : adaptive_item_rows(built_rows, a, a.items_per_sm);
+        a.item_rows ? a.item_rows : adaptive_item_rows(built_rows, a, a.items_per_sm ? a.items_per_sm : default_items_per_sm(a.slots), a.n_trees);
     auto prefix = [&](uint32_t n, uint32_t* out, auto&& chunks_of) -> uint32_t {
       uint32_t acc = 0;
       for (uint32_t e0 = 0; e0 < n; e0 += 32) {

@@ -10,6 +10,11 @@
 
 namespace mpsb {
 
+// Histogram work items per SM where the trainer sets none.
+__host__ __device__ constexpr uint32_t default_items_per_sm(uint32_t slots) {
+  return slots == uint32_t(kSlots) ? 3u : 1u;
+}
+
 constexpr uint32_t kWideVotePasses = 4;  // passes of a wide block of 32 features, at most
 
 // Device pointers and sizes of one training session, passed by value to every kernel.
