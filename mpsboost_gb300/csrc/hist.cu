@@ -27,8 +27,11 @@
 //    (the plain path): a u32 count and two FP32 reductions per cell.
 //  * The CTA flushes its non-empty cells into the node's global slot with 64-bit
 //    red.global adds (exact integer adds in fixed mode; FP64 adds in float mode).
+//  * Fixed-point training builds with hist_build_direct_kernel: a lane owns a row, holds its
+//    block of bins in registers and spreads each round over 32 features, and cells are packed
+//    words (four, or two without weights) where the item's cells allow it.
 //  * Datasets with more than 256 histogram slots per feature (u16 bins) build with
-//    hist_build_wide_kernel, at the end of this file.
+//    hist_build_wide_direct_kernel, or hist_build_wide_kernel, at the end of this file.
 #include <algorithm>
 #include <type_traits>
 

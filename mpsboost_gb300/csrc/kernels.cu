@@ -22,7 +22,8 @@
 //                  (tree.cpp:67-145): acceptance under max_leaves, ApplySplit
 //                  (tree_structure.cpp:118-148), smaller-child selection, next level.
 //   partition      PrepareSplitRows' stable partition (tree_split.cpp:273-289) as a
-//                  ballot/popc compaction: count, per-node scan, scatter.
+//                  ballot/popc compaction: count, per-node scan, scatter, in one cluster
+//                  launch for small levels.
 //   apply_leaves, apply_steps
 //                  predictions += lr * leaf (trainer.cpp:256-262) from the final row
 //                  segments: no tree traversal; the round's trees into the model.
