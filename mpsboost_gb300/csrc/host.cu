@@ -179,6 +179,8 @@ void DevicePool::close() {
 }
 
 bool DevicePool::idle() {
+  std::unique_lock<std::mutex> no_capture(capturing, std::try_to_lock);
+  if (!no_capture) return false;
   cudaStream_t s;
   {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -1158,6 +1160,7 @@ struct mpsb_cuda_trainer {
       const int gi = g_only ? 1 : 0;
       if (use_graph) {
         if (!graph_exec[gi]) {
+          std::lock_guard<std::mutex> capture(b->pool->capturing);
           CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
           uint64_t k = 0;
           try {

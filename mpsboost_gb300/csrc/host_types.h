@@ -75,6 +75,9 @@ class DevicePool {
   static constexpr size_t kBlock = size_t(2) << 20;
   static constexpr size_t kMost = size_t(8) << 30;
   const int device;
+  // Held while a session captures the backend's stream, which then must not be waited for: a
+  // session destroyed meanwhile by another thread (a garbage collector's) frees its blocks.
+  std::mutex capturing;
 
   DevicePool(int dev, cudaStream_t backend_stream);
   ~DevicePool();
@@ -84,7 +87,7 @@ class DevicePool {
   void give(void* p, size_t bytes);
   void trim();
   void close();  // the backend is going: nothing is kept from here on
-  bool idle();   // waits for the backend's stream
+  bool idle();   // waits for the backend's stream; false where it must not or fails
   size_t kept() const;
   static void trim_all();
 

@@ -251,6 +251,25 @@ def test_kept_memory_changes_nothing(threads):
         assert len(o) == 2 * len(data) and o == outs[0] and o[: len(data)] == o[len(data):]
 
 
+# Sessions that another thread drops (as a garbage collector may) while this one captures and runs
+# rounds on the same backend: their memory goes back without waiting on a stream being captured.
+def test_sessions_dropped_beside_a_capture(backend):
+    x = seeded_matrix(9, 4_000, 8, 0.0)
+    y, _ = targets(x, 9)
+    binned = mb.quantize_dense(x, 64)
+    params = dict(n_estimators=3, max_depth=4)
+    want = [t.tobytes() for t in mb.train_regressor(backend, binned, y, **params).trees]
+    idle = [mb.Trainer(backend, binned, y, **params) for _ in range(200)]
+    dropper = threading.Thread(target=lambda: [t.close() for t in idle])
+    dropper.start()
+    rounds = 0
+    while dropper.is_alive() or rounds < 20:
+        got = mb.train_regressor(backend, binned, y, **params)
+        assert [t.tobytes() for t in got.trees] == want
+        rounds += 1
+    dropper.join()
+
+
 # Node-level calls convert their inputs and results on the device: row sets around a warp and a
 # CTA, few-valued and missing features on u8 and u16 pages, bit-exact to the replica; the first
 # error in the checks' order, rows before pairs, and scales of tiny and of zero pairs.
