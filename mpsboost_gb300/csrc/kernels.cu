@@ -2858,12 +2858,15 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
     BuildEntry be{};
     SubEntry se{};
     LeafActive kid[2];
-    if (t < a.n_trees && !a.lw_done[t]) {  // the same in the whole warp
+    const bool open = t < a.n_trees && !a.lw_done[t];  // the same in the whole warp
+    __syncwarp();  // every lane has read lw_done, which lane 0 may set
+    if (open) {
       LeafActive* act = a.lw_active + size_t(t) * cap;
       uint32_t* path = a.lw_path + size_t(t) * cap * W;
       uint32_t* allowed = a.lw_allowed + size_t(t) * cap * W;
       TreeState& ts = a.trees[t];
       const uint32_t cnt = a.lw_count[t], leaf_count = ts.leaf_count, tree_nodes = ts.n_tree_nodes;
+      const uint32_t slot_top = a.lw_slot_top[t];
       uint32_t best = 0xffffffffu, best_node = 0xffffffffu;
       double best_gain = 0.0;
       if (cnt > a.lw_max_active) {
@@ -2903,7 +2906,10 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
         const uint32_t li = tree_nodes, ri = li + 1;
         const uint32_t depth = c.node.depth + 1;
         const bool grow = depth < P.max_depth;
-        const uint32_t slot_top = a.lw_slot_top[t];
+        const uint32_t new_slot = grow && slot_top ? a.lw_slots[size_t(t) * S + slot_top - 1] : 0xffffffffu;
+        // Every lane holds the chosen leaf and the tree's counters: lane 0 and the copy below
+        // overwrite them.
+        __syncwarp();
         if (ri >= a.max_tree_nodes || cnt + 2 > cap || (grow && slot_top == 0)) {
           err |= kErrCapacity;
           if (lane == 0) a.lw_done[t] = 1;
@@ -2916,7 +2922,6 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
           // Children in the other row buffer: left rows, then right rows (the partition).
           const uint32_t np = c.parity ^ 1u;
           const bool build_left = b.lcount <= b.rcount;
-          const uint32_t new_slot = grow ? a.lw_slots[size_t(t) * S + slot_top - 1] : 0xffffffffu;
           if (lane == 0) {
             write_leaf(&tn[li], lv);
             write_leaf(&tn[ri], rv);

@@ -49,6 +49,26 @@ def test_split_scan_edges(backend, port, bins, features, nan, leaves):
                           min_samples_leaf=4, min_child_weight=2.0, **growth)
 
 
+# Leaf-wise trees of several classes: the step that chooses and splits a leaf takes a warp per
+# tree, eight at a time, so class counts below, at and past that; each class's trees are those
+# of a fit of the class alone. A depth limit frees slots, an interaction list writes the paths.
+@pytest.mark.parametrize("classes", [2, 8, 9, 17])
+@pytest.mark.parametrize("extra", [{}, dict(max_depth=3), dict(interaction_constraints=[[0, 1, 2], [2, 3, 4, 5]])])
+def test_leafwise_classes_equal_single_fits(backend, classes, extra):
+    x = seeded_matrix(classes, 5000, 6, 0.05, integer_columns=2)
+    rng = np.random.default_rng(classes)
+    y = (np.argsort(np.argsort(np.nan_to_num(x[:, 0]) + rng.normal(size=5000) * 0.5)) * classes // 5000).astype(float)
+    binned = mb.quantize_dense(x, 64)
+    params = dict(n_estimators=2, learning_rate=0.3, max_depth=7, min_samples_leaf=2, objective="binary_logistic",
+                  growth_strategy="leaf_wise", max_leaves=20)
+    params.update(extra)
+    got = mb.train_ovr(backend, binned, y, classes, **params)
+    for k, m in enumerate(got):
+        want = mb.train_regressor(backend, binned, (y == k).astype(float), **params)
+        assert [t.tobytes() for t in m.trees] == [t.tobytes() for t in want.trees]
+        assert m.train_predictions.tobytes() == want.train_predictions.tobytes()
+
+
 # Rows around the 32-row flag words, a CTA's 1,024 rows, 16 CTAs of a cluster and their
 # 48 rows per thread (786,432: the last single-launch partition of a root, and one past it).
 @pytest.mark.parametrize("rows", [33, 511, 1025, 16 * 1024 - 1, 16 * 1024 + 1, 70_001, 786_432, 786_433])
