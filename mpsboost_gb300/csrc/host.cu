@@ -968,6 +968,14 @@ struct mpsb_cuda_trainer {
     return uint32_t(std::min<uint64_t>(dev.max_level_nodes, uint64_t(n_trees) << std::min<uint32_t>(d, 31)));
   }
 
+  // The split scan's CTA size and what follows from it: the one-launch scan writes a record per
+  // feature chunk, and its readers step over them by partial_stride.
+  void set_scan_threads(uint32_t threads) {
+    dev.scan_threads = threads;
+    dev.n_fchunks = (dev.features + threads / 32 - 1) / (threads / 32);
+    dev.partial_stride = dev.scan_two_phase ? 1u : dev.n_fchunks;
+  }
+
   // Captured rounds bake in the launch shape: drop them after a change.
   void reset_graphs() {
     for (int i = 0; i < 2; ++i) {
@@ -984,8 +992,7 @@ struct mpsb_cuda_trainer {
     hcfg.root_threads = int(s.root_threads);
     dev.items_per_sm = s.items_per_sm;
     blocked_levels = s.blocked_levels;
-    dev.scan_threads = s.scan_threads;
-    dev.n_fchunks = (dev.features + s.scan_threads / 32 - 1) / (s.scan_threads / 32);
+    set_scan_threads(s.scan_threads);
     reset_graphs();
   }
 
@@ -1337,7 +1344,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   // item, split-scan CTA size.
   if (const char* v = std::getenv("MPSB_SCAN_THREADS"))
     a.scan_threads = uint32_t(std::min(512, std::max(32, std::atoi(v) / 32 * 32)));
-  a.n_fchunks = (F + a.scan_threads / 32 - 1) / (a.scan_threads / 32);
+  t->set_scan_threads(a.scan_threads);
   if (const char* v = std::getenv("MPSB_HIST_THREADS")) t->hcfg.threads = std::atoi(v);
   if (const char* v = std::getenv("MPSB_HIST_STAGES")) t->hcfg.stages = std::atoi(v);
   t->hcfg.direct = true;
@@ -1538,7 +1545,6 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
     a.node_path[q] = t->alloc<uint32_t>(size_t(a.max_level_nodes) * W);
     a.node_allowed[q] = t->alloc<uint32_t>(size_t(a.max_level_nodes) * W);
   }
-  a.partial_stride = a.scan_two_phase ? 1u : a.n_fchunks;
   a.partial = t->alloc<SplitRec>(size_t(a.max_level_nodes) * a.partial_stride);
   a.node_screen = t->alloc<uint32_t>(a.max_level_nodes);
   if (a.scan_two_phase) a.feature_screen = t->alloc<uint32_t>(size_t(a.max_level_nodes) * F);

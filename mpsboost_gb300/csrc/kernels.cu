@@ -3763,6 +3763,8 @@ cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_node
   }
   const int threads = int(a.scan_threads);
   if (threads < 32 || threads > kScanThreadsMax || threads % 32) return cudaErrorInvalidValue;
+  // The readers of partial find a node's records where the scan writes them.
+  if (a.partial_stride != a.n_fchunks) return cudaErrorInvalidValue;
   if (fixed) return wide ? launch_scan_one<true, true>(a, parity, grid, threads, s)
                          : launch_scan_one<true, false>(a, parity, grid, threads, s);
   return wide ? launch_scan_one<false, true>(a, parity, grid, threads, s)

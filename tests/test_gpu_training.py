@@ -229,6 +229,26 @@ def test_autotuned_shape_gives_the_same_trees(backend):
     assert plain.train_predictions.tobytes() == again.train_predictions.tobytes()
 
 
+# The fits whose split scan leaves a record per feature chunk, of which a tuned scan has fewer
+# (40 features: 10 chunks of 4, 5 of 8; 41: an uneven last one).
+@pytest.mark.parametrize("feats", [40, 41])
+@pytest.mark.parametrize("scan", [dict(reg_alpha=0.3), dict(reg_lambda=0.0, min_child_weight=0.5),
+                                  dict(split_strategy="random_threshold", random_seed=3)])
+@pytest.mark.parametrize("growth", [{}, dict(growth_strategy="leaf_wise", max_leaves=12)])
+def test_autotuned_one_launch_scan_gives_the_same_trees(backend, feats, scan, growth):
+    x, y, w = _data(50, 20_000, feats, 0.02, 2)
+    binned = mb.quantize_dense(x, 64)
+    params = dict(n_estimators=2, learning_rate=0.2, max_depth=6, min_samples_leaf=2, **scan, **growth)
+    backend.autotune_clear()
+    plain = mb.train_regressor(backend, binned, y, w, **params)
+    tuned = backend.autotune(binned, y, w, rounds_per_trial=1, **params)
+    assert tuned["scan_threads"] in (128, 256)
+    again = mb.train_regressor(backend, binned, y, w, **params)
+    backend.autotune_clear()
+    assert [t.tobytes() for t in plain.trees] == [t.tobytes() for t in again.trees]
+    assert plain.train_predictions.tobytes() == again.train_predictions.tobytes()
+
+
 @pytest.mark.parametrize("rows", [20_000, 20_003])
 def test_dataset_upload_layouts(backend, rows):
     """The per-block upload and pack gives the same trees from u8 and from u16 bins, with
