@@ -121,6 +121,16 @@ struct SplitRec {
 static_assert(sizeof(SplitRec) % 8 == 0 && sizeof(SplitRec) / 8 <= 32,
               "a warp copies a SplitRec one 8-byte word per lane");
 
+// A split's child row counts, checked before the children's segments are published: where they
+// do not add up to the node's rows (false; the launch reports kErrPartition) they are cut to
+// them, so that what is enqueued behind stays inside the node's segment.
+__host__ __device__ inline bool fit_children(uint32_t rows, uint64_t& left, uint64_t& right) {
+  if (left <= rows && right == rows - left) return true;
+  if (left > rows) left = rows;
+  right = rows - left;
+  return false;
+}
+
 // An active leaf of leaf-wise growth (ActiveNode, tree_internal.hpp:44-53): its node, the
 // row buffer holding its segment, and its best split once scanned.
 struct LeafActive {

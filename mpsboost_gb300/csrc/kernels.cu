@@ -2033,7 +2033,9 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       v[0] = acc;
       if (acc) {
         const SplitRec& b = a.partial[size_t(i) * a.partial_stride];
-        const uint32_t built = uint32_t(b.lcount <= b.rcount ? b.lcount : b.rcount);
+        uint64_t left = b.lcount, right = b.rcount;
+        fit_children(node.seg_cnt, left, right);
+        const uint32_t built = uint32_t(left <= right ? left : right);
         if (!last) {
           v[1] = ceil_div(built, item_rows);
           v[2] = ceil_div(node.seg_cnt, kPartChunk);
@@ -2078,7 +2080,8 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
     TreeNodeOut* tn = a.tree_nodes + size_t(t) * a.max_tree_nodes;
     const bool acc = a.scratch_flags[i] != 0;
     if (acc) {
-      const SplitRec b = a.partial[size_t(i) * a.partial_stride];
+      SplitRec b = a.partial[size_t(i) * a.partial_stride];
+      if (!fit_children(node.seg_cnt, b.lcount, b.rcount)) err |= kErrPartition;
       const uint32_t k = a.scratch_prefix[i];
       const uint32_t kt = k - tree_acc_base[t];
       atomicAdd(&tree_acc[t], 1u);
@@ -2101,7 +2104,6 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       pn.gain = b.gain;
       pn.default_left = uint8_t(b.default_left);
       pn.flags = 0;
-      if (b.lcount + b.rcount != node.seg_cnt) err |= kErrPartition;
       if (!last) {
         const bool build_left = b.lcount <= b.rcount;
         const uint32_t new_slot = a.free_stack[free_top - 1 - k];
@@ -2293,6 +2295,7 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
     leaf_count = a.trees[node.tree].leaf_count;
     tree_nodes = a.trees[node.tree].n_tree_nodes;
   }
+  const bool fits = !b.valid || fit_children(node.seg_cnt, b.lcount, b.rcount);
   const uint32_t built = b.valid ? uint32_t(b.lcount <= b.rcount ? b.lcount : b.rcount) : 0u;
   // Valid splits before the node and, through its tree's ordinal in the level, before its
   // tree's first node; rows the next level builds.
@@ -2351,7 +2354,7 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
       pn.gain = b.gain;
       pn.default_left = uint8_t(b.default_left);
       pn.flags = 0;
-      if (b.lcount + b.rcount != node.seg_cnt) err |= kErrPartition;
+      if (!fits) err |= kErrPartition;
       if (!last) {
         const bool build_left = b.lcount <= b.rcount;
         NodeRec c;  // the left child, then the right one
@@ -2900,7 +2903,8 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
       if (best == 0xffffffffu) {
         if (lane == 0) a.lw_done[t] = 1;
       } else {
-        const LeafActive c = act[best];  // every lane (the loads broadcast)
+        LeafActive c = act[best];  // every lane (the loads broadcast)
+        const bool fits = fit_children(c.node.seg_cnt, c.best.lcount, c.best.rcount);
         const SplitRec& b = c.best;
         TreeNodeOut* tn = a.tree_nodes + size_t(t) * a.max_tree_nodes;
         const uint32_t li = tree_nodes, ri = li + 1;
@@ -2918,7 +2922,7 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
           double lv = 0.0, rv = 0.0;
           if (!bounded_leaf(P, b.lg, b.lh, b.ll, b.lu, &lv)) err |= kErrNonFinite;
           if (!bounded_leaf(P, b.rg, b.rh, b.rl, b.ru, &rv)) err |= kErrNonFinite;
-          if (b.lcount + b.rcount != c.node.seg_cnt) err |= kErrPartition;
+          if (!fits) err |= kErrPartition;
           // Children in the other row buffer: left rows, then right rows (the partition).
           const uint32_t np = c.parity ^ 1u;
           const bool build_left = b.lcount <= b.rcount;
