@@ -1394,11 +1394,12 @@ __device__ __forceinline__ Stat<FIXED> warp_inclusive(Stat<FIXED> x, int lane) {
   return x;
 }
 
-// Block-wide inclusive prefix of one value per thread; *total gets the page's sum. One
-// barrier; `t` may be written again after the CTA's next barrier.
+// Block-wide inclusive prefix of one value per thread; *total gets the page's sum and *below
+// (floating-point sums only) the prefix without the thread's own value. One barrier; `t` may be
+// written again after the CTA's next barrier.
 template <bool FIXED>
 __device__ __forceinline__ Stat<FIXED> page_prefix(const Stat<FIXED>& own, PageTotals<FIXED>& t,
-                                                   Stat<FIXED>* total) {
+                                                   Stat<FIXED>* total, Stat<FIXED>* below) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Stat<FIXED> incl = warp_inclusive<FIXED>(own, lane);
   if (lane == 31) {
@@ -1418,6 +1419,11 @@ __device__ __forceinline__ Stat<FIXED> page_prefix(const Stat<FIXED>& own, PageT
     all = stat_add<FIXED>(all, w);
   }
   *total = all;
+  if constexpr (!FIXED) {
+    Stat<FIXED> lower = shfl_up_stat<FIXED>(incl, 1);
+    if (lane == 0) lower = stat_zero<FIXED>();
+    *below = stat_add<FIXED>(before, lower);
+  }
   return stat_add<FIXED>(before, incl);
 }
 
@@ -1564,9 +1570,13 @@ __device__ __forceinline__ void scan_feature(const TrainerDev& a, ScanNode<FIXED
       t.miss_h = b1.h;
       b1 = stat_zero<FIXED>();
     }
-    Stat<FIXED> total;
+    // The left sums of the pair's two thresholds. Integers: the lower one by subtraction. FP64
+    // sums are only added: (a + b) - b loses what is small beside b.
+    Stat<FIXED> total, left0;
     const Stat<FIXED> left1 =
-        stat_add<FIXED>(carry, page_prefix<FIXED>(stat_add<FIXED>(b0, b1), t, &total));
+        stat_add<FIXED>(carry, page_prefix<FIXED>(stat_add<FIXED>(b0, b1), t, &total, &left0));
+    if constexpr (FIXED) left0 = stat_sub<FIXED>(left1, b1);
+    else left0 = stat_add<FIXED>(stat_add<FIXED>(carry, left0), b0);
     carry = stat_add<FIXED>(carry, total);
     if (!WIDE && hm) {
       miss.count = t.miss_count;
@@ -1600,7 +1610,7 @@ __device__ __forceinline__ void scan_feature(const TrainerDev& a, ScanNode<FIXED
       visit(stat_add<FIXED>(left, miss), right, th, 1u);
       if (miss.count != 0) visit(left, stat_add<FIXED>(right, miss), th, 0u);
     };
-    at(s, stat_sub<FIXED>(left1, b1), b0.count == 0);
+    at(s, left0, b0.count == 0);
     at(s + 1, left1, b1.count == 0);
   }
 }

@@ -49,6 +49,30 @@ def test_split_scan_edges(backend, port, bins, features, nan, leaves):
                           min_samples_leaf=4, min_child_weight=2.0, **growth)
 
 
+# Float histograms: the left sums are FP64 sums of the slots below. A slot of hessian 2e-5 beside
+# one of 2e13 keeps its candidate (left hessian 2e-5 to the FP32 rounding of a row's pair), at
+# even and odd slots, at a warp's and a page's edges and on u16 pages.
+@pytest.mark.parametrize("bins,light", [(3, 0), (64, 1), (64, 62), (255, 63), (255, 64), (256, 254), (600, 255),
+                                        (600, 256), (600, 598)])
+@pytest.mark.parametrize("growth", [{}, dict(growth_strategy="leaf_wise", max_leaves=2)])
+def test_float_left_sums_keep_small_slots(backend, bins, light, growth):
+    b = np.repeat(np.arange(bins), 20)
+    w = np.full(b.size, 1e-6)
+    w[b == light + 1] = 1e12
+    y = np.where(b == light, 1e6, 0.0)
+    ds = mb.BinnedDataset(b.size, 1, bins, b[None].astype(np.uint16 if bins > 256 else np.uint8),
+                          np.zeros((1, b.size), bool), np.arange(1, bins, dtype=np.float32), np.zeros(1, np.uint64),
+                          np.array([bins - 1], np.uint32), np.array([bins], np.uint32), np.zeros(1, np.uint64))
+    m = mb.train_regressor(backend, ds, y, w, hist_mode="float", n_estimators=1, max_depth=1, reg_lambda=1e-3, **growth)
+    g = w * (m.base_score - y)
+    left = b <= light
+    root = m.trees[0][0]
+    assert (root["flags"] & 1) == 0 and root["threshold_bin"] == light
+    # 20 rows of FP32 pairs added in FP32: 21 roundings of 2^-24, twice.
+    np.testing.assert_allclose(m.trees[0][root["left_child"]]["leaf_value"],
+                               -g[left].sum() / (w[left].sum() + 1e-3), rtol=1e-5)
+
+
 # Leaf-wise trees of several classes: the step that chooses and splits a leaf takes a warp per
 # tree, eight at a time, so class counts below, at and past that; each class's trees are those
 # of a fit of the class alone. A depth limit frees slots, an interaction list writes the paths.
