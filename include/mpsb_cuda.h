@@ -219,6 +219,10 @@ int mpsb_cuda_backend_set_hist_mode(mpsb_cuda_backend* backend, int mode);
 int mpsb_cuda_timer_begin(mpsb_cuda_backend* backend);
 int mpsb_cuda_timer_end(mpsb_cuda_backend* backend, float* milliseconds);
 int mpsb_cuda_synchronize(mpsb_cuda_backend* backend);
+/* A backend keeps the device memory of finished calls for the next ones, at most 8 GiB; it goes
+ * back to the driver when the backend is destroyed, when an allocation of this library fails, or
+ * here, at once. *given_back (or null): the bytes returned. */
+int mpsb_cuda_backend_trim(mpsb_cuda_backend* backend, uint64_t* given_back);
 /* Page-lock (pin) / release a caller-owned host buffer so copies from it run at full
    host-link bandwidth. */
 int mpsb_cuda_host_register(void* ptr, uint64_t bytes);

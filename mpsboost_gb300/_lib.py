@@ -145,6 +145,7 @@ SIGNATURES = {
     "mpsb_cuda_backend_set_hist_mode": (_I32, [_VP, _I32]),
     "mpsb_cuda_timer_begin": (_I32, [_VP]),
     "mpsb_cuda_timer_end": (_I32, [_VP, C.POINTER(C.c_float)]),
+    "mpsb_cuda_backend_trim": (_I32, [_VP, C.POINTER(_U64)]),
     "mpsb_cuda_synchronize": (_I32, [_VP]),
     "mpsb_cuda_host_register": (_I32, [_VP, _U64]),
     "mpsb_cuda_host_unregister": (_I32, [_VP]),

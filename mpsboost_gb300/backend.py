@@ -493,6 +493,14 @@ class CudaBackend:
     def synchronize(self) -> None:
         check(_lib.load().mpsb_cuda_synchronize(self.handle))
 
+    def release_memory(self) -> int:
+        """Gives the device memory kept for later calls (at most 8 GiB) back to the driver, for
+        others on the GPU; returns the bytes."""
+
+        given = C.c_uint64()
+        check(_lib.load().mpsb_cuda_backend_trim(self.handle, C.byref(given)))
+        return int(given.value)
+
 
 # --------------------------------------------------------------------------------------
 # Models and training

@@ -163,11 +163,11 @@ void DevicePool::give(void* p, size_t bytes) {
   }
 }
 
-void DevicePool::trim() {
+size_t DevicePool::trim() {
   std::lock_guard<std::mutex> lock(mutex_);
   for (auto& f : free_) cudaFree(f.first);
   free_.clear();
-  kept_ = 0;
+  return std::exchange(kept_, size_t(0));
 }
 
 void DevicePool::close() {
@@ -661,6 +661,15 @@ int mpsb_cuda_timer_end(mpsb_cuda_backend* b, float* ms) {
     CK(cudaEventRecord(b->t1, b->stream));
     CK(cudaEventSynchronize(b->t1));
     CK(cudaEventElapsedTime(ms, b->t0, b->t1));
+  });
+}
+
+int mpsb_cuda_backend_trim(mpsb_cuda_backend* b, uint64_t* given_back) {
+  return guard([&] {
+    if (!b) throw TrainingError("null argument");
+    b->activate();
+    const size_t bytes = b->pool->trim();
+    if (given_back) *given_back = bytes;
   });
 }
 

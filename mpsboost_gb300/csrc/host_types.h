@@ -85,7 +85,7 @@ class DevicePool {
   DevicePool& operator=(const DevicePool&) = delete;
   void* take(size_t* bytes);  // *bytes: the size wanted, then the block's
   void give(void* p, size_t bytes);
-  void trim();
+  size_t trim();  // the bytes given back
   void close();  // the backend is going: nothing is kept from here on
   bool idle();   // waits for the backend's stream; false where it must not or fails
   size_t kept() const;

@@ -295,6 +295,22 @@ def test_kept_memory_changes_nothing(threads):
         assert len(o) == 2 * len(data) and o == outs[0] and o[: len(data)] == o[len(data):]
 
 
+def test_kept_memory_is_given_back(backend):
+    torch = pytest.importorskip("torch")
+    x = seeded_matrix(3, 200_000, 12)
+    y, w = targets(x, 3)
+    binned = mb.quantize_dense(x, 255)
+    params = dict(n_estimators=2, max_depth=5)
+    want = mb.train_regressor(backend, binned, y, w, **params)
+    free = torch.cuda.mem_get_info(0)[0]
+    given = backend.release_memory()
+    assert 0 < given <= 8 << 30
+    assert torch.cuda.mem_get_info(0)[0] - free >= given // 2
+    assert backend.release_memory() == 0
+    got = mb.train_regressor(backend, binned, y, w, **params)
+    assert [t.tobytes() for t in got.trees] == [t.tobytes() for t in want.trees]
+
+
 # Sessions that another thread drops (as a garbage collector may) while this one captures and runs
 # rounds on the same backend: their memory goes back without waiting on a stream being captured.
 def test_sessions_dropped_beside_a_capture(backend):
