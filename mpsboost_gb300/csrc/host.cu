@@ -874,14 +874,6 @@ int mpsb_cuda_dataset_uses_tma(const mpsb_cuda_dataset* d) { return d && d->has_
 // ======================================================================================
 namespace mpsb {
 
-struct TuneKey {
-  uint32_t rows, features, depth, mode, unit_hess, weighted, leafwise;
-  bool operator<(const TuneKey& o) const {
-    return std::tie(rows, features, depth, mode, unit_hess, weighted, leafwise) <
-           std::tie(o.rows, o.features, o.depth, o.mode, o.unit_hess, o.weighted, o.leafwise);
-  }
-};
-
 std::mutex g_tune_mutex;
 std::map<TuneKey, mpsb_cuda_tuning> g_tune_table;
 
@@ -893,12 +885,17 @@ bool unit_hessian_fit(const double* weights, const mpsb_train_params& p) {
   return unit;
 }
 
+// The split scan in two launches: best splits with the FP32 screen's quadratic score.
+bool two_launch_scan(const mpsb_train_params& p) {
+  return p.split_strategy == 0 && p.reg_alpha == 0.0 && p.reg_lambda > 0.0;
+}
+
 TuneKey tune_key_of(const mpsb_cuda_dataset* ds, const double* weights, const mpsb_train_params& p,
                     uint32_t options) {
   return TuneKey{ds->n_rows, ds->features, p.max_depth,
                  uint32_t((options & MPSB_OPT_FLOAT_HIST) ? kModeFloat : kModeFixed),
                  unit_hessian_fit(weights, p) ? 1u : 0u, weights ? 1u : 0u,
-                 p.growth_strategy == 1 ? 1u : 0u};
+                 p.growth_strategy == 1 ? 1u : 0u, ds->slots, two_launch_scan(p) ? 1u : 0u};
 }
 
 bool tuned_shape(const TuneKey& k, mpsb_cuda_tuning* out) {
@@ -1306,7 +1303,7 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.bins_block_stride = kBlockFeatures;
   a.bins_fm = ds->bins_fm.as<uint8_t>();
   a.slots = ds->slots;
-  a.scan_two_phase = p->split_strategy == 0 && p->reg_alpha == 0.0 && p->reg_lambda > 0.0;
+  a.scan_two_phase = two_launch_scan(*p);
   // The split scan forms each sibling's histogram (MPSB_FUSED_SUB=0: subtract_kernel
   // does); the one-launch scan on level-wise u8 datasets only.
   a.fused_sub = a.scan_two_phase || (ds->slots == uint32_t(kSlots) && p->growth_strategy != 1);
@@ -1845,14 +1842,15 @@ int mpsb_cuda_autotune(mpsb_cuda_backend* b, const mpsb_cuda_dataset* ds, const 
         if (v == c.items_per_sm) return false;
         c.items_per_sm = v;
         return true;
-      }, {2, 3, 4});
+      }, {1, 2, 3, 4});
       try_values([&](mpsb_cuda_tuning& c, uint32_t v) {
         if (v == c.blocked_levels) return false;
         c.blocked_levels = v;
         return true;
       }, {1, 2, 3});
       try_values([&](mpsb_cuda_tuning& c, uint32_t v) {
-        if (v == c.scan_threads || v < min_scan) return false;
+        // The two-launch scan's CTAs have one size.
+        if (t->dev.scan_two_phase || v == c.scan_threads || v < min_scan) return false;
         c.scan_threads = v;
         return true;
       }, {128, 256});

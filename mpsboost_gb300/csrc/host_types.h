@@ -9,6 +9,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -114,6 +115,17 @@ class DevArena {
   std::vector<std::pair<void*, size_t>> blocks_;
   char* slab_ = nullptr;
   size_t left_ = 0;
+};
+
+// The kind of fit a tuned launch shape belongs to: everything that the built-in shape, or the
+// kernels it is for, depend on (u8 and u16 datasets have other kernels and defaults).
+struct TuneKey {
+  uint32_t rows, features, depth, mode, unit_hess, weighted, leafwise, slots, two_launch_scan;
+  bool operator<(const TuneKey& o) const {
+    return std::tie(rows, features, depth, mode, unit_hess, weighted, leafwise, slots, two_launch_scan) <
+           std::tie(o.rows, o.features, o.depth, o.mode, o.unit_hess, o.weighted, o.leafwise, o.slots,
+                    o.two_launch_scan);
+  }
 };
 
 // Owning device allocation.

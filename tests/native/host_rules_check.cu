@@ -3,6 +3,7 @@
 #include <cstdio>
 
 #include "device.cuh"
+#include "host_types.h"
 
 using namespace mpsb;
 
@@ -25,4 +26,21 @@ static bool children() {
   return true;
 }
 
-int main() { return children() ? 0 : 1; }
+// Fits that differ in any one property keep tuned shapes of their own: a u8 and a u16 dataset of
+// the same rows, features and depth (slots), and the two kinds of split scan, among them.
+static bool tune_keys() {
+  constexpr int kFields = 9;
+  static_assert(sizeof(TuneKey) == kFields * sizeof(uint32_t), "a field is not compared here");
+  const TuneKey base{1000, 8, 6, 0, 1, 0, 0, 256, 1};
+  for (int i = 0; i < kFields; ++i) {
+    TuneKey other = base;
+    reinterpret_cast<uint32_t*>(&other)[i] += 1;
+    if (!(base < other) || other < base) {
+      std::printf("tune key: field %d is not told apart\n", i);
+      return false;
+    }
+  }
+  return !(base < base);
+}
+
+int main() { return children() && tune_keys() ? 0 : 1; }
