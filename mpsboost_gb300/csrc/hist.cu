@@ -846,8 +846,15 @@ __global__ void __launch_bounds__(THREADS, 1) hist_build_direct_kernel(TrainerDe
           for (uint32_t b = uint32_t(warp); b < kSlots; b += WARPS) sum += counts[b * kBlockFeatures + lane] & kPackCountMask;
           atomicAdd(s_ok + lane, sum);
           __syncthreads();
-          // Padding features of the last block hold every row in bin 0: they are not flushed.
-          const bool good = fb * kBlockFeatures + lane >= a.features || s_ok[lane] == row_count;
+          // Features that nothing reads may overflow their cells: the padding of the last block
+          // (every row in bin 0, not flushed) and what a forest tree does not have (the padding
+          // of a subset shorter than the widest, again every row in bin 0). Feature 0 of every
+          // tree is read by the root statistics.
+          const uint32_t f = fb * kBlockFeatures + lane;
+          bool unread = f >= a.features;
+          if (a.tree_feature_masks && f != 0)
+            unread |= !((a.tree_feature_masks[size_t(e.tree) * a.params.path_words + fb] >> lane) & 1u);
+          const bool good = unread || s_ok[lane] == row_count;
           packed = __all_sync(0xffffffffu, good);  // the same in every warp
           if (tid == 0) atomicAdd(a.limb_votes + 2 * fb + (packed ? 0 : 1), 1u);
           if (!packed) {

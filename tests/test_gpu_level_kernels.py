@@ -200,6 +200,30 @@ def test_compact_forest_equals_replica(backend, port, rows, subset, extra, weigh
         assert m.trees[0].tobytes() == nodes.tobytes()
 
 
+# Subsets shorter than the widest pad a tree's block with a feature that holds all rows in one
+# bin, past the packed limbs' cells; heavy cells in features that the tree has and has not, in
+# copies of its own features (8 of 70) and in the dataset's (68 of 70).
+@pytest.mark.parametrize("widest", [8, 68])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_forest_packed_limbs_of_ragged_subsets(backend, port, widest, weighted):
+    x = seeded_matrix(widest, 9_000, 70, 0.0)
+    x[:, 0] = np.arange(9_000) < 2_048
+    x[:, 5] = np.arange(9_000) % 2
+    y, w = targets(x, widest)
+    w = w if weighted else None
+    rng = np.random.default_rng(widest)
+    counts = rng.poisson(1.0, (4, 9_000)).astype(np.uint8)
+    subsets = [rng.choice(np.arange(6, 70) if t % 2 else 70, s, replace=False)
+               for t, s in enumerate([widest, min(widest - 1, 64), widest - 4, 1])]
+    params = dict(max_depth=6, min_samples_leaf=3)
+    models = mb.train_forest(backend, mb.quantize_dense(x, 255), y, w, row_counts=counts, feature_subsets=subsets, **params)
+    ds = port.quantize_dense(x, 255)
+    for t, m in enumerate(models):
+        base, nodes = _oracle_tree(port, ds, y, w, counts[t], subsets[t], params, 0)
+        assert float(m.base_score).hex() == float(base).hex()
+        assert m.trees[0].tobytes() == nodes.tobytes()
+
+
 def _traverse(trees, lr, base, bins, missing):
     """Predictions tree by tree in FP64, as RegressionModel::Predict adds them."""
     out = np.full(bins.shape[1], base)
