@@ -1554,6 +1554,12 @@ void setup_trainer(mpsb_cuda_trainer* t, mpsb_cuda_backend* b, const mpsb_cuda_d
   a.partial = t->alloc<SplitRec>(size_t(a.max_level_nodes) * a.partial_stride);
   a.node_screen = t->alloc<uint32_t>(a.max_level_nodes);
   if (a.scan_two_phase) a.feature_screen = t->alloc<uint32_t>(size_t(a.max_level_nodes) * F);
+  if (a.scan_two_phase && F > kExactFeatures) {
+    a.exact_cap = a.sm_count * kScanCtasPerSm;
+    a.exact_part = t->alloc<SplitRec>(a.exact_cap);
+    a.exact_done = t->alloc<uint32_t>(a.exact_cap);
+    CK(cudaMemsetAsync(a.exact_done, 0, a.exact_cap * sizeof(uint32_t), s));
+  }
   a.build = t->alloc<BuildEntry>(a.max_level_nodes);
   a.build_prefix = t->alloc<uint32_t>(a.max_level_nodes + 1);
   a.sub = t->alloc<SubEntry>(a.max_level_nodes);

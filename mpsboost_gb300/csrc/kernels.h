@@ -15,6 +15,9 @@ __host__ __device__ constexpr uint32_t default_items_per_sm(uint32_t slots) {
   return slots == uint32_t(kSlots) ? 3u : 1u;
 }
 
+constexpr uint32_t kScanCtasPerSm = 6;  // resident CTAs of the two-launch split scan
+constexpr uint32_t kExactFeatures = 32;  // more features than this: a node's CTAs may share them
+
 constexpr uint32_t kWideVotePasses = 4;  // passes of a wide block of 32 features, at most
 
 // Device pointers and sizes of one training session, passed by value to every kernel.
@@ -87,6 +90,12 @@ struct TrainerDev {
   uint32_t* node_screen;
   uint32_t* feature_screen;
   uint32_t scan_two_phase;
+  // Nodes whose exact evaluation several CTAs share: each CTA's best split, [node][CTA] within
+  // exact_cap records (0: a CTA per node), and how many of a node's CTAs are done (zero between
+  // launches).
+  SplitRec* exact_part;
+  uint32_t* exact_done;
+  uint32_t exact_cap;
   uint32_t n_fchunks;           // feature chunks of the one-launch split scan (a warp each feature)
   BuildEntry* build;            // [max_level_nodes]
   uint32_t* build_prefix;       // [max_level_nodes + 1] chunk prefix

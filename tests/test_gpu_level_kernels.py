@@ -49,6 +49,28 @@ def test_split_scan_edges(backend, port, bins, features, nan, leaves):
                           min_samples_leaf=4, min_child_weight=2.0, **growth)
 
 
+# Nodes with up to 8 features to evaluate exactly, one more and all of them (equal columns tie;
+# monotone constraints and hessians at min_child_weight take every feature), which a node's CTAs
+# share from 33 features on; u8 and u16 pages, level-wise and leaf-wise.
+@pytest.mark.parametrize("features,equal", [(32, 32), (33, 8), (33, 9), (70, 70), (260, 9), (1000, 300)])
+@pytest.mark.parametrize("bins", [32, 300])
+@pytest.mark.parametrize("leaves", [0, 6])
+@pytest.mark.parametrize("extra", ["", "monotone", "hessian"])
+def test_exact_scan_shared_by_ctas(backend, port, features, equal, bins, leaves, extra):
+    x = seeded_matrix(features + equal, 1500, features, 0.05, integer_columns=3)
+    rng = np.random.default_rng(equal)
+    x[:, rng.choice(features, equal, replace=False)] = x[:, [features // 2]]
+    y = np.nan_to_num(x[:, features // 2]) + rng.normal(size=1500) * 0.2
+    params = dict(n_estimators=2, learning_rate=0.3, max_depth=4, min_samples_leaf=2)
+    if extra == "monotone":
+        params["monotonic_constraints"] = [1, 0, -1, 1] * (features // 4) + [0] * (features % 4)
+    if extra == "hessian":
+        params["min_child_weight"] = 20.0
+    if leaves:
+        params.update(growth_strategy="leaf_wise", max_leaves=leaves)
+    assert_equals_replica(backend, port, x, y, None, bins, **params)
+
+
 # Float histograms: the left sums are FP64 sums of the slots below. A slot of hessian 2e-5 beside
 # one of 2e13 keeps its candidate (left hessian 2e-5 to the FP32 rounding of a row's pair), at
 # even and odd slots, at a warp's and a page's edges and on u16 pages.
