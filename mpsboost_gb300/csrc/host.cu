@@ -2187,14 +2187,20 @@ void predict_trees(mpsb_cuda_backend* b, const std::vector<const std::vector<mps
                    double base, double lr, const mpsb_cuda_dataset* ds, double* out) {
   dataset_ready(ds);
   std::vector<uint32_t> offsets(trees.size() + 1, 0);
+  uint64_t visits = 0;  // of a row, were every tree balanced
   for (size_t t = 0; t < trees.size(); ++t) {
     offsets[t + 1] = offsets[t] + uint32_t(trees[t]->size());
-    for (const mpsb_tree_node& nd : *trees[t])
-      if (!(nd.flags & 1u) && nd.feature_index >= ds->features)
+    uint32_t leaves = 0;
+    for (const mpsb_tree_node& nd : *trees[t]) {
+      if (nd.flags & 1u) ++leaves;
+      else if (nd.feature_index >= ds->features)
         throw TrainingError("Prediction feature count does not match the tree model");
+    }
+    while (leaves >>= 1) ++visits;
   }
   HostForest packed;
-  if (!trees.empty() && predict_rows(ds->n_rows, ds->features, ds->slots == uint32_t(kSlots) ? 1 : 2) != 0 &&
+  if (!trees.empty() &&
+      predict_packed_pays(ds->n_rows, ds->features, ds->slots == uint32_t(kSlots) ? 1 : 2, offsets.back(), visits) &&
       pack_forest(trees, lr, ds, packed)) {
     // One upload and one buffer: nodes, leaf steps, tree and group tables, predictions.
     const size_t nb = packed.nodes.size() * sizeof(uint2), sb = packed.steps.size() * sizeof(double),
@@ -2224,18 +2230,18 @@ void predict_trees(mpsb_cuda_backend* b, const std::vector<const std::vector<mps
   std::vector<mpsb_tree_node> flat(offsets.back() ? offsets.back() : 1);
   for (size_t t = 0; t < trees.size(); ++t)
     std::copy(trees[t]->begin(), trees[t]->end(), flat.begin() + offsets[t]);
-  DevBuf d_nodes, d_off, d_out;
-  d_nodes.alloc(flat.size() * sizeof(mpsb_tree_node));
-  d_off.alloc(offsets.size() * sizeof(uint32_t));
-  d_out.alloc(size_t(ds->n_rows) * sizeof(double));
+  DevArena mem;
+  mem.pool = b->pool;
+  TreeNodeOut* d_nodes = static_cast<TreeNodeOut*>(mem.alloc(flat.size() * sizeof(mpsb_tree_node)));
+  uint32_t* d_off = static_cast<uint32_t*>(mem.alloc(offsets.size() * sizeof(uint32_t)));
+  double* d_out = static_cast<double*>(mem.alloc(size_t(ds->n_rows) * sizeof(double)));
   cudaStream_t s = b->stream;
-  CK(cudaMemcpyAsync(d_nodes.p, flat.data(), flat.size() * sizeof(mpsb_tree_node), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(d_off.p, offsets.data(), offsets.size() * 4, cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(d_nodes, flat.data(), flat.size() * sizeof(mpsb_tree_node), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(d_off, offsets.data(), offsets.size() * 4, cudaMemcpyHostToDevice, s));
   CK(launch_predict(ds->bins_fm.as<uint8_t>(), ds->bins16_fm.as<uint16_t>(), ds->slots, ds->n_rows,
                     ds->nfb, ds->has_missing.as<uint8_t>(),
-                    d_nodes.as<TreeNodeOut>(), d_off.as<uint32_t>(), uint32_t(trees.size()), base, lr,
-                    d_out.as<double>(), b->error.as<uint32_t>(), s));
-  CK(cudaMemcpyAsync(out, d_out.p, size_t(ds->n_rows) * sizeof(double), cudaMemcpyDeviceToHost, s));
+                    d_nodes, d_off, uint32_t(trees.size()), base, lr, d_out, b->error.as<uint32_t>(), s));
+  CK(cudaMemcpyAsync(out, d_out, size_t(ds->n_rows) * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (b->take_error()) throw TrainingError("Tree node index is out of bounds or the structure contains a cycle");
 }
 

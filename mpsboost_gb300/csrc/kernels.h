@@ -279,6 +279,27 @@ inline uint32_t predict_rows(uint32_t n_rows, uint32_t features, size_t bin_byte
     rows >>= 1;
   return kPredictTreeBytes + uint64_t(features) * (rows * bin_bytes + 4) <= kPredictSmemMax ? rows : 0u;
 }
+// Whether the packed kernel is the faster one. `entries`: inner nodes and leaves of all trees;
+// `visits`: nodes a row passes in all of them, were they balanced. Three things it spends that
+// the general kernel does not, each against what it saves, the visits' gathers (whole calls on
+// resident datasets of 255 bins, complete trees on random features, general -> packed, ms):
+//  * a CTA stages every tree: 16 of depth 10 on 30,000 rows (128 rows a CTA: 1.6 entries per row
+//    and visit) 0.43 -> 0.50, 64 of depth 8 (0.5) 0.91 -> 0.79, 8 of depth 11 on 1,000,000 x 64
+//    (1,024 rows: 0.36) 0.71 -> 0.56;
+//  * it stages every feature of its rows, used or not: 1,000,000 x 128, 4 trees of depth 6 (five
+//    bytes a visit) 0.18 -> 0.24, 16 (1.3) 0.48 -> 0.40; 30,000 x 512, 16 (5.3) 0.21 and 0.21.
+//    Up to 32 KB a CTA do not show: 1,000 x 256, one tree, 0.05 -> 0.04;
+//  * the features' bins cut the rows that an SM walks at once: 300,000 x 1,000 (an eighth) 0.05
+//    -> 1.88 with one tree, 3.5 -> 7.0 with 256; 300,000 x 512 (a quarter) 3.2 -> 3.8; 1,000,000
+//    x 256 (half) 0.10 -> 0.50 with one tree, 1.74 -> 1.55 with 64 of depth 6.
+inline bool predict_packed_pays(uint32_t n_rows, uint32_t features, size_t bin_bytes, uint64_t entries,
+                                uint64_t visits) {
+  const uint64_t rows = predict_rows(n_rows, features, bin_bytes), free_rows = predict_rows(n_rows, 0, bin_bytes);
+  const uint64_t row_bytes = features * bin_bytes;
+  if (rows == 0 || 5 * entries > 3 * rows * visits + 5120) return false;
+  if (rows == free_rows) return row_bytes * rows <= 32768 || row_bytes <= 4 * visits;
+  return 2 * rows == free_rows && 3 * row_bytes <= 2 * visits;
+}
 cudaError_t launch_predict_packed(const uint8_t* bins_fm, const uint16_t* bins16_fm, uint32_t slots,
                                   uint32_t n_rows, uint32_t features, const PackedForest& f, double base,
                                   double* out, cudaStream_t stream);

@@ -43,4 +43,25 @@ static bool tune_keys() {
   return !(base < base);
 }
 
-int main() { return children() && tune_keys() ? 0 : 1; }
+// The prediction kernel's rule at the sizes it was measured at: complete trees of a depth.
+static bool predict_rule() {
+  struct {
+    uint32_t rows, features, trees, depth;
+    bool packed;
+  } at[] = {{1000, 64, 1, 6, true},         {1000, 256, 1, 6, true},        {1000, 64, 64, 6, true},
+            {1'000'000, 128, 1, 6, false},  {1'000'000, 128, 4, 6, false},  {1'000'000, 128, 16, 6, true},
+            {1'000'000, 64, 8, 11, true},   {30'000, 64, 16, 10, false},    {30'000, 64, 64, 8, true},
+            {30'000, 512, 1, 6, false},     {30'000, 512, 256, 6, true},    {300'000, 1000, 1, 6, false},
+            {300'000, 1000, 256, 6, false}, {300'000, 512, 256, 6, false},  {1'000'000, 256, 1, 6, false},
+            {1'000'000, 256, 64, 6, true},  {1'000'000, 2000, 256, 6, false}, {1, 1, 1, 0, true}};
+  for (const auto& c : at) {
+    const uint64_t entries = uint64_t(c.trees) * ((2ull << c.depth) - 1), visits = uint64_t(c.trees) * c.depth;
+    if (predict_packed_pays(c.rows, c.features, 1, entries, visits) != c.packed) {
+      std::printf("prediction of %u x %u by %u trees of depth %u\n", c.rows, c.features, c.trees, c.depth);
+      return false;
+    }
+  }
+  return true;
+}
+
+int main() { return children() && tune_keys() && predict_rule() ? 0 : 1; }

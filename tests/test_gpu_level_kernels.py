@@ -308,6 +308,29 @@ def test_predict_edges(backend, rows, features, bins, nan, splits, shuffle):
     assert got.tobytes() == _traverse(trees, 0.1, 0.25, binned.bins, binned.missing).tobytes()
 
 
+# Both prediction kernels around the rule that chooses between them: 32 KB of bins a CTA and one
+# feature more with few visits, four bytes a visit and more, features that halve and quarter a
+# CTA's rows with few and many trees, trees in groups of the staging's 4,096 nodes on few rows
+# and on many, u8 and u16 bins.
+@pytest.mark.parametrize("rows,features,bins,splits", [
+    (5_000, 256, 32, [63]), (5_000, 257, 32, [63]), (20_000, 264, 32, [63] * 11), (20_000, 265, 32, [63] * 11),
+    (160_001, 200, 32, [15] * 3), (160_001, 200, 32, [15] * 90), (160_000, 400, 32, [15] * 90),
+    (2_000, 6, 64, [4000, 90, 10, 4096]), (160_002, 6, 64, [4000, 90, 10, 4096]), (160_003, 70, 300, [31] * 40),
+    (160_003, 130, 300, [31] * 40),
+])
+def test_predict_routes(backend, rows, features, bins, splits):
+    rng = np.random.default_rng(features)
+    counts = np.full(features, bins, np.uint32)
+    b = rng.integers(0, bins, (features, rows)).astype(np.uint16 if bins > 256 else np.uint8)
+    binned = mb.BinnedDataset(rows, features, bins, b, np.zeros(b.shape, bool),
+                              np.tile(np.arange(1, bins, dtype=np.float32), features),
+                              np.arange(features, dtype=np.uint64) * (bins - 1), counts - 1, counts,
+                              np.zeros(features, np.uint64))
+    trees = [_grown(rng, features, bins - 1, s, False) for s in splits]
+    got = mb.RegressionModel(0.25, 0.1, trees).predict(backend, binned)
+    assert got.tobytes() == _traverse(trees, 0.1, 0.25, binned.bins, binned.missing).tobytes()
+
+
 # Working memory kept between calls: fits of sizes that share, outgrow and split the kept blocks
 # give the same bytes again, on one backend and on two threads with one each; 600,000 rows also
 # take the result buffers mapped beside the training.
