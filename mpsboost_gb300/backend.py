@@ -763,8 +763,12 @@ class _ResultBuffers:
         self.rows, self.arrays, self.thread = rows, [], None
         if 4 << 20 <= 8 * count * rows <= 4 << 30:
             self.arrays = [np.empty(rows, np.float64) for _ in range(count)]
-            self.thread = threading.Thread(target=self._map, daemon=True)
-            self.thread.start()
+            thread = threading.Thread(target=self._map, daemon=True)
+            try:
+                thread.start()
+                self.thread = thread
+            except RuntimeError:  # no thread to be had (a limit, or the interpreter is exiting):
+                pass              # the copy maps the pages
 
     def _map(self) -> None:
         lib = _lib.load()

@@ -1,8 +1,12 @@
-"""The native pass over class labels against the sort and search it replaces (no GPU)."""
+"""The native pass over class labels against the sort and search it replaces, and the result buffers beside
+it (no GPU)."""
+
+import threading
 
 import numpy as np
 import pytest
 
+from mpsboost_gb300.backend import _ResultBuffers
 from mpsboost_gb300.estimators import _encode_classes
 
 
@@ -19,3 +23,16 @@ def test_class_positions(rows, values):
     np.testing.assert_array_equal(classes, want)
     np.testing.assert_array_equal(encoded, np.searchsorted(want, y).astype(np.float64))
     assert classes.dtype == want.dtype and encoded.dtype == np.float64
+
+
+# Where no thread can be started, the training results' pages are mapped by the copy instead.
+def test_result_buffers_without_a_thread(monkeypatch):
+    def refuse(self):
+        raise RuntimeError("can't start new thread")
+
+    monkeypatch.setattr(threading.Thread, "start", refuse)
+    results = _ResultBuffers(2, 600_000)
+    results.join()
+    for k in range(2):
+        assert results[k].shape == (600_000,) and results[k].dtype == np.float64
+    assert results[0] is not results[1]
