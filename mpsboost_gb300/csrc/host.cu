@@ -26,7 +26,6 @@
 #include <mutex>
 #include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -407,7 +406,7 @@ int class_ids(const double* y, uint64_t n, uint32_t limit, uint8_t* seen) {
     const uint64_t lo = n * k / workers, hi = n * (k + 1) / workers;
     try {
       pool[k] = std::thread(check, lo, hi);
-    } catch (const std::system_error&) {
+    } catch (const std::exception&) {  // no thread, or no memory for one
       check(lo, hi);
     }
   }

@@ -1,13 +1,19 @@
 """The native pass over class labels against the sort and search it replaces, and the result buffers beside
 it (no GPU)."""
 
+import os
+import shutil
+import subprocess
 import threading
 
 import numpy as np
 import pytest
 
+from mpsboost_gb300 import build
 from mpsboost_gb300.backend import _ResultBuffers
 from mpsboost_gb300.estimators import _encode_classes
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 # Class ids that are their own positions, gaps, the table's last number and one past it, a sign,
@@ -23,6 +29,17 @@ def test_class_positions(rows, values):
     np.testing.assert_array_equal(classes, want)
     np.testing.assert_array_equal(encoded, np.searchsorted(want, y).astype(np.float64))
     assert classes.dtype == want.dtype and encoded.dtype == np.float64
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no host compiler")
+def test_class_ids_without_memory(tmp_path):
+    lib = build.build()
+    exe = tmp_path / "no_memory_check"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "include"),
+                    os.path.join(ROOT, "tests", "native", "no_memory_check.cpp"), lib, "-rdynamic",
+                    f"-Wl,-rpath,{os.path.dirname(lib)}", "-o", str(exe)], check=True)
+    run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert run.returncode == 0, run.stdout + run.stderr
 
 
 # Where no thread can be started, the training results' pages are mapped by the copy instead.
