@@ -125,6 +125,23 @@ def test_partition_edges(backend, port, rows):
                           min_samples_leaf=2)
 
 
+# The cluster partition at the largest nodes that it takes: 16 rows a thread of 16 CTAs for a root
+# (262,144 rows; one more takes the three launches), twice that from four nodes on, where a node
+# may hold nearly all rows, and in leaf-wise steps up to the flag words of 16 CTAs.
+@pytest.mark.parametrize("rows,growth", [
+    (262_144, {}), (262_145, {}), (524_288, {}), (524_289, {}),
+    (1_048_576, dict(growth_strategy="leaf_wise", max_leaves=4)),
+    (1_048_577, dict(growth_strategy="leaf_wise", max_leaves=4)),
+])
+def test_partition_largest_nodes(backend, port, rows, growth):
+    x = seeded_matrix(rows, rows, 2, 0.05)
+    x[:, 1] = np.arange(rows) % 997 < 2  # nearly all rows in one child, level by level
+    rng = np.random.default_rng(rows)
+    y = 5.0 * x[:, 1] + 0.1 * np.nan_to_num(x[:, 0]) + (x[:, 0] > 2.5) * 3.0 + rng.normal(size=rows) * 0.05
+    assert_equals_replica(backend, port, x, y, None, 32, n_estimators=1, learning_rate=0.3, max_depth=4,
+                          min_samples_leaf=2, **growth)
+
+
 # A histogram cell of 2,047 rows (the packed limbs' largest), one past it, and multiples of
 # 2,048 (whose count fields read 0), in a block with continuous features; unweighted fits
 # build two packed words, weighted ones four.
