@@ -673,12 +673,6 @@ mpsb_cuda_dataset* finish_narrow(mpsb_cuda_backend* b, Scratch& ss, const Keys& 
 constexpr int kSortThreads = 256;
 constexpr uint32_t kSortTile = 4096;  // keys per (feature, tile) block
 
-__global__ void sort_keys_init_kernel(const uint32_t* keys, const uint8_t* missing, size_t cells,
-                                      uint32_t* out) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < cells; i += size_t(gridDim.x) * blockDim.x)
-    out[i] = missing[i] ? kMissingKey : keys[i];
-}
-
 // Digit counts of one (tile, feature): cnt[(f * 16 + digit) * tiles + tile].
 __global__ void __launch_bounds__(kSortThreads) sort_count_kernel(const uint32_t* keys, uint32_t n,
                                                                   uint32_t tiles, int shift, uint32_t* cnt) {
@@ -868,37 +862,34 @@ __global__ void transform_wide_kernel(const uint32_t* keys, const uint8_t* missi
 }
 
 // Sorts every feature's keys (missing rows last) into `sorted`; `tmp` is a buffer of the
-// same size. Eight passes: the result ends where it started.
-void sort_feature_keys(cudaStream_t s, Scratch& ss, const uint32_t* keys, const uint8_t* missing,
-                       uint32_t n, uint32_t features, uint32_t* sorted, uint32_t* tmp) {
-  const size_t cells = size_t(n) * features;
+// same size. Eight passes, the first out of the keys: the last one ends in `sorted`.
+void sort_feature_keys(cudaStream_t s, Scratch& ss, const uint32_t* keys, uint32_t n, uint32_t features,
+                       uint32_t* sorted, uint32_t* tmp) {
   const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
   uint32_t* cnt = ss.alloc<uint32_t>(size_t(features) * 16 * tiles);
-  sort_keys_init_kernel<<<unsigned(std::min<size_t>((cells + 255) / 256, 152 * 32)), 256, 0, s>>>(
-      keys, missing, cells, sorted);
-  CK(cudaGetLastError());
-  uint32_t* a = sorted;
-  uint32_t* b = tmp;
+  const uint32_t* in = keys;
+  uint32_t* out = tmp;
   for (int shift = 0; shift < 32; shift += 4) {
-    sort_count_kernel<<<dim3(tiles, features), kSortThreads, 0, s>>>(a, n, tiles, shift, cnt);
+    sort_count_kernel<<<dim3(tiles, features), kSortThreads, 0, s>>>(in, n, tiles, shift, cnt);
     CK(cudaGetLastError());
     sort_scan_kernel<<<features, 1024, 0, s>>>(cnt, tiles);
     CK(cudaGetLastError());
-    sort_scatter_kernel<<<dim3(tiles, features), kSortThreads, 0, s>>>(a, b, n, tiles, shift, cnt);
+    sort_scatter_kernel<<<dim3(tiles, features), kSortThreads, 0, s>>>(in, out, n, tiles, shift, cnt);
     CK(cudaGetLastError());
-    std::swap(a, b);
+    in = out;
+    out = out == tmp ? sorted : tmp;
   }
 }
 
 // QuantizeDense for max_bins > 256 on the device: u16 feature-major bins in `bins_fm`,
 // boundaries [features][max_bins - 1] in `bounds` with their counts.
-void quantize_wide(cudaStream_t s, Scratch& ss, const uint32_t* keys, const uint8_t* missing,
+void quantize_wide(cudaStream_t s, Scratch& ss, const uint32_t* keys,
                    const std::vector<uint64_t>& missing_count, uint32_t n, uint32_t features,
                    uint32_t max_bins, float* bounds, uint32_t* counts, uint16_t* bins_fm) {
   const size_t cells = size_t(n) * features;
   uint32_t* sorted = ss.alloc<uint32_t>(cells);
   uint32_t* tmp = ss.alloc<uint32_t>(cells);
-  sort_feature_keys(s, ss, keys, missing, n, features, sorted, tmp);
+  sort_feature_keys(s, ss, keys, n, features, sorted, tmp);
   uint64_t* d_miss = ss.alloc<uint64_t>(features);
   CK(cudaMemcpyAsync(d_miss, missing_count.data(), features * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
   wide_bounds_kernel<<<features, 1024, 0, s>>>(sorted, n, d_miss, max_bins, bounds, counts);
@@ -960,7 +951,7 @@ int mpsb_cuda_dataset_quantize(mpsb_cuda_backend* b, const void* data, int scala
       float* bounds = ss.alloc<float>(size_t(features) * stride);
       uint32_t* counts = ss.alloc<uint32_t>(features);
       uint16_t* bins16 = ss.alloc<uint16_t>(size_t(features) * n);
-      quantize_wide(s, ss, k.keys, k.missing, k.missing_count, n, features, max_bins, bounds, counts, bins16);
+      quantize_wide(s, ss, k.keys, k.missing_count, n, features, max_bins, bounds, counts, bins16);
       const dim3 grid(std::max(1u, std::min((n + 255) / 256, uint32_t(b->sm_count) * 4 / std::max(1u, features) + 1)),
                       features);
       transform_wide_kernel<<<grid, 256, 0, s>>>(k.keys, k.missing, n, bounds, stride, counts, bins16);

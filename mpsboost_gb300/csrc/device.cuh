@@ -194,7 +194,6 @@ struct Control {
   uint32_t part_chunks;
   uint32_t leaf_chunks;
   uint32_t free_top;       // histogram-slot free stack
-  uint32_t split_items;    // nodes x feature chunks
   uint32_t item_rows;      // rows per histogram work item of the current level
   uint32_t round;          // the round in progress
   uint32_t grad_ticket;    // CTAs of the gradient launch that have finished

@@ -273,7 +273,6 @@ __device__ __noinline__ void round_setup(const TrainerDev& a, bool g_only) {
     a.ctl->n_part = 0;
     a.ctl->hist_items = acc * a.nfb;
     a.ctl->hist_counter = 0;
-    a.ctl->split_items = a.n_trees * a.n_fchunks;
     a.ctl->item_rows = item_rows;
   }
   if (threadIdx.x >= 32) {  // beside warp 0's work items
@@ -2324,7 +2323,6 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       ctl->n_part = 0;
       ctl->hist_items = 0;
       ctl->part_chunks = 0;
-      ctl->split_items = 0;
     } else {
       ctl->free_top = free_top - n_acc + (n - n_acc);
       ctl->n_nodes = 2 * n_acc;
@@ -2335,7 +2333,6 @@ __global__ void __launch_bounds__(1024) finalize_kernel(TrainerDev a, int parity
       a.part_prefix[n_acc] = carry6[2];
       ctl->hist_items = carry6[1] * a.nfb;
       ctl->part_chunks = carry6[2];
-      ctl->split_items = 2 * n_acc * a.n_fchunks;
       ctl->item_rows = item_rows;
     }
     ctl->hist_counter = 0;
@@ -2564,7 +2561,6 @@ __global__ void __launch_bounds__(kNodeFinalizeMax) finalize_nodes_kernel(Traine
     ctl->n_part = acc_next;
     ctl->hist_items = last ? 0u : tot[1] * a.nfb;
     ctl->part_chunks = last ? 0u : tot[2];
-    ctl->split_items = 2 * acc_next * a.n_fchunks;
     if (!last) {
       ctl->free_top = free_top - n_acc + (n - n_acc);
       a.build_prefix[n_acc] = tot[1];
@@ -3184,7 +3180,6 @@ __global__ void __launch_bounds__(32 * kSelectTrees) leafwise_select_kernel(Trai
       ctl->hist_counter = 0;
       ctl->item_rows = item_rows;
       ctl->n_nodes = n_scan;
-      ctl->split_items = n_scan * a.n_fchunks;
     }
   }
 }
@@ -3247,7 +3242,7 @@ __global__ void leafwise_finish_kernel(TrainerDev a) {
     ctl->n_leafseg = n;
     ctl->leaf_chunks = chunks;
     ctl->n_nodes = ctl->n_build = ctl->n_sub = ctl->n_part = 0;
-    ctl->hist_items = ctl->part_chunks = ctl->split_items = 0;
+    ctl->hist_items = ctl->part_chunks = 0;
   }
 }
 
