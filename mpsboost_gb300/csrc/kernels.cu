@@ -1735,17 +1735,72 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
 // level's children are leaves, so no later level subtracts from a sibling's histogram: the
 // screen leaves it unwritten (a quarter of its bytes) and the few features evaluated here
 // form it again.
+// The common path is short of instructions on purpose, as each launch fetches it cold: what only
+// shared nodes need is out of line, and the features are counted at a barrier (inlined, with a
+// sum through shared memory, ordinary levels took 1 us more). A level that could share costs 0.2
+// to 0.5 us more than one CTA per node.
 constexpr uint32_t kExactAlone = 8;
 
+// Whether the thread's listed feature is one of this part's: every parts-th of the node's.
+// `before`: listed features of the blocks before, moved on. Every thread of the CTA.
+__device__ __noinline__ bool part_takes(bool listed, uint32_t* before, uint32_t part, uint32_t parts) {
+  __shared__ uint32_t s_rank[kScanCtaWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t ballot = __ballot_sync(0xffffffffu, listed);
+  if (lane == 0) s_rank[warp] = uint32_t(__popc(ballot));
+  __syncthreads();
+  uint32_t rank = *before + uint32_t(__popc(ballot & ((1u << lane) - 1u)));
+#pragma unroll
+  for (int q = 0; q < kScanCtaWarps; ++q) {
+    if (q < warp) rank += s_rank[q];
+    *before += s_rank[q];
+  }
+  return listed && rank % parts == part;
+}
+
+// The end of a shared node's part, whose record is written: the last part to come here copies
+// the best of the node's records to *out. Every thread of the CTA.
+__device__ __noinline__ void part_done(const SplitRec* records, uint32_t* done, uint32_t parts, SplitRec* out) {
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(done, 1u) == parts - 1;
+    if (s_last) *done = 0;
+  }
+  __syncthreads();
+  if (!s_last || threadIdx.x >= 32) return;
+  __threadfence();
+  uint32_t v = 0, f = 0xffffffffu, at = 0;
+  double g = 0.0;
+  auto consider_record = [&](uint32_t ov, double og, uint32_t of, uint32_t oat) {
+    if (ov && (!v || og > g || (og == g && of < f))) {  // no two records share a feature
+      v = ov;
+      g = og;
+      f = of;
+      at = oat;
+    }
+  };
+  for (uint32_t q = threadIdx.x; q < parts; q += 32)
+    consider_record(__ldcg(&records[q].valid), __ldcg(&records[q].gain), __ldcg(&records[q].feature), q);
+  for (int off = 16; off > 0; off >>= 1) {
+    const uint32_t ov = __shfl_xor_sync(0xffffffffu, v, off), of = __shfl_xor_sync(0xffffffffu, f, off);
+    const uint32_t oat = __shfl_xor_sync(0xffffffffu, at, off);
+    const double og = __shfl_xor_sync(0xffffffffu, g, off);
+    consider_record(ov, og, of, oat);
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);  // without a split: any of the records
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(records + at);
+  unsigned long long* dst = reinterpret_cast<unsigned long long*>(out);
+  if (threadIdx.x < sizeof(SplitRec) / 8) dst[threadIdx.x] = __ldcg(src + threadIdx.x);
+}
+
 template <bool FIXED, bool WIDE, bool PARTS>
-__global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, int parity, bool to_active, bool last,
-                                                                  uint32_t max_parts) {
+__global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, int parity, bool to_active, bool last) {
   __shared__ PageTotals<FIXED> s_totals[2];
   __shared__ uint32_t s_list[kScanCta], s_listed;
   __shared__ double s_gain[kScanCtaWarps];
   __shared__ uint32_t s_key[kScanCtaWarps][5];  // valid, feature, threshold, default_left, thread
-  __shared__ uint32_t s_count[kScanCtaWarps];
-  __shared__ bool s_last;
   const TreeParams& P = a.params;
   launch_order();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1753,10 +1808,13 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
   const uint32_t msl = min_leaf_rows(P);
   const uint32_t n_nodes = a.ctl->n_nodes;
   uint32_t buf = 0, err = 0;
-  // (The launch covers the level's bound.)
-  const uint32_t parts = PARTS && uint64_t(n_nodes) * max_parts <= a.exact_cap ? max_parts : 1u;
-  for (uint32_t item = blockIdx.x; item < n_nodes * parts; item += gridDim.x) {
-    const uint32_t part = PARTS ? item / n_nodes : 0u, i = PARTS ? item - part * n_nodes : item;
+  // PARTS: the grid is (the level's bound, parts).
+  const uint32_t part = PARTS ? blockIdx.y : 0u, parts = PARTS ? gridDim.y : 1u;
+  if (PARTS && n_nodes > gridDim.x) {
+    if (threadIdx.x == 0) raise(a.ctl, kErrCapacity);
+    return;
+  }
+  for (uint32_t i = blockIdx.x; i < n_nodes; i += gridDim.x) {
     const NodeRec& rec = a.nodes[parity][i];
     const TreeState& tree = a.trees[rec.tree];
     const double inv_g = tree.inv_g, inv_h = tree.inv_h;
@@ -1770,17 +1828,16 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
       return word != 0 && ((word & kFeatureExact) || !(__uint_as_float(word) < cut));
     };
     bool shared = false;  // the node's CTAs share its features; the same in all of them
-    if (PARTS && parts > 1) {
+    uint32_t mine_listed = 0;  // of the thread's first 32 features, one bit each
+    if (PARTS) {
       uint32_t all = 0;
-#pragma unroll 4
-      for (uint32_t f = threadIdx.x; f < F; f += kScanCta) all += listed_feature(f) ? 1u : 0u;
-      all = __reduce_add_sync(0xffffffffu, all);
-      if (lane == 0) s_count[warp] = all;
-      __syncthreads();
-      all = 0;
-#pragma unroll
-      for (int q = 0; q < kScanCtaWarps; ++q) all += s_count[q];
-      __syncthreads();  // s_count is written again
+      if (threadIdx.x == 0) s_listed = 0;
+#pragma unroll 1
+      for (uint32_t k = 0; k * kScanCta < F; ++k) {
+        const bool l = listed_feature(k * kScanCta + threadIdx.x);
+        if (k < 32) mine_listed |= uint32_t(l) << k;
+        all += uint32_t(__syncthreads_count(l));
+      }
       shared = all > kExactAlone;
       if (!shared && part != 0) continue;
     }
@@ -1790,22 +1847,13 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
     double gain = 0.0;
     Stat<FIXED> cl = stat_zero<FIXED>(), cr = stat_zero<FIXED>();
     for (uint32_t base = 0; base < F; base += kScanCta) {
-      if (threadIdx.x == 0) s_listed = 0;
-      __syncthreads();
-      const uint32_t mine = base + threadIdx.x;
-      bool take = listed_feature(mine);
-      if (PARTS && shared) {  // every parts-th of the listed ones
-        const uint32_t ballot = __ballot_sync(0xffffffffu, take);
-        if (lane == 0) s_count[warp] = uint32_t(__popc(ballot));
+      if (!PARTS || base) {  // PARTS: cleared with the counting above
+        if (threadIdx.x == 0) s_listed = 0;
         __syncthreads();
-        uint32_t rank = before + uint32_t(__popc(ballot & ((1u << lane) - 1u)));
-#pragma unroll
-        for (int q = 0; q < kScanCtaWarps; ++q) {
-          if (q < warp) rank += s_count[q];
-          before += s_count[q];
-        }
-        take = take && rank % parts == part;
       }
+      const uint32_t mine = base + threadIdx.x;
+      bool take = PARTS && base < 32 * kScanCta ? (mine_listed >> (base / kScanCta)) & 1u : listed_feature(mine);
+      if (PARTS && shared) take = part_takes(take, &before, part, parts);
       if (take) s_list[atomicAdd(&s_listed, 1u)] = mine;  // any order: the best split is unique
       __syncthreads();
       const uint32_t listed = s_listed;
@@ -1917,41 +1965,7 @@ __global__ void __launch_bounds__(kScanCta, 4) split_exact_kernel(TrainerDev a, 
       *out = split_record<FIXED>(P, cl, cr, inv_g, inv_h, mono, lo, hi, gain, feature, threshold,
                                  default_left);
     }
-    if (PARTS && shared) {  // the last of the node's CTAs picks among their records
-      __threadfence();
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        s_last = atomicAdd(a.exact_done + i, 1u) == parts - 1;
-        if (s_last) a.exact_done[i] = 0;
-      }
-      __syncthreads();
-      if (s_last && warp == 0) {
-        __threadfence();
-        const SplitRec* rec_of = a.exact_part + size_t(i) * parts;
-        uint32_t v = 0, f = 0xffffffffu, at = 0;
-        double g = 0.0;
-        auto consider_record = [&](uint32_t ov, double og, uint32_t of, uint32_t oat) {
-          if (ov && (!v || og > g || (og == g && of < f))) {  // no two records share a feature
-            v = ov;
-            g = og;
-            f = of;
-            at = oat;
-          }
-        };
-        for (uint32_t q = uint32_t(lane); q < parts; q += 32)
-          consider_record(__ldcg(&rec_of[q].valid), __ldcg(&rec_of[q].gain), __ldcg(&rec_of[q].feature), q);
-        for (int off = 16; off > 0; off >>= 1) {
-          const uint32_t ov = __shfl_xor_sync(0xffffffffu, v, off), of = __shfl_xor_sync(0xffffffffu, f, off);
-          const uint32_t oat = __shfl_xor_sync(0xffffffffu, at, off);
-          const double og = __shfl_xor_sync(0xffffffffu, g, off);
-          consider_record(ov, og, of, oat);
-        }
-        at = __shfl_sync(0xffffffffu, at, 0);  // without a split: any of the records
-        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(rec_of + at);
-        unsigned long long* dst = reinterpret_cast<unsigned long long*>(node_best);
-        if (lane < int(sizeof(SplitRec) / 8)) dst[lane] = __ldcg(src + lane);
-      }
-    }
+    if (PARTS && shared) part_done(a.exact_part + size_t(i) * parts, a.exact_done + i, parts, node_best);
     __syncthreads();  // the argmax arrays and the list are rewritten by the next node
   }
   if (err) raise(a.ctl, err);
@@ -3758,10 +3772,10 @@ __global__ void pack_bins16_kernel(const void* src, uint32_t width, const uint8_
 // are long. Not the histogram builds: their CTAs take a whole SM's registers while they wait
 // (logistic 24.2 -> 26.2 ms).
 template <class... Params, class... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), const TrainerDev& a, uint32_t grid, uint32_t block,
+cudaError_t launch_chained(void (*kernel)(Params...), const TrainerDev& a, dim3 grid, uint32_t block,
                            cudaStream_t s, uint32_t cluster, Args... args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.stream = s;
   cudaLaunchAttribute attr[2] = {};
@@ -3836,9 +3850,12 @@ cudaError_t launch_scan_two(const TrainerDev& a, int parity, uint32_t max_nodes,
   // nodes leave room on the SMs.
   const uint32_t parts = uint32_t(std::max<uint64_t>(
       1, std::min<uint64_t>((a.features + kExactFeatures - 1) / kExactFeatures, a.exact_cap / max_nodes)));
-  const uint32_t exact = uint32_t(std::min<uint64_t>(resident, uint64_t(max_nodes) * parts));
-  return launch_chained(parts > 1 ? split_exact_kernel<FIXED, WIDE, true> : split_exact_kernel<FIXED, WIDE, false>, a,
-                        exact, kScanCta, s, 0, parity, kind == ScanKind::kActive, last, parts);
+  const uint32_t nodes = uint32_t(std::min<uint64_t>(resident, max_nodes));
+  if (parts > 1)
+    return launch_chained(split_exact_kernel<FIXED, WIDE, true>, a, dim3(nodes, parts), kScanCta, s, 0, parity,
+                          kind == ScanKind::kActive, last);
+  return launch_chained(split_exact_kernel<FIXED, WIDE, false>, a, nodes, kScanCta, s, 0, parity,
+                        kind == ScanKind::kActive, last);
 }
 
 cudaError_t launch_split_scan(const TrainerDev& a, int parity, uint32_t max_nodes, ScanKind kind,
