@@ -102,7 +102,7 @@ typedef struct {
   uint32_t max_leaves;
   uint32_t max_active_leaves;
   uint32_t split_strategy;  /* 0 best_gain, 1 random_threshold */
-  uint32_t growth_strategy; /* 0 level_wise (1 leaf_wise is not provided here) */
+  uint32_t growth_strategy; /* 0 level_wise, 1 leaf_wise */
   uint32_t random_seed;
   uint32_t n_monotonic;
   uint32_t n_interaction_groups;

@@ -51,7 +51,7 @@ constexpr uint64_t kLongItemRows = 12288;
 // Work items per SM a level is cut into. u8 datasets: three, two while the level has fewer
 // than eight nodes. Wide ones: one, because each of an item's passes zeroes and flushes
 // 200 KB whatever its rows (three items: 12.5 -> 10.2 ms for 1,000,000 x 64 at 1,024 bins
-// with one, 18.7 -> 15.7 at 2,000, 8.3 -> 7.7 at 300).
+// with one, 18.7 -> 15.7 at 2,000, 8.3 -> 7.7 at 300, each before the whole waves below).
 __device__ __forceinline__ uint32_t level_items_per_sm(const TrainerDev& a, uint32_t nodes) {
   const uint32_t base = a.items_per_sm ? a.items_per_sm : default_items_per_sm(a.slots);
   return nodes < 8 && base > 2 ? base - 1 : base;
@@ -63,10 +63,12 @@ __device__ __forceinline__ uint32_t level_items_per_sm(const TrainerDev& a, uint
 // level overshoots its multiple of the SM count and ends in a wave of a few items
 // (one-vs-rest of ten classes 15.1 -> 14.5 ms, 1,024 bins 9.9 -> 9.4). One more per SM from
 // eight nodes on where the items still hold kLongItemRows rows: a large level ends more evenly
-// with more of them, and their flushes hardly count (10,000,000 x 128: 76.4 ms without, 75.8
-// with; the same from 8,192 rows, 76.4 from 16,384). Where the upper end
-// forces more items, their number is raised to the next multiple of the
-// SM count, so that the persistent CTAs end the level together. At the lower end an item's
+// with more of them, and their flushes hardly count (20 trees of 10,000,000 x 128 77.26 ms
+// without, 76.54 with; 8,000,000 x 128 unweighted 51.75 and 51.35, 6,000,000 x 100 53.53 and
+// 53.40, one-vs-rest of ten classes 14.72 and 14.62, of eight on 700,000 rows 11.77 and 11.88;
+// each the median of four runs in turn). Where the upper end forces more items, their number is
+// raised to the next multiple of the SM count, so that the persistent CTAs end the level
+// together. At the lower end an item's
 // reductions (about 1.5 us) weigh as much as its flush: 100,000 x 32, depth 6, 50 trees
 // take 17.5, 17.3, 17.7 and 18.7 ms with items of 512, 1,024, 2,048 and 4,096 rows.
 __device__ __forceinline__ uint32_t adaptive_item_rows(uint64_t rows, const TrainerDev& a, uint32_t per_sm,
@@ -899,12 +901,9 @@ __device__ __forceinline__ void stage_feature_hist(const unsigned long long* src
   __syncwarp();
 }
 
-// stage_feature_hist of a sibling's histogram, formed on the way: parent minus the built
-// child word by word, with subtract_kernel's checks (count underflow; float mode: finite
-// sums, non-negative hessians, the hessian difference clamped at 0 within 1e-5), and
-// written back over the parent's words in the same 16-byte chunks.
 // One word of a sibling's slot: parent minus built child, with subtract_kernel's checks
-// (word 0 count, 1 g, 2 h).
+// (word 0 count, 1 g, 2 h; count underflow; float mode: finite sums, non-negative hessians, the
+// hessian difference clamped at 0 within 1e-5).
 template <bool FIXED>
 __device__ __forceinline__ unsigned long long sibling_word(unsigned long long pw, unsigned long long cw,
                                                            uint32_t word, uint32_t& err) {
@@ -925,6 +924,8 @@ __device__ __forceinline__ unsigned long long sibling_word(unsigned long long pw
   return (unsigned long long)__double_as_longlong(diff < 0.0 ? 0.0 : diff);
 }
 
+// stage_feature_hist of a sibling's histogram, formed on the way and written back over the
+// parent's words in the same 16-byte chunks.
 template <bool FIXED>
 __device__ __forceinline__ void stage_sibling_hist(unsigned long long* parent,
                                                    const unsigned long long* built,
@@ -1729,8 +1730,9 @@ __global__ void __launch_bounds__(kScanCta, WIDE ? 5 : 6) split_screen_kernel(Tr
 // kExactAlone (features under monotone constraints, hessians at min_child_weight, equal
 // columns) every CTA takes its share, 2 to 12 us a feature, and the last one to finish picks
 // the best. Ten trees of depth 6, one CTA per node -> shared: 100,000 x 200 all monotone
-// 147 -> 30.6 ms, 2,000 x 500 with min_child_weight 20 unweighted 86.8 -> 9.5, 100,000 x 200 of eight
-// distinct columns 9.3 -> 4.9.
+// 147 -> 30.4 ms, 2,000 x 500 with min_child_weight 20 unweighted 86.9 -> 9.8, 100,000 x 200 of
+// eight distinct columns 9.3 -> 5.0, 200 x 5,000 down to single rows (whose splits tie in many
+// features) 368 -> 22.7.
 // to_active: a leaf-wise step, whose nodes' splits go to their active leaves. last: the
 // level's children are leaves, so no later level subtracts from a sibling's histogram: the
 // screen leaves it unwritten (a quarter of its bytes) and the few features evaluated here

@@ -126,7 +126,8 @@ struct TrainerDev {
   uint32_t item_rows;           // rows per histogram work item (<= kItemRowsMax); 0: the
                                 // level's adaptive value ctl->item_rows
   uint32_t sm_count;
-  uint32_t items_per_sm;        // histogram work items per SM of the adaptive item size (0: 3)
+  uint32_t items_per_sm;        // histogram work items per SM of the adaptive item size (0:
+                                // default_items_per_sm)
   uint32_t mode;                // kModeFixed / kModeFloat
   uint32_t ovr;                 // labels are class ids; tree t fits class t (logistic)
   uint32_t n_classes;           // native softmax: K classes, one tree per class in turn;
